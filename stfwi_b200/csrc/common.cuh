@@ -29,11 +29,11 @@ constexpr int NTHR = TX * NWARP;  // threads per block
 // psi (C-PML memory) arrays per shot: x-strips and z-strips
 enum { PX_SXX = 0, PX_SXZ, PX_DXU, PX_DXV, PX_NFWD };
 enum { PZ_SXZ = 0, PZ_SZZ, PZ_DZV, PZ_DZU, PZ_NFWD };
-// adjoint psi: 4 x + 4 z, double-buffered (slot 0/1)
+// adjoint psi: 4 x + 4 z
 enum { PXA_DXU = 0, PXA_DXV, PXA_XX, PXA_XXZ, PXA_N };
 enum { PZA_DZU = 0, PZA_DZV, PZA_ZXZ, PZA_ZZ, PZA_N };
-constexpr int NPX = PX_NFWD + 2 * PXA_N;  // 12
-constexpr int NPZ = PZ_NFWD + 2 * PZA_N;  // 12
+constexpr int NPX = PX_NFWD + PXA_N;  // 8
+constexpr int NPZ = PZ_NFWD + PZA_N;  // 8
 
 // field slots per shot
 enum { F_U = 0, F_V, F_EX, F_EZ, F_ES, F_N };
@@ -53,12 +53,27 @@ struct Geo {
     long long nd;              // nz_dom*nx_dom
     int snf;                   // history fields per slot: 3 (stresses) or 5 (+ U, V)
     uint32_t wait_polls;       // mbarrier polls before a tile wait gives up (WAIT3 by default)
-    // dispatch order of the tiles of the staged tilings (A: fwd_vel, fwd_str,
-    // adj_a; B: adj_b): the `heavy` tiles that touch an edge, a C-PML strip
-    // or the free surface first, or null for the plain order
-    const int *tordA, *tordB;
-    int theavyA, theavyB;
-    int goff;                  // first shot group of the launch (a pass split into two chains)
+    const float4 *pmx, *pmz;   // C-PML (b, a, 1/k) per column, (b, a, 1/k, strip index) per row; whole tiles
+    // image bands of the adjoint: columns [0, jl) and [jr, nx) of the x
+    // images, rows [0, ita) and [iba, nz) of the z images that st_adj_a
+    // reads, [0, itb) and [ibb, nz) of those that st_adj_b reads
+    int jl, jr, wxp, ita, iba, itb, ibb;
+    long long txs, tzs;        // floats of one x (z) image of a shot
+};
+
+// a launch's work: every tile (order: tile row << 16 | tile column) of the
+// shots [s0, s1); every block gets `per` items, the first `extra` one more
+struct Work {
+    const uint32_t *order;
+    int ntx, tiles, s0, s1, per, extra;
+    int part;              // number of the part of the pass that the shots are
+};
+
+// images of the adjoint fields under the transposed C-PML, [shot][2][...]:
+// of the strain adjoints (x: exx_a, exz_a; z: ezz_a, exz_a), written by
+// st_adj_b, and of the velocity adjoints (x: P, Q; z: P, Q), by st_adj_a
+struct Images {
+    float *xa, *za, *xb, *zb;
 };
 
 struct Mat {
@@ -70,6 +85,7 @@ struct Mat {
 
 struct Shots {
     const int *sx, *sz, *type;      // padded-grid source position, type
+    const int4 *pos;                // the same as (row, column, type, 0)
     const float *wav;               // [nshot][nt]
     const float *fcoef;             // dt/(dx dz) * B[src]          (force)
     const float *mcoef;             // 2 (L+M)[src] dx dz           (moment denominator)
@@ -124,14 +140,6 @@ __device__ __forceinline__ float *pz_ptr(const Geo &g, float *PZ, int s, int a)
     return PZ + ((long long)s * NPZ + a) * g.zstride;
 }
 
-// forward C-PML (fwi/forward.py:107-112): psi' = b psi + a D ; D' = D/k + psi'
-__device__ __forceinline__ float pml_fwd(float D, float b, float a, float ik, float *psi)
-{
-    float pn = b * (*psi) + a * D;
-    *psi = pn;
-    return D * ik + pn;
-}
-
 // forward outputs of the strain phase
 struct FwdOut {
     float *rec;          // [nshot][4][nt][nrec]
@@ -149,9 +157,8 @@ struct AdjIn {
     const float *rec_adj;  // [nshot][4][nt][nrec]
     const float *row0;     // forward post-PML d(vx)/dx at row 0: + (s*slots + slot)*nx_dom
     int slots, slot;
-    double *accLr;         // [groups][nx_dom] FP64: dJ/dLr on row 0
+    double *accLr;         // [nshot][nx_dom] FP64: dJ/dLr on row 0
     int want_exact;
-    int ping;              // psi slot read (ping) / written (1-ping)
 };
 
 // inputs and outputs of the adjoint strain phase
@@ -162,34 +169,19 @@ struct AdjOut {
     int slot_img;          // slot of the forward carry-out of this step (imaging), -1 if none
     int slot_next;         // slot of the carry-out of the next step (density imaging term), -1 if none
     int accp;              // accumulator planes per group (5, or 7 with the density terms)
-    double *acc;           // [groups][accp][nd]: gM, gL, gL2M (exact), glam, gmu (imaging), gB (exact), g_rho_lame (imaging)
+    int groups, parts;     // accumulator groups, parts of the pass that share them out
+    double *acc;           // [groups][accp][nd]: sC, sB, sA (exact), glam, gmu (imaging), gB (exact), g_rho_lame (imaging)
+    double *mterm;         // [nshot]: the moment sources' dJ/dL = dJ/dM terms (exact)
     int want_exact, want_img;
     float *src_a;          // [nshot][nt] or null
     const float *rec_adj;  // [nshot][4][nt][nrec]
-    int ping;
-    int hist_tma;          // two-column kernels: the carry-in stresses arrive by TMA (history map valid)
+    int hist_tma;          // the history's stresses arrive by TMA (history map valid)
 };
 
 constexpr uint32_t WAIT3 = 1u << 22; // mbarrier polls before a wait gives up
 constexpr int ST_TIMEOUT3 = 2;
 
 __host__ __device__ constexpr int al32_3(int x) { return (x + 31) / 32 * 32; }
-
-struct Ctx3 {
-    int tile, j0, i0, s0, s1;
-};
-
-// on a wait that ran out (the copy of shot `it` of the block): record the
-// timeout and, before the block returns, drain the copies still in flight,
-// which are those of shots it and it + 1 (each shot's copy is issued two
-// shots ahead, on barrier it & 1); these waits are bounded too
-__device__ __forceinline__ void abort3(uint64_t *bar, int it, int nsh, int *status)
-{
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
-        atomicOr(status, ST_TIMEOUT3);
-        for (int k = it; k < it + 2 && k < nsh; ++k) mbar_wait_bounded(bar + (k & 1), (k >> 1) & 1, WAIT3);
-    }
-}
 
 // strains from stresses at one cell (inverse of the 2x2 normal-stress law and sxz = 2 M es)
 __device__ __forceinline__ void strains_of(float sxx, float szz, float sxz, float l2m, float l, float mm,

@@ -1,19 +1,9 @@
-// Table-driven, pair-arithmetic stencil kernels (sm_100a).
+// Stencil kernels of the forward and adjoint steps (sm_100a).
 //
 // Four kernels per time step pair: fwd_vel (U, V), fwd_str (the stresses,
 // receivers, history), adj_a (P, Q) and adj_b (the strain adjoints and the
-// gradient sums), each over every tile of every shot of the batch, with the
-// tiling, TMA staging and per-term slice ranges of stencil_parts.cuh, and:
-//  * tiles that touch an edge, a C-PML strip or the free surface evaluate
-//    every stencil with per-column (x) and per-row (z) coefficient vectors
-//    from shared memory, the reference's dropped high-order terms as zero
-//    coefficients: one code path for all lanes of a warp instead of a masked
-//    and an unmasked path side by side;
-//  * interior tiles compute the z-stencils and the pointwise updates of a
-//    thread's two columns as pairs (__ffma2_rn / __fmul2_rn: one paired FP32
-//    instruction for both columns).
-// A coefficient that is zero contributes fma(0, f, d) = d exactly, so the
-// masked terms drop out as in the reference.
+// gradient sums), each over every tile of every shot of the launch, with the
+// tiling and the stencil pieces of stencil_parts.cuh.
 #pragma once
 #include <type_traits>
 
@@ -21,26 +11,42 @@
 
 namespace stfwi {
 
-// coefficient vectors of the masked stencils at index t of n (term k of the
-// vector is c_k where the reference forms it, else 0)
-template <int FD> __device__ __forceinline__ float cfk(int k) { return k <= FD / 2 ? cf<FD>(k) : 0.f; }
+__device__ __forceinline__ float f2c(const float2 &v, int c) { return c == 0 ? v.x : v.y; }
 
+// arithmetic on the two columns of a thread
+__device__ __forceinline__ float2 dup2(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+}
+
+// Coefficients of the masked stencils.  A term is dropped only within 2K cells
+// of an edge, so a table holds one entry for each of the first and the last
+// eight positions and one for all between; a block builds it in shared memory
+// while its first boxes are on their way.  A dropped term is a zero
+// coefficient: fma(0, f, d) = d exactly.
+constexpr int TAB = 17;
+__device__ __forceinline__ int tab_at(int t, int n) { return n <= TAB ? min(t, TAB - 1) : t < 8 ? t : min(max(t - n + TAB, 8), TAB - 1); }
+__device__ __forceinline__ int tab_pos(int e, int n) { return n <= TAB || e <= 8 ? e : n - TAB + e; }
+
+__device__ __forceinline__ float v4k(const float4 &v, int k) { return k == 1 ? v.x : k == 2 ? v.y : k == 3 ? v.z : v.w; }
 template <int FD, class Pred> __device__ __forceinline__ float4 cvec(Pred p)
 {
-    return make_float4(p(1) ? cfk<FD>(1) : 0.f, p(2) ? cfk<FD>(2) : 0.f, p(3) ? cfk<FD>(3) : 0.f,
-                       p(4) ? cfk<FD>(4) : 0.f);
+    auto c = [&](int k) { return k <= FD / 2 && p(k) ? cf<FD>(k) : 0.f; };
+    return make_float4(c(1), c(2), c(3), c(4));
 }
-// D+ at t: f[t+k] - f[t-k+1]
+// sets: D+ and D-; A and B of the transposed D+ and of the transposed D- (of positions below lim)
 template <int FD> __device__ __forceinline__ float4 cv_P(int t, int n)
 {
     return cvec<FD>([&](int k) { return mP(t, k, n); });
 }
-// D- at t: f[t+k-1] - f[t-k]
 template <int FD> __device__ __forceinline__ float4 cv_M(int t, int n)
 {
     return cvec<FD>([&](int k) { return mM(t, k, n); });
 }
-// transposed D+ at t: + c_k f[t-k] (A) - c_k f[t+k-1] (B)
 template <int FD> __device__ __forceinline__ float4 cv_tPA(int t, int n)
 {
     return cvec<FD>([&](int k) { return mP(t - k, k, n); });
@@ -49,7 +55,6 @@ template <int FD> __device__ __forceinline__ float4 cv_tPB(int t, int n)
 {
     return cvec<FD>([&](int k) { return mP(t + k - 1, k, n); });
 }
-// transposed D- at t below `lim`: + c_k f[t-k+1] (A) - c_k f[t+k] (B)
 template <int FD> __device__ __forceinline__ float4 cv_tMA(int t, int n, int lim)
 {
     return cvec<FD>([&](int k) { return mM(t - k + 1, k, n) && t - k + 1 < lim; });
@@ -58,368 +63,522 @@ template <int FD> __device__ __forceinline__ float4 cv_tMB(int t, int n, int lim
 {
     return cvec<FD>([&](int k) { return mM(t + k, k, n) && t + k < lim; });
 }
+// forward kernels: x sets (P, M), z sets (P, M)
+struct FwdTab { float4 x[2][TAB], z[2][TAB]; };
+// adjoint kernels: x and z sets (tPA, tPB, tMA, tMB); the strain update
+// transposes D- as formed below the last column and row
+struct AdjTab { float4 x[4][TAB], z[4][TAB]; };
 
-__device__ __forceinline__ float v4k(const float4 &v, int k)
+template <int FD> __device__ __forceinline__ void fill(FwdTab *tb, const Geo &g, int tid)
 {
-    return k == 1 ? v.x : k == 2 ? v.y : k == 3 ? v.z : v.w;
+    if (tid >= 4 * TAB) return;
+    const int set = tid / TAB, e = tid % TAB, n = set < 2 ? g.nx : g.nz, t = tab_pos(e, n);
+    float4 *o = set < 2 ? &tb->x[set][e] : &tb->z[set - 2][e];
+    *o = (set & 1) == 0 ? cv_P<FD>(t, n) : cv_M<FD>(t, n);
 }
-__device__ __forceinline__ float f2c(const float2 &v, int c) { return c == 0 ? v.x : v.y; }
+template <int FD> __device__ __forceinline__ void fill(AdjTab *tb, const Geo &g, int tid, int below)
+{
+    if (tid >= 8 * TAB) return;
+    const int set = tid / TAB, e = tid % TAB, n = set < 4 ? g.nx : g.nz, t = tab_pos(e, n), lim = n - below;
+    float4 *o = set < 4 ? &tb->x[set][e] : &tb->z[set - 4][e];
+    const int k = set & 3;
+    *o = k == 0 ? cv_tPA<FD>(t, n) : k == 1 ? cv_tPB<FD>(t, n) : k == 2 ? cv_tMA<FD>(t, n, lim) : cv_tMB<FD>(t, n, lim);
+}
 
-// table-driven stencils on the x-neighbourhood a (column c of the pair)
-template <int FD> __device__ __forceinline__ float a_dp_t(const float (&a)[10], int c, const float4 &v)
+// a table entry, loaded where it is used: the entries of a thread's columns
+// are the same for all its rows, and kept in registers they would spill
+__device__ __forceinline__ float4 entry(const float4 *p)
 {
-    float d = 0.f;
-#pragma unroll
-    for (int k = 1; k <= FD / 2; ++k) d += v4k(v, k) * (a[4 + c + k] - a[5 + c - k]);
-    return d;
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_u32(p)));
+    return v;
 }
-template <int FD> __device__ __forceinline__ float a_dm_t(const float (&a)[10], int c, const float4 &v)
+
+// x stencils of a thread's two columns from their neighbourhood a: with the
+// plain coefficients, or (XB) with those of the table rows A (and B) at e0, e1
+template <int FD, bool XB> __device__ __forceinline__ float2 x_dp(const float (&a)[10], const float4 *A, int e0, int e1)
 {
-    float d = 0.f;
-#pragma unroll
-    for (int k = 1; k <= FD / 2; ++k) d += v4k(v, k) * (a[3 + c + k] - a[4 + c - k]);
-    return d;
-}
-template <int FD>
-__device__ __forceinline__ float a_tdp_t(const float (&a)[10], int c, const float4 &A, const float4 &B)
-{
-    float d = 0.f;
-#pragma unroll
-    for (int k = 1; k <= FD / 2; ++k) {
-        d += v4k(A, k) * a[4 + c - k];
-        d -= v4k(B, k) * a[3 + c + k];
+    if (!XB) {
+        auto c = [](int k) { return cf<FD>(k); };
+        return make_float2(a_dp<FD>(a, 0, c), a_dp<FD>(a, 1, c));
     }
-    return d;
+    const float4 v0 = entry(A + e0), v1 = entry(A + e1);
+    return make_float2(a_dp<FD>(a, 0, [&](int k) { return v4k(v0, k); }), a_dp<FD>(a, 1, [&](int k) { return v4k(v1, k); }));
 }
-template <int FD>
-__device__ __forceinline__ float a_tdm_t(const float (&a)[10], int c, const float4 &A, const float4 &B)
+template <int FD, bool XB> __device__ __forceinline__ float2 x_dm(const float (&a)[10], const float4 *A, int e0, int e1)
 {
-    float d = 0.f;
-#pragma unroll
-    for (int k = 1; k <= FD / 2; ++k) {
-        d += v4k(A, k) * a[5 + c - k];
-        d -= v4k(B, k) * a[4 + c + k];
+    if (!XB) {
+        auto c = [](int k) { return cf<FD>(k); };
+        return make_float2(a_dm<FD>(a, 0, c), a_dm<FD>(a, 1, c));
     }
-    return d;
+    const float4 v0 = entry(A + e0), v1 = entry(A + e1);
+    return make_float2(a_dm<FD>(a, 0, [&](int k) { return v4k(v0, k); }), a_dm<FD>(a, 1, [&](int k) { return v4k(v1, k); }));
 }
-// table-driven z stencils on the pair's window w (row r of the thread at w[r + K])
-template <int FD, int W> __device__ __forceinline__ float w_dp_t(const float2 (&w)[W], int r, int c, const float4 &v)
+template <int FD, bool XB>
+__device__ __forceinline__ float2 x_tdp(const float (&a)[10], const float4 *A, const float4 *B, int e0, int e1)
+{
+    if (!XB) {
+        auto c = [](int k) { return cf<FD>(k); };
+        return make_float2(a_tdp<FD>(a, 0, c, c), a_tdp<FD>(a, 1, c, c));
+    }
+    const float4 u0 = entry(A + e0), v0 = entry(B + e0), u1 = entry(A + e1), v1 = entry(B + e1);
+    return make_float2(a_tdp<FD>(a, 0, [&](int k) { return v4k(u0, k); }, [&](int k) { return v4k(v0, k); }),
+                       a_tdp<FD>(a, 1, [&](int k) { return v4k(u1, k); }, [&](int k) { return v4k(v1, k); }));
+}
+template <int FD, bool XB>
+__device__ __forceinline__ float2 x_tdm(const float (&a)[10], const float4 *A, const float4 *B, int e0, int e1)
+{
+    if (!XB) {
+        auto c = [](int k) { return cf<FD>(k); };
+        return make_float2(a_tdm<FD>(a, 0, c, c), a_tdm<FD>(a, 1, c, c));
+    }
+    const float4 u0 = entry(A + e0), v0 = entry(B + e0), u1 = entry(A + e1), v1 = entry(B + e1);
+    return make_float2(a_tdm<FD>(a, 0, [&](int k) { return v4k(u0, k); }, [&](int k) { return v4k(v0, k); }),
+                       a_tdm<FD>(a, 1, [&](int k) { return v4k(u1, k); }, [&](int k) { return v4k(v1, k); }));
+}
+// z stencils of the pair at row r of the thread from its window w (row r at
+// w[r + K]): plain coefficients, or (GUARD) those of the table entry at A (and B)
+template <int FD, bool GUARD, int W>
+__device__ __forceinline__ float2 z_dp(const float2 (&w)[W], int r, const float4 *A)
 {
     constexpr int K = FD / 2;
-    float d = 0.f;
+    float4 v;
+    if (GUARD) v = entry(A);
+    float2 d = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 1; k <= K; ++k) d += v4k(v, k) * (f2c(w[r + K + k], c) - f2c(w[r + K - k + 1], c));
+    for (int k = 1; k <= K; ++k) d = fma2(dup2(GUARD ? v4k(v, k) : cf<FD>(k)), sub2(w[r + K + k], w[r + K - k + 1]), d);
     return d;
 }
-template <int FD, int W> __device__ __forceinline__ float w_dm_t(const float2 (&w)[W], int r, int c, const float4 &v)
+template <int FD, bool GUARD, int W>
+__device__ __forceinline__ float2 z_dm(const float2 (&w)[W], int r, const float4 *A)
 {
     constexpr int K = FD / 2;
-    float d = 0.f;
+    float4 v;
+    if (GUARD) v = entry(A);
+    float2 d = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 1; k <= K; ++k) d += v4k(v, k) * (f2c(w[r + K + k - 1], c) - f2c(w[r + K - k], c));
+    for (int k = 1; k <= K; ++k) d = fma2(dup2(GUARD ? v4k(v, k) : cf<FD>(k)), sub2(w[r + K + k - 1], w[r + K - k]), d);
     return d;
 }
-template <int FD, int W>
-__device__ __forceinline__ float w_tdp_t(const float2 (&w)[W], int r, int c, const float4 &A, const float4 &B)
+template <int FD, bool GUARD, int W>
+__device__ __forceinline__ float2 z_tdp(const float2 (&w)[W], int r, const float4 *A, const float4 *B)
 {
     constexpr int K = FD / 2;
-    float d = 0.f;
+    float4 u, v;
+    if (GUARD) { u = entry(A); v = entry(B); }
+    float2 d = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 1; k <= K; ++k) {
-        d += v4k(A, k) * f2c(w[r + K - k], c);
-        d -= v4k(B, k) * f2c(w[r + K + k - 1], c);
+        d = fma2(dup2(GUARD ? v4k(u, k) : cf<FD>(k)), w[r + K - k], d);
+        d = fma2(dup2(GUARD ? -v4k(v, k) : -cf<FD>(k)), w[r + K + k - 1], d);
     }
     return d;
 }
-template <int FD, int W>
-__device__ __forceinline__ float w_tdm_t(const float2 (&w)[W], int r, int c, const float4 &A, const float4 &B)
+template <int FD, bool GUARD, int W>
+__device__ __forceinline__ float2 z_tdm(const float2 (&w)[W], int r, const float4 *A, const float4 *B)
 {
     constexpr int K = FD / 2;
-    float d = 0.f;
+    float4 u, v;
+    if (GUARD) { u = entry(A); v = entry(B); }
+    float2 d = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 1; k <= K; ++k) {
-        d += v4k(A, k) * f2c(w[r + K - k + 1], c);
-        d -= v4k(B, k) * f2c(w[r + K + k], c);
+        d = fma2(dup2(GUARD ? v4k(u, k) : cf<FD>(k)), w[r + K - k + 1], d);
+        d = fma2(dup2(GUARD ? -v4k(v, k) : -cf<FD>(k)), w[r + K + k], d);
     }
     return d;
 }
 
-// paired FP32 arithmetic (both columns of a thread in one instruction)
-__device__ __forceinline__ float2 dup2(float s) { return make_float2(s, s); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup2(-1.f), a); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-// unmasked z stencils of the pair, paired
-template <int FD, int W> __device__ __forceinline__ float2 w_dp2(const float2 (&w)[W], int r)
-{
-    constexpr int K = FD / 2;
-    float2 d = mul2(dup2(cf<FD>(1)), sub2(w[r + K + 1], w[r + K]));
-#pragma unroll
-    for (int k = 2; k <= K; ++k) d = fma2(dup2(cf<FD>(k)), sub2(w[r + K + k], w[r + K - k + 1]), d);
-    return d;
-}
-template <int FD, int W> __device__ __forceinline__ float2 w_dm2(const float2 (&w)[W], int r)
-{
-    constexpr int K = FD / 2;
-    float2 d = mul2(dup2(cf<FD>(1)), sub2(w[r + K], w[r + K - 1]));
-#pragma unroll
-    for (int k = 2; k <= K; ++k) d = fma2(dup2(cf<FD>(k)), sub2(w[r + K + k - 1], w[r + K - k]), d);
-    return d;
-}
-template <int FD, int W> __device__ __forceinline__ float2 w_tdp2(const float2 (&w)[W], int r)
-{
-    constexpr int K = FD / 2;
-    float2 d = mul2(dup2(cf<FD>(1)), w[r + K - 1]);
-    d = fma2(dup2(-cf<FD>(1)), w[r + K], d);
-#pragma unroll
-    for (int k = 2; k <= K; ++k) {
-        d = fma2(dup2(cf<FD>(k)), w[r + K - k], d);
-        d = fma2(dup2(-cf<FD>(k)), w[r + K + k - 1], d);
-    }
-    return d;
-}
-template <int FD, int W> __device__ __forceinline__ float2 w_tdm2(const float2 (&w)[W], int r)
-{
-    constexpr int K = FD / 2;
-    float2 d = mul2(dup2(cf<FD>(1)), w[r + K]);
-    d = fma2(dup2(-cf<FD>(1)), w[r + K + 1], d);
-#pragma unroll
-    for (int k = 2; k <= K; ++k) {
-        d = fma2(dup2(cf<FD>(k)), w[r + K - k + 1], d);
-        d = fma2(dup2(-cf<FD>(k)), w[r + K + k], d);
-    }
-    return d;
-}
-
-// z window of the pair as float2 rows
+// z window of the pair
 template <int W, int RPT>
-__device__ __forceinline__ void zwin2p(float2 (&w)[W], const float *s, int ty, int tx)
+__device__ __forceinline__ void zwin(float2 (&w)[W], const float *s, int ty, int tx)
 {
 #pragma unroll
     for (int m = 0; m < W; ++m) w[m] = *reinterpret_cast<const float2 *>(s + (ty * RPT + m) * SW4 + XO4 + 2 * tx);
 }
+__device__ __forceinline__ float2 pair_at(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 
-// tile and shot group of this block, boundary tiles first: the blocks of
-// every (boundary tile, shot group) pair are dispatched before the interior
-// ones, so that the long blocks do not form the tail of the launch
-__device__ __forceinline__ Ctx3 ctx5(const Geo &g, int spg, int tzh, int tiles_x, const int *order, int heavy)
-{
-    const int tiles = gridDim.x, groups = gridDim.y;
-    const int b = blockIdx.y * tiles + blockIdx.x;
-    int t = blockIdx.x, grp = blockIdx.y;
-    if (order && heavy > 0 && heavy < tiles) {
-        if (b < heavy * groups) {
-            t = order[b % heavy];
-            grp = b / heavy;
-        } else {
-            const int b2 = b - heavy * groups, light = tiles - heavy;
-            t = order[heavy + b2 % light];
-            grp = b2 / light;
-        }
+// ------------------------------------------------------------- work and pipeline
+//
+// Work items are (tile, shot) pairs, ordered by tile, within a tile by shot;
+// every block takes an equal, consecutive run of them and reloads a tile's
+// constants only when the tile changes.
+//
+// The item's boxes arrive by TMA in a ring of NST stages.  Every warp waits
+// for a stage by itself and counts itself out once it has read it; the last
+// warp out of a stage refills it with the item NST further on.  No barrier
+// joins the warps of a block, and the ring keeps loads in flight across
+// tiles and groups.
+
+struct Cursor {
+    int pos, shot;        // tile position, shot
+    uint32_t cur, ahead;  // this tile (row << 16 | column) and the next, loaded while this one is at work
+    __device__ __forceinline__ int j0() const { return (cur & 0xffffu) * TX4; }
+    __device__ __forceinline__ int i0(int tzh) const { return (cur >> 16) * tzh; }
+    __device__ __forceinline__ int tile(const Work &w) const { return (cur >> 16) * w.ntx + (cur & 0xffffu); }
+    __device__ __forceinline__ void look(const Work &w) { ahead = __ldg(w.order + min(pos + 1, w.tiles - 1)); }
+    __device__ __forceinline__ void init(const Work &w, unsigned item)
+    {
+        const unsigned ns = w.s1 - w.s0;
+        pos = item / ns;
+        shot = w.s0 + (int)(item - pos * ns);
+        cur = __ldg(w.order + pos);
     }
-    Ctx3 c;
-    c.tile = t;
-    c.j0 = (t % tiles_x) * TX4;
-    c.i0 = (t / tiles_x) * tzh;
-    c.s0 = (grp + g.goff) * spg;
-    c.s1 = min(c.s0 + spg, g.nshot);
-    return c;
+    // is this the tile's last shot
+    __device__ __forceinline__ bool last(const Work &w) const { return shot + 1 == w.s1; }
+    // to the next item; true when the tile changes
+    __device__ __forceinline__ bool next(const Work &w)
+    {
+        if (++shot < w.s1) return false;
+        shot = w.s0;
+        ++pos;
+        cur = ahead;
+        look(w);
+        return true;
+    }
+};
+
+// first item of block b's share
+__device__ __forceinline__ int share(const Work &w, int b) { return b * w.per + min(b, w.extra); }
+
+// ring state in shared memory
+template <int NST> struct Ring {
+    uint64_t full[NST];
+    uint32_t out[NST];      // warps that have left each stage, over all rounds
+    uint32_t issued;        // items issued by this block; DEAD set once a warp gave up
+};
+constexpr uint32_t RING_DEAD = 1u << 31;
+
+// relaxed: a warp's reads of a stage are complete (their values are in
+// registers) before it counts itself out, and the count orders nothing else;
+// an acquire-release here would wait for the warp's global stores
+__device__ __forceinline__ uint32_t atom_add_cta(uint32_t *p, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.relaxed.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ uint32_t atom_or_cta(uint32_t *p, uint32_t v)
+{
+    uint32_t old;
+    asm volatile("atom.acq_rel.cta.shared::cta.or.b32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
+    return old;
 }
 
-// shared-memory plans of the table-driven kernels: the two-column layout
-// followed by the coefficient tables (float4 per column of the tile for
-// each x-stencil set, per row of the tile for each z-stencil set)
-template <int FD, int R> struct L5 {
-    using P4 = L4<FD, R>;
-    static constexpr int CTA = 4 * (2 * TX4 + 2 * P4::A::TZH);                    // 2 x-sets, 2 z-sets
-    static constexpr int CTB = 4 * (4 * TX4 + 4 * P4::A::TZH);                    // 4 x-sets, 4 z-sets (adj_a)
-    static constexpr int CTBB = 4 * (4 * TX4 + 4 * P4::B::TZH);                   // 4 x-sets, 4 z-sets (adj_b)
-    static constexpr int VEL = P4::VEL + CTA, STR = P4::STR + CTA;
-    static constexpr int ADA = P4::ADA + CTB, ADB = P4::ADB + CTBB;
-    static constexpr size_t bytes(int floats, int nbar) { return (size_t)floats * 4 + 8 * nbar; }
+// a wait ran out at the block's item `it`: record it, stop further issues,
+// and wait (bounded) for every copy already issued that this warp has not
+// seen land, so that the block never exits under a copy in flight
+template <int NST> __device__ __forceinline__ void ring_abort(Ring<NST> *r, int it, int *status)
+{
+    if (threadIdx.x == 0) {
+        atomicOr(status, ST_TIMEOUT3);
+        const int n = (int)(atom_or_cta(&r->issued, RING_DEAD) & ~RING_DEAD);
+        for (int k = it; k < n; ++k) mbar_wait_bounded(r->full + k % NST, (k / NST) & 1, WAIT3);
+    }
+    __syncwarp();
+}
+
+// this warp has read item `it` from its stage: true in lane 0 of the last
+// warp out, which then issues the item NST further on
+template <int NST> __device__ __forceinline__ bool ring_leave(Ring<NST> *r, int st, bool more)
+{
+    __syncwarp();
+    if (threadIdx.x != 0) return false;
+    const uint32_t old = atom_add_cta(r->out + st, 1u);
+    if (!more || old % NWARP != NWARP - 1) return false;
+    return !(atom_add_cta(&r->issued, 1u) & RING_DEAD);
+}
+
+// stage sizes (floats) and ring depths: as many stages as two blocks an SM
+// have room for
+template <int FD, int R> struct Stage {
+    using T = G4<FD, R>;
+    static constexpr int OWN2 = al32_3(2 * T::TZH * TX4), OWN3 = al32_3(3 * T::TZH * TX4);
+    static constexpr int VEL = T::S3 + OWN2, STR = T::S2 + OWN3;
+    static constexpr int ADA = al32_3(4 * T::SN) + OWN2, ADB = al32_3(4 * T::SN) + 2 * OWN3;
+    static constexpr int fit(int floats) { return imin(4, (113 * 1024 - 256 - (int)sizeof(AdjTab)) / (floats * 4)); }
+    static constexpr int imin(int a, int b) { return a < b ? a : b; }
+    static constexpr int NVEL = fit(VEL), NSTR = fit(STR), NADA = fit(ADA), NADB = fit(ADB);
+    // stages, coefficient table, ring
+    static constexpr size_t bytes(int floats, int nst) { return (size_t)floats * nst * 4 + sizeof(AdjTab) + 12 * nst + 16; }
 };
+
+// ------------------------------------------------------------- guarded paths
+//
+// Which work a cell needs is decided per tile for the columns and per warp
+// (RPT rows) for the rows: a warp takes the unguarded path when neither a
+// slice mask nor a C-PML strip applies to its cells.  GUARD rows test the
+// masks of their row, uniform over the warp, XB tiles (the first and last of
+// a tile row) also those of their columns.
+
+// columns [j0, j0 + TX4) clear of the `lo` first and `hi` last columns
+__device__ __forceinline__ bool cols_plain(const Geo &g, int j0, int lo, int hi)
+{
+    return j0 >= lo && j0 + TX4 <= g.nx - hi;
+}
+// rows [a, b] clear of the `lo` first and `hi` last rows
+__device__ __forceinline__ bool rows_plain(const Geo &g, int a, int b, int lo, int hi)
+{
+    return a >= lo && b < g.nz - hi;
+}
+
+// x-strip indices of columns jb, jb + 1 (-1 outside the strips and the grid)
+__device__ __forceinline__ int2 xstrip_pair(const Geo &g, int jb)
+{
+    return make_int2(jb < g.nx ? xstrip_index(g, jb) : -1, jb + 1 < g.nx ? xstrip_index(g, jb + 1) : -1);
+}
+
+// a 16-byte C-PML entry (constant during a launch)
+__device__ __forceinline__ float4 ldt(const float4 *p) { return __ldg(p); }
+
+// The C-PML memories of a warp's rows (two arrays a, b) and coefficients, on
+// their way into L1 before the warp waits for its stage: loaded into registers
+// there they would be live across the stencils, loaded row by row from L2 each
+// row would wait for its own.
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+template <int RPT>
+__device__ __forceinline__ void prefetch_x(const Geo &g, int iw, int2 xs, const float *a, const float *b)
+{
+    const int x = max(xs.x, xs.y);
+    if (x < 0) return;
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int o = min(iw + r, g.nz - 1) * g.xs_n + x;
+        prefetch_l1(a + o);
+        prefetch_l1(b + o);
+    }
+}
+template <int RPT>
+__device__ __forceinline__ void prefetch_z(const Geo &g, int iw, int jb, const float *a, const float *b)
+{
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int zs = zstrip_index(g, min(iw + r, g.nz - 1));
+        if (zs < 0 || jb >= g.nx) continue;
+        prefetch_l1(a + zs * g.P + jb);
+        prefetch_l1(b + zs * g.P + jb);
+    }
+}
+// a row's memories of the columns jb, jb + 1 in an x strip.  Columns outside
+// the strips load some valid element: their coefficients are (0, 0, 1).
+__device__ __forceinline__ float2 mem_x(const float *row, int2 xs)
+{
+    return make_float2(row[max(xs.x, 0)], row[max(xs.y, 0)]);
+}
+
+// C-PML of a pair of x-derivatives on one row (c0, c1: the columns' (b, a, 1/k),
+// old: their memories, p: the memory's row) / of z-derivatives (p: the pair's memory)
+__device__ __forceinline__ void pml_x2(float2 &d, const float4 &c0, const float4 &c1, int2 xs, float2 old, float *p)
+{
+    const float p0 = c0.x * old.x + c0.y * d.x, p1 = c1.x * old.y + c1.y * d.y;
+    if (xs.x >= 0) p[xs.x] = p0;
+    if (xs.y >= 0) p[xs.y] = p1;
+    d = make_float2(d.x * c0.z + p0, d.y * c1.z + p1);
+}
+__device__ __forceinline__ void pml_z2(float2 &d, const float4 &zc, float2 old, float *p)
+{
+    const float2 pn = fma2(dup2(zc.x), old, mul2(dup2(zc.y), d));
+    *reinterpret_cast<float2 *>(p) = pn;
+    d = fma2(d, dup2(zc.z), pn);
+}
+// transposed C-PML of a pair (the memory kept as phi = psi / (dt / d)): x' = (1/k + a) x + a phi, phi' = b (x + phi)
+__device__ __forceinline__ void adj_x2(float2 &v, const float4 &c0, const float4 &c1, int2 xs, float2 phi, float *p)
+{
+    if (xs.x >= 0) p[xs.x] = c0.x * (v.x + phi.x);
+    if (xs.y >= 0) p[xs.y] = c1.x * (v.y + phi.y);
+    v = make_float2((c0.z + c0.y) * v.x + c0.y * phi.x, (c1.z + c1.y) * v.y + c1.y * phi.y);
+}
+__device__ __forceinline__ void adj_z2(float2 &v, const float4 &zc, float2 phi, float *p)
+{
+    *reinterpret_cast<float2 *>(p) = mul2(dup2(zc.x), add2(v, phi));
+    v = fma2(dup2(zc.z + zc.y), v, mul2(dup2(zc.y), phi));
+}
+// the same at one cell (receiver injection): a value s added before the transform
+__device__ __forceinline__ float adj_inject(float s, const float4 &c, bool strip, float *p)
+{
+    if (strip) atomicAdd(p, c.x * s);
+    return strip ? (c.z + c.y) * s : s;
+}
+
+// add v to component k (0 or 1) of a pair, nothing for any other k
+__device__ __forceinline__ void add_at(float2 &p, int k, float v)
+{
+    if (k == 0) p.x = p.x + v;
+    if (k == 1) p.y = p.y + v;
+}
+// store a pair (XB: only its first column where it is the row's last)
+template <bool XB> __device__ __forceinline__ void store_pair(float *p, float2 v, int left)
+{
+    if (!XB || left >= 2) *reinterpret_cast<float2 *>(p) = v;
+    else if (left == 1) *p = v.x;
+}
+
+
+// a material of columns jb, jb + 1 of row i (its rows start on 128 bytes, jb
+// is even).  Off the grid it is some other cell's: nothing computed there is
+// kept, and a select on the loaded value would wait for it.
+__device__ __forceinline__ float2 mat_pair(const Geo &g, const float *a, int i, int jb)
+{
+    return *reinterpret_cast<const float2 *>(a + (long long)min(i, g.nz - 1) * g.P + (jb < g.nx ? jb : 0));
+}
+
+// start of a launch: the block's share [first, first + nit) of the items, the
+// ring's barriers, and the first NST items on their way (by the first thread,
+// before the others are waited for); the others meanwhile build the tables
+template <int NST, class Issue, class Fill>
+__device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Cursor &c, int &first, int &nit, Issue issue,
+                                           Fill fill_tab)
+{
+    first = share(w, blockIdx.x);
+    nit = share(w, blockIdx.x + 1) - first;
+    if (nit <= 0) return false;
+    c.init(w, first);
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int b = 0; b < NST; ++b) { mbar_init(ring->full + b, 1); ring->out[b] = 0; }
+        ring->issued = min(NST, nit);
+        fence_async_shared();
+        issue(c, 0);
+#pragma unroll 1
+        for (int b = 1; b < NST && b < nit; ++b) {
+            Cursor u;
+            u.init(w, first + b);
+            issue(u, b);
+        }
+    }
+    c.look(w);
+    fill_tab(threadIdx.y * TX + threadIdx.x);
+    __syncthreads();
+    return true;
+}
 
 // ------------------------------------------------------------- forward: velocities
 
 template <int FD, int RPT>
 __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
-    st_fwd_vel(Geo g, Mat m, Shots sh, float *F, float *PX, float *PZ, int n, int spg, int tiles_x, int *status,
+    st_fwd_vel(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh, float *F,
+               float *PX, float *PZ, int n, const __grid_constant__ Work w, int *status,
                const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmUo)
 {
     using T = G4<FD, RPT>;
-    constexpr int K = T::K, SN = T::SN;
-    constexpr int STG = L4<FD, RPT>::VEL_STAGE, OWNB = 2 * T::TZH * TX4 * 4;
+    using Sg = Stage<FD, RPT>;
+    constexpr int K = T::K, SN = T::SN, STG = Sg::VEL, NST = Sg::NVEL, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
-    // coefficient tables: x sets (D+ of sxx, D- of sxz), z sets (D- of sxz, D+ of szz)
-    float4 *xt = reinterpret_cast<float4 *>(sm + L4<FD, RPT>::VEL);
-    float4 *zt = xt + 2 * TX4;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L5<FD, RPT>::VEL);
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const Ctx3 c = ctx5(g, spg, T::TZH, tiles_x, g.tordA, g.theavyA);
-    const int nsh = c.s1 - c.s0;
-    if (nsh <= 0) return;
-    if (tid == 0) {
-        mbar_init(bar + 0, 1); mbar_init(bar + 1, 1);
-        fence_async_shared();
-        for (int b = 0; b < 2 && b < nsh; ++b) {
-            mbar_arrive_expect_tx(bar + b, 3 * SN * 4 + OWNB);
-            tma_load_4d(sm + b * STG, &tmS, bar + b, c.j0 - XO4, c.i0 - K, F_EX, c.s0 + b);
-            tma_load_4d(sm + b * STG + T::S3, &tmUo, bar + b, c.j0, c.i0, F_U, c.s0 + b);
-        }
-    }
-    for (int t = tid; t < 2 * TX4; t += NTHR) {
-        const int j = c.j0 + t % TX4;
-        xt[t] = t < TX4 ? cv_P<FD>(j, g.nx) : cv_M<FD>(j, g.nx);
-    }
-    for (int t = tid; t < 2 * T::TZH; t += NTHR) {
-        const int i = c.i0 + t % T::TZH;
-        zt[t] = t < T::TZH ? cv_M<FD>(i, g.nz) : cv_P<FD>(i, g.nz);
-    }
-    __syncthreads();
-    const int jb = c.j0 + 2 * tx;
-    int xs[2];
-    float bxv[2], axv[2], ikxv[2];
+    FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
+    Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    auto issue = [&](const Cursor &u, int st) {
+        mbar_arrive_expect_tx(ring->full + st, (3 * SN + 2 * PL) * 4);
+        tma_load_4d(sm + st * STG, &tmS, ring->full + st, u.j0() - XO4, u.i0(T::TZH) - K, F_EX, u.shot);
+        tma_load_4d(sm + st * STG + T::S3, &tmUo, ring->full + st, u.j0(), u.i0(T::TZH), F_U, u.shot);
+    };
+    Cursor c;   // the item at work
+    int first, nit;
+    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
+    // columns (of the tile) and rows (of this warp) where no slice mask and no
+    // C-PML strip applies; the strips are at least K wide, so they hold the
+    // masked columns and rows except those below a free surface
+    bool xin = false, zin = false;
+    int jb = 0, iw = 0, e0 = 0, e1 = 0;   // e0, e1: the columns' table entries
+    float2 B[RPT];
+    auto enter = [&]() {
+        jb = c.j0() + 2 * tx;
+        e0 = tab_at(jb, g.nx);
+        e1 = tab_at(jb + 1, g.nx);
+        iw = c.i0(T::TZH) + ty * RPT;
+        xin = cols_plain(g, c.j0(), g.pad, g.pad);
+        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
 #pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-        const int j = jb + cc;
-        xs[cc] = (j < g.nx) ? xstrip_index(g, j) : -1;
-        bxv[cc] = xs[cc] >= 0 ? m.bx[j] : 0.f;
-        axv[cc] = xs[cc] >= 0 ? m.ax[j] : 0.f;
-        ikxv[cc] = xs[cc] >= 0 ? m.ikx[j] : 1.f;
-    }
-    // dt/dx B and dt/dz B of the thread's cells
-    float2 bx2[RPT], bz2[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        float bc[2];
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int i = c.i0 + ty * RPT + r, j = jb + cc;
-            bc[cc] = (i < g.nz && j < g.nx) ? m.B[(long long)i * g.P + j] : 0.f;
-        }
-        bx2[r] = make_float2(g.dtdx * bc[0], g.dtdx * bc[1]);
-        bz2[r] = make_float2(g.dtdz * bc[0], g.dtdz * bc[1]);
-    }
-
-    const bool plain = tile_plain4(g, c.i0, c.j0, T::TZH, T::M);
-    for (int it = 0; it < nsh; ++it) {
-        const int s = c.s0 + it;
-        float *S = sm + (it & 1) * STG;
-        const float *own = S + T::S3;   // [U, V][TZH][TX4] of the tile's own cells
+        for (int r = 0; r < RPT; ++r) B[r] = mat_pair(g, m.B, iw + r, jb);
+    };
+    enter();
+    int st = 0, ph = 0;
+    for (int it = 0; it < nit; ++it) {
+        const int s = c.shot;
+        const int4 src = __ldg(sh.pos + s);
+        const float *S = sm + st * STG, *own = S + T::S3;   // own: [U, V][TZH][TX4] of the tile's own cells
         float *U = F + ((long long)s * F_N + F_U) * g.fstride;
         float *V = F + ((long long)s * F_N + F_V) * g.fstride;
-        if (!__syncthreads_and(mbar_wait_bounded(bar + (it & 1), (it >> 1) & 1, g.wait_polls))) {
-            abort3(bar, it, nsh, status);
+        float *pSXX = px_ptr(g, PX, s, PX_SXX), *pSXZx = px_ptr(g, PX, s, PX_SXZ);
+        float *pSXZz = pz_ptr(g, PZ, s, PZ_SXZ), *pSZZ = pz_ptr(g, PZ, s, PZ_SZZ);
+        auto rows = [&](auto gd, auto xb) -> bool {
+            constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
+            int2 xs = make_int2(-1, -1);
+            if (XB) {
+                xs = xstrip_pair(g, jb);
+                prefetch_x<RPT>(g, iw, xs, pSXX, pSXZx);
+                prefetch_l1(g.pmx + jb);
+            }
+            if (GUARD) {
+                prefetch_z<RPT>(g, iw, jb, pSXZz, pSZZ);
+                prefetch_l1(g.pmz + iw);
+            }
+            if (!mbar_wait_bounded(ring->full + st, ph, g.wait_polls)) return false;
+            float2 dzxz[RPT], dzz[RPT];
+            {
+                float2 wn[T::W];
+                zwin<T::W, RPT>(wn, S + 2 * SN, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) {
+                    dzxz[r] = z_dm<FD, GUARD>(wn, r, &tab->z[1][tab_at(iw + r, g.nz)]);
+                    if (GUARD && g.fs && iw + r == 0) dzxz[r] = mul2(dup2(2.f * cf<FD>(1)), wn[r + K]);
+                }
+                zwin<T::W, RPT>(wn, S + SN, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) dzz[r] = z_dp<FD, GUARD>(wn, r, &tab->z[0][tab_at(iw + r, g.nz)]);
+            }
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                const int i = iw + r, zr = ty * RPT + r, q = (zr + K) * SW4 + XO4 + 2 * tx;
+                if (GUARD && i >= g.nz - 1) continue;   // row nz - 1 keeps its value
+                float a[10];
+                xrow(a, S, q);
+                float2 dxx = x_dp<FD, XB>(a, tab->x[0], e0, e1);
+                xrow(a, S + 2 * SN, q);
+                float2 dxxz = x_dm<FD, XB>(a, tab->x[1], e0, e1);
+                const float2 u2 = pair_at(own + zr * TX4 + 2 * tx), v2 = pair_at(own + PL + zr * TX4 + 2 * tx);
+                if (XB) {
+                    const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
+                    const float2 m0 = mem_x(pSXX + i * g.xs_n, xs), m1 = mem_x(pSXZx + i * g.xs_n, xs);
+                    pml_x2(dxx, c0, c1, xs, m0, pSXX + i * g.xs_n);
+                    pml_x2(dxxz, c0, c1, xs, m1, pSXZx + i * g.xs_n);
+                }
+                if (GUARD) {
+                    const float4 zc = ldt(g.pmz + i);
+                    const int zs = __float_as_int(zc.w);
+                    if (zs >= 0 && (!XB || jb < g.nx)) {
+                        const float2 m0 = pair_at(pSXZz + zs * g.P + jb), m1 = pair_at(pSZZ + zs * g.P + jb);
+                        pml_z2(dzxz[r], zc, m0, pSXZz + zs * g.P + jb);
+                        pml_z2(dzz[r], zc, m1, pSZZ + zs * g.P + jb);
+                    }
+                }
+                const float2 bx = mul2(dup2(g.dtdx), B[r]), bz = mul2(dup2(g.dtdz), B[r]);
+                float2 un = fma2(bz, dzxz[r], fma2(bx, dxx, u2));
+                float2 vn = fma2(bz, dzz[r], fma2(bx, dxxz, v2));
+                const long long o = (long long)i * g.P + jb;
+                if (XB) {
+                    // columns 0 and nx - 1 keep their value
+                    if (jb < 1 || jb >= g.nx - 1) { un.x = u2.x; vn.x = v2.x; }
+                    if (jb + 1 >= g.nx - 1) { un.y = u2.y; vn.y = v2.y; }
+                }
+                if (src.x == i && src.z == 0 && (!XB || (src.y >= 1 && src.y < g.nx - 1)))   // force source
+                    add_at(vn, src.y - jb, sh.fcoef[s] * sh.wav[(long long)s * g.nt + n]);
+                store_pair<XB>(U + o, un, g.nx - jb);
+                store_pair<XB>(V + o, vn, g.nx - jb);
+            }
+            return true;
+        };
+        if (!(!xin ? rows(std::true_type{}, std::true_type{})
+                   : !zin ? rows(std::true_type{}, std::false_type{}) : rows(std::false_type{}, std::false_type{}))) {
+            ring_abort(ring, it, status);
             return;
         }
-        const float *sxx = S, *szz = S + SN, *sxz = S + 2 * SN;
-        float2 wxz[T::W], wzz[T::W];
-        zwin2p<T::W, RPT>(wxz, sxz, ty, tx);
-        zwin2p<T::W, RPT>(wzz, szz, ty, tx);
-        if (plain && !in_tile4(sh.sz[s], sh.sx[s], c.i0, c.j0, T::TZH)) {
-            // interior tile without this shot's source: no guards, paired arithmetic
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                float ax[10], az[10];
-                xrow(ax, sxx, q);
-                xrow(az, sxz, q);
-                const float2 u2 = *reinterpret_cast<const float2 *>(own + (ty * RPT + r) * TX4 + 2 * tx);
-                const float2 v2 = *reinterpret_cast<const float2 *>(own + (T::TZH + ty * RPT + r) * TX4 + 2 * tx);
-                const float2 dxx = make_float2(a_dp<FD, false>(ax, 0, 0, 0), a_dp<FD, false>(ax, 1, 0, 0));
-                const float2 dxxz = make_float2(a_dm<FD, false>(az, 0, 0, 0), a_dm<FD, false>(az, 1, 0, 0));
-                const float2 un = fma2(bz2[r], w_dm2<FD>(wxz, r), fma2(bx2[r], dxx, u2));
-                const float2 vn = fma2(bz2[r], w_dp2<FD>(wzz, r), fma2(bx2[r], dxxz, v2));
-                const long long o = (long long)i * g.P + jb;
-                *reinterpret_cast<float2 *>(U + o) = un;
-                *reinterpret_cast<float2 *>(V + o) = vn;
-            }
-        } else {
-            const int ssx = sh.sx[s], ssz = sh.sz[s], stype = sh.type[s];
-            float *pSXX = px_ptr(g, PX, s, PX_SXX), *pSXZx = px_ptr(g, PX, s, PX_SXZ);
-            float *pSXZz = pz_ptr(g, PZ, s, PZ_SXZ), *pSZZ = pz_ptr(g, PZ, s, PZ_SZZ);
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                float ax[10], az[10];
-                xrow(ax, sxx, q);
-                xrow(az, sxz, q);
-                const int zs = zstrip_index(g, i);
-                // this row's C-PML memories, requested before the stencils
-                float pxo[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, pzo[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-                float zb = 0.f, za = 0.f, zik = 1.f;
-                if (i < g.nz - 1) {
-#pragma unroll
-                    for (int cc = 0; cc < 2; ++cc) {
-                        const int j = jb + cc;
-                        if (j < 1 || j >= g.nx - 1) continue;
-                        if (xs[cc] >= 0) {
-                            const int px = i * g.xs_n + xs[cc];
-                            pxo[cc][0] = pSXX[px];
-                            pxo[cc][1] = pSXZx[px];
-                        }
-                        if (zs >= 0) {
-                            const int pz = zs * g.P + j;
-                            pzo[cc][0] = pSXZz[pz];
-                            pzo[cc][1] = pSZZ[pz];
-                        }
-                    }
-                    if (zs >= 0) { zb = m.bz[i]; za = m.az[i]; zik = m.ikz[i]; }
-                }
-                const float2 u2 = *reinterpret_cast<const float2 *>(own + (ty * RPT + r) * TX4 + 2 * tx);
-                const float2 v2 = *reinterpret_cast<const float2 *>(own + (T::TZH + ty * RPT + r) * TX4 + 2 * tx);
-                const float u[2] = {u2.x, u2.y}, v[2] = {v2.x, v2.y};
-                const float4 czm = zt[ty * RPT + r], czp = zt[T::TZH + ty * RPT + r];
-                float un[2], vn[2];
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int j = jb + cc;
-                    un[cc] = u[cc];
-                    vn[cc] = v[cc];
-                    if (i >= g.nz - 1 || j < 1 || j >= g.nx - 1) continue;
-                    float dxx = a_dp_t<FD>(ax, cc, xt[2 * tx + cc]);
-                    float dxxz = a_dm_t<FD>(az, cc, xt[TX4 + 2 * tx + cc]);
-                    float dzxz = (g.fs && i == 0) ? 2.f * cf<FD>(1) * f2c(wxz[r + K], cc) : w_dm_t<FD>(wxz, r, cc, czm);
-                    float dzz = w_dp_t<FD>(wzz, r, cc, czp);
-                    if (xs[cc] >= 0) {
-                        const int px = i * g.xs_n + xs[cc];
-                        dxx = pml_fwd_pre(dxx, bxv[cc], axv[cc], ikxv[cc], pxo[cc][0], pSXX + px);
-                        dxxz = pml_fwd_pre(dxxz, bxv[cc], axv[cc], ikxv[cc], pxo[cc][1], pSXZx + px);
-                    }
-                    if (zs >= 0) {
-                        const int pz = zs * g.P + j;
-                        dzxz = pml_fwd_pre(dzxz, zb, za, zik, pzo[cc][0], pSXZz + pz);
-                        dzz = pml_fwd_pre(dzz, zb, za, zik, pzo[cc][1], pSZZ + pz);
-                    }
-                    const float bxc = cc ? bx2[r].y : bx2[r].x, bzc = cc ? bz2[r].y : bz2[r].x;
-                    un[cc] = u[cc] + bxc * dxx + bzc * dzxz;
-                    float vv = v[cc] + bxc * dxxz + bzc * dzz;
-                    if (stype == 0 && i == ssz && j == ssx) vv = vv + sh.fcoef[s] * sh.wav[(long long)s * g.nt + n];
-                    vn[cc] = vv;
-                }
-                // cells outside the update region keep their value (column 0, nx-1, row nz-1)
-                if (i < g.nz - 1 && jb < g.nx) {
-                    const long long o = (long long)i * g.P + jb;
-                    if (jb + 1 < g.nx) {
-                        *reinterpret_cast<float2 *>(U + o) = make_float2(un[0], un[1]);
-                        *reinterpret_cast<float2 *>(V + o) = make_float2(vn[0], vn[1]);
-                    } else {
-                        U[o] = un[0];
-                        V[o] = vn[0];
-                    }
-                }
-            }
+        if (ring_leave(ring, st, it + NST < nit)) {
+            Cursor u;
+            u.init(w, first + it + NST);
+            issue(u, st);
         }
-        fence_async_shared();
-        __syncthreads();
-        if (tid == 0 && it + 2 < nsh) {
-            mbar_arrive_expect_tx(bar + (it & 1), 3 * SN * 4 + OWNB);
-            tma_load_4d(S, &tmS, bar + (it & 1), c.j0 - XO4, c.i0 - K, F_EX, s + 2);
-            tma_load_4d(S + T::S3, &tmUo, bar + (it & 1), c.j0, c.i0, F_U, s + 2);
-        }
+        if (++st == NST) { st = 0; ph ^= 1; }
+        if (c.next(w)) enter();
     }
 }
 
@@ -427,1022 +586,907 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
 
 template <int FD, int RPT, bool ENERGY>
 __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
-    st_fwd_str(Geo g, Mat m, Shots sh, Recv rv, float *F, float *PX, float *PZ, int n, int spg, int tiles_x,
-               FwdOut out, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmSo)
+    st_fwd_str(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh,
+               const __grid_constant__ Recv rv, float *F, float *PX, float *PZ, int n, const __grid_constant__ Work w,
+               const __grid_constant__ FwdOut out, const __grid_constant__ CUtensorMap tmV,
+               const __grid_constant__ CUtensorMap tmSo)
 {
     using T = G4<FD, RPT>;
-    constexpr int K = T::K, SN = T::SN;
-    constexpr int STG = L4<FD, RPT>::STR_STAGE, OWNB = 3 * T::TZH * TX4 * 4;
+    using Sg = Stage<FD, RPT>;
+    constexpr int K = T::K, SN = T::SN, STG = Sg::STR, NST = Sg::NSTR, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
-    // coefficient tables: x sets (D- of U, D+ of V), z sets (D- of V, D+ of U)
-    float4 *xt = reinterpret_cast<float4 *>(sm + L4<FD, RPT>::STR);
-    float4 *zt = xt + 2 * TX4;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L5<FD, RPT>::STR);
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const Ctx3 c = ctx5(g, spg, T::TZH, tiles_x, g.tordA, g.theavyA);
-    const int nsh = c.s1 - c.s0;
-    if (nsh <= 0) return;
-    if (tid == 0) {
-        mbar_init(bar + 0, 1); mbar_init(bar + 1, 1);
-        fence_async_shared();
-        for (int b = 0; b < 2 && b < nsh; ++b) {
-            mbar_arrive_expect_tx(bar + b, 2 * SN * 4 + OWNB);
-            tma_load_4d(sm + b * STG, &tmV, bar + b, c.j0 - XO4, c.i0 - K, F_U, c.s0 + b);
-            tma_load_4d(sm + b * STG + T::S2, &tmSo, bar + b, c.j0, c.i0, F_EX, c.s0 + b);
-        }
-    }
-    for (int t = tid; t < 2 * TX4; t += NTHR) {
-        const int j = c.j0 + t % TX4;
-        xt[t] = t < TX4 ? cv_M<FD>(j, g.nx) : cv_P<FD>(j, g.nx);
-    }
-    for (int t = tid; t < 2 * T::TZH; t += NTHR) {
-        const int i = c.i0 + t % T::TZH;
-        zt[t] = t < T::TZH ? cv_M<FD>(i, g.nz) : cv_P<FD>(i, g.nz);
-    }
-    __syncthreads();
-    const int jb = c.j0 + 2 * tx;
-    int xs[2];
-    float bxv[2], axv[2], ikxv[2], Lr0[2];
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-        const int j = jb + cc;
-        xs[cc] = (j < g.nx) ? xstrip_index(g, j) : -1;
-        bxv[cc] = xs[cc] >= 0 ? m.bx[j] : 0.f;
-        axv[cc] = xs[cc] >= 0 ? m.ax[j] : 0.f;
-        ikxv[cc] = xs[cc] >= 0 ? m.ikx[j] : 1.f;
-        Lr0[cc] = (g.fs && j < g.nx) ? m.Lr[j] : 0.f;
-    }
-    float2 ml2m[RPT], ml[RPT], mm2[RPT];
+    FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
+    Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    auto issue = [&](const Cursor &u, int st) {
+        mbar_arrive_expect_tx(ring->full + st, (2 * SN + 3 * PL) * 4);
+        tma_load_4d(sm + st * STG, &tmV, ring->full + st, u.j0() - XO4, u.i0(T::TZH) - K, F_U, u.shot);
+        tma_load_4d(sm + st * STG + T::S2, &tmSo, ring->full + st, u.j0(), u.i0(T::TZH), F_EX, u.shot);
+    };
+    Cursor c;
+    int first, nit;
+    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
+    bool xin = false, zin = false;   // as in st_fwd_vel
+    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+    float2 ml2m[RPT], ml[RPT], mm[RPT];
     constexpr int RG = ENERGY ? RPT : 1;
     double eacc[RG][2];
+    auto enter = [&]() {
+        jb = c.j0() + 2 * tx;
+        e0 = tab_at(jb, g.nx);
+        e1 = tab_at(jb + 1, g.nx);
+        iw = c.i0(T::TZH) + ty * RPT;
+        xin = cols_plain(g, c.j0(), g.pad, g.pad);
+        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
+        r0 = rv.tile_start[c.tile(w)];
+        r1 = rv.tile_start[c.tile(w) + 1];
 #pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        float a[2], b[2], d[2];
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int i = c.i0 + ty * RPT + r, j = jb + cc;
-            const long long o = (long long)i * g.P + j;
-            const bool ok = i < g.nz && j < g.nx;
-            a[cc] = ok ? m.L2M[o] : 0.f;
-            b[cc] = ok ? m.L[o] : 0.f;
-            d[cc] = ok ? 2.f * m.M[o] : 0.f;
-            if (r < RG) eacc[r][cc] = 0.0;
+        for (int r = 0; r < RPT; ++r) {
+            ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
+            ml[r] = mat_pair(g, m.L, iw + r, jb);
+            mm[r] = mat_pair(g, m.M, iw + r, jb);
         }
-        ml2m[r] = make_float2(a[0], a[1]);
-        ml[r] = make_float2(b[0], b[1]);
-        mm2[r] = make_float2(d[0], d[1]);
-    }
+#pragma unroll
+        for (int r = 0; r < RG; ++r) eacc[r][0] = eacc[r][1] = 0.0;
+    };
+    // energy sums of a tile's shots, when the block leaves the tile
+    auto leave = [&]() {
+        if constexpr (ENERGY) {
+#pragma unroll
+            for (int r = 0; r < RG; ++r)
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc)
+                    if (iw + r < g.nz && jb + cc < g.nx)
+                        atomicAdd(out.energy + (long long)(iw + r) * g.nx + jb + cc, eacc[r][cc]);
+        }
+    };
+    enter();
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
     // history rows as float pairs when every pair starts on 8 bytes
     const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;
-
-    const bool plain = tile_plain4(g, c.i0, c.j0, T::TZH, T::M);
-    for (int it = 0; it < nsh; ++it) {
-        const int s = c.s0 + it;
-        float *S = sm + (it & 1) * STG;
-        const float *own = S + T::S2;   // [sxx, szz, sxz][TZH][TX4] of the tile's own cells
+    int st = 0, ph = 0;
+    for (int it = 0; it < nit; ++it) {
+        const int s = c.shot;
+        const int4 src = __ldg(sh.pos + s);
+        const float *S = sm + st * STG, *own = S + T::S2;   // own: [sxx, szz, sxz][TZH][TX4] of the tile's own cells
         float *sxx = F + ((long long)s * F_N + F_EX) * g.fstride;
         float *szz = F + ((long long)s * F_N + F_EZ) * g.fstride;
         float *sxz = F + ((long long)s * F_N + F_ES) * g.fstride;
-        if (!__syncthreads_and(mbar_wait_bounded(bar + (it & 1), (it >> 1) & 1, g.wait_polls))) {
-            abort3(bar, it, nsh, out.status);
-            return;
-        }
-        const float *sU = S, *sV = S + SN;
-        float2 wU[T::W], wV[T::W];
-        zwin2p<T::W, RPT>(wU, sU, ty, tx);
-        zwin2p<T::W, RPT>(wV, sV, ty, tx);
+        float *pDXU = px_ptr(g, PX, s, PX_DXU), *pDXV = px_ptr(g, PX, s, PX_DXV);
+        float *pDZV = pz_ptr(g, PZ, s, PZ_DZV), *pDZU = pz_ptr(g, PZ, s, PZ_DZU);
         float *snap_s = out.snap ? out.snap + ((long long)s * out.slots + out.slot) * g.snf * g.nd : nullptr;
-        if (plain && !in_tile4(sh.sz[s], sh.sx[s], c.i0, c.j0, T::TZH)) {
-            // interior tile without this shot's source: no guards, paired arithmetic
+        auto rows = [&](auto gd, auto xb) -> bool {
+            constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
+            int2 xs = make_int2(-1, -1);
+            if (XB) {
+                xs = xstrip_pair(g, jb);
+                prefetch_x<RPT>(g, iw, xs, pDXU, pDXV);
+                prefetch_l1(g.pmx + jb);
+            }
+            if (GUARD) {
+                prefetch_z<RPT>(g, iw, jb, pDZV, pDZU);
+                prefetch_l1(g.pmz + iw);
+            }
+            if (!mbar_wait_bounded(ring->full + st, ph, g.wait_polls)) return false;
+            float2 dzv_[RPT], dzu_[RPT];
+            {
+                float2 wn[T::W];
+                zwin<T::W, RPT>(wn, S + SN, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) dzv_[r] = z_dm<FD, GUARD>(wn, r, &tab->z[1][tab_at(iw + r, g.nz)]);
+                zwin<T::W, RPT>(wn, S, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) dzu_[r] = z_dp<FD, GUARD>(wn, r, &tab->z[0][tab_at(iw + r, g.nz)]);
+            }
 #pragma unroll
             for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                const int qo = (ty * RPT + r) * TX4 + 2 * tx;
-                const float2 e1 = *reinterpret_cast<const float2 *>(own + qo);
-                const float2 e2 = *reinterpret_cast<const float2 *>(own + T::TZH * TX4 + qo);
-                const float2 e3 = *reinterpret_cast<const float2 *>(own + 2 * T::TZH * TX4 + qo);
-                float au[10], av[10];
-                xrow(au, sU, q);
-                xrow(av, sV, q);
-                const float2 dxu = make_float2(a_dm<FD, false>(au, 0, 0, 0), a_dm<FD, false>(au, 1, 0, 0));
-                const float2 dxv = make_float2(a_dp<FD, false>(av, 0, 0, 0), a_dp<FD, false>(av, 1, 0, 0));
-                const float2 dex = mul2(dtdx2, dxu), dez = mul2(dtdz2, w_dm2<FD>(wV, r));
-                const float2 des = mul2(dup2(0.5f), fma2(dtdx2, dxv, mul2(dtdz2, w_dp2<FD>(wU, r))));
-                const float2 axx = fma2(ml[r], dez, fma2(ml2m[r], dex, e1));
-                const float2 azz = fma2(ml2m[r], dez, fma2(ml[r], dex, e2));
-                const float2 axz = fma2(mm2[r], des, e3);
-                if (snap_s) {
-                    float *sp = snap_s + (long long)(i - g.z0) * g.nx_dom + (jb - g.pad);
+                const int i = iw + r, zr = ty * RPT + r, q = (zr + K) * SW4 + XO4 + 2 * tx, qo = zr * TX4 + 2 * tx;
+                if (GUARD && i >= g.nz) continue;
+                const bool last = GUARD && i >= g.nz - 1;
+                float a[10];
+                // column 0 has no D- term, column nx - 1 no D+ term: their
+                // derivatives and memories stay zero
+                xrow(a, S, q);
+                float2 dxu = x_dm<FD, XB>(a, tab->x[1], e0, e1);
+                const float2 uu = make_float2(a[4], a[5]);
+                xrow(a, S + SN, q);
+                float2 dxv = x_dp<FD, XB>(a, tab->x[0], e0, e1);
+                const float2 vv = make_float2(a[4], a[5]);
+                float2 dzv = dzv_[r], dzu = dzu_[r];
+                const float2 e1 = pair_at(own + qo), e2 = pair_at(own + PL + qo), e3 = pair_at(own + 2 * PL + qo);
+                if (last) dxv = make_float2(0.f, 0.f);
+                if (XB) {
+                    const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
+                    const float2 m0 = mem_x(pDXU + i * g.xs_n, xs), m1 = mem_x(pDXV + i * g.xs_n, xs);
+                    pml_x2(dxu, c0, c1, xs, m0, pDXU + i * g.xs_n);
+                    if (!last) pml_x2(dxv, c0, c1, xs, m1, pDXV + i * g.xs_n);
+                }
+                if (GUARD) {
+                    if (g.fs && i == 0) {
+                        // the free surface fixes d(vz)/dz
+                        dzv.x = ((!XB || jb < g.nx) ? m.Lr[jb] : 0.f) * dxu.x * g.dzdx;
+                        dzv.y = ((!XB || jb + 1 < g.nx) ? m.Lr[jb + 1] : 0.f) * dxu.y * g.dzdx;
+                    }
+                    if (XB) {
+                        if (jb >= g.nx - 1) dzv.x = 0.f;
+                        if (jb + 1 >= g.nx - 1) dzv.y = 0.f;
+                        if (jb < 1) dzu.x = 0.f;
+                    }
+                    const float4 zc = ldt(g.pmz + i);
+                    const int zs = __float_as_int(zc.w);
+                    if (zs >= 0 && (!XB || jb < g.nx)) {
+                        const float2 m0 = pair_at(pDZV + zs * g.P + jb), m1 = pair_at(pDZU + zs * g.P + jb);
+                        pml_z2(dzv, zc, m0, pDZV + zs * g.P + jb);
+                        pml_z2(dzu, zc, m1, pDZU + zs * g.P + jb);
+                    }
+                }
+                const float2 dex = mul2(dtdx2, dxu), dez = mul2(dtdz2, dzv);
+                float2 des = mul2(dup2(0.5f), fma2(dtdx2, dxv, mul2(dtdz2, dzu)));
+                if (last) des = make_float2(0.f, 0.f);
+                if (XB) {
+                    if (jb >= g.nx - 1) des.x = 0.f;
+                    if (jb + 1 >= g.nx - 1) des.y = 0.f;
+                }
+                float2 axx = fma2(ml[r], dez, fma2(ml2m[r], dex, e1));
+                float2 azz = fma2(ml2m[r], dez, fma2(ml[r], dex, e2));
+                const float2 axz = fma2(mul2(dup2(2.f), mm[r]), des, e3);
+                if (src.x == i && src.z == 1) {   // moment source
+                    const int sj = src.y - jb;
+                    const float stm = sh.wav[(long long)s * g.nt + n] * g.dt / sh.mcoef[s];
+                    const float f = sj == 0 ? ml2m[r].x + ml[r].x : ml2m[r].y + ml[r].y;
+                    add_at(axx, sj, f * stm);
+                    add_at(azz, sj, f * stm);
+                }
+                const int pi = i - g.z0, pj = jb - g.pad;
+                if (snap_s && (!GUARD || (pi >= 0 && pi < g.nz_dom))) {
+                    float *sp = snap_s + (long long)pi * g.nx_dom + pj;
+                    const bool px0 = !XB || (pj >= 0 && pj < g.nx_dom), px1 = !XB || (pj + 1 >= 0 && pj + 1 < g.nx_dom);
                     if (hist2) {
-                        __stcs(reinterpret_cast<float2 *>(sp), axx);
-                        __stcs(reinterpret_cast<float2 *>(sp + g.nd), azz);
-                        __stcs(reinterpret_cast<float2 *>(sp + 2 * g.nd), axz);
-                        if (g.snf == 5) {   // velocities of this step (density gradient)
-                            __stcs(reinterpret_cast<float2 *>(sp + 3 * g.nd), make_float2(au[4], au[5]));
-                            __stcs(reinterpret_cast<float2 *>(sp + 4 * g.nd), make_float2(av[4], av[5]));
+                        if (px0) {   // an even pair is inside or outside as a whole
+                            __stcs(reinterpret_cast<float2 *>(sp), axx);
+                            __stcs(reinterpret_cast<float2 *>(sp + g.nd), azz);
+                            __stcs(reinterpret_cast<float2 *>(sp + 2 * g.nd), axz);
+                            if (g.snf == 5) {   // velocities of this step (density gradient)
+                                __stcs(reinterpret_cast<float2 *>(sp + 3 * g.nd), uu);
+                                __stcs(reinterpret_cast<float2 *>(sp + 4 * g.nd), vv);
+                            }
                         }
                     } else {
-                        __stcs(sp, axx.x); __stcs(sp + 1, axx.y);
-                        __stcs(sp + g.nd, azz.x); __stcs(sp + g.nd + 1, azz.y);
-                        __stcs(sp + 2 * g.nd, axz.x); __stcs(sp + 2 * g.nd + 1, axz.y);
-                        if (g.snf == 5) {
-                            __stcs(sp + 3 * g.nd, au[4]); __stcs(sp + 3 * g.nd + 1, au[5]);
-                            __stcs(sp + 4 * g.nd, av[4]); __stcs(sp + 4 * g.nd + 1, av[5]);
+                        if (px0) {
+                            __stcs(sp, axx.x); __stcs(sp + g.nd, azz.x); __stcs(sp + 2 * g.nd, axz.x);
+                            if (g.snf == 5) { __stcs(sp + 3 * g.nd, uu.x); __stcs(sp + 4 * g.nd, vv.x); }
+                        }
+                        if (px1) {
+                            __stcs(sp + 1, axx.y); __stcs(sp + g.nd + 1, azz.y); __stcs(sp + 2 * g.nd + 1, axz.y);
+                            if (g.snf == 5) { __stcs(sp + 3 * g.nd + 1, uu.y); __stcs(sp + 4 * g.nd + 1, vv.y); }
                         }
                     }
+                }
+                if (GUARD && out.row0 && g.fs && i == 0) {
+                    float *rp = out.row0 + ((long long)s * out.slots + out.slot_row0) * g.nx_dom + pj;
+                    if (!XB || (pj >= 0 && pj < g.nx_dom)) rp[0] = dxu.x;
+                    if (!XB || (pj + 1 >= 0 && pj + 1 < g.nx_dom)) rp[1] = dxu.y;
                 }
                 if (ENERGY) {
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc) {
+                        if (XB && jb + cc >= g.nx) continue;
                         float f;
                         if (out.energy_comp < 2) {
-                            f = out.energy_comp == 0 ? au[4 + cc] : av[4 + cc];
+                            f = out.energy_comp == 0 ? f2c(uu, cc) : f2c(vv, cc);
                         } else {
                             float ex, ez, es;
                             strains_of(f2c(axx, cc), f2c(azz, cc), f2c(axz, cc), f2c(ml2m[r], cc), f2c(ml[r], cc),
-                                       0.5f * f2c(mm2[r], cc), ex, ez, es);
+                                       f2c(mm[r], cc), ex, ez, es);
                             f = out.energy_comp == 2 ? ex : ez;
                         }
                         eacc[r % RG][cc] += (double)f * (double)f;
                     }
                 }
                 const long long o = (long long)i * g.P + jb;
-                *reinterpret_cast<float2 *>(sxx + o) = axx;
-                *reinterpret_cast<float2 *>(szz + o) = azz;
-                *reinterpret_cast<float2 *>(sxz + o) = axz;
+                store_pair<XB>(sxx + o, axx, g.nx - jb);
+                store_pair<XB>(szz + o, azz, g.nx - jb);
+                store_pair<XB>(sxz + o, axz, g.nx - jb);
             }
-        } else {
-            const int ssx = sh.sx[s], ssz = sh.sz[s], stype = sh.type[s];
-            float *pDXU = px_ptr(g, PX, s, PX_DXU), *pDXV = px_ptr(g, PX, s, PX_DXV);
-            float *pDZV = pz_ptr(g, PZ, s, PZ_DZV), *pDZU = pz_ptr(g, PZ, s, PZ_DZU);
-#pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                if (i >= g.nz) continue;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                const int qo = (ty * RPT + r) * TX4 + 2 * tx;
-                const float2 a2 = *reinterpret_cast<const float2 *>(own + qo);
-                const float2 b2 = *reinterpret_cast<const float2 *>(own + T::TZH * TX4 + qo);
-                const float2 d2 = *reinterpret_cast<const float2 *>(own + 2 * T::TZH * TX4 + qo);
-                const float e1[2] = {a2.x, a2.y}, e2[2] = {b2.x, b2.y}, e3[2] = {d2.x, d2.y};
-                float au[10], av[10];
-                xrow(au, sU, q);
-                xrow(av, sV, q);
-                const int zs = zstrip_index(g, i);
-                // this row's C-PML memories, requested before the stencils
-                float pxo[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, pzo[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-                float zb = 0.f, za = 0.f, zik = 1.f;
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int j = jb + cc;
-                    if (j >= g.nx) continue;
-                    if (xs[cc] >= 0) {
-                        const int px = i * g.xs_n + xs[cc];
-                        if (j >= 1) pxo[cc][0] = pDXU[px];
-                        if (i < g.nz - 1) pxo[cc][1] = pDXV[px];
-                    }
-                    if (zs >= 0) {
-                        const int pz = zs * g.P + j;
-                        if (j < g.nx - 1) pzo[cc][0] = pDZV[pz];
-                        if (j >= 1) pzo[cc][1] = pDZU[pz];
-                    }
-                }
-                if (zs >= 0) { zb = m.bz[i]; za = m.az[i]; zik = m.ikz[i]; }
-                const float4 czm = zt[ty * RPT + r], czp = zt[T::TZH + ty * RPT + r];
-                float nxx[2], nzz[2], nxz[2];
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int j = jb + cc;
-                    nxx[cc] = e1[cc]; nzz[cc] = e2[cc]; nxz[cc] = e3[cc];
-                    if (j >= g.nx) continue;
-                    float dxu = a_dm_t<FD>(au, cc, xt[2 * tx + cc]);
-                    float dxv = a_dp_t<FD>(av, cc, xt[TX4 + 2 * tx + cc]);
-                    float dzv = w_dm_t<FD>(wV, r, cc, czm);
-                    float dzu = w_dp_t<FD>(wU, r, cc, czp);
-                    const int px = i * g.xs_n + xs[cc], pz = zs * g.P + j;
-                    if (j >= 1 && xs[cc] >= 0)
-                        dxu = pml_fwd_pre(dxu, bxv[cc], axv[cc], ikxv[cc], pxo[cc][0], pDXU + px);
-                    if (j < g.nx - 1) {
-                        if (g.fs && i == 0) dzv = Lr0[cc] * dxu * g.dzdx;
-                        if (zs >= 0) dzv = pml_fwd_pre(dzv, zb, za, zik, pzo[cc][0], pDZV + pz);
-                    } else {
-                        dzv = 0.f;
-                    }
-                    if (j >= 1) {
-                        if (zs >= 0) dzu = pml_fwd_pre(dzu, zb, za, zik, pzo[cc][1], pDZU + pz);
-                    } else {
-                        dzu = 0.f;
-                    }
-                    if (i < g.nz - 1) {
-                        if (xs[cc] >= 0) dxv = pml_fwd_pre(dxv, bxv[cc], axv[cc], ikxv[cc], pxo[cc][1], pDXV + px);
-                    } else {
-                        dxv = 0.f;
-                    }
-                    const float dex = j >= 1 ? g.dtdx * dxu : 0.f;
-                    const float dez = g.dtdz * dzv;
-                    const float des = (i < g.nz - 1 && j < g.nx - 1) ? 0.5f * (g.dtdz * dzu + g.dtdx * dxv) : 0.f;
-                    const float l2m = f2c(ml2m[r], cc), l = f2c(ml[r], cc);
-                    float axx = e1[cc] + l2m * dex + l * dez;
-                    float azz = e2[cc] + l * dex + l2m * dez;
-                    const float axz = e3[cc] + f2c(mm2[r], cc) * des;
-                    if (stype == 1 && i == ssz && j == ssx) {
-                        const float stm = sh.wav[(long long)s * g.nt + n] * g.dt / sh.mcoef[s];
-                        axx = axx + (l2m + l) * stm;
-                        azz = azz + (l + l2m) * stm;
-                    }
-                    nxx[cc] = axx; nzz[cc] = azz; nxz[cc] = axz;
-                    const int pi = i - g.z0, pj = j - g.pad;
-                    const bool phys = pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom;
-                    if (snap_s && phys) {
-                        float *sp = snap_s + (long long)pi * g.nx_dom + pj;
-                        __stcs(sp, axx);
-                        __stcs(sp + g.nd, azz);
-                        __stcs(sp + 2 * g.nd, axz);
-                        if (g.snf == 5) {   // velocities of this step (density gradient)
-                            __stcs(sp + 3 * g.nd, au[4 + cc]);
-                            __stcs(sp + 4 * g.nd, av[4 + cc]);
-                        }
-                    }
-                    if (out.row0 && g.fs && i == 0 && pj >= 0 && pj < g.nx_dom)
-                        out.row0[((long long)s * out.slots + out.slot_row0) * g.nx_dom + pj] = dxu;
-                    if (ENERGY) {
-                        float f;
-                        if (out.energy_comp < 2) {
-                            f = out.energy_comp == 0 ? au[4 + cc] : av[4 + cc];
-                        } else {
-                            float ex, ez, es;
-                            strains_of(axx, azz, axz, l2m, l, 0.5f * f2c(mm2[r], cc), ex, ez, es);
-                            f = out.energy_comp == 2 ? ex : ez;
-                        }
-                        eacc[r % RG][cc] += (double)f * (double)f;
-                    }
-                }
-                if (jb < g.nx) {
-                    const long long o = (long long)i * g.P + jb;
-                    if (jb + 1 < g.nx) {
-                        *reinterpret_cast<float2 *>(sxx + o) = make_float2(nxx[0], nxx[1]);
-                        *reinterpret_cast<float2 *>(szz + o) = make_float2(nzz[0], nzz[1]);
-                        *reinterpret_cast<float2 *>(sxz + o) = make_float2(nxz[0], nxz[1]);
-                    } else {
-                        sxx[o] = nxx[0]; szz[o] = nzz[0]; sxz[o] = nxz[0];
-                    }
-                }
+            return true;
+        };
+        if (!(!xin ? rows(std::true_type{}, std::true_type{})
+                   : !zin ? rows(std::true_type{}, std::false_type{}) : rows(std::false_type{}, std::false_type{}))) {
+            ring_abort(ring, it, out.status);
+            return;
+        }
+        if (ring_leave(ring, st, it + NST < nit)) {
+            Cursor u;
+            u.init(w, first + it + NST);
+            issue(u, st);
+        }
+        if (++st == NST) { st = 0; ph ^= 1; }
+        if (r1 > r0) {
+            // receivers on this warp's rows, which its own lanes have just written
+            __syncwarp();
+            const float *U = F + ((long long)s * F_N + F_U) * g.fstride;
+            const float *V = F + ((long long)s * F_N + F_V) * g.fstride;
+            for (int qq = r0 + tx; qq < r1; qq += TX) {
+                const int rid = rv.tile_rec[qq], ri = rv.rz[rid];
+                if (ri < iw || ri >= iw + RPT) continue;
+                const long long o = (long long)ri * g.P + rv.rx[rid];
+                float ex, ez, es;
+                strains_of(sxx[o], szz[o], sxz[o], m.L2M[o], m.L[o], m.M[o], ex, ez, es);
+                const float v0 = U[o], v1 = V[o];
+                float *dst = out.rec + (long long)s * 4 * g.nt * g.nrec + (long long)n * g.nrec + rid;
+                dst[0] = v0;
+                dst[(long long)g.nt * g.nrec] = v1;
+                dst[2LL * g.nt * g.nrec] = ex;
+                dst[3LL * g.nt * g.nrec] = ez;
+                if (!(isfinite(v0) && isfinite(v1) && isfinite(ex) && isfinite(ez))) atomicOr(out.status, 1);
             }
         }
-        fence_async_shared();
-        __syncthreads();
-        if (tid == 0 && it + 2 < nsh) {
-            mbar_arrive_expect_tx(bar + (it & 1), 2 * SN * 4 + OWNB);
-            tma_load_4d(S, &tmV, bar + (it & 1), c.j0 - XO4, c.i0 - K, F_U, s + 2);
-            tma_load_4d(S + T::S2, &tmSo, bar + (it & 1), c.j0, c.i0, F_EX, s + 2);
-        }
-        const int r0 = rv.tile_start[c.tile], r1 = rv.tile_start[c.tile + 1];
-        const float *U = F + ((long long)s * F_N + F_U) * g.fstride;
-        const float *V = F + ((long long)s * F_N + F_V) * g.fstride;
-        for (int qq = r0 + tid; qq < r1; qq += NTHR) {
-            const int rid = rv.tile_rec[qq];
-            const long long o = (long long)rv.rz[rid] * g.P + rv.rx[rid];
-            float ex, ez, es;
-            strains_of(sxx[o], szz[o], sxz[o], m.L2M[o], m.L[o], m.M[o], ex, ez, es);
-            const float v0 = U[o], v1 = V[o];
-            float *dst = out.rec + (long long)s * 4 * g.nt * g.nrec + (long long)n * g.nrec + rid;
-            dst[0] = v0;
-            dst[(long long)g.nt * g.nrec] = v1;
-            dst[2LL * g.nt * g.nrec] = ex;
-            dst[3LL * g.nt * g.nrec] = ez;
-            if (!(isfinite(v0) && isfinite(v1) && isfinite(ex) && isfinite(ez))) atomicOr(out.status, 1);
-        }
-    }
-    if (ENERGY) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                const int i = c.i0 + ty * RPT + r, j = jb + cc;
-                if (i < g.nz && j < g.nx) atomicAdd(out.energy + (long long)i * g.nx + j, eacc[r][cc]);
-            }
+        if (c.last(w) || it + 1 == nit) leave();
+        if (c.next(w)) enter();
     }
 }
+
+// ------------------------------------------------------------- adjoint
+//
+// The transposed C-PML acts on the values that a transposed stencil then
+// gathers, so a reader next to a strip needs the image of its neighbours'
+// cells.  The writer makes it: each strain (velocity) update, holding the new
+// value and the memory of its own cells in registers, also stores the images
+// that the next velocity (strain) update will differentiate, in arrays that
+// cover only the cells some strip-touching box reads ([jl, jr) x [it, ib) is
+// left out): x images in bands of columns, z images in bands of rows.  The
+// memories are then private to a cell's owner, one copy each.
+
+// does the staged box of a tile touch an x strip / a z strip
+__device__ __forceinline__ bool box_x(const Geo &g, int j0)
+{
+    return j0 - XO4 < g.pad || j0 + TX4 + XO4 > g.nx - g.pad;
+}
+__device__ __forceinline__ bool box_z(const Geo &g, int i0, int tzh, int K)
+{
+    return i0 + tzh + K > g.nz - g.pad || (!g.fs && i0 - K < g.pad);
+}
+// place of column j / row i in the image bands
+__device__ __forceinline__ int band_x(const Geo &g, int j) { return j < g.jl ? j : j - g.jr + g.jl; }
+__device__ __forceinline__ int band(int i, int lo, int hi) { return i < lo ? i : i - hi + lo; }
 
 // ------------------------------------------------------------- adjoint: P = B U_a, Q = B V_a
 
 template <int FD, int RPT>
 __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
-    st_adj_a(Geo g, Mat m, Recv rv, float *A, float *PX, float *PZ, int n, int spg, int tiles_x, AdjIn in,
-             int *status, const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmPQo)
+    st_adj_a(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Recv rv, float *A,
+             float *PX, float *PZ, const __grid_constant__ Images im, int n, const __grid_constant__ Work w,
+             const __grid_constant__ AdjIn in, int *status,
+             const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmPQo,
+             const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ)
 {
+    constexpr int SNA = al32_3(G4<FD, RPT>::SN), SOWN = al32_3(4 * SNA);
     using T = G4<FD, RPT>;
-    constexpr int K = T::K, SN = T::SN, SH = T::SH;
-    constexpr int STG = L4<FD, RPT>::ADA_STAGE, OWNB = 2 * T::TZH * TX4 * 4;
+    using Sg = Stage<FD, RPT>;
+    constexpr int K = T::K, SN = T::SN, STG = Sg::ADA, NST = Sg::NADA, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
-    constexpr int NCC = (SW4 + TX - 1) / TX;
-    float *aDxV = sm + 2 * STG;
-    float *tab = aDxV + T::S1;
-    // coefficient tables: x sets (A, B of the transposed D- of exx_a, A, B of
-    // the transposed D+ of exz_a), z sets (A, B of the transposed D+ of exz_a,
-    // A, B of the transposed D- of ezz_a)
-    float4 *xt = reinterpret_cast<float4 *>(sm + L4<FD, RPT>::ADA);
-    float4 *zt = xt + 4 * TX4;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L5<FD, RPT>::ADA);
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const Ctx3 c = ctx5(g, spg, T::TZH, tiles_x, g.tordA, g.theavyA);
-    const int nsh = c.s1 - c.s0;
-    if (nsh <= 0) return;
-    if (tid == 0) {
-        mbar_init(bar + 0, 1); mbar_init(bar + 1, 1);
-        fence_async_shared();
-        for (int b = 0; b < 2 && b < nsh; ++b) {
-            mbar_arrive_expect_tx(bar + b, 3 * SN * 4 + OWNB);
-            tma_load_4d(sm + b * STG, &tmE, bar + b, c.j0 - XO4, c.i0 - K, F_EX, c.s0 + b);
-            tma_load_4d(sm + b * STG + T::S3, &tmPQo, bar + b, c.j0, c.i0, F_U, c.s0 + b);
+    AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
+    Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    // planes of the staged box: what the step differentiates.  Away from the
+    // C-PML strips these are the strain adjoints themselves; where the box
+    // touches a strip, their transposed-C-PML images (adj_b writes them), x
+    // and z images separately, and the exz image for x is a plane of its own.
+    auto issue = [&](const Cursor &u, int st) {
+        const bool bx = box_x(g, u.j0()), bz = box_z(g, u.i0(T::TZH), T::TZH, K);
+        constexpr int PB = SN * 4, OB = 2 * T::TZH * TX4 * 4;
+        uint64_t *bar = ring->full + st;
+        float *d = sm + st * STG;
+        const int s = u.shot, x = u.j0() - XO4, y = u.i0(T::TZH) - K;
+        const int xi = x >= g.jr ? x - g.jr + g.jl : x, yi = y >= g.iba ? y - g.iba + g.ita : y;
+        mbar_arrive_expect_tx(bar, (bx || bz ? 4 : 3) * PB + OB);
+        if (bx) tma_load_4d(d, &tmX, bar, xi, y, 0, s);
+        else tma_load_4d(d, &tmE, bar, x, y, F_EX, s);
+        if (bz) {
+            tma_load_4d(d + SNA, &tmZ, bar, x, yi, 0, s);
+            tma_load_4d(d + 2 * SNA, &tmZ, bar, x, yi, 1, s);
+        } else {
+            tma_load_4d(d + SNA, &tmE, bar, x, y, F_EZ, s);
+            tma_load_4d(d + 2 * SNA, &tmE, bar, x, y, F_ES, s);
         }
-    }
-    __syncthreads();
-    const bool fix = box_special4(g, c.i0, c.j0, T::TZH, K);
-    const bool lean = !fix && tile_plain4(g, c.i0, c.j0, T::TZH, T::M);
-    if (fix) pml_table4<SH>(g, m, c.i0 - K, c.j0, tab, tid);   // ordered before use by the first wait's barrier
-    for (int t = tid; t < 4 * TX4; t += NTHR) {
-        const int j = c.j0 + t % TX4, set = t / TX4;
-        xt[t] = set == 0 ? cv_tMA<FD>(j, g.nx, g.nx) : set == 1 ? cv_tMB<FD>(j, g.nx, g.nx)
-              : set == 2 ? cv_tPA<FD>(j, g.nx) : cv_tPB<FD>(j, g.nx);
-    }
-    for (int t = tid; t < 4 * T::TZH; t += NTHR) {
-        const int i = c.i0 + t % T::TZH, set = t / T::TZH;
-        zt[t] = set == 0 ? cv_tPA<FD>(i, g.nz) : set == 1 ? cv_tPB<FD>(i, g.nz)
-              : set == 2 ? cv_tMA<FD>(i, g.nz, g.nz) : cv_tMB<FD>(i, g.nz, g.nz);
-    }
-    const int rd = in.ping, wr = 1 - in.ping;
-    const int jb = c.j0 + 2 * tx;
-    const float hdtdz = 0.5f * g.dtdz, hdtdx = 0.5f * g.dtdx;
-    float2 Bc[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        float bc[2];
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int i = c.i0 + ty * RPT + r, j = jb + cc;
-            bc[cc] = (i < g.nz && j < g.nx) ? m.B[(long long)i * g.P + j] : 0.f;
-        }
-        Bc[r] = make_float2(bc[0], bc[1]);
-    }
-    double glr[2] = {0.0, 0.0};
+        if (bx) tma_load_4d(d + 3 * SNA, &tmX, bar, xi, y, 1, s);
+        else if (bz) tma_load_4d(d + 3 * SNA, &tmE, bar, x, y, F_ES, s);
+        tma_load_4d(d + SOWN, &tmPQo, bar, u.j0(), u.i0(T::TZH), F_U, s);
+    };
 
-    for (int it = 0; it < nsh; ++it) {
-        const int s = c.s0 + it;
-        float *S = sm + (it & 1) * STG;
-        const float *own = S + T::S3;   // [P, Q][TZH][TX4] of the tile's own cells
+    Cursor c;
+    int first, nit;
+    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i, 0); })) return;
+    // transposed masks reach 2K - 1 (low edge) and 2K (high edge) cells inwards
+    const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
+    const float hdtdz = 0.5f * g.dtdz, hdtdx = 0.5f * g.dtdx;
+    bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
+    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+    float2 Bc[RPT];
+    auto enter = [&]() {
+        jb = c.j0() + 2 * tx;
+        e0 = tab_at(jb, g.nx);
+        e1 = tab_at(jb + 1, g.nx);
+        iw = c.i0(T::TZH) + ty * RPT;
+        xin = cols_plain(g, c.j0(), mlo, mhi);
+        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
+        bx = box_x(g, c.j0());
+        bz = box_z(g, c.i0(T::TZH), T::TZH, K);
+        xband = jb < g.nx && (jb < g.jl || jb >= g.jr);
+        zband = iw < g.itb || iw + RPT > g.ibb;
+        r0 = rv.tile_start[c.tile(w)];
+        r1 = rv.tile_start[c.tile(w) + 1];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) Bc[r] = mat_pair(g, m.B, iw + r, jb);
+    };
+    enter();
+    int st = 0, ph = 0;
+    for (int it = 0; it < nit; ++it) {
+        const int s = c.shot;
+        const float *S = sm + st * STG;
+        const float *own = S + SOWN;   // [P, Q][TZH][TX4] of the tile's own cells
         float *Pp = A + ((long long)s * F_N + F_U) * g.fstride;
         float *Qp = A + ((long long)s * F_N + F_V) * g.fstride;
-        if (!__syncthreads_and(mbar_wait_bounded(bar + (it & 1), (it >> 1) & 1, g.wait_polls))) {
-            abort3(bar, it, nsh, status);
-            return;
-        }
-        if (fix) {
-            const float *pDzU = pz_ptr(g, PZ, s, PZ_NFWD + rd * PZA_N + PZA_DZU);
-            const float *pDzV = pz_ptr(g, PZ, s, PZ_NFWD + rd * PZA_N + PZA_DZV);
-            const float *pDxU = px_ptr(g, PX, s, PX_NFWD + rd * PXA_N + PXA_DXU);
-            const float *pDxV = px_ptr(g, PX, s, PX_NFWD + rd * PXA_N + PXA_DXV);
-            float *wDzU = pz_ptr(g, PZ, s, PZ_NFWD + wr * PZA_N + PZA_DZU);
-            float *wDzV = pz_ptr(g, PZ, s, PZ_NFWD + wr * PZA_N + PZA_DZV);
-            float *wDxU = px_ptr(g, PX, s, PX_NFWD + wr * PXA_N + PXA_DXU);
-            float *wDxV = px_ptr(g, PX, s, PX_NFWD + wr * PXA_N + PXA_DXV);
-            // box columns [0, xl) and [xr, SW4) lie in the x-strips
-            const int xl = g.pad - (c.j0 - XO4), xr = g.nx - g.pad - (c.j0 - XO4);
-            const float *tbx = tab, *tax = tab + SW4, *tikx = tab + 2 * SW4, *tlr = tab + 3 * SW4;
-            const int *txs = reinterpret_cast<const int *>(tab + 4 * SW4);
-            const float *tbz = tab + 5 * SW4, *taz = tbz + SH, *tikz = taz + SH;
-            const int *tzs = reinterpret_cast<const int *>(tikz + SH);
-            for (int rr = ty; rr < SH; rr += NWARP) {
-                const int i = c.i0 - K + rr;
-                const int zs = tzs[rr];
-                const bool rowsp = zs >= 0 || (g.fs && i == 0);
-                const bool own_row = rr >= K && rr < K + T::TZH;
-                // the C-PML memories of this row's cells, all requested before any is used
-                float ps[NCC][4];
-#pragma unroll
-                for (int b = 0; b < NCC; ++b) {
-                    const int cc = tx + b * TX, jj = c.j0 - XO4 + cc;
-                    ps[b][0] = ps[b][1] = ps[b][2] = ps[b][3] = 0.f;
-                    if (cc >= SW4) continue;
-                    if (zs >= 0 && jj >= 0 && jj < g.nx) {
-                        const long long pz = (long long)zs * g.P + jj;
-                        ps[b][0] = pDzV[pz];
-                        ps[b][1] = pDzU[pz];
-                    }
-                    const int xs = txs[cc];
-                    if (xs >= 0 && i >= 0 && i < g.nz) {
-                        const long long px = (long long)i * g.xs_n + xs;
-                        ps[b][2] = pDxU[px];
-                        ps[b][3] = pDxV[px];
-                    }
-                }
-#pragma unroll
-                for (int b = 0; b < NCC; ++b) {
-                    const int cc = tx + b * TX;
-                    if (cc >= SW4) continue;
-                    const int jj = c.j0 - XO4 + cc, q = rr * SW4 + cc;
-                    if (!rowsp && cc >= xl && cc < xr) {
-                        // outside the strips and off the free-surface row the
-                        // transform is the identity
-                        aDxV[q] = S[2 * SN + q];
-                        continue;
-                    }
-                    const float ea = S[q], za = S[SN + q], sa = S[2 * SN + q];
-                    float vDxU = ea, vDzV = za, vDzU = sa, vDxV = sa;
-                    if (i >= 0 && i < g.nz && jj >= 0 && jj < g.nx) {
-                        const bool own = own_row && cc >= XO4 && cc < XO4 + TX4;
-                        const int xs = txs[cc];
-                        const long long pz = (long long)zs * g.P + jj, px = (long long)i * g.xs_n + xs;
-                        if (zs >= 0) vDzV = pml_adj4(za, tbz[rr], taz[rr], tikz[rr], ps[b][0], wDzV + pz, own);
-                        float din = (jj >= 1) ? ea : 0.f;
-                        if (g.fs && i == 0 && jj < g.nx - 1) din = tlr[cc] * vDzV + din;
-                        vDxU = din;
-                        if (xs >= 0) vDxU = pml_adj4(din, tbx[cc], tax[cc], tikx[cc], ps[b][2], wDxU + px, own);
-                        const float h = (i < g.nz - 1 && jj < g.nx - 1) ? sa : 0.f;
-                        vDzU = h;
-                        vDxV = h;
-                        if (zs >= 0) vDzU = pml_adj4(h, tbz[rr], taz[rr], tikz[rr], ps[b][1], wDzU + pz, own);
-                        if (xs >= 0) vDxV = pml_adj4(h, tbx[cc], tax[cc], tikx[cc], ps[b][3], wDxV + px, own);
-                    }
-                    S[q] = vDxU; S[SN + q] = vDzV; S[2 * SN + q] = vDzU; aDxV[q] = vDxV;
-                }
+        float *iXX = im.xb + (long long)s * 2 * g.txs, *iXXZ = iXX + g.txs;
+        float *iZXZ = im.zb + (long long)s * 2 * g.tzs, *iZZ = iZXZ + g.tzs;
+        const float *aDxU = S, *aDzV = S + SNA, *aDzU = S + 2 * SNA, *aDxV = (bx || bz) ? S + 3 * SNA : aDzU;
+        float *fXX = px_ptr(g, PX, s, PX_NFWD + PXA_XX), *fXXZ = px_ptr(g, PX, s, PX_NFWD + PXA_XXZ);
+        float *fZXZ = pz_ptr(g, PZ, s, PZ_NFWD + PZA_ZXZ), *fZZ = pz_ptr(g, PZ, s, PZ_NFWD + PZA_ZZ);
+        auto rows = [&](auto gd, auto xb) -> bool {
+            constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
+            int2 xs = make_int2(-1, -1);
+            if (XB) {
+                xs = xstrip_pair(g, jb);
+                prefetch_x<RPT>(g, iw, xs, fXX, fXXZ);
+                prefetch_l1(g.pmx + jb);
             }
-            __syncthreads();
-        }
-        const float *aDxU = S, *aDzV = S + SN, *aDzU = S + 2 * SN;
-        const float *aXV = fix ? aDxV : aDzU;
-        float2 wzu[T::W], wzv[T::W];
-        zwin2p<T::W, RPT>(wzu, aDzU, ty, tx);
-        zwin2p<T::W, RPT>(wzv, aDzV, ty, tx);
-        if (lean) {
-            // interior tile whose box needs no fix-up: no guards, paired arithmetic
+            if (GUARD) {
+                prefetch_z<RPT>(g, iw, jb, fZXZ, fZZ);
+                prefetch_l1(g.pmz + iw);
+            }
+            if (!mbar_wait_bounded(ring->full + st, ph, g.wait_polls)) return false;
+            float2 zu_[RPT], zv_[RPT];
+            {
+                float2 wn[T::W];
+                zwin<T::W, RPT>(wn, aDzU, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) zu_[r] = z_tdp<FD, GUARD>(wn, r, &tab->z[0][tab_at(iw + r, g.nz)], &tab->z[1][tab_at(iw + r, g.nz)]);
+                zwin<T::W, RPT>(wn, aDzV, ty, tx);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) zv_[r] = z_tdm<FD, GUARD>(wn, r, &tab->z[2][tab_at(iw + r, g.nz)], &tab->z[3][tab_at(iw + r, g.nz)]);
+            }
 #pragma unroll
             for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                float ad[10], av[10];
-                xrow(ad, aDxU, q);
-                xrow(av, aXV, q);
-                const float2 p2 = *reinterpret_cast<const float2 *>(own + (ty * RPT + r) * TX4 + 2 * tx);
-                const float2 q2 = *reinterpret_cast<const float2 *>(own + (T::TZH + ty * RPT + r) * TX4 + 2 * tx);
-                const float2 tdm = make_float2(a_tdm<FD, false>(ad, 0, 0, 0, 0), a_tdm<FD, false>(ad, 1, 0, 0, 0));
-                const float2 tdp = make_float2(a_tdp<FD, false>(av, 0, 0, 0), a_tdp<FD, false>(av, 1, 0, 0));
-                const float2 gu = fma2(dup2(g.dtdx), tdm, mul2(dup2(hdtdz), w_tdp2<FD>(wzu, r)));
-                const float2 gv = fma2(dup2(g.dtdz), w_tdm2<FD>(wzv, r), mul2(dup2(hdtdx), tdp));
-                const long long o = (long long)i * g.P + jb;
-                *reinterpret_cast<float2 *>(Pp + o) = fma2(Bc[r], gu, p2);
-                *reinterpret_cast<float2 *>(Qp + o) = fma2(Bc[r], gv, q2);
-            }
-        } else {
+                const int i = iw + r, zr = ty * RPT + r, q = (zr + K) * SW4 + XO4 + 2 * tx;
+                if (GUARD && i >= g.nz) continue;
+                const bool last = GUARD && i >= g.nz - 1;
+                float a[10];
+                xrow(a, aDxU, q);
+                if (GUARD && g.fs && i == 0 && !bx) {
+                    // free surface: d(vz)/dz is d(vx)/dx times Lr there, so
+                    // exx_a receives Lr ezz_a (the x images already hold it)
+                    float az[10];
+                    xrow(az, aDzV, q);
 #pragma unroll
-            for (int r = 0; r < RPT; ++r) {
-                const int i = c.i0 + ty * RPT + r;
-                if (i >= g.nz) continue;
-                const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-                float ad[10], av[10];
-                xrow(ad, aDxU, q);
-                xrow(av, aXV, q);
-                const float2 p2 = *reinterpret_cast<const float2 *>(own + (ty * RPT + r) * TX4 + 2 * tx);
-                const float2 q2 = *reinterpret_cast<const float2 *>(own + (T::TZH + ty * RPT + r) * TX4 + 2 * tx);
-                const float pr[2] = {p2.x, p2.y}, qr[2] = {q2.x, q2.y};
-                const int zr = ty * RPT + r;
-                const float4 zpa = zt[zr], zpb = zt[T::TZH + zr], zma = zt[2 * T::TZH + zr], zmb = zt[3 * T::TZH + zr];
-                float np[2], nq[2];
+                    for (int k = 0; k < 10; ++k) a[k] = m.Lr[jb - 4 + k] * az[k] + a[k];
+                }
+                const float2 tdm = x_tdm<FD, XB>(a, tab->x[2], tab->x[3], e0, e1);
+                xrow(a, aDxV, q);
+                float2 tdp = x_tdp<FD, XB>(a, tab->x[0], tab->x[1], e0, e1), zu = zu_[r], zv = zv_[r];
+                const float2 p2 = pair_at(own + zr * TX4 + 2 * tx), q2 = pair_at(own + PL + zr * TX4 + 2 * tx);
+                if (last) tdp = make_float2(0.f, 0.f);
+                if (XB) {
+                    if (jb < 1 || jb >= g.nx - 1) zu.x = 0.f;
+                    if (jb + 1 >= g.nx - 1) zu.y = 0.f;
+                    if (jb >= g.nx - 1) zv.x = 0.f;
+                    if (jb + 1 >= g.nx - 1) zv.y = 0.f;
+                }
+                const float2 gu = fma2(dup2(g.dtdx), tdm, mul2(dup2(hdtdz), zu));
+                const float2 gv = fma2(dup2(g.dtdz), zv, mul2(dup2(hdtdx), tdp));
+                const float2 np = fma2(Bc[r], gu, p2), nq = fma2(Bc[r], gv, q2);
+                if (GUARD && in.want_exact && g.fs && i == 0) {
+                    // dJ/dLr on the free-surface row
 #pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int j = jb + cc;
-                    np[cc] = pr[cc]; nq[cc] = qr[cc];
-                    if (j >= g.nx) continue;
-                    const int col = 2 * tx + cc;
-                    const float gu = (j >= 1 ? hdtdz * w_tdp_t<FD>(wzu, r, cc, zpa, zpb) : 0.f)
-                                   + g.dtdx * a_tdm_t<FD>(ad, cc, xt[col], xt[TX4 + col]);
-                    const float gv = (i < g.nz - 1 ? hdtdx * a_tdp_t<FD>(av, cc, xt[2 * TX4 + col], xt[3 * TX4 + col]) : 0.f)
-                                   + (j < g.nx - 1 ? g.dtdz * w_tdm_t<FD>(wzv, r, cc, zma, zmb) : 0.f);
-                    np[cc] = pr[cc] + f2c(Bc[r], cc) * gu;
-                    nq[cc] = qr[cc] + f2c(Bc[r], cc) * gv;
-                    if (in.want_exact && g.fs && i == 0) {
-                        const int pj = j - g.pad;
+                    for (int cc = 0; cc < 2; ++cc) {
+                        const int j = jb + cc, pj = j - g.pad;
                         if (pj >= 0 && pj < g.nx_dom && j < g.nx - 1) {
                             const float du = in.row0[((long long)s * in.slots + in.slot) * g.nx_dom + pj];
-                            glr[cc] += (double)(g.dtdz * f2c(wzv[r + K], cc)) * (double)du * (double)g.dzdx;
+                            in.accLr[(long long)s * g.nx_dom + pj] += (double)(g.dtdz * aDzV[q + cc]) * (double)du * (double)g.dzdx;
                         }
                     }
                 }
-                if (jb < g.nx) {
-                    const long long o = (long long)i * g.P + jb;
-                    if (jb + 1 < g.nx) {
-                        *reinterpret_cast<float2 *>(Pp + o) = make_float2(np[0], np[1]);
-                        *reinterpret_cast<float2 *>(Qp + o) = make_float2(nq[0], nq[1]);
-                    } else {
-                        Pp[o] = np[0];
-                        Qp[o] = nq[0];
+                const long long o = (long long)i * g.P + jb;
+                store_pair<XB>(Pp + o, np, g.nx - jb);
+                store_pair<XB>(Qp + o, nq, g.nx - jb);
+                if (xband || zband) {
+                    // images for the strain update, which reads P and Q on [0, nz - 1) x [1, nx - 1) only
+                    float2 pv = np, qv = nq;
+                    if (last) pv = qv = make_float2(0.f, 0.f);
+                    if (XB) {
+                        if (jb < 1 || jb >= g.nx - 1) pv.x = qv.x = 0.f;
+                        if (jb + 1 >= g.nx - 1) pv.y = qv.y = 0.f;
+                    }
+                    if (xband) {
+                        float2 vXX = pv, vXXZ = qv;
+                        if (XB) {
+                            const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
+                            const float2 m0 = mem_x(fXX + i * g.xs_n, xs), m1 = mem_x(fXXZ + i * g.xs_n, xs);
+                            adj_x2(vXX, c0, c1, xs, m0, fXX + i * g.xs_n);
+                            adj_x2(vXXZ, c0, c1, xs, m1, fXXZ + i * g.xs_n);
+                        }
+                        const long long b = (long long)i * g.wxp + band_x(g, jb);
+                        *reinterpret_cast<float2 *>(iXX + b) = vXX;
+                        *reinterpret_cast<float2 *>(iXXZ + b) = vXXZ;
+                    }
+                    if ((i < g.itb || i >= g.ibb) && (!XB || jb < g.nx)) {
+                        float2 vZXZ = pv, vZZ = qv;
+                        if (GUARD) {
+                            const float4 zc = ldt(g.pmz + i);
+                            const int zs = __float_as_int(zc.w);
+                            if (zs >= 0) {
+                                const float2 m0 = pair_at(fZXZ + zs * g.P + jb), m1 = pair_at(fZZ + zs * g.P + jb);
+                                adj_z2(vZXZ, zc, m0, fZXZ + zs * g.P + jb);
+                                adj_z2(vZZ, zc, m1, fZZ + zs * g.P + jb);
+                            }
+                        }
+                        const long long b = (long long)band(i, g.itb, g.ibb) * g.P + jb;
+                        *reinterpret_cast<float2 *>(iZXZ + b) = vZXZ;
+                        *reinterpret_cast<float2 *>(iZZ + b) = vZZ;
                     }
                 }
             }
+            return true;
+        };
+        if (!(!xin ? rows(std::true_type{}, std::true_type{})
+                   : !zin ? rows(std::true_type{}, std::false_type{}) : rows(std::false_type{}, std::false_type{}))) {
+            ring_abort(ring, it, status);
+            return;
         }
-        fence_async_shared();
-        __syncthreads();
-        if (tid == 0 && it + 2 < nsh) {
-            mbar_arrive_expect_tx(bar + (it & 1), 3 * SN * 4 + OWNB);
-            tma_load_4d(S, &tmE, bar + (it & 1), c.j0 - XO4, c.i0 - K, F_EX, s + 2);
-            tma_load_4d(S + T::S3, &tmPQo, bar + (it & 1), c.j0, c.i0, F_U, s + 2);
+        if (ring_leave(ring, st, it + NST < nit)) {
+            Cursor u;
+            u.init(w, first + it + NST);
+            issue(u, st);
         }
-        const int r0 = rv.tile_start[c.tile], r1 = rv.tile_start[c.tile + 1];
-        for (int qq = r0 + tid; qq < r1; qq += NTHR) {
-            const int rid = rv.tile_rec[qq];
-            const long long o = (long long)rv.rz[rid] * g.P + rv.rx[rid];
-            const float *src = in.rec_adj + (long long)s * 4 * g.nt * g.nrec + (long long)n * g.nrec + rid;
-            const float b = m.B[o];
-            atomicAdd(Pp + o, b * src[0]);
-            atomicAdd(Qp + o, b * src[(long long)g.nt * g.nrec]);
+        if (++st == NST) { st = 0; ph ^= 1; }
+        if (r1 > r0) {
+            // receivers on this warp's rows, whose cells its own lanes have just written
+            __syncwarp();
+            for (int qq = r0 + tx; qq < r1; qq += TX) {
+                const int rid = rv.tile_rec[qq], i = rv.rz[rid], j = rv.rx[rid];
+                if (i < iw || i >= iw + RPT) continue;
+                const long long o = (long long)i * g.P + j;
+                const float *src = in.rec_adj + (long long)s * 4 * g.nt * g.nrec + (long long)n * g.nrec + rid;
+                const float b = m.B[o], dp = b * src[0], dq = b * src[(long long)g.nt * g.nrec];
+                atomicAdd(Pp + o, dp);
+                atomicAdd(Qp + o, dq);
+                if (i >= g.nz - 1 || j < 1 || j >= g.nx - 1) continue;
+                if (j < g.jl || j >= g.jr) {
+                    const int xs = xstrip_index(g, j);
+                    const float4 xc = ldt(g.pmx + j);
+                    const long long t = (long long)i * g.wxp + band_x(g, j);
+                    atomicAdd(iXX + t, adj_inject(dp, xc, xs >= 0, fXX + i * g.xs_n + xs));
+                    atomicAdd(iXXZ + t, adj_inject(dq, xc, xs >= 0, fXXZ + i * g.xs_n + xs));
+                }
+                if (i < g.itb || i >= g.ibb) {
+                    const float4 zc = ldt(g.pmz + i);
+                    const int zs = __float_as_int(zc.w);
+                    const long long t = (long long)band(i, g.itb, g.ibb) * g.P + j, pz = (long long)zs * g.P + j;
+                    atomicAdd(iZXZ + t, adj_inject(dp, zc, zs >= 0, fZXZ + pz));
+                    atomicAdd(iZZ + t, adj_inject(dq, zc, zs >= 0, fZZ + pz));
+                }
+            }
         }
-    }
-    if (in.want_exact && g.fs && c.i0 == 0 && ty == 0) {
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int j = jb + cc, pj = j - g.pad;
-            if (pj >= 0 && pj < g.nx_dom && j < g.nx - 1) in.accLr[(long long)(c.s0 / spg) * g.nx_dom + pj] += glr[cc];
-        }
+        if (c.next(w)) enter();
     }
 }
 
 // ------------------------------------------------------------- adjoint: strains + gradient
 
+// receiver adjoints e1 (exx) and e3 (ezz) at cell (i, j) of shot s, after the
+// cell's own update: into the strain adjoints and into the images st_adj_a
+// differentiates
+__device__ __forceinline__ void inject_strain(const Geo &g, const Mat &m, const Images &im, float *A, float *PX,
+                                              float *PZ, int s, int i, int j, float e1, float e3)
+{
+    const long long o = (long long)i * g.P + j;
+    atomicAdd(A + ((long long)s * F_N + F_EX) * g.fstride + o, e1);
+    atomicAdd(A + ((long long)s * F_N + F_EZ) * g.fstride + o, e3);
+    const float4 zc = ldt(g.pmz + i);
+    const int zs = __float_as_int(zc.w);
+    float d3 = e3;
+    if (zs >= 0) d3 = adj_inject(e3, zc, true, pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZV) + (long long)zs * g.P + j);
+    if (i < g.ita || i >= g.iba)
+        atomicAdd(im.za + (long long)s * 2 * g.tzs + (long long)band(i, g.ita, g.iba) * g.P + j, d3);
+    if (j < g.jl || j >= g.jr) {
+        float d1 = j >= 1 ? e1 : 0.f;
+        if (g.fs && i == 0 && j < g.nx - 1) d1 = m.Lr[j] * d3 + d1;
+        const int xs = xstrip_index(g, j);
+        if (xs >= 0)
+            d1 = adj_inject(d1, ldt(g.pmx + j), true, px_ptr(g, PX, s, PX_NFWD + PXA_DXU) + (long long)i * g.xs_n + xs);
+        atomicAdd(im.xa + (long long)s * 2 * g.txs + (long long)i * g.wxp + band_x(g, j), d1);
+    }
+}
+
 template <int FD, int RPT, bool EXACT, bool IMG, bool RHO>
 __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
-    st_adj_b(Geo g, Mat m, Shots sh, Recv rv, float *A, float *PX, float *PZ, int n, int spg, int tiles_x,
-             AdjOut o, int *status, const __grid_constant__ CUtensorMap tmPQ,
-             const __grid_constant__ CUtensorMap tmEo, const __grid_constant__ CUtensorMap tmH)
+    st_adj_b(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh,
+             const __grid_constant__ Recv rv, float *A, float *PX, float *PZ, const __grid_constant__ Images im, int n,
+             const __grid_constant__ Work w, const __grid_constant__ AdjOut o, int *status, const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmEo,
+             const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmX,
+             const __grid_constant__ CUtensorMap tmZ)
 {
+    constexpr int SNA = al32_3(G4<FD, RPT>::SN), SOWN = al32_3(4 * SNA);
+    // one history box per item from [shot][slot * snf + field][nz_dom][nx_dom]
+    // at the tile's physical coordinates (cells outside arrive as 0): the
+    // carry-in stresses of the exact gradient, or the carry-out ones of the
+    // imaging condition
+    const int hslot = EXACT ? o.slot_in : o.slot_img;
+    const bool htma = (EXACT || IMG) && o.hist_tma && hslot >= 0;
     using T = G4<FD, RPT>;
-    constexpr int K = T::K, SN = T::SN, SH = T::SH;
-    constexpr int STG = L4<FD, RPT>::ADB_STAGE, OWNB = 3 * T::TZH * TX4 * 4, PL = T::TZH * TX4;
+    using Sg = Stage<FD, RPT>;
+    constexpr int K = T::K, SN = T::SN, STG = Sg::ADB, NST = Sg::NADB, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
-    constexpr int NCC = (SW4 + TX - 1) / TX;
-    float *aZXZ = sm + 2 * STG, *aXXZ = aZXZ + T::S1;
-    float *tab = aXXZ + T::S1;
-    // coefficient tables: x sets (A, B of the transposed D+ of P, A, B of
-    // the transposed D- of Q), z sets (A, B of the transposed D+ of Q, A, B
-    // of the transposed D- of P)
-    float4 *xt = reinterpret_cast<float4 *>(sm + L4<FD, RPT>::ADB);
-    float4 *zt = xt + 4 * TX4;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L5<FD, RPT>::ADB);
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const Ctx3 c = ctx5(g, spg, T::TZH, tiles_x, g.tordB, g.theavyB);
-    const int nsh = c.s1 - c.s0;
-    if (nsh <= 0) return;
-    // the carry-in stresses of the exact gradient: one more box per shot from
-    // the history [shot][slot * snf + field][nz_dom][nx_dom] at the tile's
-    // physical coordinates (cells outside the physical domain arrive as 0)
-    const bool htma = EXACT && o.hist_tma && o.slot_in >= 0;
-    const int hbytes = htma ? OWNB : 0;
-    const int hx = c.j0 - g.pad, hy = c.i0 - g.z0, hz = o.slot_in * g.snf;
-    if (tid == 0) {
-        mbar_init(bar + 0, 1); mbar_init(bar + 1, 1);
-        fence_async_shared();
-        for (int b = 0; b < 2 && b < nsh; ++b) {
-            mbar_arrive_expect_tx(bar + b, 2 * SN * 4 + OWNB + hbytes);
-            tma_load_4d(sm + b * STG, &tmPQ, bar + b, c.j0 - XO4, c.i0 - K, F_U, c.s0 + b);
-            tma_load_4d(sm + b * STG + T::S2, &tmEo, bar + b, c.j0, c.i0, F_EX, c.s0 + b);
-            if (htma)
-                tma_load_4d_hint(sm + b * STG + T::S2 + L4<FD, RPT>::OWNB3, &tmH, bar + b, hx, hy, hz, c.s0 + b,
-                                 l2_evict_first());
+    AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
+    Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    // planes as in st_adj_a: P and Q, or their images where the box touches a
+    // strip; the z image of P and the x image of Q are planes of their own
+    auto issue = [&](const Cursor &u, int st) {
+        const bool bx = box_x(g, u.j0()), bz = box_z(g, u.i0(T::TZH), T::TZH, K);
+        constexpr int PB = SN * 4, OB = 3 * T::TZH * TX4 * 4;
+        uint64_t *bar = ring->full + st;
+        float *d = sm + st * STG;
+        const int s = u.shot, x = u.j0() - XO4, y = u.i0(T::TZH) - K;
+        const int xi = x >= g.jr ? x - g.jr + g.jl : x, yi = y >= g.ibb ? y - g.ibb + g.itb : y;
+        mbar_arrive_expect_tx(bar, (bx || bz ? 4 : 2) * PB + OB + (htma ? OB : 0));
+        if (bx) tma_load_4d(d, &tmX, bar, xi, y, 0, s);
+        else tma_load_4d(d, &tmP, bar, x, y, F_U, s);
+        if (bz) tma_load_4d(d + SNA, &tmZ, bar, x, yi, 1, s);
+        else tma_load_4d(d + SNA, &tmP, bar, x, y, F_V, s);
+        if (bx || bz) {
+            if (bz) tma_load_4d(d + 2 * SNA, &tmZ, bar, x, yi, 0, s);
+            else tma_load_4d(d + 2 * SNA, &tmP, bar, x, y, F_U, s);
+            if (bx) tma_load_4d(d + 3 * SNA, &tmX, bar, xi, y, 1, s);
+            else tma_load_4d(d + 3 * SNA, &tmP, bar, x, y, F_V, s);
         }
-    }
-    __syncthreads();
-    const bool fix = box_strips4(g, c.i0, c.j0, T::TZH, K);
-    const bool lean = !fix && tile_plain4(g, c.i0, c.j0, T::TZH, T::M);
-    if (fix) pml_table4<SH>(g, m, c.i0 - K, c.j0, tab, tid);   // ordered before use by the first wait's barrier
-    for (int t = tid; t < 4 * TX4; t += NTHR) {
-        const int j = c.j0 + t % TX4, set = t / TX4;
-        xt[t] = set == 0 ? cv_tPA<FD>(j, g.nx) : set == 1 ? cv_tPB<FD>(j, g.nx)
-              : set == 2 ? cv_tMA<FD>(j, g.nx, g.nx - 1) : cv_tMB<FD>(j, g.nx, g.nx - 1);
-    }
-    for (int t = tid; t < 4 * T::TZH; t += NTHR) {
-        const int i = c.i0 + t % T::TZH, set = t / T::TZH;
-        zt[t] = set == 0 ? cv_tPA<FD>(i, g.nz) : set == 1 ? cv_tPB<FD>(i, g.nz)
-              : set == 2 ? cv_tMA<FD>(i, g.nz, g.nz - 1) : cv_tMB<FD>(i, g.nz, g.nz - 1);
-    }
-    const int rd = o.ping, wr = 1 - o.ping;
-    const int jb = c.j0 + 2 * tx;
+        tma_load_4d(d + SOWN, &tmEo, bar, u.j0(), u.i0(T::TZH), F_EX, s);
+        if (htma)
+            tma_load_4d_hint(d + SOWN + Sg::OWN3, &tmH, bar, u.j0() - g.pad, u.i0(T::TZH) - g.z0, hslot * g.snf, s, l2_evict_first());
+    };
+
+    Cursor c;
+    int first, nit;
+    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i, 1); })) return;
+    const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
+    const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;   // history pairs start on 8 bytes
     constexpr int RE = EXACT ? RPT : 1, RI = IMG ? RPT : 1;
-    float mL2M[RPT][2], mL[RPT][2], mM2[RPT][2], idet[RI][2], i2m[RI][2];
-    // per-launch sums over the block's shots (at most a few terms) in FP32;
-    // the sums over steps and shot groups are FP64 (the reductions below).
+    bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
+    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0, sfirst = 0;
+    float2 ml2m[RPT], ml[RPT], mm[RPT];
+    // sums over the shots that the block takes of this tile in one go, in
+    // FP32; over steps, groups and blocks in FP64 (the reductions of leave()).
     // The exact gradient sums the carry-in stresses s against the stress
     // adjoints, sA = sum(s1 sxx_a + s2 szz_a), sB = sum(s2 sxx_a + s1 szz_a),
-    // sC = sum(s3 sxz_a); the strain-recovery factors (constant per cell)
-    // are applied once at the end: g_L2M = idet (L2M sA - L sB), g_L =
-    // idet (L2M sB - L sA), g_M = sC / M.
-    float sC[RE][2], sB[RE][2], sA[RE][2], glam[RI][2], gmu[RI][2];
+    // sC = sum(s3 sxz_a); k_finalize applies the strain-recovery factors.
+    float2 sA[RE], sB[RE], sC[RE], glam[RI], gmu[RI];
     // density terms (history with velocities): dJ/dB of the exact gradient
     // and the rho term of the imaging formula
     constexpr int RB = (EXACT && RHO) ? RPT : 1, RR = (IMG && RHO) ? RPT : 1;
-    float gB[RB][2], grl[RR][2];
+    float2 gB[RB], grl[RR];
+    auto enter = [&]() {
+        jb = c.j0() + 2 * tx;
+        e0 = tab_at(jb, g.nx);
+        e1 = tab_at(jb + 1, g.nx);
+        iw = c.i0(T::TZH) + ty * RPT;
+        xin = cols_plain(g, c.j0(), mlo, mhi);
+        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
+        bx = box_x(g, c.j0());
+        bz = box_z(g, c.i0(T::TZH), T::TZH, K);
+        xband = jb < g.nx && (jb < g.jl || jb >= g.jr);
+        zband = iw < g.ita || iw + RPT > g.iba;
+        r0 = n > 0 ? rv.tile_start[c.tile(w)] : 0;
+        r1 = n > 0 ? rv.tile_start[c.tile(w) + 1] : 0;
+        sfirst = c.shot;
 #pragma unroll
-    for (int r = 0; r < RB; ++r) gB[r][0] = gB[r][1] = 0.f;
-#pragma unroll
-    for (int r = 0; r < RR; ++r) grl[r][0] = grl[r][1] = 0.f;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r)
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-            const int i = c.i0 + ty * RPT + r, j = jb + cc;
-            const bool inb = i < g.nz && j < g.nx;
-            const long long off = (long long)i * g.P + j;
-            mL2M[r][cc] = inb ? m.L2M[off] : 0.f;
-            mL[r][cc] = inb ? m.L[off] : 0.f;
-            mM2[r][cc] = inb ? 2.f * m.M[off] : 0.f;
-            if (IMG) {
-                idet[r % RI][cc] = inb ? 1.0f / ((mL2M[r][cc] - mL[r][cc]) * (mL2M[r][cc] + mL[r][cc])) : 0.f;
-                i2m[r % RI][cc] = inb ? 1.0f / mM2[r][cc] : 0.f;
-            }
+        for (int r = 0; r < RPT; ++r) {
+            ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
+            ml[r] = mat_pair(g, m.L, iw + r, jb);
+            mm[r] = mat_pair(g, m.M, iw + r, jb);
         }
+        const float2 z = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int r = 0; r < RE; ++r)
+        for (int r = 0; r < RE; ++r) sA[r] = sB[r] = sC[r] = z;
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) sC[r][cc] = sB[r][cc] = sA[r][cc] = 0.f;
+        for (int r = 0; r < RI; ++r) glam[r] = gmu[r] = z;
 #pragma unroll
-    for (int r = 0; r < RI; ++r)
+        for (int r = 0; r < RB; ++r) gB[r] = z;
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) glam[r][cc] = gmu[r][cc] = 0.f;
-
-    for (int it = 0; it < nsh; ++it) {
-        const int s = c.s0 + it;
-        float *S = sm + (it & 1) * STG;
-        const float *own = S + T::S2;   // [ex_a, ez_a, es_a][TZH][TX4] of the tile's own cells
-        const float *hown = own + L4<FD, RPT>::OWNB3;   // [sxx, szz, sxz][TZH][TX4] carry-in (htma)
+        for (int r = 0; r < RR; ++r) grl[r] = z;
+    };
+    // the tile's sums so far, into a group of FP64 planes: blocks that share a
+    // tile start on shots at least `per` apart and add to groups of their own,
+    // as far as the groups go
+    auto leave = [&]() {
+        if (!EXACT && !IMG) return;
+        const int mine = o.groups / o.parts, k = (sfirst - w.s0) / max(w.per, 1);
+        double *base = o.acc + (long long)(mine > 0 ? w.part * mine + min(k, mine - 1) : 0) * o.accp * g.nd;
+#pragma unroll
+        for (int r = 0; r < RPT; ++r)
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+                const int pi = iw + r - g.z0, pj = jb + cc - g.pad;
+                if (pi < 0 || pi >= g.nz_dom || pj < 0 || pj >= g.nx_dom) continue;
+                double *acc = base + (long long)pi * g.nx_dom + pj;
+                if (EXACT) {
+                    atomicAdd(acc, (double)f2c(sC[r % RE], cc));
+                    atomicAdd(acc + g.nd, (double)f2c(sB[r % RE], cc));
+                    atomicAdd(acc + 2 * g.nd, (double)f2c(sA[r % RE], cc));
+                }
+                if (IMG) {
+                    atomicAdd(acc + 3 * g.nd, (double)f2c(glam[r % RI], cc));
+                    atomicAdd(acc + 4 * g.nd, (double)f2c(gmu[r % RI], cc));
+                }
+                if (EXACT && RHO) atomicAdd(acc + 5 * g.nd, (double)f2c(gB[r % RB], cc));
+                if (IMG && RHO) atomicAdd(acc + 6 * g.nd, (double)f2c(grl[r % RR], cc));
+            }
+    };
+    enter();
+    int st = 0, ph = 0;
+    for (int it = 0; it < nit; ++it) {
+        const int s = c.shot;
+        const float *S = sm + st * STG;
+        const float *own = S + SOWN;             // [ex_a, ez_a, es_a][TZH][TX4] of the tile's own cells
+        const float *hown = own + Sg::OWN3;      // [sxx, szz, sxz][TZH][TX4] of the history slot (htma)
         float *exa = A + ((long long)s * F_N + F_EX) * g.fstride;
         float *eza = A + ((long long)s * F_N + F_EZ) * g.fstride;
         float *esa = A + ((long long)s * F_N + F_ES) * g.fstride;
         const float *Pp = A + ((long long)s * F_N + F_U) * g.fstride;
         const float *Qp = A + ((long long)s * F_N + F_V) * g.fstride;
+        float *iXU = im.xa + (long long)s * 2 * g.txs, *iXV = iXU + g.txs;
+        float *iZV = im.za + (long long)s * 2 * g.tzs, *iZU = iZV + g.tzs;
         const float *snap_in = ((EXACT || (IMG && RHO)) && o.slot_in >= 0)
                                    ? o.snap + ((long long)s * o.slots + o.slot_in) * g.snf * g.nd : nullptr;
         const float *snap_img = ((IMG || RHO) && o.slot_img >= 0)
                                     ? o.snap + ((long long)s * o.slots + o.slot_img) * g.snf * g.nd : nullptr;
         const float *snap_next = (IMG && RHO && o.slot_next >= 0)
                                      ? o.snap + ((long long)s * o.slots + o.slot_next) * g.snf * g.nd : nullptr;
-        if (!__syncthreads_and(mbar_wait_bounded(bar + (it & 1), (it >> 1) & 1, g.wait_polls))) {
-            abort3(bar, it, nsh, status);
-            return;
-        }
-        if (fix) {
-            const float *pXX = px_ptr(g, PX, s, PX_NFWD + rd * PXA_N + PXA_XX);
-            const float *pXXZ = px_ptr(g, PX, s, PX_NFWD + rd * PXA_N + PXA_XXZ);
-            const float *pZXZ = pz_ptr(g, PZ, s, PZ_NFWD + rd * PZA_N + PZA_ZXZ);
-            const float *pZZ = pz_ptr(g, PZ, s, PZ_NFWD + rd * PZA_N + PZA_ZZ);
-            float *wXX = px_ptr(g, PX, s, PX_NFWD + wr * PXA_N + PXA_XX);
-            float *wXXZ = px_ptr(g, PX, s, PX_NFWD + wr * PXA_N + PXA_XXZ);
-            float *wZXZ = pz_ptr(g, PZ, s, PZ_NFWD + wr * PZA_N + PZA_ZXZ);
-            float *wZZ = pz_ptr(g, PZ, s, PZ_NFWD + wr * PZA_N + PZA_ZZ);
-            const int xl = g.pad - (c.j0 - XO4), xr = g.nx - g.pad - (c.j0 - XO4);
-            const float *tbx = tab, *tax = tab + SW4, *tikx = tab + 2 * SW4;
-            const int *txs = reinterpret_cast<const int *>(tab + 4 * SW4);
-            const float *tbz = tab + 5 * SW4, *taz = tbz + SH, *tikz = taz + SH;
-            const int *tzs = reinterpret_cast<const int *>(tikz + SH);
-            for (int rr = ty; rr < SH; rr += NWARP) {
-                const int i = c.i0 - K + rr;
-                const int zs = tzs[rr];
-                const bool rowsp = zs >= 0;
-                const bool own_row = rr >= K && rr < K + T::TZH;
-                float ps[NCC][4];
+        const int4 src = __ldg(sh.pos + s);
+        const float *aXX = S, *aZZ = S + SNA;
+        const float *aZXZ = (bx || bz) ? S + 2 * SNA : aXX, *aXXZ = (bx || bz) ? S + 3 * SNA : aZZ;
+        float *fDXU = px_ptr(g, PX, s, PX_NFWD + PXA_DXU), *fDXV = px_ptr(g, PX, s, PX_NFWD + PXA_DXV);
+        float *fDZV = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZV), *fDZU = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZU);
+        auto rows = [&](auto gd, auto xb) -> bool {
+            constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
+            int2 xs = make_int2(-1, -1);
+            if (XB) {
+                xs = xstrip_pair(g, jb);
+                prefetch_x<RPT>(g, iw, xs, fDXU, fDXV);
+                prefetch_l1(g.pmx + jb);
+            }
+            if (GUARD) {
+                prefetch_z<RPT>(g, iw, jb, fDZV, fDZU);
+                prefetch_l1(g.pmz + iw);
+            }
+            if (!mbar_wait_bounded(ring->full + st, ph, g.wait_polls)) return false;
+            // centred differences of P and Q for the imaging condition come
+            // from the staged boxes where these hold P and Q themselves
+            const bool boxed = IMG && !GUARD && !bx && !bz;
+            float2 zp_[RPT], zm_[RPT], dzP[RI], dzQ[RI];
+            {
+                float2 wn[T::W];
+                zwin<T::W, RPT>(wn, aZZ, ty, tx);
 #pragma unroll
-                for (int b = 0; b < NCC; ++b) {
-                    const int cc = tx + b * TX, jj = c.j0 - XO4 + cc;
-                    ps[b][0] = ps[b][1] = ps[b][2] = ps[b][3] = 0.f;
-                    if (cc >= SW4) continue;
-                    const int xs = txs[cc];
-                    if (xs >= 0 && i >= 0 && i < g.nz) {
-                        const long long px = (long long)i * g.xs_n + xs;
-                        ps[b][0] = pXX[px];
-                        ps[b][1] = pXXZ[px];
-                    }
-                    if (zs >= 0 && jj >= 0 && jj < g.nx) {
-                        const long long pz = (long long)zs * g.P + jj;
-                        ps[b][2] = pZXZ[pz];
-                        ps[b][3] = pZZ[pz];
-                    }
+                for (int r = 0; r < RPT; ++r) {
+                    zp_[r] = z_tdp<FD, GUARD>(wn, r, &tab->z[0][tab_at(iw + r, g.nz)], &tab->z[1][tab_at(iw + r, g.nz)]);
+                    if (IMG) dzQ[r % RI] = sub2(wn[r + K + 1], wn[r + K - 1]);
                 }
+                zwin<T::W, RPT>(wn, aZXZ, ty, tx);
 #pragma unroll
-                for (int b = 0; b < NCC; ++b) {
-                    const int cc = tx + b * TX;
-                    if (cc >= SW4) continue;
-                    const int jj = c.j0 - XO4 + cc, q = rr * SW4 + cc;
-                    if (!rowsp && cc >= xl && cc < xr) {
-                        // outside the strips: identity (cells off the grid are
-                        // zero-filled by the tile copy already)
-                        aZXZ[q] = S[q];
-                        aXXZ[q] = S[SN + q];
-                        continue;
-                    }
-                    float pv = 0.f, qq = 0.f;
-                    if (i >= 0 && i < g.nz - 1 && jj >= 1 && jj < g.nx - 1) { pv = S[q]; qq = S[SN + q]; }
-                    float vXX = pv, vZXZ = pv, vXXZ = qq, vZZ = qq;
-                    if (i >= 0 && i < g.nz && jj >= 0 && jj < g.nx) {
-                        const bool own = own_row && cc >= XO4 && cc < XO4 + TX4;
-                        const int xs = txs[cc];
-                        const long long px = (long long)i * g.xs_n + xs, pz = (long long)zs * g.P + jj;
-                        if (xs >= 0) {
-                            vXX = pml_adj4(pv, tbx[cc], tax[cc], tikx[cc], ps[b][0], wXX + px, own);
-                            vXXZ = pml_adj4(qq, tbx[cc], tax[cc], tikx[cc], ps[b][1], wXXZ + px, own);
-                        }
-                        if (zs >= 0) {
-                            vZXZ = pml_adj4(pv, tbz[rr], taz[rr], tikz[rr], ps[b][2], wZXZ + pz, own);
-                            vZZ = pml_adj4(qq, tbz[rr], taz[rr], tikz[rr], ps[b][3], wZZ + pz, own);
-                        }
-                    }
-                    S[q] = vXX; S[SN + q] = vZZ; aZXZ[q] = vZXZ; aXXZ[q] = vXXZ;
+                for (int r = 0; r < RPT; ++r) {
+                    zm_[r] = z_tdm<FD, GUARD>(wn, r, &tab->z[2][tab_at(iw + r, g.nz)], &tab->z[3][tab_at(iw + r, g.nz)]);
+                    if (GUARD && g.fs && iw + r == 0) zm_[r] = fma2(dup2(2.f * cf<FD>(1)), wn[r + K], zm_[r]);
+                    if (IMG) dzP[r % RI] = sub2(wn[r + K + 1], wn[r + K - 1]);
                 }
             }
-            __syncthreads();
-        }
-        const float *aXX = S, *aZZ = S + SN;
-        const float *sZXZ = fix ? aZXZ : S, *sXXZ = fix ? aXXZ : S + SN;
-        float2 wzz[T::W], wzxz[T::W];
-        zwin2p<T::W, RPT>(wzz, aZZ, ty, tx);
-        zwin2p<T::W, RPT>(wzxz, sZXZ, ty, tx);
-        const int ssx = sh.sx[s], ssz = sh.sz[s], stype = sh.type[s];
-        // an interior tile whose box needs no fix-up, without this shot's
-        // source: no per-cell guards, paired arithmetic
-        auto lean_rows = [&]() {
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int i = c.i0 + ty * RPT + r;
-            const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-            const int qo = (ty * RPT + r) * TX4 + 2 * tx;
-            const float2 ea = *reinterpret_cast<const float2 *>(own + qo);
-            const float2 za = *reinterpret_cast<const float2 *>(own + PL + qo);
-            const float2 sa = *reinterpret_cast<const float2 *>(own + 2 * PL + qo);
-            float axx[10], axz[10];
-            xrow(axx, aXX, q);
-            xrow(axz, sXXZ, q);
-            const float2 sxx = mul2(dtdx2, make_float2(a_tdp<FD, false>(axx, 0, 0, 0), a_tdp<FD, false>(axx, 1, 0, 0)));
-            const float2 szz = mul2(dtdz2, w_tdp2<FD>(wzz, r));
-            const float2 sxz = fma2(dtdx2, make_float2(a_tdm<FD, false>(axz, 0, 0, 0, 0), a_tdm<FD, false>(axz, 1, 0, 0, 0)),
-                                    mul2(dtdz2, w_tdm2<FD>(wzxz, r)));
-            const float2 l2m = make_float2(mL2M[r][0], mL2M[r][1]), l = make_float2(mL[r][0], mL[r][1]);
-            const float2 nex = fma2(l, szz, fma2(l2m, sxx, ea));
-            const float2 nez = fma2(l2m, szz, fma2(l, sxx, za));
-            const float2 nes = fma2(make_float2(mM2[r][0], mM2[r][1]), sxz, sa);
-            const int pi = i - g.z0, pj0 = jb - g.pad;
-            if (EXACT && (htma || snap_in)) {
+            for (int r = 0; r < RPT; ++r) {
+                const int i = iw + r, zr = ty * RPT + r, q = (zr + K) * SW4 + XO4 + 2 * tx, qo = zr * TX4 + 2 * tx;
+                if (GUARD && i >= g.nz) continue;
+                const bool last = GUARD && i >= g.nz - 1;
+                float a[10];
+                xrow(a, aXX, q);
+                float2 tdp = x_tdp<FD, XB>(a, tab->x[0], tab->x[1], e0, e1);
+                const float2 dxP = make_float2(a[5] - a[3], a[6] - a[4]);
+                xrow(a, aXXZ, q);
+                float2 tdm = x_tdm<FD, XB>(a, tab->x[2], tab->x[3], e0, e1);
+                const float2 dxQ = make_float2(a[5] - a[3], a[6] - a[4]);
+                float2 zp = zp_[r], zm = zm_[r];
+                const float2 ea = pair_at(own + qo), za = pair_at(own + PL + qo), sa = pair_at(own + 2 * PL + qo);
+                if (last) tdp = tdm = make_float2(0.f, 0.f);
+                if (XB) {
+                    if (jb < 1 || jb >= g.nx - 1) zp.x = zm.x = 0.f;
+                    if (jb + 1 >= g.nx - 1) zp.y = zm.y = 0.f;
+                }
+                const float2 sxx = mul2(dtdx2, tdp), szz = mul2(dtdz2, zp);
+                const float2 sxz = fma2(dtdx2, tdm, mul2(dtdz2, zm));
+                const float2 nex = fma2(ml[r], szz, fma2(ml2m[r], sxx, ea));
+                const float2 nez = fma2(ml2m[r], szz, fma2(ml[r], sxx, za));
+                const float2 nes = fma2(mul2(dup2(2.f), mm[r]), sxz, sa);
+                const int pi = i - g.z0, pj0 = jb - g.pad;
+                const bool prow = !GUARD || (pi >= 0 && pi < g.nz_dom);
+                const bool p0 = prow && (!XB || (pj0 >= 0 && pj0 < g.nx_dom));
+                const bool p1 = prow && (!XB || (pj0 + 1 >= 0 && pj0 + 1 < g.nx_dom));
+                // a history plane's pair at this cell (outside the physical grid: 0)
+                auto hist = [&](const float *pl) {
+                    const float *a = pl + (long long)pi * g.nx_dom + pj0;
+                    float2 v = make_float2(0.f, 0.f);
+                    if (hist2) {
+                        if (p0) v = __ldcs(reinterpret_cast<const float2 *>(a));
+                    } else {
+                        if (p0) v.x = __ldcs(a);
+                        if (p1) v.y = __ldcs(a + 1);
+                    }
+                    return v;
+                };
                 float2 h1, h2, h3;
                 if (htma) {
-                    h1 = *reinterpret_cast<const float2 *>(hown + qo);
-                    h2 = *reinterpret_cast<const float2 *>(hown + PL + qo);
-                    h3 = *reinterpret_cast<const float2 *>(hown + 2 * PL + qo);
-                } else {
-                    const long long pq = (long long)pi * g.nx_dom + pj0;
-                    h1 = make_float2(__ldcs(snap_in + pq), __ldcs(snap_in + pq + 1));
-                    h2 = make_float2(__ldcs(snap_in + g.nd + pq), __ldcs(snap_in + g.nd + pq + 1));
-                    h3 = make_float2(__ldcs(snap_in + 2 * g.nd + pq), __ldcs(snap_in + 2 * g.nd + pq + 1));
+                    h1 = pair_at(hown + qo);
+                    h2 = pair_at(hown + PL + qo);
+                    h3 = pair_at(hown + 2 * PL + qo);
                 }
-                float2 ta = make_float2(sA[r % RE][0], sA[r % RE][1]);
-                float2 tb = make_float2(sB[r % RE][0], sB[r % RE][1]);
-                float2 tc = make_float2(sC[r % RE][0], sC[r % RE][1]);
-                ta = __fadd2_rn(ta, fma2(h1, sxx, mul2(h2, szz)));
-                tb = __fadd2_rn(tb, fma2(h2, sxx, mul2(h1, szz)));
-                tc = fma2(h3, sxz, tc);
-                sA[r % RE][0] = ta.x; sA[r % RE][1] = ta.y;
-                sB[r % RE][0] = tb.x; sB[r % RE][1] = tb.y;
-                sC[r % RE][0] = tc.x; sC[r % RE][1] = tc.y;
-            }
-            if (RHO || IMG) {
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int j = jb + cc, pj = pj0 + cc;
-                    const long long off = (long long)i * g.P + j, pq = (long long)pi * g.nx_dom + pj;
-                    if (RHO) {
-                        const float pc = Pp[off], qc = Qp[off], bb = m.B[off];
-                        if (EXACT && snap_in && snap_img) {
-                            const float du = snap_img[3 * g.nd + pq] - snap_in[3 * g.nd + pq];
-                            const float dv = snap_img[4 * g.nd + pq] - snap_in[4 * g.nd + pq];
-                            gB[r % RB][cc] += (pc * du + qc * dv) / (bb * bb);
-                        }
-                        if (IMG) {
-                            const float ua = pc / bb, va = qc / bb;
-                            float t = 0.f;
-                            if (n >= 2 && snap_in) t += ua * snap_in[3 * g.nd + pq] + va * snap_in[4 * g.nd + pq];
-                            if (n <= g.nt - 3 && snap_next)
-                                t -= ua * snap_next[3 * g.nd + pq] + va * snap_next[4 * g.nd + pq];
-                            grl[r % RR][cc] -= 0.5f * t;
-                        }
-                    }
-                    if (IMG && snap_img) {
-                        const int ip = (i + 1) % g.nz, im = (i - 1 + g.nz) % g.nz;
-                        const int jp = (j + 1) % g.nx, jm = (j - 1 + g.nx) % g.nx;
-                        const long long oxp = (long long)i * g.P + jp, oxm = (long long)i * g.P + jm;
-                        const long long ozp = (long long)ip * g.P + j, ozm = (long long)im * g.P + j;
-                        const float dxBU = (Pp[oxp] - Pp[oxm]) * g.inv2dx;
-                        const float dzBV = (Qp[ozp] - Qp[ozm]) * g.inv2dz;
-                        const float dzBU = (Pp[ozp] - Pp[ozm]) * g.inv2dz;
-                        const float dxBV = (Qp[oxp] - Qp[oxm]) * g.inv2dx;
-                        const float t1 = snap_img[pq], t2 = snap_img[g.nd + pq], t3 = snap_img[2 * g.nd + pq];
-                        const float e1 = (mL2M[r][cc] * t1 - mL[r][cc] * t2) * idet[r % RI][cc];
-                        const float e2 = (mL2M[r][cc] * t2 - mL[r][cc] * t1) * idet[r % RI][cc];
-                        const float e3 = t3 * i2m[r % RI][cc];
-                        glam[r % RI][cc] -= g.dt * ((e1 + e2) * (dxBU + dzBV));
-                        gmu[r % RI][cc] -= g.dt * (2.f * e1 * dxBU + 2.f * e2 * dzBV + e3 * (dzBU + dxBV));
-                    }
+                if (EXACT && snap_in) {
+                    if (!htma) { h1 = hist(snap_in); h2 = hist(snap_in + g.nd); h3 = hist(snap_in + 2 * g.nd); }
+                    sA[r % RE] = add2(sA[r % RE], fma2(h1, sxx, mul2(h2, szz)));
+                    sB[r % RE] = add2(sB[r % RE], fma2(h2, sxx, mul2(h1, szz)));
+                    sC[r % RE] = fma2(h3, sxz, sC[r % RE]);
                 }
-            }
-            const long long off = (long long)i * g.P + jb;
-            *reinterpret_cast<float2 *>(exa + off) = nex;
-            *reinterpret_cast<float2 *>(eza + off) = nez;
-            *reinterpret_cast<float2 *>(esa + off) = nes;
-        }
-        };
-        // tiles with an edge, a C-PML strip, the free surface or the source:
-        // table-driven stencils, per-cell guards
-        auto rows = [&]() {
-        constexpr bool LEAN = false;
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            const int i = c.i0 + ty * RPT + r;
-            if (!LEAN && i >= g.nz) continue;
-            const int q = (ty * RPT + r + K) * SW4 + XO4 + 2 * tx;
-            const int qo = (ty * RPT + r) * TX4 + 2 * tx;
-            const float2 a2 = *reinterpret_cast<const float2 *>(own + qo);
-            const float2 b2 = *reinterpret_cast<const float2 *>(own + PL + qo);
-            const float2 d2 = *reinterpret_cast<const float2 *>(own + 2 * PL + qo);
-            const float ea[2] = {a2.x, a2.y}, za[2] = {b2.x, b2.y}, sa[2] = {d2.x, d2.y};
-            float axx[10], axz[10];
-            xrow(axx, aXX, q);
-            xrow(axz, sXXZ, q);
-            const int zr = ty * RPT + r;
-            const float4 zpa = zt[zr], zpb = zt[T::TZH + zr], zma = zt[2 * T::TZH + zr], zmb = zt[3 * T::TZH + zr];
-            float h1[2] = {0.f, 0.f}, h2[2] = {0.f, 0.f}, h3[2] = {0.f, 0.f};
-            if (EXACT && htma) {
-                const float2 x1 = *reinterpret_cast<const float2 *>(hown + qo);
-                const float2 x2 = *reinterpret_cast<const float2 *>(hown + PL + qo);
-                const float2 x3 = *reinterpret_cast<const float2 *>(hown + 2 * PL + qo);
-                h1[0] = x1.x; h1[1] = x1.y; h2[0] = x2.x; h2[1] = x2.y; h3[0] = x3.x; h3[1] = x3.y;
-            } else if (EXACT && snap_in) {
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    const int pi = i - g.z0, pj = jb + cc - g.pad;
-                    if (LEAN || (pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom)) {
-                        const long long pq = (long long)pi * g.nx_dom + pj;
-                        h1[cc] = __ldcs(snap_in + pq);
-                        h2[cc] = __ldcs(snap_in + g.nd + pq);
-                        h3[cc] = __ldcs(snap_in + 2 * g.nd + pq);
-                    }
-                }
-            }
-            float nex[2], nez[2], nes[2];
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                const int j = jb + cc;
-                nex[cc] = ea[cc]; nez[cc] = za[cc]; nes[cc] = sa[cc];
-                if (!LEAN && j >= g.nx) continue;
-                float sxx = 0.f, szz = 0.f, sxz = 0.f;
-                const int col = 2 * tx + cc;
-                if (i < g.nz - 1) {
-                    sxx = g.dtdx * a_tdp_t<FD>(axx, cc, xt[col], xt[TX4 + col]);
-                    sxz = g.dtdx * a_tdm_t<FD>(axz, cc, xt[2 * TX4 + col], xt[3 * TX4 + col]);
-                }
-                if (j >= 1 && j < g.nx - 1) {
-                    szz = g.dtdz * w_tdp_t<FD>(wzz, r, cc, zpa, zpb);
-                    sxz += g.dtdz * w_tdm_t<FD>(wzxz, r, cc, zma, zmb);
-                    if (g.fs && i == 0) sxz += 2.f * cf<FD>(1) * g.dtdz * f2c(wzxz[r + K], cc);
-                }
-                const long long off = (long long)i * g.P + j;
-                if (!LEAN && i == ssz && j == ssx) {
-                    const float w = sh.wav[(long long)s * g.nt + n];
-                    if (stype == 0) {
-                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = g.dtdxdz * Qp[off];
+                if (src.x == i && (jb == src.y || jb + 1 == src.y)) {
+                    // the source's cell
+                    const int cc = src.y - jb;
+                    const float e = f2c(ea, cc) + f2c(za, cc);
+                    if (src.z == 0) {
+                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = g.dtdxdz * Qp[(long long)i * g.P + jb + cc];
                     } else {
-                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = (g.dt / sh.mcoef[s]) * (ea[cc] + za[cc]);
+                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = (g.dt / sh.mcoef[s]) * e;
                         if (EXACT) {
-                            // the moment factor's (L + M) term, straight into
-                            // this group's FP64 sums of the source cell
-                            const double lm = sh.lm[s];
-                            const double glm = -((double)w * g.dt / ((double)sh.mcoef[s] / lm)) / (lm * lm)
-                                               * (double)(ea[cc] + za[cc]);
-                            const int pi = i - g.z0, pj = j - g.pad;
-                            if (pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom) {
-                                double *acc = o.acc + (long long)(c.s0 / spg) * o.accp * g.nd +
-                                              (long long)pi * g.nx_dom + pj;
-                                atomicAdd(acc, glm);
-                                atomicAdd(acc + g.nd, glm);
-                            }
+                            // the moment factor's (L + M) term, one FP64 sum per shot
+                            const double lm = sh.lm[s], wv = sh.wav[(long long)s * g.nt + n];
+                            o.mterm[s] += -(wv * g.dt / ((double)sh.mcoef[s] / lm)) / (lm * lm) * (double)e;
                         }
                     }
                 }
-                nex[cc] = ea[cc] + mL2M[r][cc] * sxx + mL[r][cc] * szz;
-                nez[cc] = za[cc] + mL[r][cc] * sxx + mL2M[r][cc] * szz;
-                nes[cc] = sa[cc] + mM2[r][cc] * sxz;
-                if (EXACT) {
-                    sA[r % RE][cc] += h1[cc] * sxx + h2[cc] * szz;
-                    sB[r % RE][cc] += h2[cc] * sxx + h1[cc] * szz;
-                    sC[r % RE][cc] += h3[cc] * sxz;
-                }
-                const int pi = i - g.z0, pj = j - g.pad;
-                if (RHO && (LEAN || (pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom))) {
-                    const long long pq = (long long)pi * g.nx_dom + pj;
-                    const float pc = Pp[off], qc = Qp[off], bb = m.B[off];
+                if (RHO && (p0 || p1)) {
+                    const long long off = (long long)i * g.P + jb;
+                    const float2 pc = *reinterpret_cast<const float2 *>(Pp + off), qc = *reinterpret_cast<const float2 *>(Qp + off);
+                    const float2 bb = mat_pair(g, m.B, i, jb);
                     if (EXACT && snap_in && snap_img) {
                         // dJ/dB: U_a dU/B + V_a dV/B with U_a = P/B and the
                         // step's velocity increments from the history
-                        const float du = snap_img[3 * g.nd + pq] - snap_in[3 * g.nd + pq];
-                        const float dv = snap_img[4 * g.nd + pq] - snap_in[4 * g.nd + pq];
-                        gB[r % RB][cc] += (pc * du + qc * dv) / (bb * bb);
+                        const float2 du = sub2(hist(snap_img + 3 * g.nd), hist(snap_in + 3 * g.nd));
+                        const float2 dv = sub2(hist(snap_img + 4 * g.nd), hist(snap_in + 4 * g.nd));
+                        if (p0) gB[r % RB].x += (pc.x * du.x + qc.x * dv.x) / (bb.x * bb.x);
+                        if (p1) gB[r % RB].y += (pc.y * du.y + qc.y * dv.y) / (bb.y * bb.y);
                     }
                     if (IMG) {
                         // -1/2 U_a(n) (vx(n-1) - vx(n+1)), the rho term of the
                         // imaging formula regrouped by adjoint step
-                        const float ua = pc / bb, va = qc / bb;
-                        float t = 0.f;
-                        if (n >= 2 && snap_in) t += ua * snap_in[3 * g.nd + pq] + va * snap_in[4 * g.nd + pq];
+                        float2 t = make_float2(0.f, 0.f);
+                        const float2 ua = make_float2(p0 ? pc.x / bb.x : 0.f, p1 ? pc.y / bb.y : 0.f);
+                        const float2 va = make_float2(p0 ? qc.x / bb.x : 0.f, p1 ? qc.y / bb.y : 0.f);
+                        if (n >= 2 && snap_in)
+                            t = add2(t, fma2(ua, hist(snap_in + 3 * g.nd), mul2(va, hist(snap_in + 4 * g.nd))));
                         if (n <= g.nt - 3 && snap_next)
-                            t -= ua * snap_next[3 * g.nd + pq] + va * snap_next[4 * g.nd + pq];
-                        grl[r % RR][cc] -= 0.5f * t;
+                            t = sub2(t, fma2(ua, hist(snap_next + 3 * g.nd), mul2(va, hist(snap_next + 4 * g.nd))));
+                        grl[r % RR] = fma2(dup2(-0.5f), t, grl[r % RR]);
                     }
                 }
-                if (IMG && snap_img && (LEAN || (pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom))) {
-                    const long long pq = (long long)pi * g.nx_dom + pj;
-                    const int ip = (i + 1) % g.nz, im = (i - 1 + g.nz) % g.nz;
-                    const int jp = (j + 1) % g.nx, jm = (j - 1 + g.nx) % g.nx;
-                    const long long oxp = (long long)i * g.P + jp, oxm = (long long)i * g.P + jm;
-                    const long long ozp = (long long)ip * g.P + j, ozm = (long long)im * g.P + j;
-                    const float dxBU = (Pp[oxp] - Pp[oxm]) * g.inv2dx;
-                    const float dzBV = (Qp[ozp] - Qp[ozm]) * g.inv2dz;
-                    const float dzBU = (Pp[ozp] - Pp[ozm]) * g.inv2dz;
-                    const float dxBV = (Qp[oxp] - Qp[oxm]) * g.inv2dx;
-                    const float t1 = snap_img[pq], t2 = snap_img[g.nd + pq], t3 = snap_img[2 * g.nd + pq];
-                    const float e1 = (mL2M[r][cc] * t1 - mL[r][cc] * t2) * idet[r % RI][cc];
-                    const float e2 = (mL2M[r][cc] * t2 - mL[r][cc] * t1) * idet[r % RI][cc];
-                    const float e3 = t3 * i2m[r % RI][cc];
-                    glam[r % RI][cc] -= g.dt * ((e1 + e2) * (dxBU + dzBV));
-                    gmu[r % RI][cc] -= g.dt * (2.f * e1 * dxBU + 2.f * e2 * dzBV + e3 * (dzBU + dxBV));
+                if (IMG && snap_img && (p0 || p1)) {
+                    if (EXACT || !htma) { h1 = hist(snap_img); h2 = hist(snap_img + g.nd); h3 = hist(snap_img + 2 * g.nd); }
+#pragma unroll
+                    for (int cc = 0; cc < 2; ++cc) {
+                        if (!(cc ? p1 : p0)) continue;
+                        float dxBU, dzBU, dxBV, dzBV;
+                        if (boxed) {
+                            dxBU = f2c(dxP, cc) * g.inv2dx;
+                            dxBV = f2c(dxQ, cc) * g.inv2dx;
+                            dzBU = f2c(dzP[r % RI], cc) * g.inv2dz;
+                            dzBV = f2c(dzQ[r % RI], cc) * g.inv2dz;
+                        } else {
+                            // periodic at the edges of the padded grid, as jnp.roll
+                            const int j = jb + cc, ip = (i + 1) % g.nz, im1 = (i - 1 + g.nz) % g.nz;
+                            const int jp = (j + 1) % g.nx, jm = (j - 1 + g.nx) % g.nx;
+                            const long long oxp = (long long)i * g.P + jp, oxm = (long long)i * g.P + jm;
+                            const long long ozp = (long long)ip * g.P + j, ozm = (long long)im1 * g.P + j;
+                            dxBU = (Pp[oxp] - Pp[oxm]) * g.inv2dx;
+                            dzBV = (Qp[ozp] - Qp[ozm]) * g.inv2dz;
+                            dzBU = (Pp[ozp] - Pp[ozm]) * g.inv2dz;
+                            dxBV = (Qp[oxp] - Qp[oxm]) * g.inv2dx;
+                        }
+                        const float l2m = f2c(ml2m[r], cc), l = f2c(ml[r], cc);
+                        const float t1 = f2c(h1, cc), t2 = f2c(h2, cc), id = 1.0f / ((l2m - l) * (l2m + l));
+                        const float e1 = (l2m * t1 - l * t2) * id, e2 = (l2m * t2 - l * t1) * id;
+                        const float e3 = f2c(h3, cc) * (1.0f / (2.f * f2c(mm[r], cc)));
+                        const float gl = -g.dt * ((e1 + e2) * (dxBU + dzBV));
+                        const float gm = -g.dt * (2.f * e1 * dxBU + 2.f * e2 * dzBV + e3 * (dzBU + dxBV));
+                        if (cc) { glam[r % RI].y += gl; gmu[r % RI].y += gm; }
+                        else { glam[r % RI].x += gl; gmu[r % RI].x += gm; }
+                    }
                 }
-            }
-            if (LEAN || jb < g.nx) {
                 const long long off = (long long)i * g.P + jb;
-                if (LEAN || jb + 1 < g.nx) {
-                    *reinterpret_cast<float2 *>(exa + off) = make_float2(nex[0], nex[1]);
-                    *reinterpret_cast<float2 *>(eza + off) = make_float2(nez[0], nez[1]);
-                    *reinterpret_cast<float2 *>(esa + off) = make_float2(nes[0], nes[1]);
-                } else {
-                    exa[off] = nex[0]; eza[off] = nez[0]; esa[off] = nes[0];
+                store_pair<XB>(exa + off, nex, g.nx - jb);
+                store_pair<XB>(eza + off, nez, g.nx - jb);
+                store_pair<XB>(esa + off, nes, g.nx - jb);
+                if (xband || zband) {
+                    // images for the velocity update
+                    float2 vzv = nez, h = nes;
+                    if (last) h = make_float2(0.f, 0.f);
+                    if (XB) {
+                        if (jb >= g.nx - 1) h.x = 0.f;
+                        if (jb + 1 >= g.nx - 1) h.y = 0.f;
+                    }
+                    if (!XB || jb < g.nx) {
+                        float2 vzu = h;
+                        if (GUARD) {
+                            const float4 zc = ldt(g.pmz + i);
+                            const int zs = __float_as_int(zc.w);
+                            if (zs >= 0) {
+                                const float2 m0 = pair_at(fDZV + zs * g.P + jb), m1 = pair_at(fDZU + zs * g.P + jb);
+                                adj_z2(vzv, zc, m0, fDZV + zs * g.P + jb);
+                                adj_z2(vzu, zc, m1, fDZU + zs * g.P + jb);
+                            }
+                        }
+                        if (i < g.ita || i >= g.iba) {
+                            const long long b = (long long)band(i, g.ita, g.iba) * g.P + jb;
+                            *reinterpret_cast<float2 *>(iZV + b) = vzv;
+                            *reinterpret_cast<float2 *>(iZU + b) = vzu;
+                        }
+                    }
+                    if (xband) {
+                        float2 d = nex, v = h;
+                        if (XB && jb < 1) d.x = 0.f;
+                        if (GUARD && g.fs && i == 0) {
+                            // the free surface's d(vz)/dz term (columns below nx - 1)
+                            if (!XB || jb < g.nx - 1) d.x = m.Lr[jb] * vzv.x + d.x;
+                            if (!XB || jb + 1 < g.nx - 1) d.y = m.Lr[jb + 1] * vzv.y + d.y;
+                        }
+                        if (XB) {
+                            const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
+                            const float2 m0 = mem_x(fDXU + i * g.xs_n, xs), m1 = mem_x(fDXV + i * g.xs_n, xs);
+                            adj_x2(d, c0, c1, xs, m0, fDXU + i * g.xs_n);
+                            adj_x2(v, c0, c1, xs, m1, fDXV + i * g.xs_n);
+                        }
+                        const long long b = (long long)i * g.wxp + band_x(g, jb);
+                        *reinterpret_cast<float2 *>(iXU + b) = d;
+                        *reinterpret_cast<float2 *>(iXV + b) = v;
+                    }
                 }
             }
-        }
+            return true;
         };
-        if (lean && !in_tile4(ssz, ssx, c.i0, c.j0, T::TZH)) lean_rows();
-        else rows();
-        fence_async_shared();
-        __syncthreads();
-        if (tid == 0 && it + 2 < nsh) {
-            mbar_arrive_expect_tx(bar + (it & 1), 2 * SN * 4 + OWNB + hbytes);
-            tma_load_4d(S, &tmPQ, bar + (it & 1), c.j0 - XO4, c.i0 - K, F_U, s + 2);
-            tma_load_4d(S + T::S2, &tmEo, bar + (it & 1), c.j0, c.i0, F_EX, s + 2);
-            if (htma)
-                tma_load_4d_hint(S + T::S2 + L4<FD, RPT>::OWNB3, &tmH, bar + (it & 1), hx, hy, hz, s + 2,
-                                 l2_evict_first());
+        if (!(!xin ? rows(std::true_type{}, std::true_type{})
+                   : !zin ? rows(std::true_type{}, std::false_type{}) : rows(std::false_type{}, std::false_type{}))) {
+            ring_abort(ring, it, status);
+            return;
         }
-        if (n > 0) {
-            const int r0 = rv.tile_start[c.tile], r1 = rv.tile_start[c.tile + 1];
-            for (int qq = r0 + tid; qq < r1; qq += NTHR) {
-                const int rid = rv.tile_rec[qq];
-                const long long off = (long long)rv.rz[rid] * g.P + rv.rx[rid];
+        if (ring_leave(ring, st, it + NST < nit)) {
+            Cursor u;
+            u.init(w, first + it + NST);
+            issue(u, st);
+        }
+        if (++st == NST) { st = 0; ph ^= 1; }
+        if (r1 > r0) {
+            // receivers of step n - 1 on this warp's rows, whose cells its own lanes have just written
+            __syncwarp();
+            for (int qq = r0 + tx; qq < r1; qq += TX) {
+                const int rid = rv.tile_rec[qq], i = rv.rz[rid];
+                if (i < iw || i >= iw + RPT) continue;
                 const float *src = o.rec_adj + (long long)s * 4 * g.nt * g.nrec + (long long)(n - 1) * g.nrec + rid;
-                atomicAdd(exa + off, src[2LL * g.nt * g.nrec]);
-                atomicAdd(eza + off, src[3LL * g.nt * g.nrec]);
+                inject_strain(g, m, im, A, PX, PZ, s, i, rv.rx[rid], src[2LL * g.nt * g.nrec], src[3LL * g.nt * g.nrec]);
             }
         }
-    }
-    if (EXACT || IMG) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r)
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                const int i = c.i0 + ty * RPT + r, j = jb + cc;
-                const int pi = i - g.z0, pj = j - g.pad;
-                if (i < g.nz && j < g.nx && pi >= 0 && pi < g.nz_dom && pj >= 0 && pj < g.nx_dom) {
-                    // one block per (tile, shot group) adds to these cells in a
-                    // launch: the atomic adds only avoid waiting for the loads
-                    double *acc = o.acc + (long long)(c.s0 / spg) * o.accp * g.nd + (long long)pi * g.nx_dom + pj;
-                    if (EXACT) {
-                        const double l2m = mL2M[r][cc], l = mL[r][cc];
-                        const double id = 1.0 / ((l2m - l) * (l2m + l));
-                        const double a = sA[r % RE][cc], b = sB[r % RE][cc];
-                        atomicAdd(acc, 2.0 * (double)sC[r % RE][cc] / (double)mM2[r][cc]);
-                        atomicAdd(acc + g.nd, id * (l2m * b - l * a));
-                        atomicAdd(acc + 2 * g.nd, id * (l2m * a - l * b));
-                    }
-                    if (IMG) {
-                        atomicAdd(acc + 3 * g.nd, (double)glam[r % RI][cc]);
-                        atomicAdd(acc + 4 * g.nd, (double)gmu[r % RI][cc]);
-                    }
-                    if (EXACT && RHO) atomicAdd(acc + 5 * g.nd, (double)gB[r % RB][cc]);
-                    if (IMG && RHO) atomicAdd(acc + 6 * g.nd, (double)grl[r % RR][cc]);
-                }
-            }
+        if (c.last(w) || it + 1 == nit) leave();
+        if (c.next(w)) enter();
     }
 }
 

@@ -56,8 +56,9 @@ struct stfwi_handle {
     // tensor maps of the staged tiles and per-kernel shot groups
     int sms = 148;
     int accp = 5;   // accumulator planes per shot group (7 with the density terms)
-    CUtensorMap tmS{}, tmV{}, tmE{}, tmPQ{};
-    CUtensorMap tmUo{}, tmSo{}, tmPQo{}, tmEo{};   // own-cell boxes of the two-column kernels
+    CUtensorMap tmS{}, tmV{}, tmE{}, tmP{};        // halo boxes: stresses, velocities; one adjoint field (adj_a, adj_b tiles)
+    CUtensorMap tmUo{}, tmSo{}, tmPQo{}, tmEo{};   // own-cell boxes
+    CUtensorMap tmXa{}, tmZa{}, tmXb{}, tmZb{};    // halo boxes of the image bands
     CUtensorMap tmH{};        // history [shot][slot*snf + field][nz_dom][nx_dom] (own-cell carry-in boxes)
     bool hist_tma = false;    // tmH valid: pad and nx_dom multiples of 4 (16-byte box rows)
     // staged tilings: tiles tw columns wide; fwd_vel/fwd_str/adj_a tiles tha
@@ -68,15 +69,19 @@ struct stfwi_handle {
     int ntz_max = 1;                                       // tile rows of the lowest tiles (array sizes)
     int *tile_startA = nullptr, *tile_recA = nullptr;      // receivers grouped by the tw x tha tiles
     int *tile_startB = nullptr, *tile_recB = nullptr;      // receivers grouped by the tw x thb tiles
-    int *tordA = nullptr, *tordB = nullptr;                // tile dispatch orders, boundary tiles first
-    int grp[4] = {1, 1, 1, 1}, spgk[4] = {1, 1, 1, 1};
-    int acc_groups = 1, acc_used = 1;
-    int lr_used = 1;  // rows of accLr written by the U_a/V_a phase (one per block row of shots)
+    uint32_t *tordA = nullptr, *tordB = nullptr;           // tile orders (tile row << 16 | tile column)
+    float4 *pmx = nullptr, *pmz = nullptr;                 // C-PML per column and row
+    float *img = nullptr;                                  // image bands of the adjoint
+    Images im{};
+    std::map<const void *, int> resident;                  // blocks of a kernel that the device holds at a time
+    int spgk[4] = {1, 1, 1, 1};   // shots per block of the four stencil kernels
+    int acc_groups = 1;
     int tuned[4] = {0, 0, 0, 0};  // shots per block chosen by stfwi_autotune (0: default)
 
     // shots / receivers
     int nshot = 0;
     int *sx = nullptr, *sz = nullptr, *stype = nullptr;
+    int4 *spos = nullptr;
     float *wav = nullptr, *fcoef = nullptr, *mcoef = nullptr, *lm = nullptr;
     int *rx = nullptr, *rz = nullptr;
     bool shots_set = false, recv_set = false;
@@ -101,7 +106,7 @@ struct stfwi_handle {
     // history covers all nt steps)
     int ck = 0, ncp = 0;
     float *CKF = nullptr, *CKPX = nullptr, *CKPZ = nullptr;
-    double *acc = nullptr, *accLr = nullptr, *gtmp = nullptr;
+    double *acc = nullptr, *accLr = nullptr, *gtmp = nullptr, *mterm = nullptr;
     double *energy = nullptr;
     double *mis_trace = nullptr, *mis_shot = nullptr;
     float *src_a = nullptr;
@@ -113,7 +118,7 @@ struct stfwi_handle {
     // a pass split into chains over the shot groups: the chains it may use
     // (1-4, stfwi_set_chains), the chains of the pass being recorded, and
     // the streams of chains 1.. (chain 0 runs on the pass's own stream)
-    int chains = 2, nchain_cur = 1;
+    int chains = 2;
     cudaStream_t hsx[MAX_CHAINS - 1] = {};
     cudaEvent_t ev_in = nullptr, ev_out = nullptr, ev_fork = nullptr;
     cudaEvent_t ev_join[MAX_CHAINS - 1] = {};
@@ -123,6 +128,7 @@ struct stfwi_handle {
     double prof_ms[4] = {0, 0, 0, 0};
     long long prof_cnt[4] = {0, 0, 0, 0};
     std::map<GraphKey, cudaGraphExec_t> graphs;
+    char *slab = nullptr;   // the allocation that holds every array
     size_t bytes = 0;
 };
 
@@ -163,6 +169,42 @@ int acc_groups_of(const stfwi_desc *d)
     return std::max(1, (d->max_shots + spg0 - 1) / spg0);
 }
 
+// Image bands of the adjoint: the columns (rows) that the boxes of the tiles
+// whose box touches a C-PML strip cover.  Rows depend on the tile height th.
+struct Bands {
+    long long jl, jr, wx, wxp, txs, tzs;   // tzs: for the highest tiles, whose bands are the widest
+};
+void row_band(long long nz, int pad, int fs, int K, int th, int *lo, int *hi)
+{
+    *lo = 0;
+    *hi = (int)nz;
+    for (int i0 = 0; i0 < nz; i0 += th) {
+        if (!fs && i0 - K < pad) *lo = i0 + th + K;
+        if (i0 + th + K > nz - pad) *hi = std::min(*hi, i0 - K);
+    }
+    *lo = std::min<int>(*lo, (int)nz);
+    *hi = std::max(*hi, *lo);
+}
+Bands bands_of(long long nz, long long nx, long long P, int pad, int fs, int K)
+{
+    Bands b{};
+    b.jl = 0;
+    b.jr = nx;
+    for (long long j0 = 0; j0 < nx; j0 += TX4) {
+        if (j0 - XO4 < pad) b.jl = j0 + TX4 + XO4;
+        if (j0 + TX4 + XO4 > nx - pad) b.jr = std::min(b.jr, j0 - XO4);
+    }
+    // bands that meet are one band (band coordinates are then the grid's own)
+    if (b.jl >= b.jr) b.jr = b.jl;
+    b.wx = b.jl < b.jr ? b.jl + nx - b.jr : nx;
+    b.wxp = (std::max(b.wx, b.jl) + 2 + 31) / 32 * 32;
+    b.txs = nz * b.wxp;
+    int lo, hi;
+    row_band(nz, pad, fs, K, RPT_DEFAULT * NWARP, &lo, &hi);
+    b.tzs = (lo + nz - hi) * P;
+    return b;
+}
+
 // k: history segment length (k = nt: every step kept, no checkpoints)
 Plan make_plan(const stfwi_desc *d, int k)
 {
@@ -177,6 +219,8 @@ Plan make_plan(const stfwi_desc *d, int k)
     const int G = acc_groups_of(d);
     p.fields = (size_t)2 * S * F_N * p.nz * p.P * sizeof(float);
     p.psi = (size_t)S * (NPX * p.nz * p.xs_n + NPZ * p.zs_n * p.P) * sizeof(float);
+    const Bands bd = bands_of(p.nz, p.nx, p.P, d->pad, d->free_surface, d->fd_order / 2);
+    p.psi += (size_t)S * 4 * (bd.txs + bd.tzs) * sizeof(float);
     // history fields per slot: the stresses, plus U and V for the density
     // gradient (want_gradient == 2); with checkpoints and velocities one more
     // slot holds the first output of the following segment
@@ -186,7 +230,8 @@ Plan make_plan(const stfwi_desc *d, int k)
     p.row0 = (d->want_gradient && d->free_surface) ? (size_t)S * slots * d->nx_dom * sizeof(float) : 0;
     const long long ncp = (d->want_gradient && k < d->nt) ? (d->nt + k - 1) / k : 0;
     p.ckpt = (size_t)ncp * S * (F_N * p.nz * p.P + PX_NFWD * p.nz * p.xs_n + PZ_NFWD * p.zs_n * p.P) * sizeof(float);
-    p.acc = (size_t)G * ((snf == 5 ? 7 : 5) * p.nd + d->nx_dom) * sizeof(double) + 3 * p.nd * 2 * sizeof(double);
+    p.acc = (d->want_gradient ? (size_t)G * (snf == 5 ? 7 : 5) * p.nd * sizeof(double) : 0) +
+            (size_t)S * (d->nx_dom + 1) * sizeof(double) + 3 * p.nd * 2 * sizeof(double);
     p.rec = (size_t)2 * S * 4 * d->nt * std::max(d->nrec, 1) * sizeof(float)
           + (size_t)S * d->nt * std::max(d->nrec, 1) * sizeof(float);
     p.misc = (size_t)(8 * p.nz * p.P + 4 * p.nd) * sizeof(float) + (size_t)2 * p.nz * p.nx * sizeof(double)
@@ -236,7 +281,7 @@ __global__ void k_vpmax(const float *vp, long long n, float *out)
 // 2-D coefficient arrays are constant along rows (x) / columns (z).
 __global__ void k_pml(int nz, int nx, int nz_dom, int pad, int fs, double dx, double dt, double fc,
                       const float *vpmax, float *bx, float *ax, float *ikx, float *bz, float *az,
-                      float *ikz)
+                      float *ikz, float4 *pmx, float4 *pmz)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const double Lp = pad * dx;
@@ -261,6 +306,7 @@ __global__ void k_pml(int nz, int nx, int nz_dom, int pad, int fs, double dx, do
         if (t < pad) i = pad - 1 - t;
         else if (t >= nx - pad) i = t - (nx - pad);
         coef(i, bx + t, ax + t, ikx + t);
+        pmx[t] = i < 0 ? make_float4(0.f, 0.f, 1.f, 0.f) : make_float4(bx[t], ax[t], ikx[t], 0.f);
     }
     if (t < nz) {
         int i = -1;
@@ -268,6 +314,10 @@ __global__ void k_pml(int nz, int nx, int nz_dom, int pad, int fs, double dx, do
         if (t >= bottom) i = t - bottom;
         else if (!fs && t < pad) i = pad - 1 - t;
         coef(i, bz + t, az + t, ikz + t);
+        // the z-strip index: bottom strip first, then the top one
+        const int zs = i < 0 ? -1 : t >= bottom ? t - bottom : pad + t;
+        pmz[t] = i < 0 ? make_float4(0.f, 0.f, 1.f, __int_as_float(-1))
+                       : make_float4(bz[t], az[t], ikz[t], __int_as_float(zs));
     }
 }
 
@@ -285,15 +335,14 @@ __global__ void k_src_coefs(int nshot, const int *sx, const int *sz, int P, cons
 }
 
 // adjoint prologue: receiver injection of the last step into exx_a, ezz_a
-__global__ void k_inject_last(Geo g, const int *rx, const int *rz, const float *rec_adj, float *A)
+__global__ void k_inject_last(Geo g, Mat m, Images im, const int *rx, const int *rz, const float *rec_adj, float *A,
+                              float *PX, float *PZ)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.nshot * g.nrec) return;
     const int s = t / g.nrec, r = t % g.nrec;
-    const long long o = (long long)rz[r] * g.P + rx[r];
     const float *src = rec_adj + (long long)s * 4 * g.nt * g.nrec + (long long)(g.nt - 1) * g.nrec + r;
-    atomicAdd(A + ((long long)s * F_N + F_EX) * g.fstride + o, src[2LL * g.nt * g.nrec]);
-    atomicAdd(A + ((long long)s * F_N + F_EZ) * g.fstride + o, src[3LL * g.nt * g.nrec]);
+    inject_strain(g, m, im, A, PX, PZ, s, rz[r], rx[r], src[2LL * g.nt * g.nrec], src[3LL * g.nt * g.nrec]);
 }
 
 // Residual preparation (fwi/gradient.py:139-156, fwi/filters.py), one thread
@@ -364,33 +413,39 @@ __global__ void k_misfit_reduce(int nshot, int nrec, const double *mis_trace, do
     mis_shot[s] = a;
 }
 
-// (M, L, L2M) or (lambda, mu) partial sums -> (Vs, Vp, rho) gradients on the
-// physical grid.  EXACT: M = rho Vs^2, L2M = rho Vp^2, L = L2M - 2M; the
+// Partial sums -> (Vs, Vp, rho) gradients on the physical grid.  The exact
+// gradient's sums of stresses against stress adjoints become (M, L, L2M)
+// gradients with the strain-recovery factors, g_L2M = idet (L2M sA - L sB),
+// g_L = idet (L2M sB - L sA), g_M = sC / M; a moment source adds its term to
+// g_M and g_L of its cell.  EXACT: M = rho Vs^2, L2M = rho Vp^2, L = L2M - 2M; the
 // free-surface ratio Lr = -L/L2M contributes on row 0.  IMAGING:
 // fwi/imaging.py:165-167.
-__global__ void k_finalize(Geo g, int groups, int accp, int lr_rows, const double *acc, const double *accLr,
-                           const float *L2M, const float *L, const float *vs, const float *vp,
+__global__ void k_finalize(Geo g, int groups, int accp, const double *acc, const double *accLr, const double *mterm,
+                           Shots sh, const float *L2M, const float *L, const float *M, const float *vs, const float *vp,
                            const float *rho, int want_exact, int want_img, double *out_exact,
                            double *out_img)
 {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (q >= g.nd) return;
     const int pi = (int)(q / g.nx_dom), pj = (int)(q % g.nx_dom);
-    double gM = 0, gL = 0, gL2M = 0, gla = 0, gmu = 0, gB = 0, grl = 0;
+    double sA = 0, sB = 0, sC = 0, gla = 0, gmu = 0, gB = 0, grl = 0;
     for (int k = 0; k < groups; ++k) {
         const double *a = acc + (long long)k * accp * g.nd + q;
-        gM += a[0]; gL += a[g.nd]; gL2M += a[2 * g.nd]; gla += a[3 * g.nd]; gmu += a[4 * g.nd];
+        sC += a[0]; sB += a[g.nd]; sA += a[2 * g.nd]; gla += a[3 * g.nd]; gmu += a[4 * g.nd];
         if (accp == 7) { gB += a[5 * g.nd]; grl += a[6 * g.nd]; }
     }
     const double r = rho[q], a = vs[q], b = vp[q];
     if (want_exact) {
+        const long long oc = (long long)(pi + g.z0) * g.P + pj + g.pad;
+        const double cl2m = L2M[oc], cl = L[oc], id = 1.0 / ((cl2m - cl) * (cl2m + cl));
+        double gM = sC / (double)M[oc], gL = id * (cl2m * sB - cl * sA), gL2M = id * (cl2m * sA - cl * sB);
+        for (int s = 0; s < g.nshot; ++s)
+            if (sh.type[s] == 1 && sh.sz[s] == pi + g.z0 && sh.sx[s] == pj + g.pad) { gM += mterm[s]; gL += mterm[s]; }
         if (g.fs && pi == 0) {
             double glr = 0;
-            for (int k = 0; k < lr_rows; ++k) glr += accLr[(long long)k * g.nx_dom + pj];
-            const long long o = (long long)(pi + g.z0) * g.P + pj + g.pad;
-            const double l2m = L2M[o], l = L[o];
-            gL += -glr / l2m;
-            gL2M += glr * l / (l2m * l2m);
+            for (int k = 0; k < g.nshot; ++k) glr += accLr[(long long)k * g.nx_dom + pj];
+            gL += -glr / cl2m;
+            gL2M += glr * cl / (cl2m * cl2m);
         }
         out_exact[q] = 2.0 * r * a * (gM - 2.0 * gL);
         out_exact[g.nd + q] = 2.0 * r * b * (gL2M + gL);
@@ -412,7 +467,7 @@ Mat mat_of(stfwi_handle *h)
 }
 Shots shots_of(stfwi_handle *h)
 {
-    return Shots{h->sx, h->sz, h->stype, h->wav, h->fcoef, h->mcoef, h->lm};
+    return Shots{h->sx, h->sz, h->stype, h->spos, h->wav, h->fcoef, h->mcoef, h->lm};
 }
 
 // event pair of sampled step n around kernel k (0 fwd_vel, 1 fwd_str, 2 adj_a, 3 adj_b)
@@ -429,86 +484,127 @@ inline void prof_mark(stfwi_handle *h, int k, int n, int which, cudaStream_t st)
     else cudaEventRecord(h->pev[k][idx], st);
 }
 
-// the shot groups of kernel k that a launch covers: all of them (part < 0)
-// or chain `part`'s share of the h->nchain_cur chains of a split pass
-// (consecutive groups); the Geo of the launch carries the first group
-Geo part_geo(const stfwi_handle *h, int k, int part, int *ngroups)
+// A pass may run as chains of launches over parts of the shots, which never
+// interact (each owns its fields, C-PML memories and history; the shared sums
+// are atomic).
+struct Part {
+    int index, s0, s1;   // shots [s0, s1)
+};
+
+std::vector<Part> parts_of(const stfwi_handle *h, int parts)
 {
-    Geo g = h->g;
-    const int G = h->grp[k], C = h->nchain_cur;
-    if (part < 0) {
-        *ngroups = G;
-        return g;
-    }
-    const int a = G * part / C, b = G * (part + 1) / C;
-    g.goff = a;
-    *ngroups = b - a;
-    return g;
+    std::vector<Part> p;
+    const int n = h->nshot;
+    for (int k = 0; k < parts; ++k)
+        p.push_back(Part{k, (int)((long long)n * k / parts), (int)((long long)n * (k + 1) / parts)});
+    return p;
 }
 
-// chains a pass may run as: independent chains over the shot groups (the
-// shots never interact, the shared sums are atomic) when every stencil
-// kernel groups the shots the same way -- a chain's kernels then touch
-// exactly its own shots -- and no sampled timing is on; at most one chain
-// per group
-int pass_chains(const stfwi_handle *h)
+// the work of a launch of kernel k over a part's shots
+Work work_of(const stfwi_handle *h, int k, const Part &part)
 {
-    for (int k = 1; k < 4; ++k)
-        if (h->spgk[k] != h->spgk[0] || h->grp[k] != h->grp[0]) return 1;
-    if (h->prof_every != 0) return 1;
-    return std::max(1, std::min(h->chains, h->grp[0]));
+    Work w{};
+    w.order = k == 3 ? h->tordB : h->tordA;
+    w.ntx = h->ntx;
+    w.tiles = h->ntx * (k == 3 ? h->ntzb : h->ntza);
+    w.s0 = part.s0;
+    w.s1 = part.s1;
+    w.part = part.index;
+    return w;
+}
+
+// Blocks of a launch and each block's share of the items: runs of at most
+// `run` shots (h->spgk), but at least one block per slot of the device while
+// there are items enough.  Runs of 5-7 are the best on every grid measured
+// (exact gradient, us a step, forward + adjoint: 50 shots of 172 x 540 cells
+// 88.9 + 123.0 at 3, 81.4 + 119.7 at 5, 85.8 + 132.5 at 10; 16 shots of
+// 324 x 1040 100.0 + 134.7, 90.2 + 129.5, 98.1 + 141.7): shorter runs pay a
+// block's start and the FP64 sums of its tile more often, longer ones leave
+// the last blocks of a launch alone on the device.
+template <typename K> int blocks_of(stfwi_handle *h, K kern, size_t smem, int run, Work &w)
+{
+    int &n = h->resident[(const void *)kern];
+    if (n == 0) {
+        int per = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, NTHR, smem) != cudaSuccess) cudaGetLastError();
+        n = std::max(1, per) * h->sms;
+    }
+    const int items = w.tiles * (w.s1 - w.s0);
+    const int blocks = std::max(std::min(items, n), (items + run - 1) / run);
+    w.per = items / blocks;
+    w.extra = items % blocks;
+    return blocks;
+}
+
+// parts of a pass, each on a stream of its own.  One part while sampled
+// timing is on (one event pair per kernel and step).
+std::vector<Part> pass_parts(const stfwi_handle *h)
+{
+    return parts_of(h, h->prof_every != 0 ? 1 : std::max(1, std::min(h->chains, h->nshot)));
+}
+
+// groups of accumulator planes a pass uses: one per block that shares a tile
+// of a part, as far as there are any
+int acc_in_use(const stfwi_handle *h, int parts)
+{
+    const int n = (h->nshot + parts - 1) / parts, items = h->ntx * h->ntzb * n;
+    const int blocks = std::max(std::min(items, 2 * h->sms), (items + h->spgk[3] - 1) / h->spgk[3]);
+    const int per = std::max(1, items / blocks);
+    return std::min(h->acc_groups, parts * ((n - 1) / per + 1));
 }
 
 template <int FD, int R>
-void launch_fwd_step_r(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, int part)
+void launch_fwd_step_r(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Part &part)
 {
-    using Lk = L5<FD, R>;
-    const int tiles = h->ntx * h->ntza;
-    dim3 block(TX, NWARP);
+    using Sg = Stage<FD, R>;
+    const dim3 block(TX, NWARP);
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
-    int ng = 0;
-    const Geo g0 = part_geo(h, 0, part, &ng);
+    constexpr size_t bv = Sg::bytes(Sg::VEL, Sg::NVEL), bs = Sg::bytes(Sg::STR, Sg::NSTR);
+    Work w0 = work_of(h, 0, part), w1 = work_of(h, 1, part);
+    const int n0 = blocks_of(h, st_fwd_vel<FD, R>, bv, h->spgk[0], w0);
     prof_mark(h, 0, n, 0, st);
-    st_fwd_vel<FD, R><<<dim3(tiles, ng), block, Lk::bytes(Lk::VEL, 2), st>>>(
-        g0, mat_of(h), shots_of(h), h->F, h->PX, h->PZ, n, h->spgk[0], h->ntx, h->status, h->tmS, h->tmUo);
+    st_fwd_vel<FD, R><<<n0, block, bv, st>>>(
+        h->g, mat_of(h), shots_of(h), h->F, h->PX, h->PZ, n, w0, h->status, h->tmS, h->tmUo);
     prof_mark(h, 0, n, 1, st);
     prof_mark(h, 1, n, 0, st);
-    const Geo g1 = part_geo(h, 1, part, &ng);
     auto str = o.energy ? st_fwd_str<FD, R, true> : st_fwd_str<FD, R, false>;
-    str<<<dim3(tiles, ng), block, Lk::bytes(Lk::STR, 2), st>>>(
-        g1, mat_of(h), shots_of(h), rva, h->F, h->PX, h->PZ, n, h->spgk[1], h->ntx, o, h->tmV, h->tmSo);
+    const int n1 = blocks_of(h, str, bs, h->spgk[1], w1);
+    str<<<n1, block, bs, st>>>(
+        h->g, mat_of(h), shots_of(h), rva, h->F, h->PX, h->PZ, n, w1, o, h->tmV, h->tmSo);
     prof_mark(h, 1, n, 1, st);
 }
 
 template <int FD>
-void launch_fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, int part)
+void launch_fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Part &part)
 {
     if (h->ra == 1) launch_fwd_step_r<FD, 1>(h, n, o, st, part);
     else launch_fwd_step_r<FD, 2>(h, n, o, st, part);
 }
 
 template <int FD, int R>
-void launch_adj_a_r(stfwi_handle *h, int n, const AdjIn &ai, cudaStream_t st, int part)
+void launch_adj_a_r(stfwi_handle *h, int n, const AdjIn &ai, cudaStream_t st, const Part &part)
 {
-    using Lk = L5<FD, R>;
+    using Sg = Stage<FD, R>;
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
-    int ng = 0;
-    const Geo ga = part_geo(h, 2, part, &ng);
-    st_adj_a<FD, R><<<dim3(h->ntx * h->ntza, ng), dim3(TX, NWARP), Lk::bytes(Lk::ADA, 2), st>>>(
-        ga, mat_of(h), rva, h->A, h->PX, h->PZ, n, h->spgk[2], h->ntx, ai, h->status, h->tmE, h->tmPQo);
+    constexpr size_t bytes = Sg::bytes(Sg::ADA, Sg::NADA);
+    Work w = work_of(h, 2, part);
+    const int nb = blocks_of(h, st_adj_a<FD, R>, bytes, h->spgk[2], w);
+    st_adj_a<FD, R><<<nb, dim3(TX, NWARP), bytes, st>>>(
+        h->g, mat_of(h), rva, h->A, h->PX, h->PZ, h->im, n, w, ai, h->status, h->tmE, h->tmPQo, h->tmXa, h->tmZa);
 }
 
 template <int FD, int R>
-void launch_adj_b_r(stfwi_handle *h, int n, const AdjOut &ao, cudaStream_t st, int part)
+void launch_adj_b_r(stfwi_handle *h, int n, const AdjOut &ao, cudaStream_t st, const Part &part)
 {
-    using Lk = L5<FD, R>;
+    using Sg = Stage<FD, R>;
     Recv rvb{h->tile_startB, h->tile_recB, h->rx, h->rz};
-    int ng = 0;
-    const Geo gb = part_geo(h, 3, part, &ng);
+    constexpr size_t bytes = Sg::bytes(Sg::ADB, Sg::NADB);
+    Work w = work_of(h, 3, part);
     auto launch = [&](auto kern) {
-        kern<<<dim3(h->ntx * h->ntzb, ng), dim3(TX, NWARP), Lk::bytes(Lk::ADB, 2), st>>>(
-            gb, mat_of(h), shots_of(h), rvb, h->A, h->PX, h->PZ, n, h->spgk[3], h->ntx, ao, h->status,
-            h->tmPQ, h->tmEo, h->tmH);
+        const int nb = blocks_of(h, kern, bytes, h->spgk[3], w);
+        kern<<<nb, dim3(TX, NWARP), bytes, st>>>(
+            h->g, mat_of(h), shots_of(h), rvb, h->A, h->PX, h->PZ, h->im, n, w, ao, h->status, h->tmP, h->tmEo,
+            h->tmH, h->tmXb, h->tmZb);
     };
     const bool rho = h->g.snf == 5;
     if (ao.want_exact && ao.want_img) rho ? launch(st_adj_b<FD, R, true, true, true>) : launch(st_adj_b<FD, R, true, true, false>);
@@ -518,7 +614,7 @@ void launch_adj_b_r(stfwi_handle *h, int n, const AdjOut &ao, cudaStream_t st, i
 }
 
 template <int FD>
-void launch_adj_step(stfwi_handle *h, int n, const AdjIn &ai, const AdjOut &ao, cudaStream_t st, int part = -1)
+void launch_adj_step(stfwi_handle *h, int n, const AdjIn &ai, const AdjOut &ao, cudaStream_t st, const Part &part)
 {
     prof_mark(h, 2, n, 0, st);
     if (h->ra == 1) launch_adj_a_r<FD, 1>(h, n, ai, st, part);
@@ -535,37 +631,34 @@ stfwi_status zero_forward_state(stfwi_handle *h, cudaStream_t st)
 {
     const Geo &g = h->g;
     CK(h, cudaMemsetAsync(h->F, 0, (size_t)h->nshot * F_N * g.fstride * sizeof(float), st));
-    for (int s = 0; s < h->nshot; ++s) {
-        CK(h, cudaMemsetAsync(h->PX + (long long)s * NPX * g.xstride, 0,
-                              (size_t)PX_NFWD * g.xstride * sizeof(float), st));
-        CK(h, cudaMemsetAsync(h->PZ + (long long)s * NPZ * g.zstride, 0,
-                              (size_t)PZ_NFWD * g.zstride * sizeof(float), st));
-    }
+    // the forward memories of every shot: the first arrays of its block
+    CK(h, cudaMemset2DAsync(h->PX, NPX * g.xstride * 4, 0, PX_NFWD * g.xstride * 4, h->nshot, st));
+    CK(h, cudaMemset2DAsync(h->PZ, NPZ * g.zstride * 4, 0, PZ_NFWD * g.zstride * 4, h->nshot, st));
     CK(h, cudaMemsetAsync(h->status, 0, sizeof(int), st));
     return STFWI_OK;
 }
 
-stfwi_status zero_adjoint_state(stfwi_handle *h, cudaStream_t st)
+stfwi_status zero_adjoint_state(stfwi_handle *h, int groups, cudaStream_t st)
 {
     const Geo &g = h->g;
     CK(h, cudaMemsetAsync(h->A, 0, (size_t)h->nshot * F_N * g.fstride * sizeof(float), st));
-    for (int s = 0; s < h->nshot; ++s) {
-        CK(h, cudaMemsetAsync(h->PX + ((long long)s * NPX + PX_NFWD) * g.xstride, 0,
-                              (size_t)2 * PXA_N * g.xstride * sizeof(float), st));
-        CK(h, cudaMemsetAsync(h->PZ + ((long long)s * NPZ + PZ_NFWD) * g.zstride, 0,
-                              (size_t)2 * PZA_N * g.zstride * sizeof(float), st));
-    }
-    CK(h, cudaMemsetAsync(h->acc, 0, (size_t)h->acc_used * h->accp * g.nd * sizeof(double), st));
-    CK(h, cudaMemsetAsync(h->accLr, 0, (size_t)h->lr_used * g.nx_dom * sizeof(double), st));
+    CK(h, cudaMemset2DAsync(h->PX + PX_NFWD * g.xstride, NPX * g.xstride * 4, 0, PXA_N * g.xstride * 4, h->nshot, st));
+    CK(h, cudaMemset2DAsync(h->PZ + PZ_NFWD * g.zstride, NPZ * g.zstride * 4, 0, PZA_N * g.zstride * 4, h->nshot, st));
+    // the strains' images; st_adj_a writes the velocities' before they are read
+    CK(h, cudaMemsetAsync(h->im.xa, 0, (size_t)h->nshot * 2 * g.txs * sizeof(float), st));
+    CK(h, cudaMemsetAsync(h->im.za, 0, (size_t)h->nshot * 2 * g.tzs * sizeof(float), st));
+    if (h->acc) CK(h, cudaMemsetAsync(h->acc, 0, (size_t)groups * h->accp * g.nd * sizeof(double), st));
+    CK(h, cudaMemsetAsync(h->accLr, 0, (size_t)h->nshot * g.nx_dom * sizeof(double), st));
+    CK(h, cudaMemsetAsync(h->mterm, 0, (size_t)h->nshot * sizeof(double), st));
     return STFWI_OK;
 }
 
-// history slot 0 of every shot = the physical cells of the current state
+// history slot 0 of the shots from s0 = the physical cells of the current state
 // (the carry-in of the first step of a history segment)
-__global__ void k_snap_state(Geo g, int slots, const float *F, float *snap)
+__global__ void k_snap_state(Geo g, int s0, int slots, const float *F, float *snap)
 {
     const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int s = blockIdx.y;
+    const int s = s0 + blockIdx.y;
     if (q >= g.nd) return;
     const int pi = (int)(q / g.nx_dom), pj = (int)(q % g.nx_dom);
     const long long o = (long long)(pi + g.z0) * g.P + pj + g.pad;
@@ -578,36 +671,36 @@ __global__ void k_snap_state(Geo g, int slots, const float *F, float *snap)
     }
 }
 
-void snap_state(stfwi_handle *h, cudaStream_t st)
+void snap_state(stfwi_handle *h, const Part &p, cudaStream_t st)
 {
     const Geo &g = h->g;
-    k_snap_state<<<dim3((unsigned)((g.nd + 255) / 256), h->nshot), 256, 0, st>>>(g, h->slots, h->F, h->snap);
+    k_snap_state<<<dim3((unsigned)((g.nd + 255) / 256), p.s1 - p.s0), 256, 0, st>>>(g, p.s0, h->slots, h->F, h->snap);
 }
 
-// state of the forward (fields + forward C-PML memories) <-> checkpoint c
-stfwi_status copy_ckpt(stfwi_handle *h, int c, bool save, cudaStream_t st)
+// state of the forward (fields + forward C-PML memories) of a part <-> checkpoint c
+stfwi_status copy_ckpt(stfwi_handle *h, int c, const Part &p, bool save, cudaStream_t st)
 {
     const Geo &g = h->g;
-    const size_t S = (size_t)h->d.max_shots, ns = (size_t)h->nshot;
-    float *cf = h->CKF + (size_t)c * S * F_N * g.fstride;
-    float *cx = h->CKPX + (size_t)c * S * PX_NFWD * g.xstride;
-    float *cz = h->CKPZ + (size_t)c * S * PZ_NFWD * g.zstride;
+    const size_t S = (size_t)h->d.max_shots, ns = (size_t)(p.s1 - p.s0), at = (size_t)c * S + p.s0;
+    float *cf = h->CKF + at * F_N * g.fstride, *f = h->F + (size_t)p.s0 * F_N * g.fstride;
+    float *cx = h->CKPX + at * PX_NFWD * g.xstride, *x = h->PX + (size_t)p.s0 * NPX * g.xstride;
+    float *cz = h->CKPZ + at * PZ_NFWD * g.zstride, *z = h->PZ + (size_t)p.s0 * NPZ * g.zstride;
     const size_t fb = ns * F_N * g.fstride * 4;
     const size_t xw = PX_NFWD * g.xstride * 4, xp = NPX * g.xstride * 4;
     const size_t zw = PZ_NFWD * g.zstride * 4, zp = NPZ * g.zstride * 4;
     if (save) {
-        CK(h, cudaMemcpyAsync(cf, h->F, fb, cudaMemcpyDeviceToDevice, st));
-        CK(h, cudaMemcpy2DAsync(cx, xw, h->PX, xp, xw, ns, cudaMemcpyDeviceToDevice, st));
-        CK(h, cudaMemcpy2DAsync(cz, zw, h->PZ, zp, zw, ns, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpyAsync(cf, f, fb, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpy2DAsync(cx, xw, x, xp, xw, ns, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpy2DAsync(cz, zw, z, zp, zw, ns, cudaMemcpyDeviceToDevice, st));
     } else {
-        CK(h, cudaMemcpyAsync(h->F, cf, fb, cudaMemcpyDeviceToDevice, st));
-        CK(h, cudaMemcpy2DAsync(h->PX, xp, cx, xw, xw, ns, cudaMemcpyDeviceToDevice, st));
-        CK(h, cudaMemcpy2DAsync(h->PZ, zp, cz, zw, zw, ns, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpyAsync(f, cf, fb, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpy2DAsync(x, xp, cx, xw, xw, ns, cudaMemcpyDeviceToDevice, st));
+        CK(h, cudaMemcpy2DAsync(z, zp, cz, zw, zw, ns, cudaMemcpyDeviceToDevice, st));
     }
     return STFWI_OK;
 }
 
-void fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, int part = -1)
+void fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Part &part)
 {
     switch (h->d.fd_order) {
     case 2: launch_fwd_step<2>(h, n, o, st, part); break;
@@ -616,23 +709,23 @@ void fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, int part
     }
 }
 
-// fork the streams of chains 1 .. C-1 off `st` / join them back (event
-// edges of the captured graph); C = h->nchain_cur
-stfwi_status fork_chains(stfwi_handle *h, cudaStream_t st)
+// run fn(part, stream) for every part: their streams fork off `st` and join
+// it again (event edges of a captured graph)
+template <class Fn> stfwi_status run_parts(stfwi_handle *h, cudaStream_t st, Fn fn)
 {
-    CK(h, cudaEventRecord(h->ev_fork, st));
-    for (int c = 1; c < h->nchain_cur; ++c) CK(h, cudaStreamWaitEvent(h->hsx[c - 1], h->ev_fork, 0));
-    return STFWI_OK;
-}
-stfwi_status join_chains(stfwi_handle *h, cudaStream_t st)
-{
-    for (int c = 1; c < h->nchain_cur; ++c) {
+    const std::vector<Part> parts = pass_parts(h);
+    const int lanes = (int)parts.size();
+    if (lanes > 1) CK(h, cudaEventRecord(h->ev_fork, st));
+    for (int c = 1; c < lanes; ++c) CK(h, cudaStreamWaitEvent(h->hsx[c - 1], h->ev_fork, 0));
+    stfwi_status r = STFWI_OK;
+    for (const Part &p : parts)
+        if (!r) r = fn(p, p.index == 0 ? st : h->hsx[p.index - 1]);
+    for (int c = 1; c < lanes; ++c) {
         CK(h, cudaEventRecord(h->ev_join[c - 1], h->hsx[c - 1]));
         CK(h, cudaStreamWaitEvent(st, h->ev_join[c - 1], 0));
     }
-    return STFWI_OK;
+    return r;
 }
-cudaStream_t chain_stream(const stfwi_handle *h, cudaStream_t st, int c) { return c == 0 ? st : h->hsx[c - 1]; }
 
 // record the whole forward pass (kind 0) or illumination pass (kind 2)
 stfwi_status enqueue_forward(stfwi_handle *h, uint32_t flags, int comp, cudaStream_t st)
@@ -651,31 +744,23 @@ stfwi_status enqueue_forward(stfwi_handle *h, uint32_t flags, int comp, cudaStre
     }
     // with checkpoints the history is written later, segment by segment
     const bool hist = store && h->ncp == 0;
-    if (hist) snap_state(h, st);
-    h->nchain_cur = pass_chains(h);
-    const bool split = h->nchain_cur > 1;
     const bool ckpt = store && h->ncp > 0;
-    if (split && !ckpt && (rc = fork_chains(h, st))) return rc;
-    for (int n = 0; n < h->g.nt; ++n) {
-        if (ckpt && n % h->ck == 0) {
-            // the checkpoint copy takes every shot: the chains join before
-            // it and fork again after it
-            if (split && n > 0 && (rc = join_chains(h, st))) return rc;
-            stfwi_status r = copy_ckpt(h, n / h->ck, true, st);
-            if (r) return r;
-            if (split && (rc = fork_chains(h, st))) return rc;
+    rc = run_parts(h, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
+        if (hist) snap_state(h, p, s);
+        for (int n = 0; n < h->g.nt; ++n) {
+            if (ckpt && n % h->ck == 0) {
+                stfwi_status r = copy_ckpt(h, n / h->ck, p, true, s);
+                if (r) return r;
+            }
+            o.snap = hist ? h->snap : nullptr;
+            o.row0 = (hist && h->g.fs) ? h->row0 : nullptr;
+            o.slot = n + 1;
+            o.slot_row0 = n;
+            fwd_step(h, n, o, s, p);
         }
-        o.snap = hist ? h->snap : nullptr;
-        o.row0 = (hist && h->g.fs) ? h->row0 : nullptr;
-        o.slot = n + 1;
-        o.slot_row0 = n;
-        if (split) {
-            for (int c = 0; c < h->nchain_cur; ++c) fwd_step(h, n, o, chain_stream(h, st, c), c);
-        } else {
-            fwd_step(h, n, o, st);
-        }
-    }
-    if (split && (rc = join_chains(h, st))) return rc;
+        return STFWI_OK;
+    });
+    if (rc) return rc;
     CK(h, cudaGetLastError());
     return STFWI_OK;
 }
@@ -758,33 +843,24 @@ stfwi_status encode(stfwi_handle *h, CUtensorMap *m, void *base, int rank, const
     return STFWI_OK;
 }
 
-template <typename Lk>
-stfwi_status set_smem(stfwi_handle *h, const void *const (&kern)[7])
-{
-    const size_t bytes[] = {Lk::bytes(Lk::VEL, 2), Lk::bytes(Lk::STR, 2), Lk::bytes(Lk::ADA, 2), Lk::bytes(Lk::ADB, 2),
-                            Lk::bytes(Lk::ADB, 2), Lk::bytes(Lk::ADB, 2), Lk::bytes(Lk::ADB, 2)};
-    for (int k = 0; k < 7; ++k)
-        CK(h, cudaFuncSetAttribute(kern[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes[k]));
-    return STFWI_OK;
-}
-
 template <int FD, int R>
 stfwi_status setup_tma_kernels_r(stfwi_handle *h)
 {
-    using Lk = L5<FD, R>;
-    const void *const kern[7] = {
-        (const void *)st_fwd_vel<FD, R>, (const void *)st_fwd_str<FD, R, false>, (const void *)st_adj_a<FD, R>,
-        (const void *)st_adj_b<FD, R, true, false, false>, (const void *)st_adj_b<FD, R, true, true, false>,
-        (const void *)st_adj_b<FD, R, false, true, false>, (const void *)st_adj_b<FD, R, false, false, false>};
-    stfwi_status r = set_smem<Lk>(h, kern);
-    if (r) return r;
-    CK(h, cudaFuncSetAttribute((const void *)st_fwd_str<FD, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)Lk::bytes(Lk::STR, 2)));
-    const void *const rho_kern[3] = {(const void *)st_adj_b<FD, R, true, false, true>,
-                                     (const void *)st_adj_b<FD, R, true, true, true>,
-                                     (const void *)st_adj_b<FD, R, false, true, true>};
-    for (const void *k : rho_kern)
-        CK(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Lk::bytes(Lk::ADB, 2)));
+    using Sg = Stage<FD, R>;
+    auto limit = [&](auto kern, size_t bytes) -> stfwi_status {
+        CK(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return STFWI_OK;
+    };
+    constexpr size_t bv = Sg::bytes(Sg::VEL, Sg::NVEL), bs = Sg::bytes(Sg::STR, Sg::NSTR),
+                     ba = Sg::bytes(Sg::ADA, Sg::NADA), bb = Sg::bytes(Sg::ADB, Sg::NADB);
+    stfwi_status r;
+    if ((r = limit(st_fwd_vel<FD, R>, bv)) || (r = limit(st_fwd_str<FD, R, false>, bs)) ||
+        (r = limit(st_fwd_str<FD, R, true>, bs)) || (r = limit(st_adj_a<FD, R>, ba)) ||
+        (r = limit(st_adj_b<FD, R, true, false, false>, bb)) || (r = limit(st_adj_b<FD, R, true, true, false>, bb)) ||
+        (r = limit(st_adj_b<FD, R, false, true, false>, bb)) || (r = limit(st_adj_b<FD, R, false, false, false>, bb)) ||
+        (r = limit(st_adj_b<FD, R, true, false, true>, bb)) || (r = limit(st_adj_b<FD, R, true, true, true>, bb)) ||
+        (r = limit(st_adj_b<FD, R, false, true, true>, bb)))
+        return r;
     return STFWI_OK;
 }
 
@@ -807,12 +883,23 @@ stfwi_status setup_tensor_maps(stfwi_handle *h)
     const cuuint32_t bw = (cuuint32_t)(h->tw + 8);
     const cuuint32_t box3[4] = {bw, (cuuint32_t)(h->tha + 2 * H), 3, 1};
     const cuuint32_t box2[4] = {bw, (cuuint32_t)(h->tha + 2 * H), 2, 1};
-    const cuuint32_t box2s[4] = {bw, (cuuint32_t)(h->thb + 2 * H), 2, 1};
+    const cuuint32_t box1a[4] = {bw, (cuuint32_t)(h->tha + 2 * H), 1, 1};
+    const cuuint32_t box1b[4] = {bw, (cuuint32_t)(h->thb + 2 * H), 1, 1};
     stfwi_status r;
     if ((r = encode(h, &h->tmS, h->F, 4, fdims, fstr, box3))) return r;
     if ((r = encode(h, &h->tmV, h->F, 4, fdims, fstr, box2))) return r;
-    if ((r = encode(h, &h->tmE, h->A, 4, fdims, fstr, box3))) return r;
-    if ((r = encode(h, &h->tmPQ, h->A, 4, fdims, fstr, box2s))) return r;
+    if ((r = encode(h, &h->tmE, h->A, 4, fdims, fstr, box1a))) return r;
+    if ((r = encode(h, &h->tmP, h->A, 4, fdims, fstr, box1b))) return r;
+    // image bands: columns (rows) past the band's end arrive as zeros, as do those past the grid's
+    const cuuint64_t xstr[3] = {(cuuint64_t)g.wxp * 4, (cuuint64_t)g.txs * 4, (cuuint64_t)2 * g.txs * 4};
+    const cuuint64_t xdims[4] = {(cuuint64_t)(g.jl < g.jr ? g.jl + g.nx - g.jr : g.nx), (cuuint64_t)g.nz, 2, S};
+    const cuuint64_t zstr[3] = {(cuuint64_t)g.P * 4, (cuuint64_t)g.tzs * 4, (cuuint64_t)2 * g.tzs * 4};
+    const cuuint64_t zda[4] = {(cuuint64_t)g.nx, (cuuint64_t)(g.ita + g.nz - g.iba), 2, S};
+    const cuuint64_t zdb[4] = {(cuuint64_t)g.nx, (cuuint64_t)(g.itb + g.nz - g.ibb), 2, S};
+    if ((r = encode(h, &h->tmXa, h->im.xa, 4, xdims, xstr, box1a))) return r;
+    if ((r = encode(h, &h->tmXb, h->im.xb, 4, xdims, xstr, box1b))) return r;
+    if ((r = encode(h, &h->tmZa, h->im.za, 4, zda, zstr, box1a))) return r;
+    if ((r = encode(h, &h->tmZb, h->im.zb, 4, zdb, zstr, box1b))) return r;
     {
         const cuuint32_t own2[4] = {(cuuint32_t)h->tw, (cuuint32_t)h->tha, 2, 1};
         const cuuint32_t own3[4] = {(cuuint32_t)h->tw, (cuuint32_t)h->tha, 3, 1};
@@ -835,41 +922,28 @@ stfwi_status setup_tensor_maps(stfwi_handle *h)
     return STFWI_OK;
 }
 
-// shots per block of each staged kernel (balanced groups; the strain phase
-// keeps at most acc_groups accumulator groups)
-void set_groups(stfwi_handle *h, const int spg_in[4])
+// shots per block of each stencil kernel
+void set_groups(stfwi_handle *h, const int spg[4])
 {
-    const int nshot = h->nshot;
-    for (int k = 0; k < 4; ++k) {
-        const int spg = std::max(1, spg_in[k]);
-        int G = (nshot + spg - 1) / spg;
-        if (k == 3) G = std::min(G, h->acc_groups);
-        h->spgk[k] = (nshot + G - 1) / G;
-        h->grp[k] = (nshot + h->spgk[k] - 1) / h->spgk[k];
-    }
-    h->acc_used = h->grp[3];
-    h->lr_used = h->grp[2];
+    for (int k = 0; k < 4; ++k) h->spgk[k] = std::max(1, spg[k]);
 }
 
 }  // namespace
 
-// tiles of a tw x th tiling in dispatch order, the `heavy` tiles first: those
-// whose own cells touch an edge margin, a C-PML strip or the free-surface
-// row, or whose staged box (one halo of K rows and 4 columns) reaches a strip
-// or the free-surface row, i.e. the tiles that take the guarded path
-std::vector<int> tile_order(const Geo &g, int K, int tw, int th, int ntx, int ntz, int *heavy)
+// tiles of a tw x th tiling in the order the blocks take them: the boundary
+// tiles (those with a guarded path: an edge margin, a C-PML strip, the
+// free-surface rows) first, because they cost several interior ones and a
+// launch that ended on them would leave the other SMs idle
+std::vector<uint32_t> tile_order(const Geo &g, int K, int tw, int th, int ntx, int ntz)
 {
-    const int M = 2 * K + 1;
-    std::vector<int> hv, lt;
+    const int M = 2 * K;
+    std::vector<uint32_t> hv, lt;
     for (int t = 0; t < ntx * ntz; ++t) {
         const int i0 = (t / ntx) * th, j0 = (t % ntx) * tw, i1 = i0 + th - 1, j1 = j0 + tw - 1;
-        bool plain = i0 >= M && i1 <= g.nz - 1 - M && j0 >= M && j1 <= g.nx - 1 - M && j0 >= g.pad &&
-                     j1 < g.nx - g.pad && i1 < g.nz - g.pad && (g.fs || i0 >= g.pad);
-        const int r0 = i0 - K, r1 = i1 + K, c0 = j0 - 4, c1 = j1 + 4;
-        const bool box = c0 < g.pad || c1 >= g.nx - g.pad || r1 >= g.nz - g.pad || r0 <= 0 || (!g.fs && r0 < g.pad);
-        (plain && !box ? lt : hv).push_back(t);
+        const int lo = std::max(g.pad, M);
+        const bool plain = i0 >= (g.fs ? M : lo) && i1 < g.nz - lo && j0 >= lo && j1 < g.nx - lo;
+        (plain ? lt : hv).push_back((uint32_t)(t / ntx) << 16 | (uint32_t)(t % ntx));
     }
-    *heavy = (int)hv.size();
     hv.insert(hv.end(), lt.begin(), lt.end());
     return hv;
 }
@@ -911,12 +985,12 @@ static stfwi_status set_tiling(stfwi_handle *h, int ra, int rb)
     h->ntza = (g.nz + h->tha - 1) / h->tha;
     h->ntzb = (g.nz + h->thb - 1) / h->thb;
     const int K = h->d.fd_order / 2;
-    int ha = 0, hb = 0;
-    const std::vector<int> oa = tile_order(g, K, h->tw, h->tha, h->ntx, h->ntza, &ha);
-    const std::vector<int> ob = tile_order(g, K, h->tw, h->thb, h->ntx, h->ntzb, &hb);
+    const std::vector<uint32_t> oa = tile_order(g, K, h->tw, h->tha, h->ntx, h->ntza);
+    const std::vector<uint32_t> ob = tile_order(g, K, h->tw, h->thb, h->ntx, h->ntzb);
     CK(h, cudaMemcpy(h->tordA, oa.data(), oa.size() * 4, cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(h->tordB, ob.data(), ob.size() * 4, cudaMemcpyHostToDevice));
-    g.tordA = h->tordA; g.tordB = h->tordB; g.theavyA = ha; g.theavyB = hb;
+    row_band(g.nz, g.pad, g.fs, K, h->tha, &g.ita, &g.iba);
+    row_band(g.nz, g.pad, g.fs, K, h->thb, &g.itb, &g.ibb);
     stfwi_status r = setup_tensor_maps(h);
     if (r) return r;
     if (h->recv_set && (r = group_receivers(h))) return r;
@@ -1168,13 +1242,14 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
         if (r) { delete h; return r; }
         h->acc_groups = acc_groups_of(d);
     }
-    h->acc_used = h->acc_groups;
     h->slots = k + 1 + ((g.snf == 5 && h->ncp > 0) ? 1 : 0);
 
+    // one device allocation for everything (a cudaMalloc costs about 0.1 ms),
+    // each array on 256 bytes
+    std::vector<std::pair<void **, size_t>> want;
     auto alloc = [&](void **ptr, size_t bytes) -> bool {
         if (bytes == 0) { *ptr = nullptr; return true; }
-        if (cudaMalloc(ptr, bytes) != cudaSuccess) return false;
-        h->bytes += bytes;
+        want.emplace_back(ptr, bytes);
         return true;
     };
     const long long S = d->max_shots, NP = p.nz * p.P, nd = p.nd;
@@ -1182,11 +1257,11 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     bool ok = true;
     ok &= alloc((void **)&h->vs, nd * 4) && alloc((void **)&h->vp, nd * 4) && alloc((void **)&h->rho, nd * 4);
     ok &= alloc((void **)&h->MATS, 4 * NP * 4) && alloc((void **)&h->Lr, p.P * 4);
-    if (ok) { h->B = h->MATS; h->L2M = h->MATS + NP; h->L = h->MATS + 2 * NP; h->M = h->MATS + 3 * NP; }
     ok &= alloc((void **)&h->bx, p.P * 4) && alloc((void **)&h->ax, p.P * 4) && alloc((void **)&h->ikx, p.P * 4);
     ok &= alloc((void **)&h->bz, p.nz * 4) && alloc((void **)&h->az, p.nz * 4) && alloc((void **)&h->ikz, p.nz * 4);
     ok &= alloc((void **)&h->vpmax, 16) && alloc((void **)&h->status, 16);
-    ok &= alloc((void **)&h->sx, S * 4) && alloc((void **)&h->sz, S * 4) && alloc((void **)&h->stype, S * 4);
+    ok &= alloc((void **)&h->sx, S * 4) && alloc((void **)&h->sz, S * 4) && alloc((void **)&h->stype, S * 4) &&
+          alloc((void **)&h->spos, S * sizeof(int4));
     ok &= alloc((void **)&h->wav, S * d->nt * 4) && alloc((void **)&h->fcoef, S * 4) &&
           alloc((void **)&h->mcoef, S * 4) && alloc((void **)&h->lm, S * 4);
     // tile arrays sized for the lowest tiles (set_tiling picks the heights)
@@ -1195,6 +1270,12 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
           alloc((void **)&h->tile_startB, (ntl_max + 1) * 4) && alloc((void **)&h->tile_recB, nrec * 4);
     ok &= alloc((void **)&h->rx, nrec * 4) && alloc((void **)&h->rz, nrec * 4);
     ok &= alloc((void **)&h->tordA, ntl_max * 4) && alloc((void **)&h->tordB, ntl_max * 4);
+    // C-PML tables of whole tiles
+    const int ncx = h->ntx * h->tw, ncz = (int)((p.nz + RPT_DEFAULT * NWARP - 1) / (RPT_DEFAULT * NWARP)) * RPT_DEFAULT * NWARP;
+    ok &= alloc((void **)&h->pmx, (size_t)(ncx + ncz) * sizeof(float4));
+    const Bands bd = bands_of(p.nz, p.nx, p.P, d->pad, g.fs, H);
+    g.jl = (int)bd.jl; g.jr = (int)bd.jr; g.wxp = (int)bd.wxp; g.txs = bd.txs; g.tzs = bd.tzs;
+    ok &= alloc((void **)&h->img, (size_t)S * 4 * (bd.txs + bd.tzs) * sizeof(float));
     ok &= alloc((void **)&h->F, (size_t)S * F_N * NP * 4) && alloc((void **)&h->A, (size_t)S * F_N * NP * 4);
     ok &= alloc((void **)&h->PX, (size_t)S * NPX * p.nz * p.xs_n * 4) &&
           alloc((void **)&h->PZ, (size_t)S * NPZ * p.zs_n * p.P * 4);
@@ -1207,8 +1288,9 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
               alloc((void **)&h->CKPX, (size_t)h->ncp * S * PX_NFWD * p.nz * p.xs_n * 4) &&
               alloc((void **)&h->CKPZ, (size_t)h->ncp * S * PZ_NFWD * p.zs_n * p.P * 4);
     }
-    ok &= alloc((void **)&h->acc, (size_t)h->acc_groups * h->accp * nd * 8) &&
-          alloc((void **)&h->accLr, (size_t)std::max(h->acc_groups, d->max_shots) * std::max(d->nx_dom, 1) * 8) &&
+    // the sums of the model gradients, which need a history
+    ok &= alloc((void **)&h->acc, d->want_gradient ? (size_t)h->acc_groups * h->accp * nd * 8 : 0) &&
+          alloc((void **)&h->accLr, (size_t)S * std::max(d->nx_dom, 1) * 8) && alloc((void **)&h->mterm, (size_t)S * 8) &&
           alloc((void **)&h->gtmp, (size_t)6 * nd * 8);
     ok &= alloc((void **)&h->energy, (size_t)p.nz * p.nx * 8);
     ok &= alloc((void **)&h->pw, (2 * POST_MAX_RADIUS + 1) * 8) && alloc((void **)&h->ptaper, (size_t)nd * 8) &&
@@ -1216,6 +1298,18 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
           alloc((void **)&h->pscr, (size_t)p.nz * p.nx * 8) && alloc((void **)&h->pmax, 64);
     ok &= alloc((void **)&h->mis_trace, (size_t)S * nrec * 8) && alloc((void **)&h->mis_shot, (size_t)S * 8);
     ok &= alloc((void **)&h->src_a, (size_t)S * d->nt * 4);
+    size_t slab = 0;
+    for (const auto &q : want) slab += (q.second + 255) / 256 * 256;
+    ok = ok && cudaMalloc((void **)&h->slab, slab) == cudaSuccess;
+    if (ok) {
+        char *at = h->slab;
+        for (const auto &q : want) {
+            *q.first = at;
+            at += (q.second + 255) / 256 * 256;
+        }
+        h->bytes = slab;
+        h->B = h->MATS; h->L2M = h->MATS + NP; h->L = h->MATS + 2 * NP; h->M = h->MATS + 3 * NP;
+    }
     if (!ok) {
         cudaGetLastError();
         stfwi_destroy(h);
@@ -1237,6 +1331,14 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     cudaMemset(h->MATS, 0, (size_t)4 * NP * 4);
     cudaMemset(h->F, 0, (size_t)S * F_N * NP * 4);
     cudaMemset(h->A, 0, (size_t)S * F_N * NP * 4);
+    cudaMemset(h->img, 0, (size_t)S * 4 * (g.txs + g.tzs) * 4);
+    h->im.xa = h->img;
+    h->im.xb = h->im.xa + S * 2 * g.txs;
+    h->im.za = h->im.xb + S * 2 * g.txs;
+    h->im.zb = h->im.za + S * 2 * g.tzs;
+    cudaMemset(h->pmx, 0, (size_t)(ncx + ncz) * sizeof(float4));
+    h->pmz = h->pmx + ncx;
+    g.pmx = h->pmx; g.pmz = h->pmz;
     {
         stfwi_status r = set_tiling(h, RPT_DEFAULT, RPT_DEFAULT);
         if (r) {
@@ -1254,15 +1356,7 @@ void stfwi_destroy(stfwi_handle *h)
     if (!h) return;
     if (h->hs) cudaStreamSynchronize(h->hs);
     drop_graphs(h);
-    void *bufs[] = {h->vs, h->vp, h->rho, h->MATS, h->Lr, h->bx, h->ax, h->ikx, h->bz,
-                    h->az, h->ikz, h->vpmax, h->status, h->sx, h->sz, h->stype, h->wav, h->fcoef, h->mcoef,
-                    h->lm, h->rx, h->rz, h->F, h->A, h->PX, h->PZ, h->rec,
-                    h->rec_adj, h->obs, h->snap, h->row0, h->acc, h->accLr, h->gtmp, h->energy,
-                    h->mis_trace, h->mis_shot, h->src_a, h->pw, h->ptaper, h->pillum, h->ptmp, h->pscr, h->pmax,
-                    h->tile_startA, h->tile_recA, h->tile_startB, h->tile_recB, h->tordA, h->tordB, h->CKF, h->CKPX,
-                    h->CKPZ};
-    for (void *b : bufs)
-        if (b) cudaFree(b);
+    if (h->slab) cudaFree(h->slab);
     for (int k = 0; k < 4; ++k)
         for (cudaEvent_t e : h->pev[k]) cudaEventDestroy(e);
     if (h->ev_in) cudaEventDestroy(h->ev_in);
@@ -1292,7 +1386,7 @@ stfwi_status stfwi_set_model(stfwi_handle *h, const float *vs, const float *vp, 
     k_vpmax<<<1, 1024, 0, st>>>(h->vp, g.nd, h->vpmax);
     const int nmax = std::max(g.nx, g.nz);
     k_pml<<<(nmax + 127) / 128, 128, 0, st>>>(g.nz, g.nx, g.nz_dom, g.pad, g.fs, h->d.dx, h->d.dt, h->d.fc,
-                                              h->vpmax, h->bx, h->ax, h->ikx, h->bz, h->az, h->ikz);
+                                              h->vpmax, h->bx, h->ax, h->ikx, h->bz, h->az, h->ikz, h->pmx, h->pmz);
     CK(h, cudaGetLastError());
     h->model_set = true;
     if (h->shots_set) {
@@ -1338,6 +1432,7 @@ stfwi_status stfwi_set_shots(stfwi_handle *h, int32_t nshot, const int32_t *src,
     cudaStream_t st = (cudaStream_t)stream;
     Geo &g = h->g;
     std::vector<int> sx(nshot), sz(nshot), ty(nshot);
+    std::vector<int4> pos(nshot);
     for (int s = 0; s < nshot; ++s) {
         sx[s] = src[3 * s] + g.pad;
         sz[s] = src[3 * s + 1] + g.z0;
@@ -1347,7 +1442,9 @@ stfwi_status stfwi_set_shots(stfwi_handle *h, int32_t nshot, const int32_t *src,
         if (sx[s] < 0 || sx[s] >= g.nx || sz[s] < 0 || sz[s] >= g.nz)
             return fail(h, STFWI_ERR_INVALID, "source %d at (%d,%d) is outside the grid", s, src[3 * s + 1], src[3 * s]);
     }
+    for (int s = 0; s < nshot; ++s) pos[s] = make_int4(sz[s], sx[s], ty[s], 0);
     CK(h, cudaStreamSynchronize(st));
+    CK(h, cudaMemcpy(h->spos, pos.data(), nshot * sizeof(int4), cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(h->sx, sx.data(), nshot * 4, cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(h->sz, sz.data(), nshot * 4, cudaMemcpyHostToDevice));
     CK(h, cudaMemcpy(h->stype, ty.data(), nshot * 4, cudaMemcpyHostToDevice));
@@ -1356,11 +1453,7 @@ stfwi_status stfwi_set_shots(stfwi_handle *h, int32_t nshot, const int32_t *src,
     h->nshot = nshot;
     g.nshot = nshot;
     {
-        // shots per block by default (measured on B200, 50 shots of 172 x 540):
-        // enough blocks to keep every SM busy, copies of the next shots in
-        // flight while one computes; the strain phase keeps FP64 sums per cell
-        // over its shots and gains from larger groups
-        static const int dflt4[4] = {3, 3, 3, 4};
+        static const int dflt4[4] = {6, 6, 6, 6};   // see blocks_of
         int spg[4];
         for (int k = 0; k < 4; ++k)
             spg[k] = h->d.shot_group > 0 ? h->d.shot_group : h->tuned[k] > 0 ? h->tuned[k] : dflt4[k];
@@ -1471,31 +1564,36 @@ stfwi_status stfwi_gradient(stfwi_handle *h, uint32_t mode, double *g_out, float
     float *src_dev = sr ? h->src_a : nullptr;
     GraphKey key{1, mode, h->nshot};
     rc = run_graph(h, key, st, [&](cudaStream_t s) {
-        stfwi_status r = zero_adjoint_state(h, s);
+        const int parts = (int)pass_parts(h).size(), groups = acc_in_use(h, parts);
+        stfwi_status r = zero_adjoint_state(h, groups, s);
         if (r) return r;
         const int thr = 256;
         if (g.nrec > 0)
-            k_inject_last<<<(g.nshot * g.nrec + thr - 1) / thr, thr, 0, s>>>(g, h->rx, h->rz, h->rec_adj, h->A);
-        auto adj = [&](int n, int seg0, int seg1, cudaStream_t as, int part) {
-            const int ping = (g.nt - 1 - n) & 1;
+            k_inject_last<<<(g.nshot * g.nrec + thr - 1) / thr, thr, 0, s>>>(g, mat_of(h), h->im, h->rx, h->rz,
+                                                                             h->rec_adj, h->A, h->PX, h->PZ);
+        auto adj = [&](int n, int seg0, int seg1, cudaStream_t as, const Part &part) {
             AdjIn ai{};
             ai.rec_adj = h->rec_adj; ai.row0 = h->row0; ai.slots = h->slots; ai.slot = n - seg0;
-            ai.accLr = h->accLr; ai.want_exact = ex; ai.ping = ping;
+            ai.accLr = h->accLr; ai.want_exact = ex;
             AdjOut ao{};
             ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = n - seg0; ao.slot_img = n - seg0 + 1;
-            ao.accp = h->accp;
+            ao.accp = h->accp; ao.groups = groups; ao.parts = parts; ao.mterm = h->mterm;
             // outputs of step n + 1: the next slot inside a segment, else the
             // extra slot filled from the following segment (checkpoints)
             ao.slot_next = (n + 1 < seg1) ? n - seg0 + 2 : (h->ncp > 0 && n + 1 < g.nt ? h->ck + 1 : -1);
             ao.acc = h->acc; ao.want_exact = ex; ao.want_img = im; ao.hist_tma = h->hist_tma ? 1 : 0;
-            ao.src_a = sr ? src_dev : nullptr; ao.rec_adj = h->rec_adj; ao.ping = ping;
+            ao.src_a = sr ? src_dev : nullptr; ao.rec_adj = h->rec_adj;
             switch (h->d.fd_order) {
             case 2: launch_adj_step<2>(h, n, ai, ao, as, part); break;
             case 4: launch_adj_step<4>(h, n, ai, ao, as, part); break;
             default: launch_adj_step<8>(h, n, ai, ao, as, part); break;
             }
         };
-        if ((ex || im) && h->ncp > 0) {
+        r = run_parts(h, s, [&](const Part &p, cudaStream_t ps) -> stfwi_status {
+            if (!((ex || im) && h->ncp > 0)) {
+                for (int n = g.nt - 1; n >= 0; --n) adj(n, 0, g.nt, ps, p);
+                return STFWI_OK;
+            }
             // segments from the last: restore the checkpoint, recompute the
             // segment's history, run its adjoint steps
             for (int c = h->ncp - 1; c >= 0; --c) {
@@ -1503,49 +1601,32 @@ stfwi_status stfwi_gradient(stfwi_handle *h, uint32_t mode, double *g_out, float
                 if (g.snf == 5 && c + 1 < h->ncp) {
                     // keep the velocities of step seg1 (slot 1 of the segment
                     // just processed) for the density term of step seg1 - 1
-                    const size_t ps = (size_t)h->slots * g.snf * g.nd * sizeof(float);
-                    CK(h, cudaMemcpy2DAsync(h->snap + ((size_t)h->ck + 1) * g.snf * g.nd + 3 * g.nd, ps,
-                                            h->snap + (size_t)g.snf * g.nd + 3 * g.nd, ps,
-                                            (size_t)2 * g.nd * sizeof(float), h->nshot, cudaMemcpyDeviceToDevice, s));
+                    const size_t pitch = (size_t)h->slots * g.snf * g.nd * sizeof(float);
+                    float *base = h->snap + (size_t)p.s0 * h->slots * g.snf * g.nd + 3 * g.nd;
+                    CK(h, cudaMemcpy2DAsync(base + ((size_t)h->ck + 1) * g.snf * g.nd, pitch, base + (size_t)g.snf * g.nd,
+                                            pitch, (size_t)2 * g.nd * sizeof(float), p.s1 - p.s0,
+                                            cudaMemcpyDeviceToDevice, ps));
                 }
-                r = copy_ckpt(h, c, false, s);
-                if (r) return r;
-                snap_state(h, s);
+                stfwi_status q = copy_ckpt(h, c, p, false, ps);
+                if (q) return q;
+                snap_state(h, p, ps);
                 FwdOut o{};
                 o.rec = h->rec; o.status = h->status; o.slots = h->slots;
                 o.snap = h->snap; o.row0 = g.fs ? h->row0 : nullptr;
-                // the segment's recompute and adjoint steps in chains over
-                // the shot groups; the copies above take every shot
-                const int C = h->nchain_cur = pass_chains(h);
-                if (C > 1 && (r = fork_chains(h, s))) return r;
                 for (int n = seg0; n < seg1; ++n) {
                     o.slot = n - seg0 + 1;
                     o.slot_row0 = n - seg0;
-                    if (C > 1)
-                        for (int q = 0; q < C; ++q) fwd_step(h, n, o, chain_stream(h, s, q), q);
-                    else
-                        fwd_step(h, n, o, s);
+                    fwd_step(h, n, o, ps, p);
                 }
-                for (int n = seg1 - 1; n >= seg0; --n) {
-                    if (C > 1)
-                        for (int q = 0; q < C; ++q) adj(n, seg0, seg1, chain_stream(h, s, q), q);
-                    else
-                        adj(n, seg0, seg1, s, -1);
-                }
-                if (C > 1 && (r = join_chains(h, s))) return r;
+                for (int n = seg1 - 1; n >= seg0; --n) adj(n, seg0, seg1, ps, p);
             }
-        } else if ((h->nchain_cur = pass_chains(h)) > 1) {
-            if ((r = fork_chains(h, s))) return r;
-            for (int n = g.nt - 1; n >= 0; --n)
-                for (int c = 0; c < h->nchain_cur; ++c) adj(n, 0, g.nt, chain_stream(h, s, c), c);
-            if ((r = join_chains(h, s))) return r;
-        } else {
-            for (int n = g.nt - 1; n >= 0; --n) adj(n, 0, g.nt, s, -1);
-        }
+            return STFWI_OK;
+        });
+        if (r) return r;
         if (ex || im)
-            k_finalize<<<(unsigned)((g.nd + 255) / 256), 256, 0, s>>>(g, h->acc_used, h->accp, h->lr_used, h->acc, h->accLr, h->L2M,
-                                                                      h->L, h->vs, h->vp, h->rho, ex, im,
-                                                                      h->gtmp, h->gtmp + 3 * g.nd);
+            k_finalize<<<(unsigned)((g.nd + 255) / 256), 256, 0, s>>>(g, groups, h->accp, h->acc, h->accLr, h->mterm,
+                                                                      shots_of(h), h->L2M, h->L, h->M, h->vs, h->vp,
+                                                                      h->rho, ex, im, h->gtmp, h->gtmp + 3 * g.nd);
         CK(h, cudaGetLastError());
         return STFWI_OK;
     });
@@ -1759,34 +1840,29 @@ static stfwi_status enqueue_timing_steps(stfwi_handle *h, int steps, cudaStream_
 {
     const Geo &g = h->g;
     stfwi_status r;
-    if ((r = zero_forward_state(h, st)) || (r = zero_adjoint_state(h, st))) return r;
-    const int C = h->nchain_cur = pass_chains(h);
-    if (C > 1 && (r = fork_chains(h, st))) return r;
+    const int parts = (int)pass_parts(h).size(), groups = acc_in_use(h, parts);
+    if ((r = zero_forward_state(h, st)) || (r = zero_adjoint_state(h, groups, st))) return r;
     FwdOut o{};
     o.rec = h->rec; o.status = h->status; o.slots = h->slots;
-    for (int n = 0; n < steps; ++n)
-        for (int q = 0; q < C; ++q) fwd_step(h, n, o, chain_stream(h, st, q), C > 1 ? q : -1);
     const bool ex = h->snap != nullptr;
-    for (int n = steps - 1; n >= 0; --n) {
-        AdjIn ai{};
-        ai.rec_adj = h->rec_adj; ai.row0 = h->row0; ai.slots = h->slots; ai.slot = 0;
-        ai.accLr = h->accLr; ai.want_exact = ex && g.fs; ai.ping = n & 1;
-        AdjOut ao{};
-        ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = 0; ao.slot_img = h->slots > 1 ? 1 : -1;
-        ao.slot_next = -1; ao.accp = h->accp; ao.acc = h->acc; ao.want_exact = ex; ao.want_img = 0;
-        ao.rec_adj = h->rec_adj; ao.ping = n & 1; ao.hist_tma = h->hist_tma ? 1 : 0;
-        for (int q = 0; q < C; ++q) {
-            cudaStream_t cs = chain_stream(h, st, q);
-            const int part = C > 1 ? q : -1;
+    return run_parts(h, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
+        for (int n = 0; n < steps; ++n) fwd_step(h, n, o, s, p);
+        for (int n = steps - 1; n >= 0; --n) {
+            AdjIn ai{};
+            ai.rec_adj = h->rec_adj; ai.row0 = h->row0; ai.slots = h->slots; ai.slot = 0;
+            ai.accLr = h->accLr; ai.want_exact = ex && g.fs;
+            AdjOut ao{};
+            ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = 0; ao.slot_img = h->slots > 1 ? 1 : -1;
+            ao.slot_next = -1; ao.accp = h->accp; ao.groups = groups; ao.parts = parts; ao.mterm = h->mterm; ao.acc = h->acc;
+            ao.want_exact = ex; ao.want_img = 0; ao.rec_adj = h->rec_adj; ao.hist_tma = h->hist_tma ? 1 : 0;
             switch (h->d.fd_order) {
-            case 2: launch_adj_step<2>(h, n, ai, ao, cs, part); break;
-            case 4: launch_adj_step<4>(h, n, ai, ao, cs, part); break;
-            default: launch_adj_step<8>(h, n, ai, ao, cs, part); break;
+            case 2: launch_adj_step<2>(h, n, ai, ao, s, p); break;
+            case 4: launch_adj_step<4>(h, n, ai, ao, s, p); break;
+            default: launch_adj_step<8>(h, n, ai, ao, s, p); break;
             }
         }
-    }
-    if (C > 1 && (r = join_chains(h, st))) return r;
-    return STFWI_OK;
+        return STFWI_OK;
+    });
 }
 
 stfwi_status stfwi_autotune(stfwi_handle *h, int32_t steps, int32_t *spg_out, void *stream)
@@ -1992,8 +2068,9 @@ stfwi_status stfwi_forward_frames(stfwi_handle *h, uint32_t fields, float *frame
     o.status = h->status;
     o.slots = h->slots;
     const dim3 grid((unsigned)((N + 255) / 256), h->nshot);
+    const Part all = parts_of(h, 1)[0];
     for (int n = 0; n < g.nt; ++n) {
-        fwd_step(h, n, o, st);
+        fwd_step(h, n, o, st, all);
         k_frames_fwd<<<grid, 256, 0, st>>>(g, mat_of(h), h->F, fields, nf, stage);
         // frame n of every (shot, field) plane: rows of N floats, nt frames apart
         cudaError_t e = cudaMemcpy2DAsync(frames + (size_t)n * N, (size_t)g.nt * N * sizeof(float), stage,
@@ -2032,24 +2109,24 @@ stfwi_status stfwi_adjoint_frames(stfwi_handle *h, uint32_t fields, float *frame
         cudaGetLastError();
         return fail(h, STFWI_ERR_OOM, "no room for the %zu-byte frame staging buffer", sbytes);
     }
-    rc = zero_adjoint_state(h, st);
+    rc = zero_adjoint_state(h, 1, st);
     if (rc) { cudaFreeAsync(stage, st); return rc; }
     const int thr = 256;
     const unsigned nrb = (unsigned)((g.nshot * std::max(g.nrec, 1) + thr - 1) / thr);
-    if (g.nrec > 0) k_inject_last<<<nrb, thr, 0, st>>>(g, h->rx, h->rz, h->rec_adj, h->A);
+    if (g.nrec > 0) k_inject_last<<<nrb, thr, 0, st>>>(g, mat_of(h), h->im, h->rx, h->rz, h->rec_adj, h->A, h->PX, h->PZ);
     const dim3 grid((unsigned)((N + 255) / 256), h->nshot);
+    const Part all = parts_of(h, 1)[0];
     for (int n = g.nt - 1; n >= 0; --n) {
-        const int ping = (g.nt - 1 - n) & 1;
         AdjIn ai{};
         ai.rec_adj = h->rec_adj; ai.row0 = h->row0; ai.slots = h->slots; ai.slot = 0;
-        ai.accLr = h->accLr; ai.want_exact = 0; ai.ping = ping;
+        ai.accLr = h->accLr; ai.want_exact = 0;
         AdjOut ao{};
         ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = -1; ao.slot_img = -1; ao.slot_next = -1;
-        ao.accp = h->accp; ao.acc = h->acc; ao.src_a = h->src_a; ao.rec_adj = h->rec_adj; ao.ping = ping;
+        ao.accp = h->accp; ao.groups = 1; ao.parts = 1; ao.acc = h->acc; ao.src_a = h->src_a; ao.rec_adj = h->rec_adj;
         switch (h->d.fd_order) {
-        case 2: launch_adj_step<2>(h, n, ai, ao, st); break;
-        case 4: launch_adj_step<4>(h, n, ai, ao, st); break;
-        default: launch_adj_step<8>(h, n, ai, ao, st); break;
+        case 2: launch_adj_step<2>(h, n, ai, ao, st, all); break;
+        case 4: launch_adj_step<4>(h, n, ai, ao, st, all); break;
+        default: launch_adj_step<8>(h, n, ai, ao, st, all); break;
         }
         k_frames_adj<<<grid, 256, 0, st>>>(g, mat_of(h), h->A, fields, nf, stage);
         if (g.nrec > 0 && n > 0 && (kex >= 0 || kez >= 0))
