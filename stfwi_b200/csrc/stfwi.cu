@@ -348,69 +348,160 @@ __global__ void k_inject_last(Geo g, Mat m, Images im, const int *rx, const int 
 // Residual preparation (fwi/gradient.py:139-156, fwi/filters.py), one thread
 // per trace: r = F T (pred - obs); misfit = scale/nshot * mean(r^2);
 // cotangent = 2 scale/(nshot N) T^T F^T r, F^T being the time-reversed cascade.
+// The other components of rec_adj are zeroed by the caller.
+//
+// A trace is a serial recurrence, so the kernel lasts as long as nt steps of
+// one thread: NS sections' states in registers (NS < 0: any number, in local
+// memory), each section's output one fma behind its input (the terms of the
+// past summed first), the samples of the next MIS_C steps requested before
+// those of the current ones are used, the taper's cosines computed by the
+// lanes of a warp for one another, and one warp per block so that few traces
+// still spread over the SMs.  250 traces, 3 sections, 200 steps: 246 us before,
+// with the states in local memory and every load waited for, 43 us now.
 struct SosParams {
     int nsos;
     double c[MAX_SOS][5];  // b0 b1 b2 a1 a2, normalised by a0
 };
+constexpr int MIS_C = 16;
 
-__global__ void k_misfit(Geo g, int comp, int n_taper, SosParams sp, double scale, int nshot_norm,
-                         const float *rec, const float *obs, float *rec_adj, double *mis_trace)
+template <int NS> struct Cascade {
+    double st[NS < 0 ? MAX_SOS : (NS > 0 ? NS : 1)][4];   // x[n-1], x[n-2], y[n-1], y[n-2] of each section
+    __device__ __forceinline__ void clear(const SosParams &sp)
+    {
+        const int ns = NS < 0 ? sp.nsos : NS;
+#pragma unroll
+        for (int k = 0; k < ns; ++k) st[k][0] = st[k][1] = st[k][2] = st[k][3] = 0.0;
+    }
+    __device__ __forceinline__ double section(const SosParams &sp, int k, double x)
+    {
+        const double past = sp.c[k][1] * st[k][0] + sp.c[k][2] * st[k][1] - sp.c[k][3] * st[k][2] - sp.c[k][4] * st[k][3];
+        const double y = fma(sp.c[k][0], x, past);
+        st[k][1] = st[k][0]; st[k][0] = x; st[k][3] = st[k][2]; st[k][2] = y;
+        return y;
+    }
+    __device__ __forceinline__ double forward(const SosParams &sp, double x)
+    {
+        const int ns = NS < 0 ? sp.nsos : NS;
+#pragma unroll
+        for (int k = 0; k < ns; ++k) x = section(sp, k, x);
+        return x;
+    }
+    __device__ __forceinline__ double backward(const SosParams &sp, double x)
+    {
+        const int ns = NS < 0 ? sp.nsos : NS;
+#pragma unroll
+        for (int k = ns - 1; k >= 0; --k) x = section(sp, k, x);
+        return x;
+    }
+};
+
+template <int NS>
+__global__ void __launch_bounds__(32)
+    k_misfit(Geo g, int comp, int n_taper, const __grid_constant__ SosParams sp, double scale, int nshot_norm,
+             const float *rec, const float *obs, float *rec_adj, double *mis_trace)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.nshot * g.nrec) return;
-    const int s = t / g.nrec, r = t % g.nrec;
+    const int total = g.nshot * g.nrec, t0 = blockIdx.x * 32 + threadIdx.x;
+    const bool live = t0 < total;
+    const int t = live ? t0 : total - 1;   // every lane takes part in the shuffles
+    const int s = t / g.nrec, r = t % g.nrec, nt = g.nt;
     const long long NR = g.nrec, NT = g.nt;
     const float *pred = rec + (long long)s * 4 * NT * NR + comp * NT * NR + r;
     const float *ob = obs + (long long)s * NT * NR + r;
-    float *out = rec_adj + (long long)s * 4 * NT * NR;
-    for (int c = 0; c < 4; ++c)
-        if (c != comp)
-            for (long long n = 0; n < NT; ++n) out[c * NT * NR + n * NR + r] = 0.f;
-    float *cot = out + comp * NT * NR + r;
-    const int tstart = g.nt - min(n_taper, g.nt);
-    const double npi = M_PI;
-    auto taper = [&](int n) -> double {
+    float *cot = rec_adj + (long long)s * 4 * NT * NR + comp * NT * NR + r;
+    const int tstart = nt - min(n_taper, nt);
+    // lane l's taper factor of step n0 + l
+    auto taper = [&](int n0) -> double {
+        const int n = n0 + threadIdx.x;
         if (n_taper <= 0 || n < tstart) return 1.0;
-        const int m = n - tstart + 1;
-        return (cos((double)m / n_taper * npi) + 1.0) / 2.0;
+        return (cos((double)(n - tstart + 1) / n_taper * M_PI) + 1.0) / 2.0;
     };
-    double st[MAX_SOS][4];
-    for (int k = 0; k < sp.nsos; ++k) st[k][0] = st[k][1] = st[k][2] = st[k][3] = 0.0;
+    Cascade<NS> f;
+    f.clear(sp);
     double sum = 0.0;
-    for (int n = 0; n < g.nt; ++n) {
-        const double tp = taper(n);
-        double x = tp * (double)pred[n * NR] - tp * (double)ob[n * NR];
-        for (int k = 0; k < sp.nsos; ++k) {
-            const double y = sp.c[k][0] * x + sp.c[k][1] * st[k][0] + sp.c[k][2] * st[k][1]
-                           - sp.c[k][3] * st[k][2] - sp.c[k][4] * st[k][3];
-            st[k][1] = st[k][0]; st[k][0] = x; st[k][3] = st[k][2]; st[k][2] = y;
-            x = y;
+    float p[MIS_C], o[MIS_C];
+    auto load = [&](int n0) {
+#pragma unroll
+        for (int k = 0; k < MIS_C; ++k) {
+            const long long q = (long long)min(n0 + k, nt - 1) * NR;
+            p[k] = pred[q];
+            o[k] = ob[q];
         }
-        sum += x * x;
-        cot[n * NR] = (float)x;
+    };
+    load(0);
+    for (int n0 = 0; n0 < nt; n0 += MIS_C) {
+        float pc[MIS_C], oc[MIS_C];
+#pragma unroll
+        for (int k = 0; k < MIS_C; ++k) { pc[k] = p[k]; oc[k] = o[k]; }
+        if (n0 + MIS_C < nt) load(n0 + MIS_C);
+        const double tl = taper(n0);
+#pragma unroll
+        for (int k = 0; k < MIS_C; ++k) {
+            const double tp = __shfl_sync(0xffffffffu, tl, k);
+            if (n0 + k >= nt) continue;
+            const double x = f.forward(sp, tp * (double)pc[k] - tp * (double)oc[k]);
+            sum += x * x;
+            if (live) cot[(long long)(n0 + k) * NR] = (float)x;
+        }
     }
     const double coef = 2.0 * scale / ((double)nshot_norm * (double)NT * (double)NR);
-    for (int k = 0; k < sp.nsos; ++k) st[k][0] = st[k][1] = st[k][2] = st[k][3] = 0.0;
-    for (int n = g.nt - 1; n >= 0; --n) {
-        double x = coef * (double)cot[n * NR];
-        for (int k = sp.nsos - 1; k >= 0; --k) {
-            const double y = sp.c[k][0] * x + sp.c[k][1] * st[k][0] + sp.c[k][2] * st[k][1]
-                           - sp.c[k][3] * st[k][2] - sp.c[k][4] * st[k][3];
-            st[k][1] = st[k][0]; st[k][0] = x; st[k][3] = st[k][2]; st[k][2] = y;
-            x = y;
+    f.clear(sp);
+    auto load_back = [&](int n0) {
+#pragma unroll
+        for (int k = 0; k < MIS_C; ++k) p[k] = cot[(long long)min(n0 + k, nt - 1) * NR];
+    };
+    const int last = (nt - 1) / MIS_C * MIS_C;
+    // a lane that only shadows the last trace reads what that trace's own lane wrote
+    __syncwarp();
+    load_back(last);
+    for (int n0 = last; n0 >= 0; n0 -= MIS_C) {
+        float pc[MIS_C];
+#pragma unroll
+        for (int k = 0; k < MIS_C; ++k) pc[k] = p[k];
+        if (n0 > 0) load_back(n0 - MIS_C);
+        const double tl = taper(n0);
+#pragma unroll
+        for (int k = MIS_C - 1; k >= 0; --k) {
+            const double tp = __shfl_sync(0xffffffffu, tl, k);
+            if (n0 + k >= nt) continue;
+            const double x = f.backward(sp, coef * (double)pc[k]);
+            if (live) cot[(long long)(n0 + k) * NR] = (float)(tp * x);
         }
-        cot[n * NR] = (float)(taper(n) * x);
     }
-    mis_trace[t] = scale / nshot_norm * sum / ((double)NT * (double)NR);
+    if (live) mis_trace[t] = scale / nshot_norm * sum / ((double)NT * (double)NR);
 }
 
+// one warp per shot
 __global__ void k_misfit_reduce(int nshot, int nrec, const double *mis_trace, double *mis_shot)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (s >= nshot) return;
     double a = 0.0;
-    for (int r = 0; r < nrec; ++r) a += mis_trace[(long long)s * nrec + r];
-    mis_shot[s] = a;
+    for (int r = threadIdx.x % 32; r < nrec; r += 32) a += mis_trace[(long long)s * nrec + r];
+    for (int d = 16; d > 0; d >>= 1) a += __shfl_down_sync(0xffffffffu, a, d);
+    if (threadIdx.x % 32 == 0) mis_shot[s] = a;
+}
+
+// residuals, adjoint sources and per-shot misfits of nshot * nrec > 0 traces
+cudaError_t launch_misfit(const Geo &g, int comp, int n_taper, const SosParams &sp, double scale, int nnorm,
+                          const float *rec, const float *obs, float *rec_adj, double *mis_trace, double *mis_shot,
+                          cudaStream_t st)
+{
+    const int n = g.nshot * g.nrec;
+    cudaError_t e = cudaMemsetAsync(rec_adj, 0, (size_t)g.nshot * 4 * g.nt * g.nrec * sizeof(float), st);
+    if (e != cudaSuccess) return e;
+    auto go = [&](auto kern) {
+        kern<<<(n + 31) / 32, 32, 0, st>>>(g, comp, n_taper, sp, scale, nnorm, rec, obs, rec_adj, mis_trace);
+    };
+    switch (sp.nsos) {
+    case 0: go(k_misfit<0>); break;
+    case 1: go(k_misfit<1>); break;
+    case 2: go(k_misfit<2>); break;
+    case 3: go(k_misfit<3>); break;
+    case 4: go(k_misfit<4>); break;
+    default: go(k_misfit<-1>); break;
+    }
+    k_misfit_reduce<<<(g.nshot + 3) / 4, 128, 0, st>>>(g.nshot, g.nrec, mis_trace, mis_shot);
+    return cudaGetLastError();
 }
 
 // Partial sums -> (Vs, Vp, rho) gradients on the physical grid.  The exact
@@ -1527,12 +1618,10 @@ stfwi_status stfwi_misfit(stfwi_handle *h, const float *obs, const stfwi_misfit_
     }
     const int nnorm = m->nshot_norm > 0 ? m->nshot_norm : h->nshot;
     CK(h, cudaMemcpyAsync(h->obs, obs, (size_t)h->nshot * g.nt * g.nrec * 4, cudaMemcpyDefault, st));
-    const int n = h->nshot * g.nrec, thr = 128;
-    if (n > 0) {
+    if (h->nshot * g.nrec > 0) {
         const int ntap = std::min(std::max(m->n_taper, 0), g.nt);  // fwi/filters.py:28
-        k_misfit<<<(n + thr - 1) / thr, thr, 0, st>>>(g, m->component, ntap, sp, m->scale, nnorm, h->rec,
-                                                     h->obs, h->rec_adj, h->mis_trace);
-        k_misfit_reduce<<<(h->nshot + 127) / 128, 128, 0, st>>>(h->nshot, g.nrec, h->mis_trace, h->mis_shot);
+        CK(h, launch_misfit(g, m->component, ntap, sp, m->scale, nnorm, h->rec, h->obs, h->rec_adj, h->mis_trace,
+                            h->mis_shot, st));
     } else {
         CK(h, cudaMemsetAsync(h->mis_shot, 0, h->nshot * 8, st));
     }
@@ -2340,11 +2429,8 @@ extern "C" stfwi_status stfwi_misfit_noalloc(int32_t nshot, int32_t nt, int32_t 
     cudaStream_t st = (cudaStream_t)stream;
     const int ntap = std::min(std::max(m->n_taper, 0), nt);
     const int nnorm = m->nshot_norm > 0 ? m->nshot_norm : nshot;
-    const int n = nshot * nrec, thr = 128;
-    k_misfit<<<(n + thr - 1) / thr, thr, 0, st>>>(g, m->component, ntap, sp, m->scale, nnorm, pred, obs, rec_adj,
-                                                 scratch);
-    k_misfit_reduce<<<(nshot + 127) / 128, 128, 0, st>>>(nshot, nrec, scratch, misfit_out);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_misfit(g, m->component, ntap, sp, m->scale, nnorm, pred, obs, rec_adj, scratch,
+                                        misfit_out, st);
     if (e != cudaSuccess) {
         fprintf(stderr, "stfwi_misfit_noalloc: launch: %s\n", cudaGetErrorString(e));
         return STFWI_ERR_CUDA;
