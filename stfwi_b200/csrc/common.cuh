@@ -67,6 +67,7 @@ struct Work {
     const uint32_t *order;
     int ntx, tiles, s0, s1, per, extra;
     int part;              // number of the part of the pass that the shots are
+    int single;            // every block has one item
 };
 
 // images of the adjoint fields under the transposed C-PML, [shot][2][...]:

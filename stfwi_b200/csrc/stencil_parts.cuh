@@ -15,17 +15,14 @@
 
 namespace stfwi {
 
-#ifndef STFWI_MINBLOCKS
-#define STFWI_MINBLOCKS 2
-#endif
-
 constexpr int TX4 = 64;               // tile width: 32 lanes x 2 columns
 constexpr int XO4 = 4;                // x halo of the staged tile
 constexpr int SW4 = TX4 + 2 * XO4;    // 72 floats = 288 B rows
 
-template <int FD, int RPT> struct G4 {
+// tiles of NW warps of RPT rows each
+template <int FD, int RPT, int NW> struct G4 {
     static constexpr int K = FD / 2;
-    static constexpr int TZH = RPT * NWARP;
+    static constexpr int TZH = RPT * NW;
     static constexpr int SH = TZH + 2 * K;
     static constexpr int SN = SH * SW4;
     static constexpr int W = RPT + 2 * K;

@@ -280,19 +280,19 @@ template <int NST> __device__ __forceinline__ void ring_abort(Ring<NST> *r, int 
 
 // this warp has read item `it` from its stage: true in lane 0 of the last
 // warp out, which then issues the item NST further on
-template <int NST> __device__ __forceinline__ bool ring_leave(Ring<NST> *r, int st, bool more)
+template <int NW, int NST> __device__ __forceinline__ bool ring_leave(Ring<NST> *r, int st, bool more)
 {
     __syncwarp();
     if (threadIdx.x != 0) return false;
     const uint32_t old = atom_add_cta(r->out + st, 1u);
-    if (!more || old % NWARP != NWARP - 1) return false;
+    if (!more || old % NW != NW - 1) return false;
     return !(atom_add_cta(&r->issued, 1u) & RING_DEAD);
 }
 
 // stage sizes (floats) and ring depths: as many stages as two blocks an SM
 // have room for
-template <int FD, int R> struct Stage {
-    using T = G4<FD, R>;
+template <int FD, int R, int NW> struct Stage {
+    using T = G4<FD, R, NW>;
     static constexpr int OWN2 = al32_3(2 * T::TZH * TX4), OWN3 = al32_3(3 * T::TZH * TX4);
     static constexpr int VEL = T::S3 + OWN2, STR = T::S2 + OWN3;
     static constexpr int ADA = al32_3(4 * T::SN) + OWN2, ADB = al32_3(4 * T::SN) + 2 * OWN3;
@@ -423,20 +423,37 @@ __device__ __forceinline__ float2 mat_pair(const Geo &g, const float *a, int i, 
 }
 
 // start of a launch: the block's share [first, first + nit) of the items, the
-// ring's barriers, and the first NST items on their way (by the first thread,
-// before the others are waited for); the others meanwhile build the tables
+// ring's barriers, the first NST items on their way (by the first warp's
+// first lane), and meanwhile, by the other warps, the coefficient tables.  All
+// that reads what the launch before wrote comes after the dependency wait:
+// where a launch may start before its predecessor ends, only the part before
+// the wait overlaps.
 template <int NST, class Issue, class Fill>
-__device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Cursor &c, int &first, int &nit, Issue issue,
+__device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Cursor &c, int &nit, Issue issue,
                                            Fill fill_tab)
 {
-    first = share(w, blockIdx.x);
+    const int first = share(w, blockIdx.x);
     nit = share(w, blockIdx.x + 1) - first;
-    if (nit <= 0) return false;
-    c.init(w, first);
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
+    const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
+    if (lead) {
         for (int b = 0; b < NST; ++b) { mbar_init(ring->full + b, 1); ring->out[b] = 0; }
         ring->issued = min(NST, nit);
         fence_async_shared();
+    }
+    if (w.single) {
+        // one item a block, the grid being (tile columns, tile rows, shots):
+        // nothing to look up before the first copy can start
+        nit = 1;
+        c.pos = 0;
+        c.shot = w.s0 + blockIdx.z;
+        c.cur = blockIdx.y << 16 | blockIdx.x;
+    } else {
+        c.init(w, first);
+    }
+    if (threadIdx.y > 0) fill_tab((threadIdx.y - 1) * TX + threadIdx.x);
+    grid_dependency_start();
+    grid_dependency_wait();
+    if (lead) {
         issue(c, 0);
 #pragma unroll 1
         for (int b = 1; b < NST && b < nit; ++b) {
@@ -446,21 +463,20 @@ __device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Curso
         }
     }
     c.look(w);
-    fill_tab(threadIdx.y * TX + threadIdx.x);
     __syncthreads();
-    return true;
+    return nit > 0;
 }
 
 // ------------------------------------------------------------- forward: velocities
 
-template <int FD, int RPT>
-__global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
+template <int FD, int RPT, int NW>
+__global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     st_fwd_vel(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh, float *F,
                float *PX, float *PZ, int n, const __grid_constant__ Work w, int *status,
                const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmUo)
 {
-    using T = G4<FD, RPT>;
-    using Sg = Stage<FD, RPT>;
+    using T = G4<FD, RPT, NW>;
+    using Sg = Stage<FD, RPT, NW>;
     constexpr int K = T::K, SN = T::SN, STG = Sg::VEL, NST = Sg::NVEL, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
@@ -472,18 +488,16 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         tma_load_4d(sm + st * STG + T::S3, &tmUo, ring->full + st, u.j0(), u.i0(T::TZH), F_U, u.shot);
     };
     Cursor c;   // the item at work
-    int first, nit;
-    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
+    int nit;
+    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
     // columns (of the tile) and rows (of this warp) where no slice mask and no
     // C-PML strip applies; the strips are at least K wide, so they hold the
     // masked columns and rows except those below a free surface
     bool xin = false, zin = false;
-    int jb = 0, iw = 0, e0 = 0, e1 = 0;   // e0, e1: the columns' table entries
+    int jb = 0, iw = 0;
     float2 B[RPT];
     auto enter = [&]() {
         jb = c.j0() + 2 * tx;
-        e0 = tab_at(jb, g.nx);
-        e1 = tab_at(jb + 1, g.nx);
         iw = c.i0(T::TZH) + ty * RPT;
         xin = cols_plain(g, c.j0(), g.pad, g.pad);
         zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
@@ -503,6 +517,7 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
             int2 xs = make_int2(-1, -1);
+            const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
                 prefetch_x<RPT>(g, iw, xs, pSXX, pSXZx);
@@ -572,9 +587,9 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, it + NST < nit)) {
+        if (ring_leave<NW>(ring, st, it + NST < nit)) {
             Cursor u;
-            u.init(w, first + it + NST);
+            u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
         if (++st == NST) { st = 0; ph ^= 1; }
@@ -584,15 +599,15 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
 
 // ------------------------------------------------------------- forward: stresses
 
-template <int FD, int RPT, bool ENERGY>
-__global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
+template <int FD, int RPT, int NW, bool ENERGY>
+__global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     st_fwd_str(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh,
                const __grid_constant__ Recv rv, float *F, float *PX, float *PZ, int n, const __grid_constant__ Work w,
                const __grid_constant__ FwdOut out, const __grid_constant__ CUtensorMap tmV,
                const __grid_constant__ CUtensorMap tmSo)
 {
-    using T = G4<FD, RPT>;
-    using Sg = Stage<FD, RPT>;
+    using T = G4<FD, RPT, NW>;
+    using Sg = Stage<FD, RPT, NW>;
     constexpr int K = T::K, SN = T::SN, STG = Sg::STR, NST = Sg::NSTR, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
@@ -604,17 +619,15 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         tma_load_4d(sm + st * STG + T::S2, &tmSo, ring->full + st, u.j0(), u.i0(T::TZH), F_EX, u.shot);
     };
     Cursor c;
-    int first, nit;
-    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
+    int nit;
+    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
     bool xin = false, zin = false;   // as in st_fwd_vel
-    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+    int jb = 0, iw = 0, r0 = 0, r1 = 0;
     float2 ml2m[RPT], ml[RPT], mm[RPT];
     constexpr int RG = ENERGY ? RPT : 1;
     double eacc[RG][2];
     auto enter = [&]() {
         jb = c.j0() + 2 * tx;
-        e0 = tab_at(jb, g.nx);
-        e1 = tab_at(jb + 1, g.nx);
         iw = c.i0(T::TZH) + ty * RPT;
         xin = cols_plain(g, c.j0(), g.pad, g.pad);
         zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
@@ -658,6 +671,7 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
             int2 xs = make_int2(-1, -1);
+            const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
                 prefetch_x<RPT>(g, iw, xs, pDXU, pDXV);
@@ -795,9 +809,9 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
             ring_abort(ring, it, out.status);
             return;
         }
-        if (ring_leave(ring, st, it + NST < nit)) {
+        if (ring_leave<NW>(ring, st, it + NST < nit)) {
             Cursor u;
-            u.init(w, first + it + NST);
+            u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
         if (++st == NST) { st = 0; ph ^= 1; }
@@ -852,17 +866,17 @@ __device__ __forceinline__ int band(int i, int lo, int hi) { return i < lo ? i :
 
 // ------------------------------------------------------------- adjoint: P = B U_a, Q = B V_a
 
-template <int FD, int RPT>
-__global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
+template <int FD, int RPT, int NW>
+__global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     st_adj_a(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Recv rv, float *A,
              float *PX, float *PZ, const __grid_constant__ Images im, int n, const __grid_constant__ Work w,
              const __grid_constant__ AdjIn in, int *status,
              const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmPQo,
              const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ)
 {
-    constexpr int SNA = al32_3(G4<FD, RPT>::SN), SOWN = al32_3(4 * SNA);
-    using T = G4<FD, RPT>;
-    using Sg = Stage<FD, RPT>;
+    constexpr int SNA = al32_3(G4<FD, RPT, NW>::SN), SOWN = al32_3(4 * SNA);
+    using T = G4<FD, RPT, NW>;
+    using Sg = Stage<FD, RPT, NW>;
     constexpr int K = T::K, SN = T::SN, STG = Sg::ADA, NST = Sg::NADA, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
@@ -895,18 +909,16 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
     };
 
     Cursor c;
-    int first, nit;
-    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i, 0); })) return;
+    int nit;
+    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i, 0); })) return;
     // transposed masks reach 2K - 1 (low edge) and 2K (high edge) cells inwards
     const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
     const float hdtdz = 0.5f * g.dtdz, hdtdx = 0.5f * g.dtdx;
     bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
-    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0;
+    int jb = 0, iw = 0, r0 = 0, r1 = 0;
     float2 Bc[RPT];
     auto enter = [&]() {
         jb = c.j0() + 2 * tx;
-        e0 = tab_at(jb, g.nx);
-        e1 = tab_at(jb + 1, g.nx);
         iw = c.i0(T::TZH) + ty * RPT;
         xin = cols_plain(g, c.j0(), mlo, mhi);
         zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
@@ -935,6 +947,7 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
             int2 xs = make_int2(-1, -1);
+            const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
                 prefetch_x<RPT>(g, iw, xs, fXX, fXXZ);
@@ -1042,9 +1055,9 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, it + NST < nit)) {
+        if (ring_leave<NW>(ring, st, it + NST < nit)) {
             Cursor u;
-            u.init(w, first + it + NST);
+            u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
         if (++st == NST) { st = 0; ph ^= 1; }
@@ -1107,23 +1120,23 @@ __device__ __forceinline__ void inject_strain(const Geo &g, const Mat &m, const 
     }
 }
 
-template <int FD, int RPT, bool EXACT, bool IMG, bool RHO>
-__global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
+template <int FD, int RPT, int NW, bool EXACT, bool IMG, bool RHO>
+__global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     st_adj_b(const __grid_constant__ Geo g, const __grid_constant__ Mat m, const __grid_constant__ Shots sh,
              const __grid_constant__ Recv rv, float *A, float *PX, float *PZ, const __grid_constant__ Images im, int n,
              const __grid_constant__ Work w, const __grid_constant__ AdjOut o, int *status, const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmEo,
              const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmX,
              const __grid_constant__ CUtensorMap tmZ)
 {
-    constexpr int SNA = al32_3(G4<FD, RPT>::SN), SOWN = al32_3(4 * SNA);
+    constexpr int SNA = al32_3(G4<FD, RPT, NW>::SN), SOWN = al32_3(4 * SNA);
     // one history box per item from [shot][slot * snf + field][nz_dom][nx_dom]
     // at the tile's physical coordinates (cells outside arrive as 0): the
     // carry-in stresses of the exact gradient, or the carry-out ones of the
     // imaging condition
     const int hslot = EXACT ? o.slot_in : o.slot_img;
     const bool htma = (EXACT || IMG) && o.hist_tma && hslot >= 0;
-    using T = G4<FD, RPT>;
-    using Sg = Stage<FD, RPT>;
+    using T = G4<FD, RPT, NW>;
+    using Sg = Stage<FD, RPT, NW>;
     constexpr int K = T::K, SN = T::SN, STG = Sg::ADB, NST = Sg::NADB, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
@@ -1155,14 +1168,14 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
     };
 
     Cursor c;
-    int first, nit;
-    if (!ring_start(ring, w, c, first, nit, issue, [&](int i) { fill<FD>(tab, g, i, 1); })) return;
+    int nit;
+    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i, 1); })) return;
     const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
     const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;   // history pairs start on 8 bytes
     constexpr int RE = EXACT ? RPT : 1, RI = IMG ? RPT : 1;
     bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
-    int jb = 0, iw = 0, e0 = 0, e1 = 0, r0 = 0, r1 = 0, sfirst = 0;
+    int jb = 0, iw = 0, r0 = 0, r1 = 0, sfirst = 0;
     float2 ml2m[RPT], ml[RPT], mm[RPT];
     // sums over the shots that the block takes of this tile in one go, in
     // FP32; over steps, groups and blocks in FP64 (the reductions of leave()).
@@ -1176,8 +1189,6 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
     float2 gB[RB], grl[RR];
     auto enter = [&]() {
         jb = c.j0() + 2 * tx;
-        e0 = tab_at(jb, g.nx);
-        e1 = tab_at(jb + 1, g.nx);
         iw = c.i0(T::TZH) + ty * RPT;
         xin = cols_plain(g, c.j0(), mlo, mhi);
         zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
@@ -1238,34 +1249,24 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
         const float *S = sm + st * STG;
         const float *own = S + SOWN;             // [ex_a, ez_a, es_a][TZH][TX4] of the tile's own cells
         const float *hown = own + Sg::OWN3;      // [sxx, szz, sxz][TZH][TX4] of the history slot (htma)
-        float *exa = A + ((long long)s * F_N + F_EX) * g.fstride;
-        float *eza = A + ((long long)s * F_N + F_EZ) * g.fstride;
-        float *esa = A + ((long long)s * F_N + F_ES) * g.fstride;
-        const float *Pp = A + ((long long)s * F_N + F_U) * g.fstride;
-        const float *Qp = A + ((long long)s * F_N + F_V) * g.fstride;
-        float *iXU = im.xa + (long long)s * 2 * g.txs, *iXV = iXU + g.txs;
-        float *iZV = im.za + (long long)s * 2 * g.tzs, *iZU = iZV + g.tzs;
-        const float *snap_in = ((EXACT || (IMG && RHO)) && o.slot_in >= 0)
-                                   ? o.snap + ((long long)s * o.slots + o.slot_in) * g.snf * g.nd : nullptr;
-        const float *snap_img = ((IMG || RHO) && o.slot_img >= 0)
-                                    ? o.snap + ((long long)s * o.slots + o.slot_img) * g.snf * g.nd : nullptr;
-        const float *snap_next = (IMG && RHO && o.slot_next >= 0)
-                                     ? o.snap + ((long long)s * o.slots + o.slot_next) * g.snf * g.nd : nullptr;
+        float *E = A + ((long long)s * F_N + F_EX) * g.fstride;   // exx_a, ezz_a, exz_a follow one another
+        const float *Pp = A + ((long long)s * F_N + F_U) * g.fstride, *Qp = Pp + g.fstride;
+        // history slots of the shot: carry-in, carry-out, and the next step's carry-out (none below 0)
+        auto slot = [&](int k) { return o.snap + ((long long)s * o.slots + k) * g.snf * g.nd; };
         const int4 src = __ldg(sh.pos + s);
         const float *aXX = S, *aZZ = S + SNA;
         const float *aZXZ = (bx || bz) ? S + 2 * SNA : aXX, *aXXZ = (bx || bz) ? S + 3 * SNA : aZZ;
-        float *fDXU = px_ptr(g, PX, s, PX_NFWD + PXA_DXU), *fDXV = px_ptr(g, PX, s, PX_NFWD + PXA_DXV);
-        float *fDZV = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZV), *fDZU = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZU);
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
             int2 xs = make_int2(-1, -1);
+            const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
-                prefetch_x<RPT>(g, iw, xs, fDXU, fDXV);
+                prefetch_x<RPT>(g, iw, xs, px_ptr(g, PX, s, PX_NFWD + PXA_DXU), px_ptr(g, PX, s, PX_NFWD + PXA_DXV));
                 prefetch_l1(g.pmx + jb);
             }
             if (GUARD) {
-                prefetch_z<RPT>(g, iw, jb, fDZV, fDZU);
+                prefetch_z<RPT>(g, iw, jb, pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZV), pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZU));
                 prefetch_l1(g.pmz + iw);
             }
             if (!mbar_wait_bounded(ring->full + st, ph, g.wait_polls)) return false;
@@ -1313,6 +1314,73 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
                 const float2 nex = fma2(ml[r], szz, fma2(ml2m[r], sxx, ea));
                 const float2 nez = fma2(ml2m[r], szz, fma2(ml[r], sxx, za));
                 const float2 nes = fma2(mul2(dup2(2.f), mm[r]), sxz, sa);
+                if (src.x == i && (jb == src.y || jb + 1 == src.y)) {
+                    // the source's cell
+                    const int cc = src.y - jb;
+                    const float e = f2c(ea, cc) + f2c(za, cc);
+                    if (src.z == 0) {
+                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = g.dtdxdz * Qp[(long long)i * g.P + jb + cc];
+                    } else {
+                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = (g.dt / sh.mcoef[s]) * e;
+                        if (EXACT) {
+                            // the moment factor's (L + M) term, one FP64 sum per shot
+                            const double lm = sh.lm[s], wv = sh.wav[(long long)s * g.nt + n];
+                            o.mterm[s] += -(wv * g.dt / ((double)sh.mcoef[s] / lm)) / (lm * lm) * (double)e;
+                        }
+                    }
+                }
+                const long long off = (long long)i * g.P + jb;
+                store_pair<XB>(E + off, nex, g.nx - jb);
+                store_pair<XB>(E + g.fstride + off, nez, g.nx - jb);
+                store_pair<XB>(E + 2 * g.fstride + off, nes, g.nx - jb);
+                if (xband || zband) {
+                    // images for the velocity update
+                    float2 vzv = nez, h = nes;
+                    if (last) h = make_float2(0.f, 0.f);
+                    if (XB) {
+                        if (jb >= g.nx - 1) h.x = 0.f;
+                        if (jb + 1 >= g.nx - 1) h.y = 0.f;
+                    }
+                    if (!XB || jb < g.nx) {
+                        float2 vzu = h;
+                        if (GUARD) {
+                            const float4 zc = ldt(g.pmz + i);
+                            const int zs = __float_as_int(zc.w);
+                            if (zs >= 0) {
+                                float *fDZV = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZV), *fDZU = pz_ptr(g, PZ, s, PZ_NFWD + PZA_DZU);
+                                const float2 m0 = pair_at(fDZV + zs * g.P + jb), m1 = pair_at(fDZU + zs * g.P + jb);
+                                adj_z2(vzv, zc, m0, fDZV + zs * g.P + jb);
+                                adj_z2(vzu, zc, m1, fDZU + zs * g.P + jb);
+                            }
+                        }
+                        if (i < g.ita || i >= g.iba) {
+                            const long long b = (long long)band(i, g.ita, g.iba) * g.P + jb;
+                            float *iz = im.za + (long long)s * 2 * g.tzs + b;
+                            *reinterpret_cast<float2 *>(iz) = vzv;
+                            *reinterpret_cast<float2 *>(iz + g.tzs) = vzu;
+                        }
+                    }
+                    if (xband) {
+                        float2 d = nex, v = h;
+                        if (XB && jb < 1) d.x = 0.f;
+                        if (GUARD && g.fs && i == 0) {
+                            // the free surface's d(vz)/dz term (columns below nx - 1)
+                            if (!XB || jb < g.nx - 1) d.x = m.Lr[jb] * vzv.x + d.x;
+                            if (!XB || jb + 1 < g.nx - 1) d.y = m.Lr[jb + 1] * vzv.y + d.y;
+                        }
+                        if (XB) {
+                            float *fDXU = px_ptr(g, PX, s, PX_NFWD + PXA_DXU), *fDXV = px_ptr(g, PX, s, PX_NFWD + PXA_DXV);
+                            const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
+                            const float2 m0 = mem_x(fDXU + i * g.xs_n, xs), m1 = mem_x(fDXV + i * g.xs_n, xs);
+                            adj_x2(d, c0, c1, xs, m0, fDXU + i * g.xs_n);
+                            adj_x2(v, c0, c1, xs, m1, fDXV + i * g.xs_n);
+                        }
+                        const long long b = (long long)i * g.wxp + band_x(g, jb);
+                        float *ix = im.xa + (long long)s * 2 * g.txs + b;
+                        *reinterpret_cast<float2 *>(ix) = d;
+                        *reinterpret_cast<float2 *>(ix + g.txs) = v;
+                    }
+                }
                 const int pi = i - g.z0, pj0 = jb - g.pad;
                 const bool prow = !GUARD || (pi >= 0 && pi < g.nz_dom);
                 const bool p0 = prow && (!XB || (pj0 >= 0 && pj0 < g.nx_dom));
@@ -1335,36 +1403,25 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
                     h2 = pair_at(hown + PL + qo);
                     h3 = pair_at(hown + 2 * PL + qo);
                 }
-                if (EXACT && snap_in) {
-                    if (!htma) { h1 = hist(snap_in); h2 = hist(snap_in + g.nd); h3 = hist(snap_in + 2 * g.nd); }
+                if (EXACT && o.slot_in >= 0) {
+                    if (!htma) {
+                        const float *in = slot(o.slot_in);
+                        h1 = hist(in); h2 = hist(in + g.nd); h3 = hist(in + 2 * g.nd);
+                    }
                     sA[r % RE] = add2(sA[r % RE], fma2(h1, sxx, mul2(h2, szz)));
                     sB[r % RE] = add2(sB[r % RE], fma2(h2, sxx, mul2(h1, szz)));
                     sC[r % RE] = fma2(h3, sxz, sC[r % RE]);
-                }
-                if (src.x == i && (jb == src.y || jb + 1 == src.y)) {
-                    // the source's cell
-                    const int cc = src.y - jb;
-                    const float e = f2c(ea, cc) + f2c(za, cc);
-                    if (src.z == 0) {
-                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = g.dtdxdz * Qp[(long long)i * g.P + jb + cc];
-                    } else {
-                        if (o.src_a) o.src_a[(long long)s * g.nt + n] = (g.dt / sh.mcoef[s]) * e;
-                        if (EXACT) {
-                            // the moment factor's (L + M) term, one FP64 sum per shot
-                            const double lm = sh.lm[s], wv = sh.wav[(long long)s * g.nt + n];
-                            o.mterm[s] += -(wv * g.dt / ((double)sh.mcoef[s] / lm)) / (lm * lm) * (double)e;
-                        }
-                    }
                 }
                 if (RHO && (p0 || p1)) {
                     const long long off = (long long)i * g.P + jb;
                     const float2 pc = *reinterpret_cast<const float2 *>(Pp + off), qc = *reinterpret_cast<const float2 *>(Qp + off);
                     const float2 bb = mat_pair(g, m.B, i, jb);
-                    if (EXACT && snap_in && snap_img) {
+                    const float *in = slot(o.slot_in), *img = slot(o.slot_img), *nxt = slot(o.slot_next);
+                    if (EXACT && o.slot_in >= 0 && o.slot_img >= 0) {
                         // dJ/dB: U_a dU/B + V_a dV/B with U_a = P/B and the
                         // step's velocity increments from the history
-                        const float2 du = sub2(hist(snap_img + 3 * g.nd), hist(snap_in + 3 * g.nd));
-                        const float2 dv = sub2(hist(snap_img + 4 * g.nd), hist(snap_in + 4 * g.nd));
+                        const float2 du = sub2(hist(img + 3 * g.nd), hist(in + 3 * g.nd));
+                        const float2 dv = sub2(hist(img + 4 * g.nd), hist(in + 4 * g.nd));
                         if (p0) gB[r % RB].x += (pc.x * du.x + qc.x * dv.x) / (bb.x * bb.x);
                         if (p1) gB[r % RB].y += (pc.y * du.y + qc.y * dv.y) / (bb.y * bb.y);
                     }
@@ -1374,15 +1431,18 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
                         float2 t = make_float2(0.f, 0.f);
                         const float2 ua = make_float2(p0 ? pc.x / bb.x : 0.f, p1 ? pc.y / bb.y : 0.f);
                         const float2 va = make_float2(p0 ? qc.x / bb.x : 0.f, p1 ? qc.y / bb.y : 0.f);
-                        if (n >= 2 && snap_in)
-                            t = add2(t, fma2(ua, hist(snap_in + 3 * g.nd), mul2(va, hist(snap_in + 4 * g.nd))));
-                        if (n <= g.nt - 3 && snap_next)
-                            t = sub2(t, fma2(ua, hist(snap_next + 3 * g.nd), mul2(va, hist(snap_next + 4 * g.nd))));
+                        if (n >= 2 && o.slot_in >= 0)
+                            t = add2(t, fma2(ua, hist(in + 3 * g.nd), mul2(va, hist(in + 4 * g.nd))));
+                        if (n <= g.nt - 3 && o.slot_next >= 0)
+                            t = sub2(t, fma2(ua, hist(nxt + 3 * g.nd), mul2(va, hist(nxt + 4 * g.nd))));
                         grl[r % RR] = fma2(dup2(-0.5f), t, grl[r % RR]);
                     }
                 }
-                if (IMG && snap_img && (p0 || p1)) {
-                    if (EXACT || !htma) { h1 = hist(snap_img); h2 = hist(snap_img + g.nd); h3 = hist(snap_img + 2 * g.nd); }
+                if (IMG && o.slot_img >= 0 && (p0 || p1)) {
+                    if (EXACT || !htma) {
+                        const float *img = slot(o.slot_img);
+                        h1 = hist(img); h2 = hist(img + g.nd); h3 = hist(img + 2 * g.nd);
+                    }
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc) {
                         if (!(cc ? p1 : p0)) continue;
@@ -1413,54 +1473,6 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
                         else { glam[r % RI].x += gl; gmu[r % RI].x += gm; }
                     }
                 }
-                const long long off = (long long)i * g.P + jb;
-                store_pair<XB>(exa + off, nex, g.nx - jb);
-                store_pair<XB>(eza + off, nez, g.nx - jb);
-                store_pair<XB>(esa + off, nes, g.nx - jb);
-                if (xband || zband) {
-                    // images for the velocity update
-                    float2 vzv = nez, h = nes;
-                    if (last) h = make_float2(0.f, 0.f);
-                    if (XB) {
-                        if (jb >= g.nx - 1) h.x = 0.f;
-                        if (jb + 1 >= g.nx - 1) h.y = 0.f;
-                    }
-                    if (!XB || jb < g.nx) {
-                        float2 vzu = h;
-                        if (GUARD) {
-                            const float4 zc = ldt(g.pmz + i);
-                            const int zs = __float_as_int(zc.w);
-                            if (zs >= 0) {
-                                const float2 m0 = pair_at(fDZV + zs * g.P + jb), m1 = pair_at(fDZU + zs * g.P + jb);
-                                adj_z2(vzv, zc, m0, fDZV + zs * g.P + jb);
-                                adj_z2(vzu, zc, m1, fDZU + zs * g.P + jb);
-                            }
-                        }
-                        if (i < g.ita || i >= g.iba) {
-                            const long long b = (long long)band(i, g.ita, g.iba) * g.P + jb;
-                            *reinterpret_cast<float2 *>(iZV + b) = vzv;
-                            *reinterpret_cast<float2 *>(iZU + b) = vzu;
-                        }
-                    }
-                    if (xband) {
-                        float2 d = nex, v = h;
-                        if (XB && jb < 1) d.x = 0.f;
-                        if (GUARD && g.fs && i == 0) {
-                            // the free surface's d(vz)/dz term (columns below nx - 1)
-                            if (!XB || jb < g.nx - 1) d.x = m.Lr[jb] * vzv.x + d.x;
-                            if (!XB || jb + 1 < g.nx - 1) d.y = m.Lr[jb + 1] * vzv.y + d.y;
-                        }
-                        if (XB) {
-                            const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
-                            const float2 m0 = mem_x(fDXU + i * g.xs_n, xs), m1 = mem_x(fDXV + i * g.xs_n, xs);
-                            adj_x2(d, c0, c1, xs, m0, fDXU + i * g.xs_n);
-                            adj_x2(v, c0, c1, xs, m1, fDXV + i * g.xs_n);
-                        }
-                        const long long b = (long long)i * g.wxp + band_x(g, jb);
-                        *reinterpret_cast<float2 *>(iXU + b) = d;
-                        *reinterpret_cast<float2 *>(iXV + b) = v;
-                    }
-                }
             }
             return true;
         };
@@ -1469,9 +1481,9 @@ __global__ void __launch_bounds__(NTHR, STFWI_MINBLOCKS)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, it + NST < nit)) {
+        if (ring_leave<NW>(ring, st, it + NST < nit)) {
             Cursor u;
-            u.init(w, first + it + NST);
+            u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
         if (++st == NST) { st = 0; ph ^= 1; }

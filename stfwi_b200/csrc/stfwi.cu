@@ -580,6 +580,7 @@ inline void prof_mark(stfwi_handle *h, int k, int n, int which, cudaStream_t st)
 // are atomic).
 struct Part {
     int index, s0, s1;   // shots [s0, s1)
+    bool early;          // its launches may overlap the end of the one before
 };
 
 std::vector<Part> parts_of(const stfwi_handle *h, int parts)
@@ -587,7 +588,8 @@ std::vector<Part> parts_of(const stfwi_handle *h, int parts)
     std::vector<Part> p;
     const int n = h->nshot;
     for (int k = 0; k < parts; ++k)
-        p.push_back(Part{k, (int)((long long)n * k / parts), (int)((long long)n * (k + 1) / parts)});
+        p.push_back(Part{k, (int)((long long)n * k / parts), (int)((long long)n * (k + 1) / parts),
+                         h->prof_every == 0});
     return p;
 }
 
@@ -612,19 +614,20 @@ Work work_of(const stfwi_handle *h, int k, const Part &part)
 // 324 x 1040 100.0 + 134.7, 90.2 + 129.5, 98.1 + 141.7): shorter runs pay a
 // block's start and the FP64 sums of its tile more often, longer ones leave
 // the last blocks of a launch alone on the device.
-template <typename K> int blocks_of(stfwi_handle *h, K kern, size_t smem, int run, Work &w)
+template <typename K> dim3 blocks_of(stfwi_handle *h, K kern, int threads, size_t smem, int run, Work &w)
 {
     int &n = h->resident[(const void *)kern];
     if (n == 0) {
         int per = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, NTHR, smem) != cudaSuccess) cudaGetLastError();
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess) cudaGetLastError();
         n = std::max(1, per) * h->sms;
     }
     const int items = w.tiles * (w.s1 - w.s0);
     const int blocks = std::max(std::min(items, n), (items + run - 1) / run);
     w.per = items / blocks;
     w.extra = items % blocks;
-    return blocks;
+    w.single = blocks == items;
+    return w.single ? dim3(w.ntx, w.tiles / w.ntx, w.s1 - w.s0) : dim3(blocks);
 }
 
 // parts of a pass, each on a stream of its own.  One part while sampled
@@ -644,76 +647,102 @@ int acc_in_use(const stfwi_handle *h, int parts)
     return std::min(h->acc_groups, parts * ((n - 1) / per + 1));
 }
 
-template <int FD, int R>
+// launch a stencil kernel; early: it may start its prologue before the launch
+// ahead of it in the stream ends
+template <typename... P, typename... A>
+void launch_stencil(void (*kern)(P...), dim3 blocks, int warps, size_t smem, cudaStream_t st, bool early, A &&...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = blocks;
+    cfg.blockDim = dim3(TX, warps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+// 16-row tiles by 16 warps of one row each instead of 8 of two: one block then
+// fills an SM, so only where there is no second one for it
+bool few_items(const stfwi_handle *h, int ntz, const Part &part)
+{
+    return h->ntx * ntz * (part.s1 - part.s0) <= h->sms;
+}
+
+template <int FD, int R, int NW>
 void launch_fwd_step_r(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Part &part)
 {
-    using Sg = Stage<FD, R>;
-    const dim3 block(TX, NWARP);
+    using Sg = Stage<FD, R, NW>;
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
     constexpr size_t bv = Sg::bytes(Sg::VEL, Sg::NVEL), bs = Sg::bytes(Sg::STR, Sg::NSTR);
     Work w0 = work_of(h, 0, part), w1 = work_of(h, 1, part);
-    const int n0 = blocks_of(h, st_fwd_vel<FD, R>, bv, h->spgk[0], w0);
+    const dim3 n0 = blocks_of(h, st_fwd_vel<FD, R, NW>, TX * NW, bv, h->spgk[0], w0);
     prof_mark(h, 0, n, 0, st);
-    st_fwd_vel<FD, R><<<n0, block, bv, st>>>(
-        h->g, mat_of(h), shots_of(h), h->F, h->PX, h->PZ, n, w0, h->status, h->tmS, h->tmUo);
+    launch_stencil(st_fwd_vel<FD, R, NW>, n0, NW, bv, st, part.early, h->g, mat_of(h), shots_of(h), h->F, h->PX, h->PZ, n, w0,
+                   h->status, h->tmS, h->tmUo);
     prof_mark(h, 0, n, 1, st);
     prof_mark(h, 1, n, 0, st);
-    auto str = o.energy ? st_fwd_str<FD, R, true> : st_fwd_str<FD, R, false>;
-    const int n1 = blocks_of(h, str, bs, h->spgk[1], w1);
-    str<<<n1, block, bs, st>>>(
-        h->g, mat_of(h), shots_of(h), rva, h->F, h->PX, h->PZ, n, w1, o, h->tmV, h->tmSo);
+    auto str = o.energy ? st_fwd_str<FD, R, NW, true> : st_fwd_str<FD, R, NW, false>;
+    const dim3 n1 = blocks_of(h, str, TX * NW, bs, h->spgk[1], w1);
+    launch_stencil(str, n1, NW, bs, st, part.early, h->g, mat_of(h), shots_of(h), rva, h->F, h->PX, h->PZ, n, w1, o, h->tmV,
+                   h->tmSo);
     prof_mark(h, 1, n, 1, st);
 }
 
 template <int FD>
 void launch_fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Part &part)
 {
-    if (h->ra == 1) launch_fwd_step_r<FD, 1>(h, n, o, st, part);
-    else launch_fwd_step_r<FD, 2>(h, n, o, st, part);
+    if (h->ra == 1) launch_fwd_step_r<FD, 1, 8>(h, n, o, st, part);
+    else if (few_items(h, h->ntza, part)) launch_fwd_step_r<FD, 1, 16>(h, n, o, st, part);
+    else launch_fwd_step_r<FD, 2, 8>(h, n, o, st, part);
 }
 
-template <int FD, int R>
+template <int FD, int R, int NW>
 void launch_adj_a_r(stfwi_handle *h, int n, const AdjIn &ai, cudaStream_t st, const Part &part)
 {
-    using Sg = Stage<FD, R>;
+    using Sg = Stage<FD, R, NW>;
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
     constexpr size_t bytes = Sg::bytes(Sg::ADA, Sg::NADA);
     Work w = work_of(h, 2, part);
-    const int nb = blocks_of(h, st_adj_a<FD, R>, bytes, h->spgk[2], w);
-    st_adj_a<FD, R><<<nb, dim3(TX, NWARP), bytes, st>>>(
-        h->g, mat_of(h), rva, h->A, h->PX, h->PZ, h->im, n, w, ai, h->status, h->tmE, h->tmPQo, h->tmXa, h->tmZa);
+    const dim3 nb = blocks_of(h, st_adj_a<FD, R, NW>, TX * NW, bytes, h->spgk[2], w);
+    launch_stencil(st_adj_a<FD, R, NW>, nb, NW, bytes, st, part.early, h->g, mat_of(h), rva, h->A, h->PX, h->PZ, h->im, n, w, ai,
+                   h->status, h->tmE, h->tmPQo, h->tmXa, h->tmZa);
 }
 
-template <int FD, int R>
+template <int FD, int R, int NW>
 void launch_adj_b_r(stfwi_handle *h, int n, const AdjOut &ao, cudaStream_t st, const Part &part)
 {
-    using Sg = Stage<FD, R>;
+    using Sg = Stage<FD, R, NW>;
     Recv rvb{h->tile_startB, h->tile_recB, h->rx, h->rz};
     constexpr size_t bytes = Sg::bytes(Sg::ADB, Sg::NADB);
     Work w = work_of(h, 3, part);
     auto launch = [&](auto kern) {
-        const int nb = blocks_of(h, kern, bytes, h->spgk[3], w);
-        kern<<<nb, dim3(TX, NWARP), bytes, st>>>(
-            h->g, mat_of(h), shots_of(h), rvb, h->A, h->PX, h->PZ, h->im, n, w, ao, h->status, h->tmP, h->tmEo,
-            h->tmH, h->tmXb, h->tmZb);
+        const dim3 nb = blocks_of(h, kern, TX * NW, bytes, h->spgk[3], w);
+        launch_stencil(kern, nb, NW, bytes, st, part.early, h->g, mat_of(h), shots_of(h), rvb, h->A, h->PX, h->PZ, h->im, n, w,
+                       ao, h->status, h->tmP, h->tmEo, h->tmH, h->tmXb, h->tmZb);
     };
     const bool rho = h->g.snf == 5;
-    if (ao.want_exact && ao.want_img) rho ? launch(st_adj_b<FD, R, true, true, true>) : launch(st_adj_b<FD, R, true, true, false>);
-    else if (ao.want_exact) rho ? launch(st_adj_b<FD, R, true, false, true>) : launch(st_adj_b<FD, R, true, false, false>);
-    else if (ao.want_img) rho ? launch(st_adj_b<FD, R, false, true, true>) : launch(st_adj_b<FD, R, false, true, false>);
-    else launch(st_adj_b<FD, R, false, false, false>);
+    if (ao.want_exact && ao.want_img) rho ? launch(st_adj_b<FD, R, NW, true, true, true>) : launch(st_adj_b<FD, R, NW, true, true, false>);
+    else if (ao.want_exact) rho ? launch(st_adj_b<FD, R, NW, true, false, true>) : launch(st_adj_b<FD, R, NW, true, false, false>);
+    else if (ao.want_img) rho ? launch(st_adj_b<FD, R, NW, false, true, true>) : launch(st_adj_b<FD, R, NW, false, true, false>);
+    else launch(st_adj_b<FD, R, NW, false, false, false>);
 }
 
 template <int FD>
 void launch_adj_step(stfwi_handle *h, int n, const AdjIn &ai, const AdjOut &ao, cudaStream_t st, const Part &part)
 {
     prof_mark(h, 2, n, 0, st);
-    if (h->ra == 1) launch_adj_a_r<FD, 1>(h, n, ai, st, part);
-    else launch_adj_a_r<FD, 2>(h, n, ai, st, part);
+    if (h->ra == 1) launch_adj_a_r<FD, 1, 8>(h, n, ai, st, part);
+    else if (few_items(h, h->ntza, part)) launch_adj_a_r<FD, 1, 16>(h, n, ai, st, part);
+    else launch_adj_a_r<FD, 2, 8>(h, n, ai, st, part);
     prof_mark(h, 2, n, 1, st);
     prof_mark(h, 3, n, 0, st);
-    if (h->rb == 1) launch_adj_b_r<FD, 1>(h, n, ao, st, part);
-    else launch_adj_b_r<FD, 2>(h, n, ao, st, part);
+    if (h->rb == 1) launch_adj_b_r<FD, 1, 8>(h, n, ao, st, part);
+    else if (few_items(h, h->ntzb, part)) launch_adj_b_r<FD, 1, 16>(h, n, ao, st, part);
+    else launch_adj_b_r<FD, 2, 8>(h, n, ao, st, part);
     prof_mark(h, 3, n, 1, st);
 }
 
@@ -934,10 +963,10 @@ stfwi_status encode(stfwi_handle *h, CUtensorMap *m, void *base, int rank, const
     return STFWI_OK;
 }
 
-template <int FD, int R>
+template <int FD, int R, int NW>
 stfwi_status setup_tma_kernels_r(stfwi_handle *h)
 {
-    using Sg = Stage<FD, R>;
+    using Sg = Stage<FD, R, NW>;
     auto limit = [&](auto kern, size_t bytes) -> stfwi_status {
         CK(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         return STFWI_OK;
@@ -945,12 +974,12 @@ stfwi_status setup_tma_kernels_r(stfwi_handle *h)
     constexpr size_t bv = Sg::bytes(Sg::VEL, Sg::NVEL), bs = Sg::bytes(Sg::STR, Sg::NSTR),
                      ba = Sg::bytes(Sg::ADA, Sg::NADA), bb = Sg::bytes(Sg::ADB, Sg::NADB);
     stfwi_status r;
-    if ((r = limit(st_fwd_vel<FD, R>, bv)) || (r = limit(st_fwd_str<FD, R, false>, bs)) ||
-        (r = limit(st_fwd_str<FD, R, true>, bs)) || (r = limit(st_adj_a<FD, R>, ba)) ||
-        (r = limit(st_adj_b<FD, R, true, false, false>, bb)) || (r = limit(st_adj_b<FD, R, true, true, false>, bb)) ||
-        (r = limit(st_adj_b<FD, R, false, true, false>, bb)) || (r = limit(st_adj_b<FD, R, false, false, false>, bb)) ||
-        (r = limit(st_adj_b<FD, R, true, false, true>, bb)) || (r = limit(st_adj_b<FD, R, true, true, true>, bb)) ||
-        (r = limit(st_adj_b<FD, R, false, true, true>, bb)))
+    if ((r = limit(st_fwd_vel<FD, R, NW>, bv)) || (r = limit(st_fwd_str<FD, R, NW, false>, bs)) ||
+        (r = limit(st_fwd_str<FD, R, NW, true>, bs)) || (r = limit(st_adj_a<FD, R, NW>, ba)) ||
+        (r = limit(st_adj_b<FD, R, NW, true, false, false>, bb)) || (r = limit(st_adj_b<FD, R, NW, true, true, false>, bb)) ||
+        (r = limit(st_adj_b<FD, R, NW, false, true, false>, bb)) || (r = limit(st_adj_b<FD, R, NW, false, false, false>, bb)) ||
+        (r = limit(st_adj_b<FD, R, NW, true, false, true>, bb)) || (r = limit(st_adj_b<FD, R, NW, true, true, true>, bb)) ||
+        (r = limit(st_adj_b<FD, R, NW, false, true, true>, bb)))
         return r;
     return STFWI_OK;
 }
@@ -959,8 +988,9 @@ stfwi_status setup_tma_kernels_r(stfwi_handle *h)
 template <int FD>
 stfwi_status setup_tma_kernels(stfwi_handle *h)
 {
-    stfwi_status r = setup_tma_kernels_r<FD, 1>(h);
-    return r ? r : setup_tma_kernels_r<FD, 2>(h);
+    stfwi_status r = setup_tma_kernels_r<FD, 1, 8>(h);
+    if (!r) r = setup_tma_kernels_r<FD, 1, 16>(h);
+    return r ? r : setup_tma_kernels_r<FD, 2, 8>(h);
 }
 
 stfwi_status setup_tensor_maps(stfwi_handle *h)

@@ -61,6 +61,13 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, u
         : "memory");
 }
 
+// Programmatic launch: let the next launch of the stream start its prologue
+// once every block of this one runs / wait until the launches this one depends
+// on are complete and their writes visible.  Without the launch attribute both
+// return at once.
+__device__ __forceinline__ void grid_dependency_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // L2 policy for data read once (the gradient history): its lines are the
 // first to go, so the fields that the next kernels read stay resident
 __device__ __forceinline__ uint64_t l2_evict_first()
