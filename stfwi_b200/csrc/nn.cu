@@ -390,73 +390,131 @@ __global__ void k_pack_input(const float *__restrict__ f, int n, int hd, int wd,
     }
 }
 
-// 2x2 average pool of a channel slice: in [n][h][w][in_cstride] at in_coff -> out [n][h/2][w/2][c]
-__global__ void k_avgpool2(const __nv_bfloat16 *__restrict__ in, int n, int h, int w, int c, int in_cstride,
-                           int in_coff, __nv_bfloat16 *__restrict__ out)
-{
-    const int ho = h / 2, wo = w / 2;
-    const size_t total = (size_t)n * ho * wo * c;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(e % c);
-        size_t p = e / c;
-        const int j = (int)(p % wo), i = (int)((p / wo) % ho), img = (int)(p / ((size_t)wo * ho));
-        const size_t r0 = ((size_t)img * h + 2 * i) * w + 2 * j;
-        const __nv_bfloat16 *q = in + in_coff + ch;
-        const float s = __bfloat162float(q[r0 * in_cstride]) + __bfloat162float(q[(r0 + 1) * in_cstride]) +
-                        __bfloat162float(q[(r0 + w) * in_cstride]) + __bfloat162float(q[(r0 + w + 1) * in_cstride]);
-        out[e] = __float2bfloat16_rn(0.25f * s);
+// The resampling kernels are memory-bound.  A block takes part of one image
+// row (blockIdx.x = image * rows + row, blockIdx.y the part), so the only
+// division left is a column's, and a thread moves V channels: 8 (16 bytes)
+// where channel counts, strides, offsets and pointers allow it, else one.
+// us at batch 8, 160 x 512, one channel a thread before -> 8: upsampling of the
+// three levels 382 -> 35, its gradient 123 -> 43, skip gradients 223 -> 56, pooling 69 -> 22.
+template <int V> struct Vec {
+    float v[V];
+    __device__ __forceinline__ void load(const __nv_bfloat16 *p)
+    {
+        if constexpr (V == 1) {
+            v[0] = __bfloat162float(*p);
+        } else {
+            const uint4 q = *reinterpret_cast<const uint4 *>(p);
+            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 f = __bfloat1622float2(h[i]);
+                v[2 * i] = f.x;
+                v[2 * i + 1] = f.y;
+            }
+        }
     }
+    __device__ __forceinline__ void store(__nv_bfloat16 *p) const
+    {
+        if constexpr (V == 1) {
+            *p = __float2bfloat16_rn(v[0]);
+        } else {
+            uint4 q;
+            __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            *reinterpret_cast<uint4 *>(p) = q;
+        }
+    }
+};
+
+// f(row, column, channel) over this block's part of a row of w columns and c channels
+template <int V, class F> __device__ __forceinline__ void for_row(int w, int c, F f)
+{
+    const unsigned cg = c / V, total = (unsigned)w * cg;
+    for (unsigned e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
+        const unsigned j = e / cg;
+        f((size_t)blockIdx.x, (int)j, (int)((e - j * cg) * V));
+    }
+}
+
+// 2x2 average pool of a channel slice: in [n][h][w][in_cstride] at in_coff -> out [n][h/2][w/2][c]
+template <int V>
+__global__ void k_avgpool2(const __nv_bfloat16 *__restrict__ in, int w, int c, int in_cstride, int in_coff,
+                           __nv_bfloat16 *__restrict__ out)
+{
+    const int wo = w / 2;
+    for_row<V>(wo, c, [&](size_t row, int j, int ch) {
+        // output rows of all images follow one another, and so do pairs of input rows
+        const __nv_bfloat16 *q = in + (2 * row * w + 2 * j) * in_cstride + in_coff + ch;
+        Vec<V> a, b, d, e;
+        a.load(q);
+        b.load(q + in_cstride);
+        d.load(q + (size_t)w * in_cstride);
+        e.load(q + (size_t)(w + 1) * in_cstride);
+#pragma unroll
+        for (int k = 0; k < V; ++k) a.v[k] = 0.25f * (a.v[k] + b.v[k] + d.v[k] + e.v[k]);
+        a.store(out + (row * wo + j) * c + ch);
+    });
 }
 
 // gradient of a skip tensor y (a ReLU output stored in a concatenation buffer slice):
 // dz = (dcat[slice] + 1/4 dpool[parent]) * [y > 0]  -> contiguous [n][h][w][c]
+template <int V>
 __global__ void k_skip_grad(const __nv_bfloat16 *__restrict__ dcat, const __nv_bfloat16 *__restrict__ ycat,
-                            int cstride, int coff, const __nv_bfloat16 *__restrict__ dpool, int n, int h, int w, int c,
+                            int cstride, int coff, const __nv_bfloat16 *__restrict__ dpool, int h, int w, int c,
                             __nv_bfloat16 *__restrict__ dz)
 {
-    const size_t total = (size_t)n * h * w * c;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(e % c);
-        const size_t p = e / c;
-        const int j = (int)(p % w), i = (int)((p / w) % h), img = (int)(p / ((size_t)w * h));
-        const size_t pp = ((size_t)img * (h / 2) + i / 2) * (w / 2) + j / 2;
-        float v = 0.25f * __bfloat162float(dpool[pp * c + ch]);
-        if (dcat) v += __bfloat162float(dcat[p * cstride + coff + ch]);
-        dz[e] = __float2bfloat16_rn(__bfloat162float(ycat[p * cstride + coff + ch]) > 0.f ? v : 0.f);
-    }
+    for_row<V>(w, c, [&](size_t row, int j, int ch) {
+        const size_t p = row * w + j;
+        Vec<V> g, y, d;
+        const unsigned img = blockIdx.x / (unsigned)h, i = blockIdx.x - img * h;
+        g.load(dpool + (((size_t)img * (h / 2) + i / 2) * (w / 2) + j / 2) * c + ch);
+        y.load(ycat + p * cstride + coff + ch);
+        if (dcat) d.load(dcat + p * cstride + coff + ch);
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            float v = 0.25f * g.v[k];
+            if (dcat) v += d.v[k];
+            g.v[k] = y.v[k] > 0.f ? v : 0.f;
+        }
+        g.store(dz + p * c + ch);
+    });
 }
 
-// nearest 2x upsampling of low [n][h][w][c] into channels [0, c) of out [n][2h][2w][out_cstride]
-__global__ void k_upsample2(const __nv_bfloat16 *__restrict__ low, int n, int h, int w, int c, int out_cstride,
+// nearest 2x upsampling of low [n][h][w][c] into channels [0, c) of out [n][2h][2w][out_cstride]; a
+// block's row is one of low, whose four copies a thread writes
+template <int V>
+__global__ void k_upsample2(const __nv_bfloat16 *__restrict__ low, int w, int c, int out_cstride,
                             __nv_bfloat16 *__restrict__ out)
 {
-    const int ho = 2 * h, wo = 2 * w;
-    const size_t total = (size_t)n * ho * wo * c;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(e % c);
-        const size_t p = e / c;
-        const int j = (int)(p % wo), i = (int)((p / wo) % ho), img = (int)(p / ((size_t)wo * ho));
-        out[p * out_cstride + ch] = low[(((size_t)img * h + i / 2) * w + j / 2) * c + ch];
-    }
+    for_row<V>(w, c, [&](size_t row, int j, int ch) {
+        Vec<V> v;
+        v.load(low + (row * w + j) * c + ch);
+        __nv_bfloat16 *q = out + (2 * row * 2 * w + 2 * j) * out_cstride + ch;
+        v.store(q);
+        v.store(q + out_cstride);
+        v.store(q + (size_t)2 * w * out_cstride);
+        v.store(q + (size_t)(2 * w + 1) * out_cstride);
+    });
 }
 
 // gradient through the upsampling into a ReLU output: dz[low] = sum_{2x2} dcat[.., 0:c] * [low > 0]
+template <int V>
 __global__ void k_upsample2_grad(const __nv_bfloat16 *__restrict__ dcat, int cstride,
-                                 const __nv_bfloat16 *__restrict__ low, int n, int h, int w, int c,
-                                 __nv_bfloat16 *__restrict__ dz)
+                                 const __nv_bfloat16 *__restrict__ low, int w, int c, __nv_bfloat16 *__restrict__ dz)
 {
-    const size_t total = (size_t)n * h * w * c;
-    const int wo = 2 * w;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(e % c);
-        const size_t p = e / c;
-        const int j = (int)(p % w), i = (int)((p / w) % h), img = (int)(p / ((size_t)w * h));
-        const size_t r0 = ((size_t)img * 2 * h + 2 * i) * wo + 2 * j;
-        const float s = __bfloat162float(dcat[r0 * cstride + ch]) + __bfloat162float(dcat[(r0 + 1) * cstride + ch]) +
-                        __bfloat162float(dcat[(r0 + wo) * cstride + ch]) +
-                        __bfloat162float(dcat[(r0 + wo + 1) * cstride + ch]);
-        dz[e] = __float2bfloat16_rn(__bfloat162float(low[e]) > 0.f ? s : 0.f);
-    }
+    for_row<V>(w, c, [&](size_t row, int j, int ch) {
+        const __nv_bfloat16 *q = dcat + (2 * row * 2 * w + 2 * j) * cstride + ch;
+        Vec<V> a, b, d, e, l;
+        a.load(q);
+        b.load(q + cstride);
+        d.load(q + (size_t)2 * w * cstride);
+        e.load(q + (size_t)(2 * w + 1) * cstride);
+        l.load(low + (row * w + j) * c + ch);
+#pragma unroll
+        for (int k = 0; k < V; ++k) a.v[k] = l.v[k] > 0.f ? a.v[k] + b.v[k] + d.v[k] + e.v[k] : 0.f;
+        a.store(dz + (row * w + j) * c + ch);
+    });
 }
 
 // 1x1 output head: out[p] = b + sum_c wt[c] y[p][c], y [npix][c] BF16 (c <= 64)
@@ -477,68 +535,104 @@ __global__ void k_head_fwd(const __nv_bfloat16 *__restrict__ y, size_t npix, int
 
 // masked mean-square loss of the head and its gradient:
 // L = sum_p wgt[p] (out - target)^2 / norm;  dz[p][c] = dL/dout * wt[c] * [y > 0];
-// dwt[c] += sum_p dL/dout y[p][c];  db += sum_p dL/dout;  loss (FP64) += L
-__global__ void k_head_loss_grad(const __nv_bfloat16 *__restrict__ y, size_t npix, int c,
-                                 const float *__restrict__ wt, const float *__restrict__ out,
-                                 const float *__restrict__ target, const float *__restrict__ wgt, float inv_norm,
-                                 __nv_bfloat16 *__restrict__ dz, float *__restrict__ dwt, float *__restrict__ db,
-                                 double *__restrict__ loss)
+// dwt[c] += sum_p dL/dout y[p][c];  db += sum_p dL/dout;  loss (FP64) += L.
+// C channels at compile time: the weight sums stay in registers (with a
+// run-time count they lay in local memory: 270 us then, 39 now, at 8 x 160 x 512, 32 channels).
+template <int C>   // 0: the loss and db alone
+__global__ void k_head_loss_grad(const __nv_bfloat16 *__restrict__ y, size_t npix, const float *__restrict__ wt,
+                                 const float *__restrict__ out, const float *__restrict__ target,
+                                 const float *__restrict__ wgt, float inv_norm, __nv_bfloat16 *__restrict__ dz,
+                                 float *__restrict__ dwt, float *__restrict__ db, double *__restrict__ loss)
 {
-    __shared__ float s_dw[64];
+    __shared__ float s_dw[C ? C : 1];
     __shared__ float s_db;
     __shared__ double s_l;
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) s_dw[i] = 0.f;
+    for (int i = threadIdx.x; i < C; i += blockDim.x) s_dw[i] = 0.f;
     if (threadIdx.x == 0) {
         s_db = 0.f;
         s_l = 0.0;
     }
     __syncthreads();
-    float acc_db = 0.f;
+    float acc_db = 0.f, acc_dw[C ? C : 1];
     double acc_l = 0.0;
-    float acc_dw[64];
-    for (int i = 0; i < 64; ++i) acc_dw[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < C; ++i) acc_dw[i] = 0.f;
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x) {
         const float r = out[p] - target[p];
         const float wp = wgt[p];
         acc_l += (double)wp * r * r * inv_norm;
         const float g = 2.f * wp * r * inv_norm;
         acc_db += g;
-        for (int k = 0; k < c; k += 16) {
+#pragma unroll
+        for (int k = 0; k < C; k += 16) {
             float v[16], d[16];
-            load_bf16x16(y + p * c + k, v);
+            load_bf16x16(y + p * C + k, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 acc_dw[k + i] = fmaf(g, v[i], acc_dw[k + i]);
                 d[i] = v[i] > 0.f ? g * __ldg(wt + k + i) : 0.f;
             }
-            store_bf16x16(dz + p * c + k, d);
+            store_bf16x16(dz + p * C + k, d);
         }
     }
-    for (int i = 0; i < c; ++i) atomicAdd(&s_dw[i], acc_dw[i]);
-    atomicAdd(&s_db, acc_db);
-    atomicAdd(&s_l, acc_l);
+    // over the lanes of a warp, then over the block's warps
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+        float s = acc_dw[i];
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+        if (threadIdx.x % 32 == 0) atomicAdd(&s_dw[i], s);
+    }
+    for (int d = 16; d > 0; d >>= 1) {
+        acc_db += __shfl_down_sync(0xffffffffu, acc_db, d);
+        acc_l += __shfl_down_sync(0xffffffffu, acc_l, d);
+    }
+    if (threadIdx.x % 32 == 0) {
+        atomicAdd(&s_db, acc_db);
+        atomicAdd(&s_l, acc_l);
+    }
     __syncthreads();
-    if (threadIdx.x < c) atomicAdd(dwt + threadIdx.x, s_dw[threadIdx.x]);
+    if ((int)threadIdx.x < C) atomicAdd(dwt + threadIdx.x, s_dw[threadIdx.x]);
     if (threadIdx.x == 0) {
         atomicAdd(db, s_db);
         atomicAdd(loss, s_l);
     }
 }
 
-// db[c] += sum over pixels of dz[p][c] (NHWC contiguous, c <= 1024)
+// db[c] += sum over pixels of dz[p][c] (NHWC contiguous, c <= 1024): a thread
+// keeps to V channels (8, 16 bytes a load, where c and the pointer allow it),
+// a block sums its threads' in shared memory.  Four pixels are in flight per
+// thread.  us for the 14 layers of a batch of 8: 397 with one 2-byte load in flight a thread, 152 now.
+template <int V>
 __global__ void k_bias_grad(const __nv_bfloat16 *__restrict__ dz, size_t npix, int c, float *__restrict__ db)
 {
     extern __shared__ float s_b[];
     for (int i = threadIdx.x; i < c; i += blockDim.x) s_b[i] = 0.f;
     __syncthreads();
-    const size_t total = npix * c;
-    // the stride is a multiple of c, so each thread stays on one channel
-    const size_t stride = (size_t)gridDim.x * blockDim.x / c * c;
-    const size_t start = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (stride > 0 && start < stride) {
-        float s = 0.f;
-        for (size_t e = start; e < total; e += stride) s += __bfloat162float(dz[e]);
-        atomicAdd(&s_b[start % c], s);
+    // threads of the grid in whole pixels: thread t takes channel group t % cg of pixels t / cg, + step, ...
+    const unsigned cg = c / V, t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x / cg;
+    const unsigned p0 = t / cg, ch = (t - p0 * cg) * V;
+    if (p0 < step) {
+        float s[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) s[k] = 0.f;
+        size_t p = p0;
+        for (; p + 3 * (size_t)step < npix; p += 4 * (size_t)step) {
+            Vec<V> a[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[q].load(dz + (p + q * (size_t)step) * c + ch);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int k = 0; k < V; ++k) s[k] += a[q].v[k];
+        }
+        for (; p < npix; p += step) {
+            Vec<V> a;
+            a.load(dz + p * c + ch);
+#pragma unroll
+            for (int k = 0; k < V; ++k) s[k] += a.v[k];
+        }
+#pragma unroll
+        for (int k = 0; k < V; ++k) atomicAdd(&s_b[ch + k], s[k]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < c; i += blockDim.x) atomicAdd(db + i, s_b[i]);
@@ -757,6 +851,19 @@ unsigned blocks_for(size_t n, int threads)
     return (unsigned)(b < 1 ? 1 : b > 4 * 148 * 8 ? 4 * 148 * 8 : b);
 }
 
+// grid of a row kernel: rows x parts of a row of `per_row` thread items, about four items a thread
+dim3 row_grid(size_t rows, size_t per_row)
+{
+    const size_t parts = (per_row + 1023) / 1024;
+    return dim3((unsigned)rows, (unsigned)(parts < 1 ? 1 : parts > 64 ? 64 : parts));
+}
+
+// may a row kernel move 8 channels a thread
+bool by8(int c, int cstride, int coff, const void *a, const void *b, const void *d = nullptr, const void *e = nullptr)
+{
+    return c % 8 == 0 && cstride % 8 == 0 && coff % 8 == 0 && aligned16(a) && aligned16(b) && aligned16(d) && aligned16(e);
+}
+
 }  // namespace
 
 extern "C" {
@@ -850,37 +957,49 @@ int stfwi_nn_avgpool2(const void *in, int n, int h, int w, int c, int in_cstride
                       void *stream)
 {
     if (h % 2 || w % 2) return nn_fail(STFWI_ERR_INVALID, "avgpool2: odd size");
-    const size_t total = (size_t)n * (h / 2) * (w / 2) * c;
-    k_avgpool2<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16 *>(in), n, h, w, c, in_cstride, in_coff, static_cast<__nv_bfloat16 *>(out));
+    const bool v8 = by8(c, in_cstride, in_coff, in, out);
+    const size_t rows = (size_t)n * (h / 2);
+    if (n > 0 && h > 0 && w > 0 && c > 0)
+        (v8 ? k_avgpool2<8> : k_avgpool2<1>)<<<row_grid(rows, (size_t)(w / 2) * c / (v8 ? 8 : 1)), 256, 0,
+                                               static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16 *>(in), w, c, in_cstride, in_coff, static_cast<__nv_bfloat16 *>(out));
     return check_launch("k_avgpool2");
 }
 
 int stfwi_nn_skip_grad(const void *dcat, const void *ycat, int cstride, int coff, const void *dpool, int n, int h,
                        int w, int c, void *dz, void *stream)
 {
-    const size_t total = (size_t)n * h * w * c;
-    k_skip_grad<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16 *>(dcat), static_cast<const __nv_bfloat16 *>(ycat), cstride, coff,
-        static_cast<const __nv_bfloat16 *>(dpool), n, h, w, c, static_cast<__nv_bfloat16 *>(dz));
+    const bool v8 = by8(c, cstride, coff, dcat, ycat, dpool, dz);
+    const size_t rows = (size_t)n * h;
+    if (n > 0 && h > 0 && w > 0 && c > 0)
+        (v8 ? k_skip_grad<8> : k_skip_grad<1>)<<<row_grid(rows, (size_t)w * c / (v8 ? 8 : 1)), 256, 0,
+                                                 static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16 *>(dcat), static_cast<const __nv_bfloat16 *>(ycat), cstride, coff,
+            static_cast<const __nv_bfloat16 *>(dpool), h, w, c, static_cast<__nv_bfloat16 *>(dz));
     return check_launch("k_skip_grad");
 }
 
 int stfwi_nn_upsample2(const void *low, int n, int h, int w, int c, int out_cstride, void *out, void *stream)
 {
-    const size_t total = (size_t)n * 4 * h * w * c;
-    k_upsample2<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16 *>(low), n, h, w, c, out_cstride, static_cast<__nv_bfloat16 *>(out));
+    const bool v8 = by8(c, out_cstride, 0, low, out);
+    const size_t rows = (size_t)n * h;
+    if (n > 0 && h > 0 && w > 0 && c > 0)
+        (v8 ? k_upsample2<8> : k_upsample2<1>)<<<row_grid(rows, (size_t)w * c / (v8 ? 8 : 1)), 256, 0,
+                                                 static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16 *>(low), w, c, out_cstride, static_cast<__nv_bfloat16 *>(out));
     return check_launch("k_upsample2");
 }
 
 int stfwi_nn_upsample2_grad(const void *dcat, int cstride, const void *low, int n, int h, int w, int c, void *dz,
                             void *stream)
 {
-    const size_t total = (size_t)n * h * w * c;
-    k_upsample2_grad<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16 *>(dcat), cstride, static_cast<const __nv_bfloat16 *>(low), n, h, w, c,
-        static_cast<__nv_bfloat16 *>(dz));
+    const bool v8 = by8(c, cstride, 0, dcat, low, dz);
+    const size_t rows = (size_t)n * h;
+    if (n > 0 && h > 0 && w > 0 && c > 0)
+        (v8 ? k_upsample2_grad<8> : k_upsample2_grad<1>)<<<row_grid(rows, (size_t)w * c / (v8 ? 8 : 1)), 256, 0,
+                                                           static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16 *>(dcat), cstride, static_cast<const __nv_bfloat16 *>(low), w, c,
+            static_cast<__nv_bfloat16 *>(dz));
     return check_launch("k_upsample2_grad");
 }
 
@@ -899,9 +1018,18 @@ int stfwi_nn_head_loss_grad(const void *y, size_t npix, int c, const float *wt, 
     if (c % 16 || c > 64) return nn_fail(STFWI_ERR_INVALID, "head: channels must be a multiple of 16, <= 64");
     unsigned blocks = blocks_for(npix, 256);
     if (blocks > 1184) blocks = 1184;
-    k_head_loss_grad<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16 *>(y), npix, c, wt, out, target, wgt, inv_norm,
-        static_cast<__nv_bfloat16 *>(dz), dwt, db, loss);
+    auto go = [&](auto kern) {
+        kern<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16 *>(y), npix, wt, out, target, wgt, inv_norm, static_cast<__nv_bfloat16 *>(dz),
+            dwt, db, loss);
+    };
+    switch (c) {
+    default: go(k_head_loss_grad<0>); break;
+    case 16: go(k_head_loss_grad<16>); break;
+    case 32: go(k_head_loss_grad<32>); break;
+    case 48: go(k_head_loss_grad<48>); break;
+    case 64: go(k_head_loss_grad<64>); break;
+    }
     return check_launch("k_head_loss_grad");
 }
 
@@ -909,9 +1037,12 @@ int stfwi_nn_bias_grad(const void *dz, size_t npix, int c, float *db, void *stre
 {
     if (c <= 0 || c > 1024) return nn_fail(STFWI_ERR_INVALID, "bias_grad: channel count %d", c);
     const int threads = 256;
-    unsigned blocks = blocks_for(npix * c / 64, threads);
+    const bool v8 = c % 8 == 0 && aligned16(dz);
+    unsigned blocks = blocks_for(npix * c / (v8 ? 128 : 64), threads);
+    if (blocks > 8 * 148) blocks = 8 * 148;
+    // at least one whole pixel's channels among the threads of the grid
     if (blocks * threads < (unsigned)c) blocks = (c + threads - 1) / threads;
-    k_bias_grad<<<blocks, threads, c * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
+    (v8 ? k_bias_grad<8> : k_bias_grad<1>)<<<blocks, threads, c * sizeof(float), static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16 *>(dz), npix, c, db);
     return check_launch("k_bias_grad");
 }

@@ -164,6 +164,82 @@ def test_pool_upsample_skip_head_and_bias_kernels():
     assert _rel(_nchw(dzh), ref) < 4e-3
 
 
+@pytest.mark.parametrize("n,h,w,c,extra,coff", [
+    (1, 2, 2, 8, 0, 0),        # one 16-byte group, one output pixel
+    (2, 4, 6, 16, 8, 8),       # a slice of a wider buffer, still in 16-byte groups
+    (2, 4, 6, 16, 4, 0),       # stride not a multiple of 8: one channel a thread
+    (1, 2, 10, 24, 16, 4),     # offset not a multiple of 8
+    (3, 6, 258, 7, 1, 1),      # odd channels, more than one block to a row
+    (1, 2, 514, 64, 64, 64),   # more than one block to a row in groups
+])
+def test_row_kernels_equal_torch(n, h, w, c, extra, coff):
+    """Additions in the kernels' order in FP32 and one BF16 rounding: no difference is allowed."""
+    import torch
+    from stfwi_b200 import _native as N
+    L = N.load()
+    cs = c + max(extra, coff)
+    big, low = _bf16((n, h, w, cs), 1), _bf16((n, h // 2, w // 2, c), 2)
+    d = _bf16((n, h, w, cs), 3)
+    quad = lambda x: ((x[:, 0::2, 0::2] + x[:, 0::2, 1::2]) + x[:, 1::2, 0::2]) + x[:, 1::2, 1::2]
+    twice = lambda x: x.repeat_interleave(2, 1).repeat_interleave(2, 2)
+    sl, dsl = big[..., coff:coff + c].float(), d[..., coff:coff + c].float()
+
+    out = torch.full((n, h // 2, w // 2, c), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert L.stfwi_nn_avgpool2(big.data_ptr(), n, h, w, c, cs, coff, out.data_ptr(), None) == 0
+    assert torch.equal(out, (0.25 * quad(sl)).to(torch.bfloat16))
+
+    up = torch.full((n, h, w, cs), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert L.stfwi_nn_upsample2(low.data_ptr(), n, h // 2, w // 2, c, cs, up.data_ptr(), None) == 0
+    assert torch.equal(up[..., :c], twice(low)) and bool((up[..., c:] == 7.0).all())
+
+    assert L.stfwi_nn_upsample2_grad(d.data_ptr(), cs, low.data_ptr(), n, h // 2, w // 2, c, out.data_ptr(),
+                                     None) == 0
+    assert torch.equal(out, torch.where(low > 0, quad(d[..., :c].float()), 0.0).to(torch.bfloat16))
+
+    dz = torch.full((n, h, w, c), 7.0, dtype=torch.bfloat16, device="cuda")
+    for dcat in (d, None):
+        assert L.stfwi_nn_skip_grad(dcat.data_ptr() if dcat is not None else None, big.data_ptr(), cs, coff,
+                                    low.data_ptr(), n, h, w, c, dz.data_ptr(), None) == 0
+        v = 0.25 * twice(low).float() + (dsl if dcat is not None else 0.0)
+        assert torch.equal(dz, torch.where(sl > 0, v, 0.0).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("npix,c", [(1, 16), (3, 1), (257, 7), (70001, 24), (300, 1000), (5, 1024)])
+def test_bias_gradient_sums_all_pixels(npix, c):
+    """FP32 sums in any order of n terms: |error| <= n 2^-24 sum |x|, and far less in practice."""
+    import torch
+    from stfwi_b200 import _native as N
+    dz = _bf16((npix, c), 4)
+    db = torch.full((c,), 2.0, dtype=torch.float32, device="cuda")
+    assert N.load().stfwi_nn_bias_grad(dz.data_ptr(), npix, c, db.data_ptr(), None) == 0
+    ref = 2.0 + dz.double().sum(0)
+    assert bool(((db.double() - ref).abs() <= (npix + 1) * 2.0 ** -24 * (2.0 + dz.double().abs().sum(0))).all())
+
+
+@pytest.mark.parametrize("npix,c", [(1, 16), (255, 32), (70001, 48), (300, 64)])
+def test_head_loss_and_gradient(npix, c):
+    import torch
+    from stfwi_b200 import _native as N
+    y, wt = _bf16((npix, c), 5), torch.randn(c, generator=torch.Generator().manual_seed(6)).cuda()
+    out, tgt = _bf16((npix,), 7).float(), _bf16((npix,), 8).float()
+    wgt = (_bf16((npix,), 9) > 0).float()
+    dz = torch.zeros((npix, c), dtype=torch.bfloat16, device="cuda")
+    dwt, db = torch.zeros(c, device="cuda"), torch.zeros(1, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float64, device="cuda")
+    assert N.load().stfwi_nn_head_loss_grad(
+        y.data_ptr(), npix, c, wt.data_ptr(), out.data_ptr(), tgt.data_ptr(), wgt.data_ptr(), 1.0 / npix, dz.data_ptr(),
+        dwt.data_ptr(), db.data_ptr(), loss.data_ptr(), None) == 0
+    r, y64 = (out - tgt).double(), y.double()
+    g = 2.0 * wgt.double() * r / npix
+    # FP32 terms and sums of npix of them: relative to the sums of magnitudes
+    eps = (npix + 8) * 2.0 ** -24
+    assert abs(float(loss) - float((wgt * r * r).sum()) / npix) <= 8 * 2.0 ** -24 * float((wgt * r * r).sum()) / npix
+    assert abs(float(db) - float(g.sum())) <= eps * float(g.abs().sum())
+    assert bool(((dwt.double() - y64.T @ g).abs() <= eps * (y64.abs().T @ g.abs())).all())
+    ref = torch.where(y64 > 0, g[:, None] * wt.double(), 0.0)
+    assert bool(((dz.double() - ref).abs() <= 2.0 ** -8 * ref.abs()).all())
+
+
 def _network_case(B=2, seed=0):
     import torch
     from stfwi_b200.learned import UNet
