@@ -106,6 +106,20 @@ def test_conv_weight_gradient_matches_torch(n, h, w, cin, cout):
     assert _rel(dw.double().cpu() - 0.5, w9.grad) < 1e-4     # FP32 accumulation of exact BF16 products
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout", [
+    (1, 1, 64, 16, 16),      # one chunk; 9 taps of 16 rows: two tiles, the second with one live atom column
+    (3, 5, 192, 48, 48),     # three atom columns a tap: 27 over four tiles, two groups; 48 columns of N
+    (1, 3, 64, 96, 32),      # 96 columns of N
+    (2, 7, 128, 32, 64),     # nine columns over five tiles
+    (1, 2, 64, 80, 272),     # 17 atom columns a tap, over 20 groups
+    (8, 40, 64, 64, 128),    # more chunks than splits: ragged shares
+])
+def test_conv_weight_gradient_tiles(n, h, w, cin, cout):
+    """Edges of the (tap, channel) tiles: FP32 sums of K exact products differ from
+    FP64's by far less than rel-L2 1e-4."""
+    test_conv_weight_gradient_matches_torch(n, h, w, cin, cout)
+
+
 def test_pool_upsample_skip_head_and_bias_kernels():
     import torch
     import torch.nn.functional as F
