@@ -57,6 +57,7 @@ struct ConvGeo {
     int y_cstride, y_coff;
     int act;              // 0 none, 1 ReLU
     int m_cstride, m_coff;  // mask (input gradient): multiply by [mask > 0]
+    int rows, strips, stages;  // row kernel: output rows of a CTA, strips of them, pipeline stages
 };
 
 struct WgradGeo {
@@ -112,6 +113,33 @@ __device__ __forceinline__ void load_bf16x16(const __nv_bfloat16 *src, float (&v
 extern __shared__ uint8_t nn_smem[];
 
 // ------------------------------------------------------------------ conv (K-major)
+
+// accumulator row of one pixel -> bias, ReLU or mask, BF16
+__device__ __forceinline__ void conv_store(const ConvGeo &g, uint32_t taddr, size_t pix, int n0, bool ok,
+                                           const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask,
+                                           __nv_bfloat16 *__restrict__ y)
+{
+    for (int c = 0; c < g.bn; c += 16) {
+        float v[16];
+        tmem_ld16(taddr + (uint32_t)c, v);
+        const int ch = n0 + c;
+        if (bias) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += __ldg(bias + ch + i);
+        }
+        if (g.act == 1) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+        }
+        if (mask) {
+            float mk[16];
+            load_bf16x16(mask + pix * g.m_cstride + g.m_coff + ch, mk);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = mk[i] > 0.f ? v[i] : 0.f;
+        }
+        if (ok) store_bf16x16(y + pix * g.y_cstride + g.y_coff + ch, v);
+    }
+}
 
 __global__ void __launch_bounds__(CONV_THREADS, 1)
     k_conv_kmajor(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, ConvGeo g,
@@ -214,25 +242,174 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     tmem_fence_after();
     const int m = threadIdx.x;
     const size_t pix = ((size_t)img * g.h + h0 + m / g.bw) * g.w + w0 + m % g.bw;
-    for (int c = 0; c < g.bn; c += 16) {
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-        const int ch = n0 + c;
-        if (bias) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] += __ldg(bias + ch + i);
+    conv_store(g, tmem + ((uint32_t)(warp * 32) << 16), pix, n0, ok, bias, mask, y);
+    tmem_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tmem_fence_after();
+        tmem_dealloc(tmem, ncols);
+    }
+}
+
+// The same convolution down a strip of image rows, 128 pixels wide.  The kernel
+// above is bound by its operands' way from L2 into shared memory: nine boxes of
+// the input and nine of the weights for each 128 pixels.  Here all weights of the
+// CTA's output channels stay in shared memory, and an input row is loaded once for
+// each horizontal tap and used for the three output rows that it reaches, whose
+// accumulators are in tensor memory (a fourth is being stored meanwhile).  Each
+// output row still adds its taps and channels in the order of the kernel above,
+// so the results are the same bits.  us at 8 x 160 x 512 (before -> now): 32 ->
+// 32 channels 60 -> 33, 96 -> 32 116 -> 88, 32 -> 96 161 -> 74; 64 -> 64
+// at 8 x 80 x 256 45 -> 29; 128 -> 384 at 8 x 40 x 128 85 -> 60.
+constexpr int ROW_ACC = 4, ROW_STAGES = 8;
+template <int KC>
+__global__ void __launch_bounds__(PIPE_THREADS, 1)
+    k_conv_rows(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, ConvGeo g,
+                const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ mask,
+                __nv_bfloat16 *__restrict__ y, int *err)
+{
+    constexpr uint32_t aw = 2u * KC, a_bytes = 128u * aw;
+    const uint32_t b_bytes = (uint32_t)g.bn * aw;            // whole swizzle atoms
+    const int nkc = g.cin / KC;
+    uint8_t *wbase = align1024(nn_smem);
+    uint8_t *base = wbase + ((9 * nkc * b_bytes + 1023u) & ~1023u);
+    uint64_t *full = reinterpret_cast<uint64_t *>(base + g.stages * a_bytes);
+    uint64_t *empty = full + ROW_STAGES;
+    uint64_t *wfull = empty + ROW_STAGES;
+    uint64_t *done = wfull + 1, *drained = done + ROW_ACC;   // per accumulator: complete; read by the epilogue
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(drained + ROW_ACC);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles_w = g.w / 128;
+    int t = blockIdx.x;
+    const int w0 = (t % tiles_w) * 128;
+    t /= tiles_w;
+    const int h0 = (t % g.strips) * g.rows, h1 = min(g.h, h0 + g.rows);
+    const int img = t / g.strips;
+    const int n0 = blockIdx.y * g.bn;
+    const uint32_t ncols = tmem_cols_for(ROW_ACC * g.bn);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < g.stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
         }
-        if (g.act == 1) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+        mbar_init(wfull, 1);
+        for (int s = 0; s < ROW_ACC; ++s) {
+            mbar_init(&done[s], 1);
+            mbar_init(&drained[s], 4);
         }
-        if (mask) {
-            float mk[16];
-            load_bf16x16(mask + pix * g.m_cstride + g.m_coff + ch, mk);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = mk[i] > 0.f ? v[i] : 0.f;
+        fence_async_shared();
+    }
+    __syncwarp();
+    if (warp == 0) tmem_alloc(tslot, ncols);
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    const uint32_t tmem = *tslot;
+
+    // boxes of the strip: input rows h0 - 1 .. h1 (rows outside the image are zeros), for
+    // each the three horizontal taps and for each the input-channel blocks
+    if (warp == 4) {
+        if (lane == 0) {
+            mbar_arrive_expect_tx(wfull, 9u * nkc * b_bytes);
+            // per (horizontal tap, channel block): vertical taps 2, 1, 0 one below the other
+            for (int i = 0; i < 9 * nkc; ++i)
+                tma_load_3d(wbase + i * b_bytes, &tmW, wfull, i / 3 % nkc * KC, n0, (2 - i % 3) * 3 + i / 3 / nkc);
+            bool ok = true;
+            int s = 0, round = 0;
+            for (int r = h0 - 1; r <= h1 && ok; ++r)
+                for (int dx = 0; dx < 3 && ok; ++dx)
+                    for (int c = 0; c < nkc && ok; ++c) {
+                        ok = round == 0 || mbar_wait_bounded(&empty[s], (round - 1) & 1, NN_WAIT);
+                        if (ok) {
+                            mbar_arrive_expect_tx(&full[s], a_bytes);
+                            tma_load_4d(base + s * a_bytes, &tmX, &full[s], c * KC, w0 + dx - 1, r, img);
+                        }
+                        if (++s == g.stages) {
+                            s = 0;
+                            ++round;
+                        }
+                    }
+            if (!ok) atomicExch(err, 1);
         }
-        if (ok) store_bf16x16(y + pix * g.y_cstride + g.y_coff + ch, v);
+        __syncwarp();
+    } else if (warp == 5) {
+        if (lane == 0) {
+            const uint32_t layout = umma_layout_for((int)aw);
+            const uint64_t a0 = umma_smem_desc(smem_u32(base), 16u, 8u * aw, layout);
+            const uint64_t b0 = umma_smem_desc(smem_u32(wbase), 16u, 8u * aw, layout);
+            int s = 0, round = 0;
+            bool ok = mbar_wait_bounded(wfull, 0, NN_WAIT);
+            for (int r = h0 - 1; r <= h1 && ok; ++r) {
+                // output row r + 1 begins here, in the accumulator of row r - 3
+                const int first = r + 1 - h0;
+                if (r + 1 < h1 && first >= ROW_ACC)
+                    ok = mbar_wait_bounded(&drained[first % ROW_ACC], (first / ROW_ACC - 1) & 1, NN_WAIT);
+                for (int dx = 0; dx < 3 && ok; ++dx)
+                    for (int c = 0; c < nkc && ok; ++c) {
+                        ok = mbar_wait_bounded(&full[s], round & 1, NN_WAIT);
+                        if (!ok) break;
+                        tmem_fence_after();
+                        // This row adds to output rows r - 1, r, r + 1 (vertical taps 2, 1, 0), whose
+                        // accumulators lie side by side but for the ring's end.  With 64-channel blocks
+                        // one MMA serves as many of them as N <= 256 holds, but for row r + 1 where its
+                        // accumulator begins (64 -> 64 channels 32 -> 29 us); with smaller blocks the
+                        // few K steps of a box do not pay for the longer loop (96 -> 32: 88 -> 97 us).
+                        const uint64_t ad = a0 + ((s * a_bytes) >> 4);
+                        const uint64_t bd = b0 + (((dx * nkc + c) * 3 * b_bytes) >> 4);
+                        const int end = min(h1, r + 2);
+                        if constexpr (KC == 64) {
+                            for (int o = max(h0, r - 1); o < end;) {
+                                const int slot = (o - h0) % ROW_ACC;
+                                const bool begins = o == r + 1 && (dx | c) == 0;
+                                int m = min(min(end - o, ROW_ACC - slot), 256 / g.bn);
+                                if ((dx | c) == 0 && !begins && o + m == r + 2) --m;
+                                const uint32_t idesc = umma_idesc_bf16(128, m * g.bn, 0, 0);
+                                const uint64_t bo = bd + (((o + 1 - r) * b_bytes) >> 4);
+                                // a K step of 16 is +32 bytes inside the swizzle atom (2 in the descriptor)
+#pragma unroll
+                                for (int k = 0; k < KC / 16; ++k)
+                                    umma_bf16(tmem + (uint32_t)(slot * g.bn), ad + 2u * k, bo + 2u * k, idesc,
+                                              !begins || k != 0);
+                                o += m;
+                            }
+                        } else {
+                            const uint32_t idesc = umma_idesc_bf16(128, g.bn, 0, 0);
+#pragma unroll
+                            for (int k = 0; k < KC / 16; ++k)
+#pragma unroll
+                                for (int j = 0; j < 3; ++j) {
+                                    const int o = r - 1 + j;
+                                    if (o < h0 || o >= end) continue;
+                                    umma_bf16(tmem + (uint32_t)(o - h0) % ROW_ACC * g.bn, ad + 2u * k,
+                                              bd + ((j * b_bytes) >> 4) + 2u * k, idesc, (dx | c | k) != 0 || j < 2);
+                                }
+                        }
+                        umma_commit(&empty[s]);
+                        if (++s == g.stages) {
+                            s = 0;
+                            ++round;
+                        }
+                    }
+                if (ok && r - 1 >= h0) umma_commit(&done[(r - 1 - h0) % ROW_ACC]);
+            }
+            if (!ok) atomicExch(err, 2);
+        }
+        __syncwarp();
+    } else {
+        for (int o = h0; o < h1; ++o) {
+            const int k = o - h0, slot = k % ROW_ACC;
+            const bool ok = mbar_wait_bounded(&done[slot], (k / ROW_ACC) & 1, NN_WAIT);
+            if (!ok && lane == 0) atomicExch(err, 3);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            tmem_fence_after();
+            const size_t pix = ((size_t)img * g.h + o) * g.w + w0 + threadIdx.x;
+            conv_store(g, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(slot * g.bn), pix, n0, true, bias, mask, y);
+            tmem_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&drained[slot]);
+        }
     }
     tmem_fence_before();
     __syncthreads();
@@ -846,6 +1023,55 @@ size_t wgrad_smem(int mt, int bn, int stages)
     return need > WGRAD_SMEM_MIN ? need : WGRAD_SMEM_MIN;
 }
 
+// How a convolution is cut into CTAs: strips of rows where the weights of all (or 64 or
+// more) output channels fit shared memory and one wave of CTAs has strips of ROWS_MIN
+// rows at least, else boxes.  Shorter strips load their two outer rows too often and wait
+// for all weights first, narrower pieces read the input again for each: us, boxes against
+// strips, 96 -> 32 channels at 1 x 160 x 512 (strips of 3 rows) 21, 23; 192 -> 64 at 8 x 80
+// x 256 (32 channels a piece) 87, 117; 128 -> 128 at 8 x 40 x 128 (strips of 5) 41, 29.
+constexpr int ROWS_MIN = 4;
+
+struct ConvPlan {
+    int bn = 0, rows = 0, strips = 0, stages = 0;   // rows 0: boxes
+    size_t smem = 0;
+};
+
+ConvPlan conv_plan(int n, int h, int w, int cin, int cout, int kc)
+{
+    ConvPlan p;
+    const size_t sm_smem = 228 * 1024, aw = 2 * kc, a = 128 * aw;
+    for (int bn = 128; bn >= 16 && w % 128 == 0; bn -= 16) {
+        if (cout % bn || (bn < cout && bn < 64)) continue;
+        const size_t fixed = 1024 + ((9 * (cin / kc) * bn * aw + 1023) & ~(size_t)1023) +
+                             (2 * ROW_STAGES + 1 + 2 * ROW_ACC) * 8 + 16;
+        const size_t cols = tmem_cols_for(ROW_ACC * bn);
+        for (int occ = 4; occ >= 1; occ >>= 1) {
+            // as many CTAs per SM as tensor memory and shared memory hold
+            const size_t cap = occ == 1 ? 227 * 1024 : sm_smem / occ - 1024;
+            if (occ * cols > 512 || fixed + 4 * a > cap) continue;
+            const double want = occ * 148.0 / ((double)n * (w / 128) * (cout / bn));
+            p.strips = want < 1 ? 1 : want > h ? h : (int)want;
+            p.rows = (h + p.strips - 1) / p.strips;
+            if (p.rows < ROWS_MIN) break;
+            p.strips = (h + p.rows - 1) / p.rows;
+            p.bn = bn;
+            p.stages = (int)((cap - fixed) / a < (size_t)ROW_STAGES ? (cap - fixed) / a : ROW_STAGES);
+            p.smem = fixed + p.stages * a;
+            // and no more of them, so that tcgen05.alloc never waits for a CTA of the same kernel
+            const size_t least = sm_smem / (512 / cols + 1) - 1024 + 16;
+            if (p.smem < least) p.smem = least;
+            return p;
+        }
+    }
+    // boxes: all output channels that a tile holds, or fewer while the grid is smaller than the
+    // chip (us at batch 1, 128 -> 128 at 40 x 128: 14.8 -> 13.2, 256 -> 256 at 20 x 64: 22 -> 19)
+    p = ConvPlan();
+    p.bn = cout % 128 == 0 ? 128 : cout % 64 == 0 ? 64 : cout % 32 == 0 ? 32 : 16;
+    while (p.bn > 16 && 2.0 * ((double)n * h * w / 128) * (cout / p.bn) <= 148) p.bn /= 2;
+    p.smem = conv_smem(kc, p.bn);
+    return p;
+}
+
 int conv_common(const void *x, int n, int h, int w, int cin, const void *wt, int cout, const float *bias, int act,
                 const void *mask, int m_cstride, int m_coff, void *y, int y_cstride, int y_coff, cudaStream_t st)
 {
@@ -864,7 +1090,9 @@ int conv_common(const void *x, int n, int h, int w, int cin, const void *wt, int
     ConvGeo g{};
     g.n = n; g.h = h; g.w = w; g.cin = cin; g.cout = cout;
     g.kc = largest_atom(cin);
-    g.bn = cout % 128 == 0 ? 128 : cout % 64 == 0 ? 64 : cout % 32 == 0 ? 32 : 16;
+    const ConvPlan plan = conv_plan(n, h, w, cin, cout, g.kc);
+    g.bn = plan.bn;
+    g.rows = plan.rows; g.strips = plan.strips; g.stages = plan.stages;
     g.bw = bw; g.bh = 128 / bw;
     g.y_cstride = y_cstride; g.y_coff = y_coff; g.act = act;
     g.m_cstride = m_cstride; g.m_coff = m_coff;
@@ -879,13 +1107,22 @@ int conv_common(const void *x, int n, int h, int w, int cin, const void *wt, int
     if (rc) return rc;
     int *err = err_flag();
     if (!err) return nn_fail(STFWI_ERR_CUDA, "conv: the error flag of this device could not be looked up");
-    static bool attr[NN_MAX_DEVICES] = {};
-    rc = smem_limit_once(k_conv_kmajor, conv_smem(64, 128), attr, "conv: shared-memory attribute");
-    if (rc) return rc;
-    const dim3 grid((unsigned)((size_t)n * (h / g.bh) * (w / g.bw)), (unsigned)(cout / g.bn));
-    k_conv_kmajor<<<grid, CONV_THREADS, conv_smem(g.kc, g.bn), st>>>(
-        tx, tw, g, bias, static_cast<const __nv_bfloat16 *>(mask), static_cast<__nv_bfloat16 *>(y), err);
-    return check_launch("k_conv_kmajor");
+    static bool attr[4][NN_MAX_DEVICES] = {};
+    auto go = [&](auto kern, size_t limit, bool (&done)[NN_MAX_DEVICES], dim3 grid, int threads) {
+        const int e = smem_limit_once(kern, limit, done, "conv: shared-memory attribute");
+        if (e) return e;
+        kern<<<grid, threads, plan.smem, st>>>(tx, tw, g, bias, static_cast<const __nv_bfloat16 *>(mask),
+                                               static_cast<__nv_bfloat16 *>(y), err);
+        return check_launch("convolution");
+    };
+    const unsigned groups = (unsigned)(cout / g.bn);
+    if (!g.rows)
+        return go(k_conv_kmajor, conv_smem(64, 128), attr[0],
+                  dim3((unsigned)((size_t)n * (h / g.bh) * (w / g.bw)), groups), CONV_THREADS);
+    const dim3 grid((unsigned)((size_t)n * g.strips * (w / 128)), groups);
+    return g.kc == 64   ? go(k_conv_rows<64>, 227 * 1024, attr[1], grid, PIPE_THREADS)
+           : g.kc == 32 ? go(k_conv_rows<32>, 227 * 1024, attr[2], grid, PIPE_THREADS)
+                        : go(k_conv_rows<16>, 227 * 1024, attr[3], grid, PIPE_THREADS);
 }
 
 unsigned blocks_for(size_t n, int threads)

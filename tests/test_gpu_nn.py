@@ -61,6 +61,21 @@ def test_conv_forward_matches_torch(n, h, w, cin, cout):
     assert float(y[..., :16].abs().max()) == 0.0 and float(y[..., 16 + cout:].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("n,h,w,cin,cout", [
+    (1, 1, 128, 16, 16),      # one row: both vertical neighbours are padding
+    (1, 3, 256, 48, 112),     # 16-channel blocks, 112 columns
+    (3, 37, 128, 32, 96),     # 96 columns; strips of unequal length
+    (2, 80, 640, 16, 32),     # more strips than SMs hold at a time
+    (40, 13, 128, 64, 64),    # long strips: the four accumulators are used again
+    (1, 5, 128, 192, 64),     # weights of a part of the output channels fit
+    (1, 40, 128, 384, 128),   # weights that do not fit: boxes
+])
+def test_conv_strips(n, h, w, cin, cout):
+    """Forward and (masked) input gradient over the ways a convolution is cut."""
+    test_conv_forward_matches_torch(n, h, w, cin, cout)
+    test_conv_input_gradient_matches_torch(n, h, w, cout, cin)
+
+
 @pytest.mark.parametrize("n,h,w,cin,cout", [(1, 4, 128, 32, 64), (2, 2, 64, 96, 32), (1, 4, 64, 16, 32)])
 def test_conv_input_gradient_matches_torch(n, h, w, cin, cout):
     """dgrad with the tap-flipped transposed weights and the ReLU mask."""
