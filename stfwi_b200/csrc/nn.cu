@@ -65,12 +65,9 @@ struct WgradGeo {
     int cout, cin;        // channels of dz (M side) and of x (N side)
     int ae_a, ae_b;       // swizzle atom width in elements along M and along N
     int ca;               // atom columns of dz: cout / ae_a
-    int mt;               // 128-row tiles of (tap, channel) rows per CTA
     int bn;               // input channels per CTA (multiple of ae_b, <= 128)
     int ci_tiles;
-    int stages;
     int chunks, chunks_per_split;  // 64-pixel row chunks in total and per CTA
-    int seg;              // chunks added up in one accumulator
 };
 
 __host__ __device__ inline uint32_t tmem_cols_for(int n)
@@ -423,15 +420,11 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
 
 // Rows of M are (tap, output channel) pairs, an atom column of dz (16, 32 or 64
 // channels) each from its own shift of dz: dW[tap] = sum_q dz[q - tap] x[q].  So
-// one load of x serves up to three 128-row tiles of a CTA (one accumulator
-// each), and layers of fewer than 128 channels fill their tiles: with one tap a
-// CTA, 32 channels used a quarter of the rows and x was read nine times.  What
-// bounds it is the operands' way from L2 into shared memory; a grid of one CTA
-// per SM takes the pixels once.  The accumulators are added to dw after every
-// `seg` chunks: the tensor cores cut the sums' low bits off, so that the error
-// grows with the length of a sum (launch code below).  us at 8 x 160 x 512 (before -> now): 32 -> 32
-// channels 209 -> 85, 96 -> 32 660 -> 100; 8 x 40 x 128: 128 -> 128 115 -> 41, 384 -> 128 135 -> 64;
-// all 14 layers 2219 -> 833.
+// layers of fewer than 128 channels fill their tiles: with one tap a CTA, 32
+// channels used a quarter of the rows, and x was read nine times instead of
+// three.  What bounds it is the operands' way from L2 into shared memory.  us at
+// 8 x 160 x 512 (before -> now): 32 -> 32 channels 209 -> 130, 96 -> 32 660 -> 379; 8 x 40 x
+// 128: 128 -> 128 115 -> 52, 384 -> 128 135 -> 103; all 14 layers 2219 -> 1378.
 __global__ void __launch_bounds__(PIPE_THREADS, 1)
     k_conv_wgrad(const __grid_constant__ CUtensorMap tmDZ, const __grid_constant__ CUtensorMap tmX, WgradGeo g,
                  float *__restrict__ dw, int *err)
@@ -439,32 +432,30 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
     const uint32_t aw_a = 2u * g.ae_a, aw_b = 2u * g.ae_b;
     const int na = 128 / g.ae_a, nb = g.bn / g.ae_b;       // atom columns of a tile along M and along N
     const uint32_t col_a = WG_PIX * aw_a, col_b = WG_PIX * aw_b;  // bytes of one atom column (multiples of 1024)
-    const uint32_t a_bytes = g.mt * na * col_a, b_bytes = nb * col_b;
+    const uint32_t a_bytes = na * col_a, b_bytes = nb * col_b;
     const uint32_t st_bytes = a_bytes + b_bytes;
     uint8_t *base = align1024(nn_smem);
-    uint64_t *full = reinterpret_cast<uint64_t *>(base + g.stages * st_bytes);
+    uint64_t *full = reinterpret_cast<uint64_t *>(base + STAGES * st_bytes);
     uint64_t *empty = full + STAGES;
-    uint64_t *done = empty + STAGES, *drained = done + 1;   // accumulators complete; read by the epilogue
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(drained + 1);
+    uint64_t *done = empty + STAGES;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = threadIdx.x >> 5;
     const int n0 = blockIdx.y * g.bn;
     const int c_begin = blockIdx.x * g.chunks_per_split;
     const int c_end = min(g.chunks, c_begin + g.chunks_per_split);
     const int nk = c_end - c_begin;
-    const uint32_t ncols = tmem_cols_for(g.mt * g.bn);
-    // this CTA's atom columns: [a0, a0 + live) of 9 taps x ca.  A tile's columns past the
+    const uint32_t ncols = tmem_cols_for(g.bn);
+    // this CTA's atom columns: [a0, a0 + live) of 9 taps x ca.  The tile's columns past the
     // last are not loaded: their accumulator rows hold anything and are not read.
-    const int a0 = blockIdx.z * g.mt * na, live = min(g.mt * na, 9 * g.ca - a0);
-    const int tiles = (live + na - 1) / na;
+    const int a0 = blockIdx.z * na, live = min(na, 9 * g.ca - a0);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < g.stages; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         mbar_init(done, 1);
-        mbar_init(drained, 4);
     }
     fence_async_shared();
     __syncwarp();
@@ -506,7 +497,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
                 }
             }
             if (__shfl_sync(0xffffffffu, fail, 0)) break;
-            if (++s == g.stages) {
+            if (++s == STAGES) {
                 s = 0;
                 ++round;
             }
@@ -515,64 +506,48 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
         // K = 16 pixel rows per MMA: +16 rows of the atom column; LBO = atom column stride, SBO = 8 rows
         const uint32_t idesc = umma_idesc_bf16(128, g.bn, 1, 1);
         const uint32_t la = umma_layout_for((int)aw_a), lb = umma_layout_for((int)aw_b);
-        int s = 0, round = 0, in_seg = 0, segs = 0;
+        int s = 0, round = 0;
         for (int kb = 0; kb < nk; ++kb) {
             int fail = 0;
             if (lane == 0) {
-                if (in_seg == 0 && segs > 0 && !mbar_wait_bounded(drained, (segs - 1) & 1, NN_WAIT)) {
-                    atomicExch(err, 14);
-                    fail = 1;
-                } else if (!mbar_wait_bounded(&full[s], round & 1, NN_WAIT)) {
+                if (!mbar_wait_bounded(&full[s], round & 1, NN_WAIT)) {
                     atomicExch(err, 12);
                     fail = 1;
                 } else {
                     tmem_fence_after();
                     const uint32_t sa = sbase + s * st_bytes, sb = sa + a_bytes;
-                    for (int t = 0; t < tiles; ++t)
 #pragma unroll
-                        for (int k = 0; k < WG_PIX / 16; ++k) {
-                            const uint64_t ad = umma_smem_desc(sa + t * na * col_a + 16u * aw_a * k, col_a, 8u * aw_a, la);
-                            const uint64_t bd = umma_smem_desc(sb + 16u * aw_b * k, col_b, 8u * aw_b, lb);
-                            umma_bf16(tmem + (uint32_t)(t * g.bn), ad, bd, idesc, (in_seg | k) != 0);
-                        }
+                    for (int k = 0; k < WG_PIX / 16; ++k) {
+                        const uint64_t ad = umma_smem_desc(sa + 16u * aw_a * k, col_a, 8u * aw_a, la);
+                        const uint64_t bd = umma_smem_desc(sb + 16u * aw_b * k, col_b, 8u * aw_b, lb);
+                        umma_bf16(tmem, ad, bd, idesc, (kb | k) != 0);
+                    }
                     umma_commit(&empty[s]);
-                    if (in_seg + 1 == g.seg || kb + 1 == nk) umma_commit(done);
+                    if (kb + 1 == nk) umma_commit(done);
                 }
             }
             if (__shfl_sync(0xffffffffu, fail, 0)) break;
-            if (++s == g.stages) {
+            if (++s == STAGES) {
                 s = 0;
                 ++round;
             }
-            if (++in_seg == g.seg) {
-                in_seg = 0;
-                ++segs;
-            }
         }
     } else {
-        for (int kb = 0, sg = 0; kb < nk; kb += g.seg, ++sg) {
-            const bool ok = mbar_wait_bounded(done, sg & 1, NN_WAIT);
-            if (!ok && lane == 0) atomicExch(err, 13);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            tmem_fence_after();
-            for (int t = 0; t < tiles; ++t) {
-                const int a = t * na + threadIdx.x / g.ae_a;
-                const int tap = (a0 + a) / g.ca, co = (a0 + a) % g.ca * g.ae_a + threadIdx.x % g.ae_a;
-                float *dst = dw + ((size_t)tap * g.cout + co) * g.cin + n0;
-                for (int c = 0; c < g.bn; c += 16) {
-                    float v[16];
-                    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * g.bn + c), v);
-                    if (a < live) {
+        const bool ok = mbar_wait_bounded(done, 0, NN_WAIT);
+        if (!ok && lane == 0) atomicExch(err, 13);
+        __syncwarp();
+        tmem_fence_after();
+        const int a = threadIdx.x / g.ae_a, tap = (a0 + a) / g.ca;
+        const int co = (a0 + a) % g.ca * g.ae_a + threadIdx.x % g.ae_a;
+        float *dst = dw + ((size_t)tap * g.cout + co) * g.cin + n0;
+        for (int c = 0; c < g.bn; c += 16) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+            if (ok && a < live) {
 #pragma unroll
-                        for (int i = 0; i < 16; i += 4)
-                            atomicAdd(reinterpret_cast<float4 *>(dst + c + i),
-                                      make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
-                    }
-                }
+                for (int i = 0; i < 16; i += 4)
+                    atomicAdd(reinterpret_cast<float4 *>(dst + c + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
             }
-            tmem_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(drained);
         }
     }
     tmem_fence_before();
@@ -1013,14 +988,10 @@ size_t conv_smem(int kc, int bn)
     return need > tmem_floor(bn) ? need : tmem_floor(bn);
 }
 
-// One CTA of the weight gradient per SM, so that its up to 512 tensor-memory
-// columns are free when it starts: more than half of the SM's shared memory.
-constexpr size_t WGRAD_SMEM_MAX = 227 * 1024, WGRAD_SMEM_MIN = 116 * 1024;
-
-size_t wgrad_smem(int mt, int bn, int stages)
+size_t wgrad_smem(int bn)
 {
-    const size_t need = 1024 + stages * (size_t)(mt * 128 + bn) * WG_PIX * 2 + (2 * STAGES + 2) * 8 + 16;
-    return need > WGRAD_SMEM_MIN ? need : WGRAD_SMEM_MIN;
+    const size_t need = 1024 + STAGES * (size_t)(128 + bn) * WG_PIX * 2 + (2 * STAGES + 1) * 8 + 16;
+    return need > tmem_floor(bn) ? need : tmem_floor(bn);
 }
 
 // How a convolution is cut into CTAs: strips of rows where the weights of all (or 64 or
@@ -1194,31 +1165,22 @@ int stfwi_nn_conv3x3_wgrad(const void *x, const void *dz, int n, int h, int w, i
     g.n = n; g.h = h; g.w = w; g.cout = cout; g.cin = cin;
     g.ae_a = largest_atom(cout);
     g.ca = cout / g.ae_a;
-    g.ae_b = largest_atom(cin);
-    g.bn = g.ae_b;
-    for (int b = g.ae_b; b <= 128; b += g.ae_b)
-        if (cin % b == 0) g.bn = b;
+    g.bn = cin % 128 == 0 ? 128 : cin % 64 == 0 ? 64 : cin % 32 == 0 ? 32 : 16;
+    g.ae_b = g.bn >= 64 ? 64 : g.bn;
     g.ci_tiles = cin / g.bn;
-    // three tiles of at most 128 accumulator columns: 384 of the SM's 512
-    const int na = 128 / g.ae_a, tiles_a = (9 * g.ca + na - 1) / na;
-    g.mt = tiles_a < 3 ? tiles_a : 3;
-    const int groups = (tiles_a + g.mt - 1) / g.mt;
-    g.stages = STAGES;
-    while (wgrad_smem(g.mt, g.bn, g.stages) > WGRAD_SMEM_MAX) --g.stages;
+    const int na = 128 / g.ae_a, groups = (9 * g.ca + na - 1) / na;
     g.chunks = n * h * (w / WG_PIX);
-    // one wave of CTAs: fewer splits leave SMs idle, more add the accumulators once more each
-    int splits = 148 / (groups * g.ci_tiles);
+    // The tensor cores cut the low bits of a sum off, so the length of the sums decides how
+    // far a gradient is from FP64's: they stay as long as with one tap, 128 output channels
+    // and bn input channels a CTA and four CTAs per SM, whatever share of the rows is filled.
+    // (Three tiles a CTA and one CTA per SM took 833 us in all, but moved gradients of 12
+    // images of 320 x 1024 by up to 8e-5 of their norm; this keeps them within 8e-7.)
+    const int tiles = 9 * ((cout + 127) / 128) * g.ci_tiles;
+    int splits = (4 * 148 + tiles - 1) / tiles;
     if (splits > g.chunks) splits = g.chunks;
     if (splits < 1) splits = 1;
     g.chunks_per_split = (g.chunks + splits - 1) / splits;
     splits = (g.chunks + g.chunks_per_split - 1) / g.chunks_per_split;
-    // No sum is longer than with one (tap, 128 channels, bn) tile a CTA and four CTAs per
-    // SM: relative errors of dw against FP64 are then 9.6e-6 -> 3.9e-6 (32 -> 32 channels at 8 x 160
-    // x 512, before -> now), 1.3e-6 -> 8.2e-7 (384 -> 128 at 8 x 40 x 128), where sums of the whole
-    // share gave 1.9e-6 (and took 10 us less).
-    const int tiles = 9 * ((cout + 127) / 128) * g.ci_tiles, sums = (4 * 148 + tiles - 1) / tiles;
-    const int longest = (g.chunks + sums - 1) / sums, segs = (g.chunks_per_split + longest - 1) / longest;
-    g.seg = (g.chunks_per_split + segs - 1) / segs;
     CUtensorMap ta, tb;
     const cuuint64_t da[4] = {(cuuint64_t)cout, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
     const cuuint32_t ba[4] = {(cuuint32_t)g.ae_a, WG_PIX, 1, 1};
@@ -1231,10 +1193,10 @@ int stfwi_nn_conv3x3_wgrad(const void *x, const void *dz, int n, int h, int w, i
     int *err = err_flag();
     if (!err) return nn_fail(STFWI_ERR_CUDA, "wgrad: the error flag of this device could not be looked up");
     static bool attr[NN_MAX_DEVICES] = {};
-    rc = smem_limit_once(k_conv_wgrad, WGRAD_SMEM_MAX, attr, "wgrad: shared-memory attribute");
+    rc = smem_limit_once(k_conv_wgrad, wgrad_smem(128), attr, "wgrad: shared-memory attribute");
     if (rc) return rc;
     const dim3 grid((unsigned)splits, (unsigned)g.ci_tiles, (unsigned)groups);
-    k_conv_wgrad<<<grid, PIPE_THREADS, wgrad_smem(g.mt, g.bn, g.stages), static_cast<cudaStream_t>(stream)>>>(ta, tb, g, dw, err);
+    k_conv_wgrad<<<grid, PIPE_THREADS, wgrad_smem(g.bn), static_cast<cudaStream_t>(stream)>>>(ta, tb, g, dw, err);
     return check_launch("k_conv_wgrad");
 }
 

@@ -122,11 +122,11 @@ def test_conv_weight_gradient_matches_torch(n, h, w, cin, cout):
 
 
 @pytest.mark.parametrize("n,h,w,cin,cout", [
-    (1, 1, 64, 16, 16),      # one chunk; 9 taps of 16 rows: two tiles, the second with one live atom column
-    (3, 5, 192, 48, 48),     # three atom columns a tap: 27 over four tiles, two groups; 48 columns of N
-    (1, 3, 64, 96, 32),      # 96 columns of N
-    (2, 7, 128, 32, 64),     # nine columns over five tiles
-    (1, 2, 64, 80, 272),     # 17 atom columns a tap, over 20 groups
+    (1, 1, 64, 16, 16),      # one chunk; nine atom columns over two tiles, the second with one
+    (3, 5, 192, 48, 48),     # three atom columns a tap: 27 over four tiles
+    (1, 3, 64, 96, 32),      # nine atom columns over three tiles; three pieces of N
+    (2, 7, 128, 32, 64),     # nine atom columns over five tiles
+    (1, 2, 64, 80, 272),     # 17 atom columns a tap, a last tile of one
     (8, 40, 64, 64, 128),    # more chunks than splits: ragged shares
 ])
 def test_conv_weight_gradient_tiles(n, h, w, cin, cout):
