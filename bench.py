@@ -418,7 +418,7 @@ def main():
             "kernel_times": "one-chain pass sampled after the timed loop"}
     # the whole step against the same peak: the algorithmic bytes of all four
     # kernels per step, over the timed ms per step (the timed loop runs the
-    # pass as two concurrent chains when the shots are grouped alike)
+    # pass as two concurrent chains)
     step_bytes = nt * sum(kb.values())
     roof["step_achieved"] = step_bytes / (ms_step * 1e-3) / 1e9
     roof["step_frac"] = roof["step_achieved"] / peak
@@ -426,10 +426,8 @@ def main():
     roof["frac_of_nominal_7700"] = achieved / 7700.0
     roof["step_frac_of_nominal_7700"] = roof["step_achieved"] / 7700.0
     # stencil launches: 2 per forward step and 2 per adjoint step, once per
-    # chain when the pass is split (every kernel with the same shots per
-    # block: at most one chain per shot group); plus set-up, misfit, finalize
-    spg = set(schedule.values()) if schedule else set()
-    chains = min(args.chains or 2, -(-ns // spg.pop())) if len(spg) == 1 else 1
+    # chain of the pass; plus set-up, misfit, finalize
+    chains = min(args.chains or 2, ns)
     launches = 4 * nt * chains + 6
 
     cpu = None

@@ -1953,7 +1953,7 @@ stfwi_status stfwi_kernel_times(stfwi_handle *h, double *out)
 
 // `steps` forward then `steps` adjoint steps of the handle's current
 // schedule, launched directly (not captured) on `st`, split into chains
-// exactly as a captured pass would be (pass_chains); the timing passes of
+// exactly as a captured pass would be (pass_parts); the timing passes of
 // the autotuner
 static stfwi_status enqueue_timing_steps(stfwi_handle *h, int steps, cudaStream_t st)
 {
@@ -2054,10 +2054,10 @@ stfwi_status stfwi_autotune(stfwi_handle *h, int32_t steps, int32_t *spg_out, vo
     const int qa = sa[0] < sa[1] ? 0 : 1, qb = best[0][3] < best[1][3] ? 0 : 1;
     if ((r = set_tiling(h, qa + 1, qb + 1))) return r;
     int spg[4] = {pick[qa][0], pick[qa][1], pick[qa][2], pick[qb][3]};
-    // stage 2: whole steps, split into chains as the passes will be.  The
-    // per-kernel picks let a pass split only when they coincide; a uniform
-    // grouping always does.  Time the picks and every uniform grouping and
-    // keep the fastest.
+    // stage 2: whole steps, split into chains as the passes will be: there a
+    // kernel overlaps the other chain's, so that the best run length of each
+    // alone need not be the best of all.  Time the picks and every length
+    // alike for all kernels and keep the fastest.
     if (h->d.shot_group <= 0 && h->chains > 1) {
         // no sampled timing while timing whole steps (it would also keep
         // the passes in one chain)

@@ -309,7 +309,7 @@ class Solver:
         return int(out[0]), int(out[1])
 
     def set_chains(self, chains):
-        """Chains (1-4) a pass may be split into over the shot groups; see stfwi_set_chains."""
+        """Chains (1-4) a pass may be split into over the shots; see stfwi_set_chains."""
         self._ok(self.lib.stfwi_set_chains(self.h, int(chains)), "set_chains")
 
     def set_tile_rows(self, rows_a, rows_b):
