@@ -12,6 +12,8 @@
 //    ReLU output, and stores BF16 NHWC with any channel stride / offset.
 //    The same kernel computes the input gradient with the tap-flipped,
 //    transposed weights.
+//  * k_conv_rows    the same convolution down strips of rows, with the weights
+//    resident and each input row used for three output rows; the same bits.
 //  * k_conv_wgrad   weight gradient dW[tap][co][ci] = sum_p dz[p][co] x[p+tap][ci]
 //    as a GEMM with M = (tap, output channel) pairs, N = input channels,
 //    K = pixels, both operands MN-major (channels contiguous in NHWC), split
