@@ -161,12 +161,18 @@ struct Plan {
     size_t total() const { return fields + psi + snap + row0 + acc + rec + misc + ckpt; }
 };
 
-// FP64 gradient accumulator groups: one per group of shots of the strain
-// phase, at least two shots per group unless the descriptor asks otherwise
+// FP64 gradient accumulator groups.  A block adds to a group of its own, so that
+// two passes give the same bits; blocks take runs of at least two shots of a
+// tile where there is work for every SM (acc_in_use), and there one group per two
+// shots is enough.  Where there is not, blocks take single shots: one group for each,
+// and one more for each uneven part; those grids are small (at most 140 MB in
+// all).  Never fewer than a pass has parts.
 int acc_groups_of(const stfwi_desc *d)
 {
-    const int spg0 = d->shot_group > 0 ? d->shot_group : 2;
-    return std::max(1, (d->max_shots + spg0 - 1) / spg0);
+    const int spg0 = d->shot_group > 0 ? d->shot_group : 2, n = d->max_shots;
+    const long long tiles = ((d->nx_dom + 2LL * d->pad + 63) / 64) * ((d->nz_dom + 2LL * d->pad + 15) / 16);
+    if (tiles * n < 4LL * 2 * 2 * 148) return std::max(1, n + MAX_CHAINS - 1);
+    return std::max(1, std::max((n + spg0 - 1) / spg0, std::min(n, MAX_CHAINS)));
 }
 
 // Image bands of the adjoint: the columns (rows) that the boxes of the tiles
