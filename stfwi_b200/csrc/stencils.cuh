@@ -295,7 +295,13 @@ template <int FD, int R, int NW> struct Stage {
     using T = G4<FD, R, NW>;
     static constexpr int OWN2 = al32_3(2 * T::TZH * TX4), OWN3 = al32_3(3 * T::TZH * TX4);
     static constexpr int VEL = T::S3 + OWN2, STR = T::S2 + OWN3;
-    static constexpr int ADA = al32_3(4 * T::SN) + OWN2, ADB = al32_3(4 * T::SN) + 2 * OWN3;
+    // adjoint stages: four planes, each a copy of its own that starts on 128
+    // bytes, then the own boxes; at FD 2 a plane's rows do not end on 128 bytes
+    static constexpr int SNA = al32_3(T::SN), SOWN = 4 * SNA;
+    static constexpr int ADA = SOWN + OWN2, ADB = SOWN + 2 * OWN3;
+    static_assert(SNA % 32 == 0 && SOWN >= 3 * SNA + T::SN && ADA >= SOWN + 2 * T::TZH * TX4 &&
+                      ADB >= SOWN + OWN3 + 3 * T::TZH * TX4,
+                  "a stage holds all that its copies write");
     static constexpr int fit(int floats) { return imin(4, (113 * 1024 - 256 - (int)sizeof(AdjTab)) / (floats * 4)); }
     static constexpr int imin(int a, int b) { return a < b ? a : b; }
     static constexpr int NVEL = fit(VEL), NSTR = fit(STR), NADA = fit(ADA), NADB = fit(ADB);
@@ -874,9 +880,9 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
              const __grid_constant__ CUtensorMap tmE, const __grid_constant__ CUtensorMap tmPQo,
              const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ)
 {
-    constexpr int SNA = al32_3(G4<FD, RPT, NW>::SN), SOWN = al32_3(4 * SNA);
     using T = G4<FD, RPT, NW>;
     using Sg = Stage<FD, RPT, NW>;
+    constexpr int SNA = Sg::SNA, SOWN = Sg::SOWN;
     constexpr int K = T::K, SN = T::SN, STG = Sg::ADA, NST = Sg::NADA, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
@@ -1128,7 +1134,6 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
              const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmX,
              const __grid_constant__ CUtensorMap tmZ)
 {
-    constexpr int SNA = al32_3(G4<FD, RPT, NW>::SN), SOWN = al32_3(4 * SNA);
     // one history box per item from [shot][slot * snf + field][nz_dom][nx_dom]
     // at the tile's physical coordinates (cells outside arrive as 0): the
     // carry-in stresses of the exact gradient, or the carry-out ones of the
@@ -1137,6 +1142,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     const bool htma = (EXACT || IMG) && o.hist_tma && hslot >= 0;
     using T = G4<FD, RPT, NW>;
     using Sg = Stage<FD, RPT, NW>;
+    constexpr int SNA = Sg::SNA, SOWN = Sg::SOWN;
     constexpr int K = T::K, SN = T::SN, STG = Sg::ADB, NST = Sg::NADB, PL = T::TZH * TX4;
     extern __shared__ __align__(128) float sm[];
     AdjTab *tab = reinterpret_cast<AdjTab *>(sm + STG * NST);
