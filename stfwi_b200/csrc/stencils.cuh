@@ -205,10 +205,10 @@ __device__ __forceinline__ float2 pair_at(const float *p) { return *reinterpret_
 // constants only when the tile changes.
 //
 // The item's boxes arrive by TMA in a ring of NST stages.  Every warp waits
-// for a stage by itself and counts itself out once it has read it; the last
-// warp out of a stage refills it with the item NST further on.  No barrier
-// joins the warps of a block, and the ring keeps loads in flight across
-// tiles and groups.
+// for a stage by itself and arrives at the stage's second barrier once it has
+// read it; the last warp to arrive refills the stage with the item NST further
+// on.  No barrier joins the warps of a block, and the ring keeps loads in
+// flight across tiles and groups.
 
 struct Cursor {
     int pos, shot;        // tile position, shot
@@ -243,50 +243,37 @@ __device__ __forceinline__ int share(const Work &w, int b) { return b * w.per + 
 
 // ring state in shared memory
 template <int NST> struct Ring {
-    uint64_t full[NST];
-    uint32_t out[NST];      // warps that have left each stage, over all rounds
-    uint32_t issued;        // items issued by this block; DEAD set once a warp gave up
+    uint64_t full[NST];     // a stage's copies have landed
+    uint64_t empty[NST];    // every warp has read the stage
+    uint32_t issued;        // items issued by this block
 };
-constexpr uint32_t RING_DEAD = 1u << 31;
 
-// relaxed: a warp's reads of a stage are complete (their values are in
-// registers) before it counts itself out, and the count orders nothing else;
-// an acquire-release here would wait for the warp's global stores
-__device__ __forceinline__ uint32_t atom_add_cta(uint32_t *p, uint32_t v)
-{
-    uint32_t old;
-    asm volatile("atom.relaxed.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
-    return old;
-}
-__device__ __forceinline__ uint32_t atom_or_cta(uint32_t *p, uint32_t v)
-{
-    uint32_t old;
-    asm volatile("atom.acq_rel.cta.shared::cta.or.b32 %0, [%1], %2;" : "=r"(old) : "r"(smem_u32(p)), "r"(v) : "memory");
-    return old;
-}
-
-// a wait ran out at the block's item `it`: record it, stop further issues,
-// and wait (bounded) for every copy already issued that this warp has not
-// seen land, so that the block never exits under a copy in flight
+// a wait ran out at the block's item `it`: record it and wait (bounded) for
+// every copy issued that this warp has not seen land.  A warp sees land or
+// waits here for all that it issued itself, so the block never exits under a
+// copy in flight; and as this warp leaves no stage from `it` on, the others
+// issue at most one round more.
 template <int NST> __device__ __forceinline__ void ring_abort(Ring<NST> *r, int it, int *status)
 {
     if (threadIdx.x == 0) {
         atomicOr(status, ST_TIMEOUT3);
-        const int n = (int)(atom_or_cta(&r->issued, RING_DEAD) & ~RING_DEAD);
+        const int n = (int)*(volatile uint32_t *)&r->issued;
         for (int k = it; k < n; ++k) mbar_wait_bounded(r->full + k % NST, (k / NST) & 1, WAIT3);
     }
     __syncwarp();
 }
 
-// this warp has read item `it` from its stage: true in lane 0 of the last
-// warp out, which then issues the item NST further on
-template <int NW, int NST> __device__ __forceinline__ bool ring_leave(Ring<NST> *r, int st, bool more)
+// this warp has read its item from stage st (round parity ph): true in lane 0
+// of the last warp out, which then issues the item NST further on.  The
+// arrivals release the warps' reads and the wait, which finds the phase
+// complete, acquires them, so the copy comes after all of them.
+template <int NST> __device__ __forceinline__ bool ring_leave(Ring<NST> *r, int st, int ph, bool more)
 {
     __syncwarp();
-    if (threadIdx.x != 0) return false;
-    const uint32_t old = atom_add_cta(r->out + st, 1u);
-    if (!more || old % NW != NW - 1) return false;
-    return !(atom_add_cta(&r->issued, 1u) & RING_DEAD);
+    if (threadIdx.x != 0 || !more) return false;
+    if (mbar_arrive_pending(r->empty + st) != 1 || !mbar_try_wait(r->empty + st, ph)) return false;
+    asm volatile("red.relaxed.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(&r->issued)) : "memory");
+    return true;
 }
 
 // stage sizes (floats) and ring depths: as many stages as two blocks an SM
@@ -306,7 +293,7 @@ template <int FD, int R, int NW> struct Stage {
     static constexpr int imin(int a, int b) { return a < b ? a : b; }
     static constexpr int NVEL = fit(VEL), NSTR = fit(STR), NADA = fit(ADA), NADB = fit(ADB);
     // stages, coefficient table, ring
-    static constexpr size_t bytes(int floats, int nst) { return (size_t)floats * nst * 4 + sizeof(AdjTab) + 12 * nst + 16; }
+    static constexpr size_t bytes(int floats, int nst) { return (size_t)floats * nst * 4 + sizeof(AdjTab) + 16 * nst + 16; }
 };
 
 // ------------------------------------------------------------- guarded paths
@@ -442,7 +429,10 @@ __device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Curso
     nit = share(w, blockIdx.x + 1) - first;
     const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
     if (lead) {
-        for (int b = 0; b < NST; ++b) { mbar_init(ring->full + b, 1); ring->out[b] = 0; }
+        for (int b = 0; b < NST; ++b) {
+            mbar_init(ring->full + b, 1);
+            mbar_init(ring->empty + b, blockDim.y);
+        }
         ring->issued = min(NST, nit);
         fence_async_shared();
     }
@@ -511,8 +501,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         for (int r = 0; r < RPT; ++r) B[r] = mat_pair(g, m.B, iw + r, jb);
     };
     enter();
-    int st = 0, ph = 0;
     for (int it = 0; it < nit; ++it) {
+        const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
         const int s = c.shot;
         const int4 src = __ldg(sh.pos + s);
         const float *S = sm + st * STG, *own = S + T::S3;   // own: [U, V][TZH][TX4] of the tile's own cells
@@ -593,12 +583,11 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave<NW>(ring, st, it + NST < nit)) {
+        if (ring_leave(ring, st, ph, it + NST < nit)) {
             Cursor u;
             u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
-        if (++st == NST) { st = 0; ph ^= 1; }
         if (c.next(w)) enter();
     }
 }
@@ -663,8 +652,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
     // history rows as float pairs when every pair starts on 8 bytes
     const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;
-    int st = 0, ph = 0;
     for (int it = 0; it < nit; ++it) {
+        const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
         const int s = c.shot;
         const int4 src = __ldg(sh.pos + s);
         const float *S = sm + st * STG, *own = S + T::S2;   // own: [sxx, szz, sxz][TZH][TX4] of the tile's own cells
@@ -815,12 +804,11 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, out.status);
             return;
         }
-        if (ring_leave<NW>(ring, st, it + NST < nit)) {
+        if (ring_leave(ring, st, ph, it + NST < nit)) {
             Cursor u;
             u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
-        if (++st == NST) { st = 0; ph ^= 1; }
         if (r1 > r0) {
             // receivers on this warp's rows, which its own lanes have just written
             __syncwarp();
@@ -938,8 +926,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         for (int r = 0; r < RPT; ++r) Bc[r] = mat_pair(g, m.B, iw + r, jb);
     };
     enter();
-    int st = 0, ph = 0;
     for (int it = 0; it < nit; ++it) {
+        const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
         const int s = c.shot;
         const float *S = sm + st * STG;
         const float *own = S + SOWN;   // [P, Q][TZH][TX4] of the tile's own cells
@@ -1061,12 +1049,11 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave<NW>(ring, st, it + NST < nit)) {
+        if (ring_leave(ring, st, ph, it + NST < nit)) {
             Cursor u;
             u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
-        if (++st == NST) { st = 0; ph ^= 1; }
         if (r1 > r0) {
             // receivers on this warp's rows, whose cells its own lanes have just written
             __syncwarp();
@@ -1249,8 +1236,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             }
     };
     enter();
-    int st = 0, ph = 0;
     for (int it = 0; it < nit; ++it) {
+        const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
         const int s = c.shot;
         const float *S = sm + st * STG;
         const float *own = S + SOWN;             // [ex_a, ez_a, es_a][TZH][TX4] of the tile's own cells
@@ -1487,12 +1474,11 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave<NW>(ring, st, it + NST < nit)) {
+        if (ring_leave(ring, st, ph, it + NST < nit)) {
             Cursor u;
             u.init(w, share(w, blockIdx.x) + it + NST);
             issue(u, st);
         }
-        if (++st == NST) { st = 0; ph ^= 1; }
         if (r1 > r0) {
             // receivers of step n - 1 on this warp's rows, whose cells its own lanes have just written
             __syncwarp();

@@ -34,6 +34,20 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// arrive (release); how many arrivals the phase still lacked before this one
+__device__ __forceinline__ uint32_t mbar_arrive_pending(uint64_t *bar)
+{
+    uint32_t n;
+    asm volatile(
+        "{\n\t.reg .b64 s;\n\t"
+        "mbarrier.arrive.shared::cta.b64 s, [%1];\n\t"
+        "mbarrier.pending_count.b64 %0, s;\n\t}"
+        : "=r"(n)
+        : "r"(smem_u32(bar))
+        : "memory");
+    return n;
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
