@@ -65,7 +65,7 @@ typedef struct {
     int32_t want_gradient;  /* 1: reserve the stress history + accumulators (g_Vs, g_Vp);
                                2: also keep the velocities in the history, for the density
                                gradient g_rho of both modes */
-    int32_t shot_group;     /* longest run of (tile, shot) items of a block (0: automatic) */
+    int32_t shot_group;     /* shots of a tile that a block of a stencil kernel takes (0: automatic) */
     double mem_budget_gb;   /* device memory the handle may use (0: 85% of free) */
     int32_t kernel_variant; /* must be 0 (the library has one stencil-kernel family; other values
                                return STFWI_ERR_UNSUPPORTED) */
@@ -172,16 +172,16 @@ stfwi_status stfwi_kernel_times(stfwi_handle *h, double *out);
 
 /* Tile-schedule autotuner (no counterpart in the reference): times `steps`
  * forward and adjoint steps of the handle's configuration for both tile
- * shapes (64 x 8 and 64 x 16 cells) and several run lengths (the (tile, shot)
- * items of a block, "shots per block", 1-25) with CUDA events around every kernel, and keeps the fastest: one
+ * shapes (64 x 8 and 64 x 16 cells) and several numbers of shots per block
+ * (1-25) with CUDA events around every kernel, and keeps the fastest: one
  * tile shape for fwd_vel, fwd_str and adj_a (they share the receivers' tile
  * lists), one for adj_b, and the shots per block of each of the four
  * stencil kernels (also across later stfwi_set_shots calls); spg_out [4]
  * (optional) receives the shots per block of fwd_vel, fwd_str, adj_a, adj_b,
  * stfwi_tile_rows the tile shapes.  A second stage times whole steps split
  * into chains as the passes will be (stfwi_set_chains) for those picks and
- * for each run length alike for all kernels, and keeps the fastest.  Overwrites the fields
- * and history: call it before the forward whose history a gradient will
+ * for each number of shots alike for all kernels, and keeps the fastest.  Overwrites
+ * the fields and history: call it before the forward whose history a gradient will
  * use.  A descriptor shot_group > 0 overrides the shots per block. */
 stfwi_status stfwi_autotune(stfwi_handle *h, int32_t steps, int32_t *spg_out, void *stream);
 
@@ -194,11 +194,10 @@ stfwi_status stfwi_tile_rows(const stfwi_handle *h, int32_t *rows_out);
 
 /* Chains a forward or adjoint pass may be split into (1-4, default 2; no
  * counterpart in the reference).  The shots never interact, so a pass without
- * sampled timing is recorded as min(chains, shots) independent chains of
- * launches over consecutive shots, on separate streams joined at its end (at
- * the end of each checkpoint segment); their launches overlap on the GPU.  Traces are the
- * same bit for bit; the FP64 sums differ only in the order of their atomic
- * additions. */
+ * sampled timing is recorded as independent chains of launches over consecutive
+ * shots, at most one chain for each run of shots that a block takes, on
+ * separate streams joined at its end; their launches overlap on the GPU.
+ * Traces and gradients are the same bit for bit whatever the chains. */
 stfwi_status stfwi_set_chains(stfwi_handle *h, int32_t chains);
 
 /* Residual preparation that allocates nothing (no counterpart in the

@@ -61,13 +61,15 @@ struct Geo {
     long long txs, tzs;        // floats of one x (z) image of a shot
 };
 
-// a launch's work: every tile (order: tile row << 16 | tile column) of the
-// shots [s0, s1); every block gets `per` items, the first `extra` one more
+// a launch's work: every tile (order: tile row << 16 | tile column) of some
+// shots, in blocks of a run of shots of a tile.  Runs have `base` shots, the
+// first `longer` of them one more, from shot s0 on; the launch takes the `runs`
+// of them from run0 on.
 struct Work {
     const uint32_t *order;
-    int ntx, tiles, s0, s1, per, extra;
-    int part;              // number of the part of the pass that the shots are
+    int ntx, s0, base, longer, runs, run0;
     int single;            // every block has one item
+    __host__ __device__ int first(int q) const { return s0 + q * base + (q < longer ? q : longer); }
 };
 
 // images of the adjoint fields under the transposed C-PML, [shot][2][...]:
@@ -170,7 +172,6 @@ struct AdjOut {
     int slot_img;          // slot of the forward carry-out of this step (imaging), -1 if none
     int slot_next;         // slot of the carry-out of the next step (density imaging term), -1 if none
     int accp;              // accumulator planes per group (5, or 7 with the density terms)
-    int groups, parts;     // accumulator groups, parts of the pass that share them out
     double *acc;           // [groups][accp][nd]: sC, sB, sA (exact), glam, gmu (imaging), gB (exact), g_rho_lame (imaging)
     double *mterm;         // [nshot]: the moment sources' dJ/dL = dJ/dM terms (exact)
     int want_exact, want_img;

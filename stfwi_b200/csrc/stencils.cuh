@@ -200,46 +200,21 @@ __device__ __forceinline__ float2 pair_at(const float *p) { return *reinterpret_
 
 // ------------------------------------------------------------- work and pipeline
 //
-// Work items are (tile, shot) pairs, ordered by tile, within a tile by shot;
-// every block takes an equal, consecutive run of them and reloads a tile's
-// constants only when the tile changes.
+// A block takes a run of shots of one tile (an item is one of them), and
+// loads the tile's constants once.
 //
-// The item's boxes arrive by TMA in a ring of NST stages.  Every warp waits
+// The items' boxes arrive by TMA in a ring of NST stages.  Every warp waits
 // for a stage by itself and arrives at the stage's second barrier once it has
 // read it; the last warp to arrive refills the stage with the item NST further
-// on.  No barrier joins the warps of a block, and the ring keeps loads in
-// flight across tiles and groups.
+// on.  No barrier joins the warps of a block.
 
-struct Cursor {
-    int pos, shot;        // tile position, shot
-    uint32_t cur, ahead;  // this tile (row << 16 | column) and the next, loaded while this one is at work
-    __device__ __forceinline__ int j0() const { return (cur & 0xffffu) * TX4; }
-    __device__ __forceinline__ int i0(int tzh) const { return (cur >> 16) * tzh; }
-    __device__ __forceinline__ int tile(const Work &w) const { return (cur >> 16) * w.ntx + (cur & 0xffffu); }
-    __device__ __forceinline__ void look(const Work &w) { ahead = __ldg(w.order + min(pos + 1, w.tiles - 1)); }
-    __device__ __forceinline__ void init(const Work &w, unsigned item)
-    {
-        const unsigned ns = w.s1 - w.s0;
-        pos = item / ns;
-        shot = w.s0 + (int)(item - pos * ns);
-        cur = __ldg(w.order + pos);
-    }
-    // is this the tile's last shot
-    __device__ __forceinline__ bool last(const Work &w) const { return shot + 1 == w.s1; }
-    // to the next item; true when the tile changes
-    __device__ __forceinline__ bool next(const Work &w)
-    {
-        if (++shot < w.s1) return false;
-        shot = w.s0;
-        ++pos;
-        cur = ahead;
-        look(w);
-        return true;
-    }
+struct Run {
+    uint32_t tile;      // row << 16 | column
+    int q, shot, n;     // number of the run, its first shot, its shots
+    __device__ __forceinline__ int j0() const { return (tile & 0xffffu) * TX4; }
+    __device__ __forceinline__ int i0(int tzh) const { return (tile >> 16) * tzh; }
+    __device__ __forceinline__ int number(const Work &w) const { return (tile >> 16) * w.ntx + (tile & 0xffffu); }
 };
-
-// first item of block b's share
-__device__ __forceinline__ int share(const Work &w, int b) { return b * w.per + min(b, w.extra); }
 
 // ring state in shared memory
 template <int NST> struct Ring {
@@ -415,52 +390,45 @@ __device__ __forceinline__ float2 mat_pair(const Geo &g, const float *a, int i, 
     return *reinterpret_cast<const float2 *>(a + (long long)min(i, g.nz - 1) * g.P + (jb < g.nx ? jb : 0));
 }
 
-// start of a launch: the block's share [first, first + nit) of the items, the
-// ring's barriers, the first NST items on their way (by the first warp's
-// first lane), and meanwhile, by the other warps, the coefficient tables.  All
-// that reads what the launch before wrote comes after the dependency wait:
-// where a launch may start before its predecessor ends, only the part before
-// the wait overlaps.
+// start of a launch: the block's run, the ring's barriers, the first NST items
+// on their way (by the first warp's first lane), and meanwhile, by the other
+// warps, the coefficient tables.  All that reads what the launch before wrote
+// comes after the dependency wait: where a launch may start before its
+// predecessor ends, only the part before the wait overlaps.
 template <int NST, class Issue, class Fill>
-__device__ __forceinline__ bool ring_start(Ring<NST> *ring, const Work &w, Cursor &c, int &nit, Issue issue,
-                                           Fill fill_tab)
+__device__ __forceinline__ void ring_start(Ring<NST> *ring, const Work &w, Run &c, Issue issue, Fill fill_tab)
 {
-    const int first = share(w, blockIdx.x);
-    nit = share(w, blockIdx.x + 1) - first;
+    if (w.single) {
+        // one item a block, the grid being (tile columns, tile rows, shots):
+        // nothing to look up before the first copy can start
+        c.tile = blockIdx.y << 16 | blockIdx.x;
+        c.q = w.run0 + blockIdx.z;
+        c.shot = w.s0 + c.q;
+        c.n = 1;
+    } else {
+        const unsigned pos = blockIdx.x / (unsigned)w.runs;
+        c.tile = __ldg(w.order + pos);
+        c.q = w.run0 + (int)(blockIdx.x - pos * w.runs);
+        c.shot = w.first(c.q);
+        c.n = w.base + (c.q < w.longer ? 1 : 0);
+    }
     const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
     if (lead) {
         for (int b = 0; b < NST; ++b) {
             mbar_init(ring->full + b, 1);
             mbar_init(ring->empty + b, blockDim.y);
         }
-        ring->issued = min(NST, nit);
+        ring->issued = min(NST, c.n);
         fence_async_shared();
-    }
-    if (w.single) {
-        // one item a block, the grid being (tile columns, tile rows, shots):
-        // nothing to look up before the first copy can start
-        nit = 1;
-        c.pos = 0;
-        c.shot = w.s0 + blockIdx.z;
-        c.cur = blockIdx.y << 16 | blockIdx.x;
-    } else {
-        c.init(w, first);
     }
     if (threadIdx.y > 0) fill_tab((threadIdx.y - 1) * TX + threadIdx.x);
     grid_dependency_start();
     grid_dependency_wait();
     if (lead) {
-        issue(c, 0);
 #pragma unroll 1
-        for (int b = 1; b < NST && b < nit; ++b) {
-            Cursor u;
-            u.init(w, first + b);
-            issue(u, b);
-        }
+        for (int b = 0; b < NST && b < c.n; ++b) issue(c.shot + b, b);
     }
-    c.look(w);
     __syncthreads();
-    return nit > 0;
 }
 
 // ------------------------------------------------------------- forward: velocities
@@ -478,32 +446,25 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
     Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
     const int tx = threadIdx.x, ty = threadIdx.y;
-    auto issue = [&](const Cursor &u, int st) {
+    Run c;
+    auto issue = [&](int s, int st) {
         mbar_arrive_expect_tx(ring->full + st, (3 * SN + 2 * PL) * 4);
-        tma_load_4d(sm + st * STG, &tmS, ring->full + st, u.j0() - XO4, u.i0(T::TZH) - K, F_EX, u.shot);
-        tma_load_4d(sm + st * STG + T::S3, &tmUo, ring->full + st, u.j0(), u.i0(T::TZH), F_U, u.shot);
+        tma_load_4d(sm + st * STG, &tmS, ring->full + st, c.j0() - XO4, c.i0(T::TZH) - K, F_EX, s);
+        tma_load_4d(sm + st * STG + T::S3, &tmUo, ring->full + st, c.j0(), c.i0(T::TZH), F_U, s);
     };
-    Cursor c;   // the item at work
-    int nit;
-    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
+    ring_start(ring, w, c, issue, [&](int i) { fill<FD>(tab, g, i); });
     // columns (of the tile) and rows (of this warp) where no slice mask and no
     // C-PML strip applies; the strips are at least K wide, so they hold the
     // masked columns and rows except those below a free surface
-    bool xin = false, zin = false;
-    int jb = 0, iw = 0;
+    const int jb = c.j0() + 2 * tx, iw = c.i0(T::TZH) + ty * RPT;
+    const bool xin = cols_plain(g, c.j0(), g.pad, g.pad);
+    const bool zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
     float2 B[RPT];
-    auto enter = [&]() {
-        jb = c.j0() + 2 * tx;
-        iw = c.i0(T::TZH) + ty * RPT;
-        xin = cols_plain(g, c.j0(), g.pad, g.pad);
-        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) B[r] = mat_pair(g, m.B, iw + r, jb);
-    };
-    enter();
-    for (int it = 0; it < nit; ++it) {
+    for (int r = 0; r < RPT; ++r) B[r] = mat_pair(g, m.B, iw + r, jb);
+    for (int it = 0; it < c.n; ++it) {
         const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
-        const int s = c.shot;
+        const int s = c.shot + it;
         const int4 src = __ldg(sh.pos + s);
         const float *S = sm + st * STG, *own = S + T::S3;   // own: [U, V][TZH][TX4] of the tile's own cells
         float *U = F + ((long long)s * F_N + F_U) * g.fstride;
@@ -583,12 +544,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, ph, it + NST < nit)) {
-            Cursor u;
-            u.init(w, share(w, blockIdx.x) + it + NST);
-            issue(u, st);
-        }
-        if (c.next(w)) enter();
+        if (ring_leave(ring, st, ph, it + NST < c.n)) issue(s + NST, st);
     }
 }
 
@@ -608,36 +564,29 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     FwdTab *tab = reinterpret_cast<FwdTab *>(sm + STG * NST);
     Ring<NST> *ring = reinterpret_cast<Ring<NST> *>(tab + 1);
     const int tx = threadIdx.x, ty = threadIdx.y;
-    auto issue = [&](const Cursor &u, int st) {
+    Run c;
+    auto issue = [&](int s, int st) {
         mbar_arrive_expect_tx(ring->full + st, (2 * SN + 3 * PL) * 4);
-        tma_load_4d(sm + st * STG, &tmV, ring->full + st, u.j0() - XO4, u.i0(T::TZH) - K, F_U, u.shot);
-        tma_load_4d(sm + st * STG + T::S2, &tmSo, ring->full + st, u.j0(), u.i0(T::TZH), F_EX, u.shot);
+        tma_load_4d(sm + st * STG, &tmV, ring->full + st, c.j0() - XO4, c.i0(T::TZH) - K, F_U, s);
+        tma_load_4d(sm + st * STG + T::S2, &tmSo, ring->full + st, c.j0(), c.i0(T::TZH), F_EX, s);
     };
-    Cursor c;
-    int nit;
-    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i); })) return;
-    bool xin = false, zin = false;   // as in st_fwd_vel
-    int jb = 0, iw = 0, r0 = 0, r1 = 0;
+    ring_start(ring, w, c, issue, [&](int i) { fill<FD>(tab, g, i); });
+    const int jb = c.j0() + 2 * tx, iw = c.i0(T::TZH) + ty * RPT;
+    const bool xin = cols_plain(g, c.j0(), g.pad, g.pad);   // as in st_fwd_vel
+    const bool zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
+    const int r0 = rv.tile_start[c.number(w)], r1 = rv.tile_start[c.number(w) + 1];
     float2 ml2m[RPT], ml[RPT], mm[RPT];
     constexpr int RG = ENERGY ? RPT : 1;
     double eacc[RG][2];
-    auto enter = [&]() {
-        jb = c.j0() + 2 * tx;
-        iw = c.i0(T::TZH) + ty * RPT;
-        xin = cols_plain(g, c.j0(), g.pad, g.pad);
-        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? K : g.pad, g.pad);
-        r0 = rv.tile_start[c.tile(w)];
-        r1 = rv.tile_start[c.tile(w) + 1];
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
-            ml[r] = mat_pair(g, m.L, iw + r, jb);
-            mm[r] = mat_pair(g, m.M, iw + r, jb);
-        }
+    for (int r = 0; r < RPT; ++r) {
+        ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
+        ml[r] = mat_pair(g, m.L, iw + r, jb);
+        mm[r] = mat_pair(g, m.M, iw + r, jb);
+    }
 #pragma unroll
-        for (int r = 0; r < RG; ++r) eacc[r][0] = eacc[r][1] = 0.0;
-    };
-    // energy sums of a tile's shots, when the block leaves the tile
+    for (int r = 0; r < RG; ++r) eacc[r][0] = eacc[r][1] = 0.0;
+    // energy sums of the run's shots
     auto leave = [&]() {
         if constexpr (ENERGY) {
 #pragma unroll
@@ -648,13 +597,12 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                         atomicAdd(out.energy + (long long)(iw + r) * g.nx + jb + cc, eacc[r][cc]);
         }
     };
-    enter();
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
     // history rows as float pairs when every pair starts on 8 bytes
     const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;
-    for (int it = 0; it < nit; ++it) {
+    for (int it = 0; it < c.n; ++it) {
         const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
-        const int s = c.shot;
+        const int s = c.shot + it;
         const int4 src = __ldg(sh.pos + s);
         const float *S = sm + st * STG, *own = S + T::S2;   // own: [sxx, szz, sxz][TZH][TX4] of the tile's own cells
         float *sxx = F + ((long long)s * F_N + F_EX) * g.fstride;
@@ -804,11 +752,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, out.status);
             return;
         }
-        if (ring_leave(ring, st, ph, it + NST < nit)) {
-            Cursor u;
-            u.init(w, share(w, blockIdx.x) + it + NST);
-            issue(u, st);
-        }
+        if (ring_leave(ring, st, ph, it + NST < c.n)) issue(s + NST, st);
         if (r1 > r0) {
             // receivers on this warp's rows, which its own lanes have just written
             __syncwarp();
@@ -829,9 +773,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 if (!(isfinite(v0) && isfinite(v1) && isfinite(ex) && isfinite(ez))) atomicOr(out.status, 1);
             }
         }
-        if (c.last(w) || it + 1 == nit) leave();
-        if (c.next(w)) enter();
     }
+    leave();
 }
 
 // ------------------------------------------------------------- adjoint
@@ -880,12 +823,13 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     // C-PML strips these are the strain adjoints themselves; where the box
     // touches a strip, their transposed-C-PML images (adj_b writes them), x
     // and z images separately, and the exz image for x is a plane of its own.
-    auto issue = [&](const Cursor &u, int st) {
-        const bool bx = box_x(g, u.j0()), bz = box_z(g, u.i0(T::TZH), T::TZH, K);
+    Run c;
+    auto issue = [&](int s, int st) {
+        const bool bx = box_x(g, c.j0()), bz = box_z(g, c.i0(T::TZH), T::TZH, K);
         constexpr int PB = SN * 4, OB = 2 * T::TZH * TX4 * 4;
         uint64_t *bar = ring->full + st;
         float *d = sm + st * STG;
-        const int s = u.shot, x = u.j0() - XO4, y = u.i0(T::TZH) - K;
+        const int x = c.j0() - XO4, y = c.i0(T::TZH) - K;
         const int xi = x >= g.jr ? x - g.jr + g.jl : x, yi = y >= g.iba ? y - g.iba + g.ita : y;
         mbar_arrive_expect_tx(bar, (bx || bz ? 4 : 3) * PB + OB);
         if (bx) tma_load_4d(d, &tmX, bar, xi, y, 0, s);
@@ -899,36 +843,24 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         }
         if (bx) tma_load_4d(d + 3 * SNA, &tmX, bar, xi, y, 1, s);
         else if (bz) tma_load_4d(d + 3 * SNA, &tmE, bar, x, y, F_ES, s);
-        tma_load_4d(d + SOWN, &tmPQo, bar, u.j0(), u.i0(T::TZH), F_U, s);
+        tma_load_4d(d + SOWN, &tmPQo, bar, c.j0(), c.i0(T::TZH), F_U, s);
     };
-
-    Cursor c;
-    int nit;
-    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i, 0); })) return;
+    ring_start(ring, w, c, issue, [&](int i) { fill<FD>(tab, g, i, 0); });
     // transposed masks reach 2K - 1 (low edge) and 2K (high edge) cells inwards
     const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
     const float hdtdz = 0.5f * g.dtdz, hdtdx = 0.5f * g.dtdx;
-    bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
-    int jb = 0, iw = 0, r0 = 0, r1 = 0;
+    const int jb = c.j0() + 2 * tx, iw = c.i0(T::TZH) + ty * RPT;
+    const bool xin = cols_plain(g, c.j0(), mlo, mhi);
+    const bool zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
+    const bool bx = box_x(g, c.j0()), bz = box_z(g, c.i0(T::TZH), T::TZH, K);
+    const bool xband = jb < g.nx && (jb < g.jl || jb >= g.jr), zband = iw < g.itb || iw + RPT > g.ibb;
+    const int r0 = rv.tile_start[c.number(w)], r1 = rv.tile_start[c.number(w) + 1];
     float2 Bc[RPT];
-    auto enter = [&]() {
-        jb = c.j0() + 2 * tx;
-        iw = c.i0(T::TZH) + ty * RPT;
-        xin = cols_plain(g, c.j0(), mlo, mhi);
-        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
-        bx = box_x(g, c.j0());
-        bz = box_z(g, c.i0(T::TZH), T::TZH, K);
-        xband = jb < g.nx && (jb < g.jl || jb >= g.jr);
-        zband = iw < g.itb || iw + RPT > g.ibb;
-        r0 = rv.tile_start[c.tile(w)];
-        r1 = rv.tile_start[c.tile(w) + 1];
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) Bc[r] = mat_pair(g, m.B, iw + r, jb);
-    };
-    enter();
-    for (int it = 0; it < nit; ++it) {
+    for (int r = 0; r < RPT; ++r) Bc[r] = mat_pair(g, m.B, iw + r, jb);
+    for (int it = 0; it < c.n; ++it) {
         const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
-        const int s = c.shot;
+        const int s = c.shot + it;
         const float *S = sm + st * STG;
         const float *own = S + SOWN;   // [P, Q][TZH][TX4] of the tile's own cells
         float *Pp = A + ((long long)s * F_N + F_U) * g.fstride;
@@ -1049,11 +981,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, ph, it + NST < nit)) {
-            Cursor u;
-            u.init(w, share(w, blockIdx.x) + it + NST);
-            issue(u, st);
-        }
+        if (ring_leave(ring, st, ph, it + NST < c.n)) issue(s + NST, st);
         if (r1 > r0) {
             // receivers on this warp's rows, whose cells its own lanes have just written
             __syncwarp();
@@ -1082,7 +1010,6 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 }
             }
         }
-        if (c.next(w)) enter();
     }
 }
 
@@ -1137,12 +1064,13 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
     const int tx = threadIdx.x, ty = threadIdx.y;
     // planes as in st_adj_a: P and Q, or their images where the box touches a
     // strip; the z image of P and the x image of Q are planes of their own
-    auto issue = [&](const Cursor &u, int st) {
-        const bool bx = box_x(g, u.j0()), bz = box_z(g, u.i0(T::TZH), T::TZH, K);
+    Run c;
+    auto issue = [&](int s, int st) {
+        const bool bx = box_x(g, c.j0()), bz = box_z(g, c.i0(T::TZH), T::TZH, K);
         constexpr int PB = SN * 4, OB = 3 * T::TZH * TX4 * 4;
         uint64_t *bar = ring->full + st;
         float *d = sm + st * STG;
-        const int s = u.shot, x = u.j0() - XO4, y = u.i0(T::TZH) - K;
+        const int x = c.j0() - XO4, y = c.i0(T::TZH) - K;
         const int xi = x >= g.jr ? x - g.jr + g.jl : x, yi = y >= g.ibb ? y - g.ibb + g.itb : y;
         mbar_arrive_expect_tx(bar, (bx || bz ? 4 : 2) * PB + OB + (htma ? OB : 0));
         if (bx) tma_load_4d(d, &tmX, bar, xi, y, 0, s);
@@ -1155,66 +1083,52 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             if (bx) tma_load_4d(d + 3 * SNA, &tmX, bar, xi, y, 1, s);
             else tma_load_4d(d + 3 * SNA, &tmP, bar, x, y, F_V, s);
         }
-        tma_load_4d(d + SOWN, &tmEo, bar, u.j0(), u.i0(T::TZH), F_EX, s);
+        tma_load_4d(d + SOWN, &tmEo, bar, c.j0(), c.i0(T::TZH), F_EX, s);
         if (htma)
-            tma_load_4d_hint(d + SOWN + Sg::OWN3, &tmH, bar, u.j0() - g.pad, u.i0(T::TZH) - g.z0, hslot * g.snf, s, l2_evict_first());
+            tma_load_4d_hint(d + SOWN + Sg::OWN3, &tmH, bar, c.j0() - g.pad, c.i0(T::TZH) - g.z0, hslot * g.snf, s, l2_evict_first());
     };
-
-    Cursor c;
-    int nit;
-    if (!ring_start(ring, w, c, nit, issue, [&](int i) { fill<FD>(tab, g, i, 1); })) return;
+    ring_start(ring, w, c, issue, [&](int i) { fill<FD>(tab, g, i, 1); });
     const int mlo = max(g.pad, 2 * K - 1), mhi = max(g.pad, 2 * K);
     const float2 dtdx2 = dup2(g.dtdx), dtdz2 = dup2(g.dtdz);
     const bool hist2 = ((g.pad | g.nx_dom) & 1) == 0;   // history pairs start on 8 bytes
     constexpr int RE = EXACT ? RPT : 1, RI = IMG ? RPT : 1;
-    bool xin = false, zin = false, bx = false, bz = false, xband = false, zband = false;
-    int jb = 0, iw = 0, r0 = 0, r1 = 0, sfirst = 0;
+    const int jb = c.j0() + 2 * tx, iw = c.i0(T::TZH) + ty * RPT;
+    const bool xin = cols_plain(g, c.j0(), mlo, mhi);
+    const bool zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
+    const bool bx = box_x(g, c.j0()), bz = box_z(g, c.i0(T::TZH), T::TZH, K);
+    const bool xband = jb < g.nx && (jb < g.jl || jb >= g.jr), zband = iw < g.ita || iw + RPT > g.iba;
+    const int r0 = n > 0 ? rv.tile_start[c.number(w)] : 0, r1 = n > 0 ? rv.tile_start[c.number(w) + 1] : 0;
     float2 ml2m[RPT], ml[RPT], mm[RPT];
-    // sums over the shots that the block takes of this tile in one go, in
-    // FP32; over steps, groups and blocks in FP64 (the reductions of leave()).
-    // The exact gradient sums the carry-in stresses s against the stress
-    // adjoints, sA = sum(s1 sxx_a + s2 szz_a), sB = sum(s2 sxx_a + s1 szz_a),
-    // sC = sum(s3 sxz_a); k_finalize applies the strain-recovery factors.
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
+        ml[r] = mat_pair(g, m.L, iw + r, jb);
+        mm[r] = mat_pair(g, m.M, iw + r, jb);
+    }
+    // sums over the run's shots, in FP32; over steps and runs in FP64 (the
+    // reductions of leave() and k_finalize).  The exact gradient sums the
+    // carry-in stresses s against the stress adjoints, sA = sum(s1 sxx_a + s2
+    // szz_a), sB = sum(s2 sxx_a + s1 szz_a), sC = sum(s3 sxz_a); k_finalize
+    // applies the strain-recovery factors.
     float2 sA[RE], sB[RE], sC[RE], glam[RI], gmu[RI];
     // density terms (history with velocities): dJ/dB of the exact gradient
     // and the rho term of the imaging formula
     constexpr int RB = (EXACT && RHO) ? RPT : 1, RR = (IMG && RHO) ? RPT : 1;
     float2 gB[RB], grl[RR];
-    auto enter = [&]() {
-        jb = c.j0() + 2 * tx;
-        iw = c.i0(T::TZH) + ty * RPT;
-        xin = cols_plain(g, c.j0(), mlo, mhi);
-        zin = rows_plain(g, iw, iw + RPT - 1, g.fs ? 2 * K - 1 : mlo, mhi);
-        bx = box_x(g, c.j0());
-        bz = box_z(g, c.i0(T::TZH), T::TZH, K);
-        xband = jb < g.nx && (jb < g.jl || jb >= g.jr);
-        zband = iw < g.ita || iw + RPT > g.iba;
-        r0 = n > 0 ? rv.tile_start[c.tile(w)] : 0;
-        r1 = n > 0 ? rv.tile_start[c.tile(w) + 1] : 0;
-        sfirst = c.shot;
+    const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-            ml2m[r] = mat_pair(g, m.L2M, iw + r, jb);
-            ml[r] = mat_pair(g, m.L, iw + r, jb);
-            mm[r] = mat_pair(g, m.M, iw + r, jb);
-        }
-        const float2 z = make_float2(0.f, 0.f);
+    for (int r = 0; r < RE; ++r) sA[r] = sB[r] = sC[r] = zero;
 #pragma unroll
-        for (int r = 0; r < RE; ++r) sA[r] = sB[r] = sC[r] = z;
+    for (int r = 0; r < RI; ++r) glam[r] = gmu[r] = zero;
 #pragma unroll
-        for (int r = 0; r < RI; ++r) glam[r] = gmu[r] = z;
+    for (int r = 0; r < RB; ++r) gB[r] = zero;
 #pragma unroll
-        for (int r = 0; r < RB; ++r) gB[r] = z;
-#pragma unroll
-        for (int r = 0; r < RR; ++r) grl[r] = z;
-    };
-    // the tile's sums so far, into a group of FP64 planes: blocks that share a
-    // tile start on shots at least `per` apart and add to groups of their own,
-    // as far as the groups go
+    for (int r = 0; r < RR; ++r) grl[r] = zero;
+    // the run's sums into its group's FP64 planes, to which no other block
+    // adds at these cells: the order of the additions is that of the steps
     auto leave = [&]() {
         if (!EXACT && !IMG) return;
-        const int mine = o.groups / o.parts, k = (sfirst - w.s0) / max(w.per, 1);
-        double *base = o.acc + (long long)(mine > 0 ? w.part * mine + min(k, mine - 1) : 0) * o.accp * g.nd;
+        double *base = o.acc + (long long)c.q * o.accp * g.nd;
 #pragma unroll
         for (int r = 0; r < RPT; ++r)
 #pragma unroll
@@ -1235,10 +1149,9 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 if (IMG && RHO) atomicAdd(acc + 6 * g.nd, (double)f2c(grl[r % RR], cc));
             }
     };
-    enter();
-    for (int it = 0; it < nit; ++it) {
+    for (int it = 0; it < c.n; ++it) {
         const int st = it % NST, ph = it / NST & 1;   // stage, parity of its round
-        const int s = c.shot;
+        const int s = c.shot + it;
         const float *S = sm + st * STG;
         const float *own = S + SOWN;             // [ex_a, ez_a, es_a][TZH][TX4] of the tile's own cells
         const float *hown = own + Sg::OWN3;      // [sxx, szz, sxz][TZH][TX4] of the history slot (htma)
@@ -1474,11 +1387,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
             ring_abort(ring, it, status);
             return;
         }
-        if (ring_leave(ring, st, ph, it + NST < nit)) {
-            Cursor u;
-            u.init(w, share(w, blockIdx.x) + it + NST);
-            issue(u, st);
-        }
+        if (ring_leave(ring, st, ph, it + NST < c.n)) issue(s + NST, st);
         if (r1 > r0) {
             // receivers of step n - 1 on this warp's rows, whose cells its own lanes have just written
             __syncwarp();
@@ -1489,9 +1398,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 inject_strain(g, m, im, A, PX, PZ, s, i, rv.rx[rid], src[2LL * g.nt * g.nrec], src[3LL * g.nt * g.nrec]);
             }
         }
-        if (c.last(w) || it + 1 == nit) leave();
-        if (c.next(w)) enter();
     }
+    leave();
 }
 
 }  // namespace stfwi

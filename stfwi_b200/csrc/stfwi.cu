@@ -73,8 +73,7 @@ struct stfwi_handle {
     float4 *pmx = nullptr, *pmz = nullptr;                 // C-PML per column and row
     float *img = nullptr;                                  // image bands of the adjoint
     Images im{};
-    std::map<const void *, int> resident;                  // blocks of a kernel that the device holds at a time
-    int spgk[4] = {1, 1, 1, 1};   // shots per block of the four stencil kernels
+    int spgk[4] = {0, 0, 0, 0};   // shots per block of the four stencil kernels (0: by runs_of's rule)
     int acc_groups = 1;
     int tuned[4] = {0, 0, 0, 0};  // shots per block chosen by stfwi_autotune (0: default)
 
@@ -161,18 +160,54 @@ struct Plan {
     size_t total() const { return fields + psi + snap + row0 + acc + rec + misc + ckpt; }
 };
 
-// FP64 gradient accumulator groups.  A block adds to a group of its own, so that
-// two passes give the same bits; blocks take runs of at least two shots of a
-// tile where there is work for every SM (acc_in_use), and there one group per two
-// shots is enough.  Where there is not, blocks take single shots: one group for each,
-// and one more for each uneven part; those grids are small (at most 140 MB in
-// all).  Never fewer than a pass has parts.
-int acc_groups_of(const stfwi_desc *d)
+// Shots per block where neither the descriptor nor the tuner says: at most
+// RUN_FWD, or RUN_ADJ_B in adj_b, whose FP32 sums are as long.  Below that, what
+// leaves about two waves of blocks (two blocks an SM), counted over all chains:
+// one shot a block costs the block's start for each (us of modelling 200 steps of
+// 152 x 500, 16-row tiles, FD 8: 13 shots 4848 with runs of one, 4060 with two;
+// 25 shots 7420 with two, 7020 with four), few long blocks leave the device
+// idle at the end (10 shots: 3555 with two, 4864 with three; 17 shots: 5176 with
+// three, 6325 with four).  Just above two whole waves the longer run waits for a
+// third (34 shots in six runs 9635, in seven 8910), hence 2.1.  Longer runs than
+// eight gain little more (us of 60 steps of 16 shots of 304 x 1000: runs of four
+// 4654, eight 4313; 20 steps of 32 shots of 608 x 2000: four 10076, eight 9161,
+// sixteen 8789; 120 of 50 shots of 152 x 500: four 8655, eight 7926, ten 9732).
+constexpr int RUN_FWD = 8, RUN_ADJ_B = 4;
+int default_run(long long items, int sms, int most)
 {
-    const int spg0 = d->shot_group > 0 ? d->shot_group : 2, n = d->max_shots;
-    const long long tiles = ((d->nx_dom + 2LL * d->pad + 63) / 64) * ((d->nz_dom + 2LL * d->pad + 15) / 16);
-    if (tiles * n < 4LL * 2 * 2 * 148) return std::max(1, n + MAX_CHAINS - 1);
-    return std::max(1, std::max((n + spg0 - 1) / spg0, std::min(n, MAX_CHAINS)));
+    const long long slots = 2LL * sms;
+    return (int)std::max(1LL, std::min((long long)most, 10 * (items + slots) / (21 * slots)));
+}
+
+// runs of at most `run` shots that n shots make, as many for each of two chains
+int level_runs(int n, int run)
+{
+    const int runs = (n + run - 1) / run;
+    return runs > 1 ? std::min(n, (runs + 1) / 2 * 2) : 1;
+}
+
+// FP64 gradient accumulator groups, one for each run of shots of adj_b:
+// every block adds to planes of its own, in the order of the steps, so that
+// two passes give the same bits whatever the chains.  One group a shot where
+// the default rule's runs are single shots (at most 60 MB in all: there are fewer
+// than 3.2 tiles and shots for each block that the device holds), else one for
+// two shots; or as many as the descriptor's runs.  `narrow`: one for two shots
+// at most, where memory is short.
+int acc_groups_of(const stfwi_desc *d, int sms, bool narrow)
+{
+    const int n = d->max_shots;
+    if (d->shot_group > 0) return (n + d->shot_group - 1) / d->shot_group;
+    if (narrow) return (n + 1) / 2;
+    const long long rows = d->nz_dom + (d->free_surface ? 1LL : 2LL) * d->pad;
+    const long long tiles = ((d->nx_dom + 2LL * d->pad + TX4 - 1) / TX4) * ((rows + 15) / 16);
+    return level_runs(n, std::min(2, default_run(tiles * n, sms, RUN_ADJ_B)));
+}
+
+int sm_count(int device)
+{
+    int n = 148;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) cudaGetLastError();
+    return n;
 }
 
 // Image bands of the adjoint: the columns (rows) that the boxes of the tiles
@@ -211,8 +246,8 @@ Bands bands_of(long long nz, long long nx, long long P, int pad, int fs, int K)
     return b;
 }
 
-// k: history segment length (k = nt: every step kept, no checkpoints)
-Plan make_plan(const stfwi_desc *d, int k)
+// k: history segment length (k = nt: every step kept, no checkpoints); G: accumulator groups
+Plan make_plan(const stfwi_desc *d, int k, int G)
 {
     Plan p{};
     p.nx = d->nx_dom + 2LL * d->pad;
@@ -222,7 +257,6 @@ Plan make_plan(const stfwi_desc *d, int k)
     p.xs_n = 2LL * d->pad;
     p.zs_n = d->free_surface ? d->pad : 2LL * d->pad;
     const long long S = d->max_shots;
-    const int G = acc_groups_of(d);
     p.fields = (size_t)2 * S * F_N * p.nz * p.P * sizeof(float);
     p.psi = (size_t)S * (NPX * p.nz * p.xs_n + NPZ * p.zs_n * p.P) * sizeof(float);
     const Bands bd = bands_of(p.nz, p.nx, p.P, d->pad, d->free_surface, d->fd_order / 2);
@@ -586,71 +620,70 @@ inline void prof_mark(stfwi_handle *h, int k, int n, int which, cudaStream_t st)
 // are atomic).
 struct Part {
     int index, s0, s1;   // shots [s0, s1)
+    int run0, runs;      // runs of the kernel that the parts were cut by
     bool early;          // its launches may overlap the end of the one before
 };
 
-std::vector<Part> parts_of(const stfwi_handle *h, int parts)
+// Runs that the pass's shots make in kernel k.  A launch has a block for
+// each run on every tile, tiles with guarded paths first: boundary tiles take two
+// to three times as long as interior ones, and it is the hardware's handing
+// out of blocks that levels them.  (A single wave of blocks with a fixed share of
+// the tiles each, the first shares all boundary tiles, took 3292 us for 200
+// steps of one shot of 304 x 1000 and 7439 for 400 of 7 of 152 x 500; this
+// takes 2042 and 5284.)
+int runs_of(const stfwi_handle *h, int k)
 {
-    std::vector<Part> p;
-    const int n = h->nshot;
-    for (int k = 0; k < parts; ++k)
-        p.push_back(Part{k, (int)((long long)n * k / parts), (int)((long long)n * (k + 1) / parts),
-                         h->prof_every == 0});
-    return p;
+    const int n = std::max(1, h->nshot), run = h->spgk[k];
+    const long long items = (long long)h->ntx * (k == 3 ? h->ntzb : h->ntza) * n;
+    const int runs = run > 0 ? (n + run - 1) / run : level_runs(n, default_run(items, h->sms, k == 3 ? RUN_ADJ_B : RUN_FWD));
+    return k == 3 ? std::min(runs, h->acc_groups) : runs;
 }
 
-// the work of a launch of kernel k over a part's shots
-Work work_of(const stfwi_handle *h, int k, const Part &part)
+// n shots in `runs` runs as equal as can be
+void cut_runs(Work &w, int n, int runs)
+{
+    w.base = n / runs;
+    w.longer = n % runs;
+    w.runs = runs;
+}
+
+// parts of a pass, each on a stream of its own, of whole runs of kernel k (adj_b,
+// whose sums then do not depend on the parts, or fwd_str in a forward pass).  One
+// part while sampled timing is on (one event pair per kernel and step).
+std::vector<Part> pass_parts(const stfwi_handle *h, int k)
 {
     Work w{};
+    cut_runs(w, h->nshot, runs_of(h, k));
+    const int parts = h->prof_every != 0 ? 1 : std::min(h->chains, w.runs);
+    std::vector<Part> out;
+    for (int c = 0; c < parts; ++c) {
+        const int a = (int)((long long)w.runs * c / parts), b = (int)((long long)w.runs * (c + 1) / parts);
+        out.push_back(Part{c, w.first(a), w.first(b), a, b - a, h->prof_every == 0});
+    }
+    return out;
+}
+
+// all shots as one part
+Part whole_pass(const stfwi_handle *h) { return Part{0, 0, h->nshot, 0, runs_of(h, 3), h->prof_every == 0}; }
+
+// a launch of kernel k over a part's shots: its work and its grid
+dim3 work_of(const stfwi_handle *h, int k, const Part &part, Work &w)
+{
+    const int ntz = k == 3 ? h->ntzb : h->ntza, tiles = h->ntx * ntz, n = part.s1 - part.s0;
     w.order = k == 3 ? h->tordB : h->tordA;
     w.ntx = h->ntx;
-    w.tiles = h->ntx * (k == 3 ? h->ntzb : h->ntza);
-    w.s0 = part.s0;
-    w.s1 = part.s1;
-    w.part = part.index;
-    return w;
-}
-
-// Blocks of a launch and each block's share of the items: runs of at most
-// `run` shots (h->spgk), but at least one block per slot of the device while
-// there are items enough.  Runs of 5-7 are the best on every grid measured
-// (exact gradient, us a step, forward + adjoint: 50 shots of 172 x 540 cells
-// 88.9 + 123.0 at 3, 81.4 + 119.7 at 5, 85.8 + 132.5 at 10; 16 shots of
-// 324 x 1040 100.0 + 134.7, 90.2 + 129.5, 98.1 + 141.7): shorter runs pay a
-// block's start and the FP64 sums of its tile more often, longer ones leave
-// the last blocks of a launch alone on the device.
-template <typename K> dim3 blocks_of(stfwi_handle *h, K kern, int threads, size_t smem, int run, Work &w)
-{
-    int &n = h->resident[(const void *)kern];
-    if (n == 0) {
-        int per = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess) cudaGetLastError();
-        n = std::max(1, per) * h->sms;
+    if (k == 3) {   // the pass's runs
+        cut_runs(w, h->nshot, runs_of(h, 3));
+        w.run0 = part.run0;
+        w.runs = part.runs;
+    } else {        // runs as long as the pass's, of the part's shots
+        const int all = runs_of(h, k), run = (h->nshot + all - 1) / all;
+        w.s0 = part.s0;
+        cut_runs(w, n, (n + run - 1) / run);
     }
-    const int items = w.tiles * (w.s1 - w.s0);
-    const int blocks = std::max(std::min(items, n), (items + run - 1) / run);
-    w.per = items / blocks;
-    w.extra = items % blocks;
-    w.single = blocks == items;
-    return w.single ? dim3(w.ntx, w.tiles / w.ntx, w.s1 - w.s0) : dim3(blocks);
-}
-
-// parts of a pass, each on a stream of its own.  One part while sampled
-// timing is on (one event pair per kernel and step).
-std::vector<Part> pass_parts(const stfwi_handle *h)
-{
-    return parts_of(h, h->prof_every != 0 ? 1 : std::max(1, std::min(h->chains, h->nshot)));
-}
-
-// groups of accumulator planes a pass uses: one per block that shares a tile
-// of a part, as far as there are any
-int acc_in_use(const stfwi_handle *h, int parts)
-{
-    const int n = (h->nshot + parts - 1) / parts, items = h->ntx * h->ntzb * n;
-    const int blocks = std::max(std::min(items, 2 * h->sms), (items + h->spgk[3] - 1) / h->spgk[3]);
-    const int per = std::max(1, items / blocks);
-    return std::min(h->acc_groups, parts * ((n - 1) / per + 1));
+    // as few items as the device holds need no order
+    w.single = w.base == 1 && w.longer == 0 && (long long)tiles * h->nshot <= 2LL * h->sms;
+    return w.single ? dim3(h->ntx, ntz, n) : dim3((unsigned)tiles * w.runs);
 }
 
 // launch a stencil kernel; early: it may start its prologue before the launch
@@ -675,7 +708,7 @@ void launch_stencil(void (*kern)(P...), dim3 blocks, int warps, size_t smem, cud
 // fills an SM, so only where there is no second one for it
 bool few_items(const stfwi_handle *h, int ntz, const Part &part)
 {
-    return h->ntx * ntz * (part.s1 - part.s0) <= h->sms;
+    return (long long)h->ntx * ntz * (part.s1 - part.s0) <= h->sms;
 }
 
 template <int FD, int R, int NW>
@@ -684,15 +717,14 @@ void launch_fwd_step_r(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st,
     using Sg = Stage<FD, R, NW>;
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
     constexpr size_t bv = Sg::bytes(Sg::VEL, Sg::NVEL), bs = Sg::bytes(Sg::STR, Sg::NSTR);
-    Work w0 = work_of(h, 0, part), w1 = work_of(h, 1, part);
-    const dim3 n0 = blocks_of(h, st_fwd_vel<FD, R, NW>, TX * NW, bv, h->spgk[0], w0);
+    Work w0{}, w1{};
+    const dim3 n0 = work_of(h, 0, part, w0), n1 = work_of(h, 1, part, w1);
     prof_mark(h, 0, n, 0, st);
     launch_stencil(st_fwd_vel<FD, R, NW>, n0, NW, bv, st, part.early, h->g, mat_of(h), shots_of(h), h->F, h->PX, h->PZ, n, w0,
                    h->status, h->tmS, h->tmUo);
     prof_mark(h, 0, n, 1, st);
     prof_mark(h, 1, n, 0, st);
     auto str = o.energy ? st_fwd_str<FD, R, NW, true> : st_fwd_str<FD, R, NW, false>;
-    const dim3 n1 = blocks_of(h, str, TX * NW, bs, h->spgk[1], w1);
     launch_stencil(str, n1, NW, bs, st, part.early, h->g, mat_of(h), shots_of(h), rva, h->F, h->PX, h->PZ, n, w1, o, h->tmV,
                    h->tmSo);
     prof_mark(h, 1, n, 1, st);
@@ -712,8 +744,8 @@ void launch_adj_a_r(stfwi_handle *h, int n, const AdjIn &ai, cudaStream_t st, co
     using Sg = Stage<FD, R, NW>;
     Recv rva{h->tile_startA, h->tile_recA, h->rx, h->rz};
     constexpr size_t bytes = Sg::bytes(Sg::ADA, Sg::NADA);
-    Work w = work_of(h, 2, part);
-    const dim3 nb = blocks_of(h, st_adj_a<FD, R, NW>, TX * NW, bytes, h->spgk[2], w);
+    Work w{};
+    const dim3 nb = work_of(h, 2, part, w);
     launch_stencil(st_adj_a<FD, R, NW>, nb, NW, bytes, st, part.early, h->g, mat_of(h), rva, h->A, h->PX, h->PZ, h->im, n, w, ai,
                    h->status, h->tmE, h->tmPQo, h->tmXa, h->tmZa);
 }
@@ -724,9 +756,9 @@ void launch_adj_b_r(stfwi_handle *h, int n, const AdjOut &ao, cudaStream_t st, c
     using Sg = Stage<FD, R, NW>;
     Recv rvb{h->tile_startB, h->tile_recB, h->rx, h->rz};
     constexpr size_t bytes = Sg::bytes(Sg::ADB, Sg::NADB);
-    Work w = work_of(h, 3, part);
+    Work w{};
+    const dim3 nb = work_of(h, 3, part, w);
     auto launch = [&](auto kern) {
-        const dim3 nb = blocks_of(h, kern, TX * NW, bytes, h->spgk[3], w);
         launch_stencil(kern, nb, NW, bytes, st, part.early, h->g, mat_of(h), shots_of(h), rvb, h->A, h->PX, h->PZ, h->im, n, w,
                        ao, h->status, h->tmP, h->tmEo, h->tmH, h->tmXb, h->tmZb);
     };
@@ -835,11 +867,11 @@ void fwd_step(stfwi_handle *h, int n, const FwdOut &o, cudaStream_t st, const Pa
     }
 }
 
-// run fn(part, stream) for every part: their streams fork off `st` and join
+// run fn(part, stream) for every part of whole runs of kernel k: their streams fork off `st` and join
 // it again (event edges of a captured graph)
-template <class Fn> stfwi_status run_parts(stfwi_handle *h, cudaStream_t st, Fn fn)
+template <class Fn> stfwi_status run_parts(stfwi_handle *h, int k, cudaStream_t st, Fn fn)
 {
-    const std::vector<Part> parts = pass_parts(h);
+    const std::vector<Part> parts = pass_parts(h, k);
     const int lanes = (int)parts.size();
     if (lanes > 1) CK(h, cudaEventRecord(h->ev_fork, st));
     for (int c = 1; c < lanes; ++c) CK(h, cudaStreamWaitEvent(h->hsx[c - 1], h->ev_fork, 0));
@@ -871,7 +903,7 @@ stfwi_status enqueue_forward(stfwi_handle *h, uint32_t flags, int comp, cudaStre
     // with checkpoints the history is written later, segment by segment
     const bool hist = store && h->ncp == 0;
     const bool ckpt = store && h->ncp > 0;
-    rc = run_parts(h, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
+    rc = run_parts(h, 1, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
         if (hist) snap_state(h, p, s);
         for (int n = 0; n < h->g.nt; ++n) {
             if (ckpt && n % h->ck == 0) {
@@ -1049,10 +1081,10 @@ stfwi_status setup_tensor_maps(stfwi_handle *h)
     return STFWI_OK;
 }
 
-// shots per block of each stencil kernel
+// shots per block of each stencil kernel (0: by runs_of's rule)
 void set_groups(stfwi_handle *h, const int spg[4])
 {
-    for (int k = 0; k < 4; ++k) h->spgk[k] = std::max(1, spg[k]);
+    for (int k = 0; k < 4; ++k) h->spgk[k] = spg[k];
 }
 
 }  // namespace
@@ -1292,7 +1324,9 @@ size_t stfwi_workspace_bytes(const stfwi_desc *d)
 {
     if (!d || d->nt < 1) return 0;
     const int k = d->ckpt_interval > 0 ? std::min(d->ckpt_interval, d->nt) : d->nt;
-    return make_plan(d, k).total();
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return make_plan(d, k, acc_groups_of(d, sm_count(dev), false)).total();
 }
 
 const char *stfwi_last_error(const stfwi_handle *h) { return h ? h->err.c_str() : "null handle"; }
@@ -1321,17 +1355,20 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     // history plan: every step if it fits, else the longest checkpoint
     // segment that fits (the recompute costs one forward whatever k is)
     int k = d->nt;
+    h->sms = sm_count(h->device);
+    h->acc_groups = acc_groups_of(d, h->sms, false);
     if (d->want_gradient) {
-        if (d->ckpt_interval > 0) {
-            k = std::min(d->ckpt_interval, d->nt);
-        } else if ((double)make_plan(d, d->nt).total() > budget) {
+        if (d->ckpt_interval > 0) k = std::min(d->ckpt_interval, d->nt);
+        // fewer groups before fewer steps
+        if ((double)make_plan(d, k, h->acc_groups).total() > budget) h->acc_groups = acc_groups_of(d, h->sms, true);
+        if (d->ckpt_interval <= 0 && (double)make_plan(d, k, h->acc_groups).total() > budget) {
             k = 0;
             for (int kk = d->nt - 1; kk >= 1; --kk)
-                if ((double)make_plan(d, kk).total() <= budget) { k = kk; break; }
+                if ((double)make_plan(d, kk, h->acc_groups).total() <= budget) { k = kk; break; }
             if (k == 0) k = 1;
         }
     }
-    Plan p = make_plan(d, k);
+    Plan p = make_plan(d, k, h->acc_groups);
     h->ck = k;
     h->ncp = (d->want_gradient && k < d->nt) ? (d->nt + k - 1) / k : 0;
     if ((double)p.total() > budget) {
@@ -1358,7 +1395,6 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     h->tw = TX4;
     h->ntx = (int)((p.nx + h->tw - 1) / h->tw);
     h->ntz_max = (int)((p.nz + RPT_MIN * NWARP - 1) / (RPT_MIN * NWARP));
-    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
     {
         stfwi_status r = STFWI_OK;
         switch (d->fd_order) {
@@ -1367,7 +1403,6 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
         default: r = setup_tma_kernels<8>(h); break;
         }
         if (r) { delete h; return r; }
-        h->acc_groups = acc_groups_of(d);
     }
     h->slots = k + 1 + ((g.snf == 5 && h->ncp > 0) ? 1 : 0);
 
@@ -1580,10 +1615,8 @@ stfwi_status stfwi_set_shots(stfwi_handle *h, int32_t nshot, const int32_t *src,
     h->nshot = nshot;
     g.nshot = nshot;
     {
-        static const int dflt4[4] = {6, 6, 6, 6};   // see blocks_of
         int spg[4];
-        for (int k = 0; k < 4; ++k)
-            spg[k] = h->d.shot_group > 0 ? h->d.shot_group : h->tuned[k] > 0 ? h->tuned[k] : dflt4[k];
+        for (int k = 0; k < 4; ++k) spg[k] = h->d.shot_group > 0 ? h->d.shot_group : h->tuned[k];
         set_groups(h, spg);
     }
     h->shots_set = true;
@@ -1689,7 +1722,7 @@ stfwi_status stfwi_gradient(stfwi_handle *h, uint32_t mode, double *g_out, float
     float *src_dev = sr ? h->src_a : nullptr;
     GraphKey key{1, mode, h->nshot};
     rc = run_graph(h, key, st, [&](cudaStream_t s) {
-        const int parts = (int)pass_parts(h).size(), groups = acc_in_use(h, parts);
+        const int groups = runs_of(h, 3);
         stfwi_status r = zero_adjoint_state(h, groups, s);
         if (r) return r;
         const int thr = 256;
@@ -1702,7 +1735,7 @@ stfwi_status stfwi_gradient(stfwi_handle *h, uint32_t mode, double *g_out, float
             ai.accLr = h->accLr; ai.want_exact = ex;
             AdjOut ao{};
             ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = n - seg0; ao.slot_img = n - seg0 + 1;
-            ao.accp = h->accp; ao.groups = groups; ao.parts = parts; ao.mterm = h->mterm;
+            ao.accp = h->accp; ao.mterm = h->mterm;
             // outputs of step n + 1: the next slot inside a segment, else the
             // extra slot filled from the following segment (checkpoints)
             ao.slot_next = (n + 1 < seg1) ? n - seg0 + 2 : (h->ncp > 0 && n + 1 < g.nt ? h->ck + 1 : -1);
@@ -1714,7 +1747,7 @@ stfwi_status stfwi_gradient(stfwi_handle *h, uint32_t mode, double *g_out, float
             default: launch_adj_step<8>(h, n, ai, ao, as, part); break;
             }
         };
-        r = run_parts(h, s, [&](const Part &p, cudaStream_t ps) -> stfwi_status {
+        r = run_parts(h, 3, s, [&](const Part &p, cudaStream_t ps) -> stfwi_status {
             if (!((ex || im) && h->ncp > 0)) {
                 for (int n = g.nt - 1; n >= 0; --n) adj(n, 0, g.nt, ps, p);
                 return STFWI_OK;
@@ -1965,12 +1998,11 @@ static stfwi_status enqueue_timing_steps(stfwi_handle *h, int steps, cudaStream_
 {
     const Geo &g = h->g;
     stfwi_status r;
-    const int parts = (int)pass_parts(h).size(), groups = acc_in_use(h, parts);
-    if ((r = zero_forward_state(h, st)) || (r = zero_adjoint_state(h, groups, st))) return r;
+    if ((r = zero_forward_state(h, st)) || (r = zero_adjoint_state(h, runs_of(h, 3), st))) return r;
     FwdOut o{};
     o.rec = h->rec; o.status = h->status; o.slots = h->slots;
     const bool ex = h->snap != nullptr;
-    return run_parts(h, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
+    return run_parts(h, 3, st, [&](const Part &p, cudaStream_t s) -> stfwi_status {
         for (int n = 0; n < steps; ++n) fwd_step(h, n, o, s, p);
         for (int n = steps - 1; n >= 0; --n) {
             AdjIn ai{};
@@ -1978,7 +2010,7 @@ static stfwi_status enqueue_timing_steps(stfwi_handle *h, int steps, cudaStream_
             ai.accLr = h->accLr; ai.want_exact = ex && g.fs;
             AdjOut ao{};
             ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = 0; ao.slot_img = h->slots > 1 ? 1 : -1;
-            ao.slot_next = -1; ao.accp = h->accp; ao.groups = groups; ao.parts = parts; ao.mterm = h->mterm; ao.acc = h->acc;
+            ao.slot_next = -1; ao.accp = h->accp; ao.mterm = h->mterm; ao.acc = h->acc;
             ao.want_exact = ex; ao.want_img = 0; ao.rec_adj = h->rec_adj; ao.hist_tma = h->hist_tma ? 1 : 0;
             switch (h->d.fd_order) {
             case 2: launch_adj_step<2>(h, n, ai, ao, s, p); break;
@@ -2193,7 +2225,7 @@ stfwi_status stfwi_forward_frames(stfwi_handle *h, uint32_t fields, float *frame
     o.status = h->status;
     o.slots = h->slots;
     const dim3 grid((unsigned)((N + 255) / 256), h->nshot);
-    const Part all = parts_of(h, 1)[0];
+    const Part all = whole_pass(h);
     for (int n = 0; n < g.nt; ++n) {
         fwd_step(h, n, o, st, all);
         k_frames_fwd<<<grid, 256, 0, st>>>(g, mat_of(h), h->F, fields, nf, stage);
@@ -2240,14 +2272,14 @@ stfwi_status stfwi_adjoint_frames(stfwi_handle *h, uint32_t fields, float *frame
     const unsigned nrb = (unsigned)((g.nshot * std::max(g.nrec, 1) + thr - 1) / thr);
     if (g.nrec > 0) k_inject_last<<<nrb, thr, 0, st>>>(g, mat_of(h), h->im, h->rx, h->rz, h->rec_adj, h->A, h->PX, h->PZ);
     const dim3 grid((unsigned)((N + 255) / 256), h->nshot);
-    const Part all = parts_of(h, 1)[0];
+    const Part all = whole_pass(h);
     for (int n = g.nt - 1; n >= 0; --n) {
         AdjIn ai{};
         ai.rec_adj = h->rec_adj; ai.row0 = h->row0; ai.slots = h->slots; ai.slot = 0;
         ai.accLr = h->accLr; ai.want_exact = 0;
         AdjOut ao{};
         ao.snap = h->snap; ao.slots = h->slots; ao.slot_in = -1; ao.slot_img = -1; ao.slot_next = -1;
-        ao.accp = h->accp; ao.groups = 1; ao.parts = 1; ao.acc = h->acc; ao.src_a = h->src_a; ao.rec_adj = h->rec_adj;
+        ao.accp = h->accp; ao.acc = h->acc; ao.src_a = h->src_a; ao.rec_adj = h->rec_adj;
         switch (h->d.fd_order) {
         case 2: launch_adj_step<2>(h, n, ai, ao, st, all); break;
         case 4: launch_adj_step<4>(h, n, ai, ao, st, all); break;

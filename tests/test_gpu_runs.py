@@ -74,3 +74,25 @@ def test_runs_of_shots_vs_oracle(fd, fs, tiles):
         errs["exact_" + name] = _rel(g["exact"][k], exact[k])
         errs["img_" + name] = _rel(g["imaging"][k], imaging[k])
     assert all(e < tol for e in errs.values()), (tol, errs)
+
+
+@pytest.mark.parametrize("group", [0, 1, 7])
+@pytest.mark.parametrize("density", [False, True])
+def test_gradients_repeat_bit_for_bit(group, density):
+    """Every block's FP32 sums go to FP64 planes of its own, step by step: a
+    second pass, and a pass in another number of chains, gives the same bits,
+    for the default runs, for runs of one shot and for long ones."""
+    fd, fs = 8, True
+    obs = _case(fd, fs)[4].astype(np.float32)
+    S = _solver(fd, fs, density=density, shot_group=group)
+    out = []
+    for chains in (2, 2, 1, 3, 4):
+        S.set_chains(chains)
+        S.forward(store=True)
+        S.misfit(obs, 1, 1.0)
+        g = S.gradient(exact=True, imaging=True)
+        out.append((S.records(), g["exact"], g["imaging"]))
+    S.close()
+    for k in range(1, len(out)):
+        for a, b in zip(out[0], out[k]):
+            assert np.array_equal(a, b), k
