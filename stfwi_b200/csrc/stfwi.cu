@@ -620,6 +620,7 @@ inline void prof_mark(stfwi_handle *h, int k, int n, int which, cudaStream_t st)
 // are atomic).
 struct Part {
     int index, s0, s1;   // shots [s0, s1)
+    int most;            // shots of the pass's longest part
     int run0, runs;      // runs of the kernel that the parts were cut by
     bool early;          // its launches may overlap the end of the one before
 };
@@ -656,15 +657,18 @@ std::vector<Part> pass_parts(const stfwi_handle *h, int k)
     cut_runs(w, h->nshot, runs_of(h, k));
     const int parts = h->prof_every != 0 ? 1 : std::min(h->chains, w.runs);
     std::vector<Part> out;
+    int most = 0;
     for (int c = 0; c < parts; ++c) {
         const int a = (int)((long long)w.runs * c / parts), b = (int)((long long)w.runs * (c + 1) / parts);
-        out.push_back(Part{c, w.first(a), w.first(b), a, b - a, h->prof_every == 0});
+        out.push_back(Part{c, w.first(a), w.first(b), 0, a, b - a, h->prof_every == 0});
+        most = std::max(most, out[c].s1 - out[c].s0);
     }
+    for (Part &p : out) p.most = most;
     return out;
 }
 
 // all shots as one part
-Part whole_pass(const stfwi_handle *h) { return Part{0, 0, h->nshot, 0, runs_of(h, 3), h->prof_every == 0}; }
+Part whole_pass(const stfwi_handle *h) { return Part{0, 0, h->nshot, h->nshot, 0, runs_of(h, 3), h->prof_every == 0}; }
 
 // a launch of kernel k over a part's shots: its work and its grid
 dim3 work_of(const stfwi_handle *h, int k, const Part &part, Work &w)
@@ -705,10 +709,13 @@ void launch_stencil(void (*kern)(P...), dim3 blocks, int warps, size_t smem, cud
 }
 
 // 16-row tiles by 16 warps of one row each instead of 8 of two: one block then
-// fills an SM, so only where there is no second one for it
+// fills an SM, so only where no launch of the pass has a second one for it.  The
+// chains' launches need not be counted together: us of modelling 200 steps of two
+// shots of 152 x 500 in two chains, 99 tiles each, 1583 with 16 warps, 1945 with 8;
+// but all chains alike (three shots: 2071 with 8, 2173 with both).
 bool few_items(const stfwi_handle *h, int ntz, const Part &part)
 {
-    return (long long)h->ntx * ntz * (part.s1 - part.s0) <= h->sms;
+    return (long long)h->ntx * ntz * part.most <= h->sms;
 }
 
 template <int FD, int R, int NW>
