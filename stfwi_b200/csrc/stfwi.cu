@@ -527,7 +527,20 @@ cudaError_t launch_misfit(const Geo &g, int comp, int n_taper, const SosParams &
                           cudaStream_t st)
 {
     const int n = g.nshot * g.nrec;
-    cudaError_t e = cudaMemsetAsync(rec_adj, 0, (size_t)g.nshot * 4 * g.nt * g.nrec * sizeof(float), st);
+    // the other components' cotangents are zero.  Component `comp` stays: where a
+    // caller gives the traces' own array as rec_adj, it holds the traces until the
+    // kernel, a trace a thread, writes their cotangents over them.
+    const size_t plane = (size_t)g.nt * g.nrec * sizeof(float), pitch = 4 * plane;
+    auto zero = [&](int c0, int c1) -> cudaError_t {
+        char *p = reinterpret_cast<char *>(rec_adj) + c0 * plane;
+        if (c0 == c1) return cudaSuccess;
+        if (pitch <= INT32_MAX) return cudaMemset2DAsync(p, pitch, 0, (c1 - c0) * plane, g.nshot, st);
+        cudaError_t e = cudaSuccess;
+        for (int s = 0; s < g.nshot && e == cudaSuccess; ++s) e = cudaMemsetAsync(p + s * pitch, 0, (c1 - c0) * plane, st);
+        return e;
+    };
+    cudaError_t e = zero(0, comp);
+    if (e == cudaSuccess) e = zero(comp + 1, 4);
     if (e != cudaSuccess) return e;
     auto go = [&](auto kern) {
         kern<<<(n + 31) / 32, 32, 0, st>>>(g, comp, n_taper, sp, scale, nnorm, rec, obs, rec_adj, mis_trace);

@@ -98,3 +98,32 @@ def test_noalloc_rejects_oversized_batches():
     st = lib.stfwi_misfit_noalloc(100, 10, too_many, buf.data_ptr(), buf.data_ptr(), ct.byref(d),
                                   buf.data_ptr(), buf.data_ptr(), None)
     assert st == N.STFWI_ERR_INVALID
+
+
+@pytest.mark.parametrize("comp", [0, 1, 3])
+def test_noalloc_in_place(comp):
+    """The traces' own array as rec_adj: the cotangents take the traces'
+    place, with the bits that a separate array gets."""
+    import torch
+
+    from stfwi_b200 import _native as N
+
+    torch.cuda.init()
+    lib = N.load()
+    ns, nt, nrec = 3, 37, 21      # 63 traces: a block of 32 and one with a lane to spare
+    g = torch.Generator(device="cuda").manual_seed(comp)
+    pred = torch.randn(ns, 4, nt, nrec, generator=g, device="cuda")
+    obs = torch.randn(ns, nt, nrec, generator=g, device="cuda")
+    sos = np.array([[0.2, 0.3, 0.2, 1.0, -0.5, 0.2]])
+    out = []
+    for adj in (torch.full_like(pred, float("nan")), pred.clone()):
+        src = pred if len(out) == 0 else adj
+        mis = torch.zeros(ns, dtype=torch.float64, device="cuda")
+        d, keep = _desc(N, comp, 1.5, sos, 5, 0)
+        st = lib.stfwi_misfit_noalloc(ns, nt, nrec, src.data_ptr(), obs.data_ptr(), ct.byref(d), adj.data_ptr(),
+                                      mis.data_ptr(), ct.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0
+        out.append((adj, mis))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    rest = [c for c in range(4) if c != comp]
+    assert out[0][0][:, comp].abs().max() > 0 and (out[0][0][:, rest] == 0).all()
