@@ -276,7 +276,8 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
     uint64_t *empty = full + ROW_STAGES;
     uint64_t *wfull = empty + ROW_STAGES;
     uint64_t *done = wfull + 1, *drained = done + ROW_ACC;   // per accumulator: complete; read by the epilogue
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(drained + ROW_ACC);
+    uint64_t *idle = drained + ROW_ACC;                      // every MMA issued is complete
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(idle + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_w = g.w / 128;
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
             mbar_init(&empty[s], 1);
         }
         mbar_init(wfull, 1);
+        mbar_init(idle, 1);
         for (int s = 0; s < ROW_ACC; ++s) {
             mbar_init(&done[s], 1);
             mbar_init(&drained[s], 4);
@@ -321,16 +323,19 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
                 for (int dx = 0; dx < 3 && ok; ++dx)
                     for (int c = 0; c < nkc && ok; ++c) {
                         ok = round == 0 || mbar_wait_bounded(&empty[s], (round - 1) & 1, NN_WAIT);
-                        if (ok) {
-                            mbar_arrive_expect_tx(&full[s], a_bytes);
-                            tma_load_4d(base + s * a_bytes, &tmX, &full[s], c * KC, w0 + dx - 1, r, img);
-                        }
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(&full[s], a_bytes);
+                        tma_load_4d(base + s * a_bytes, &tmX, &full[s], c * KC, w0 + dx - 1, r, img);
                         if (++s == g.stages) {
                             s = 0;
                             ++round;
                         }
                     }
             if (!ok) atomicExch(err, 1);
+            // the CTA does not end under a copy in flight, whoever gave up
+            mbar_wait_bounded(wfull, 0, NN_WAIT);
+            for (int i = 0; i < g.stages; ++i)
+                if (i < s || round > 0) mbar_wait_bounded(&full[i], (i < s ? round : round - 1) & 1, NN_WAIT);
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
                 if (ok && r - 1 >= h0) umma_commit(&done[(r - 1 - h0) % ROW_ACC]);
             }
             if (!ok) atomicExch(err, 2);
+            umma_commit(idle);
         }
         __syncwarp();
     } else {
@@ -413,6 +419,7 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
     tmem_fence_before();
     __syncthreads();
     if (warp == 0) {
+        mbar_wait_bounded(idle, 0, NN_WAIT);   // nor under an MMA
         tmem_fence_after();
         tmem_dealloc(tmem, ncols);
     }
@@ -525,7 +532,6 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
                         umma_bf16(tmem, ad, bd, idesc, (kb | k) != 0);
                     }
                     umma_commit(&empty[s]);
-                    if (kb + 1 == nk) umma_commit(done);
                 }
             }
             if (__shfl_sync(0xffffffffu, fail, 0)) break;
@@ -534,6 +540,9 @@ __global__ void __launch_bounds__(PIPE_THREADS, 1)
                 ++round;
             }
         }
+        // also where a wait gave up: the accumulators are freed once the MMAs issued are complete
+        if (lane == 0) umma_commit(done);
+        __syncwarp();
     } else {
         const bool ok = mbar_wait_bounded(done, 0, NN_WAIT);
         if (!ok && lane == 0) atomicExch(err, 13);
@@ -1016,7 +1025,7 @@ ConvPlan conv_plan(int n, int h, int w, int cin, int cout, int kc)
     for (int bn = 128; bn >= 16 && w % 128 == 0; bn -= 16) {
         if (cout % bn || (bn < cout && bn < 64)) continue;
         const size_t fixed = 1024 + ((9 * (cin / kc) * bn * aw + 1023) & ~(size_t)1023) +
-                             (2 * ROW_STAGES + 1 + 2 * ROW_ACC) * 8 + 16;
+                             (2 * ROW_STAGES + 2 + 2 * ROW_ACC) * 8 + 8;
         const size_t cols = tmem_cols_for(ROW_ACC * bn);
         for (int occ = 4; occ >= 1; occ >>= 1) {
             // as many CTAs per SM as tensor memory and shared memory hold
