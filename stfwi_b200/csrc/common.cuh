@@ -42,7 +42,7 @@ struct Geo {
     int nz, nx, P;             // padded grid and row pitch (floats)
     int nz_dom, nx_dom, z0, pad;
     int fs;                    // free surface
-    int xs_n, zs_n;            // strip widths: 2*pad columns, pad or 2*pad rows
+    int xs_n, zs_n;            // memories of a row in the x strips: 2*pad columns and one that stays 0; rows of the z strips: pad or 2*pad
     int nt, nrec, nshot;
     float dtdx, dtdz, dzdx, dt;
     float inv2dx, inv2dz;      // 1/(2 dx), 1/(2 dz) (imaging condition)

@@ -290,10 +290,12 @@ __device__ __forceinline__ bool rows_plain(const Geo &g, int a, int b, int lo, i
     return a >= lo && b < g.nz - hi;
 }
 
-// x-strip indices of columns jb, jb + 1 (-1 outside the strips and the grid)
+// x-strip indices of columns jb, jb + 1; outside the strips and the grid the
+// index of the row's last memory, which stays zero
 __device__ __forceinline__ int2 xstrip_pair(const Geo &g, int jb)
 {
-    return make_int2(jb < g.nx ? xstrip_index(g, jb) : -1, jb + 1 < g.nx ? xstrip_index(g, jb + 1) : -1);
+    const int a = jb < g.nx ? xstrip_index(g, jb) : -1, b = jb + 1 < g.nx ? xstrip_index(g, jb + 1) : -1;
+    return make_int2(a < 0 ? g.xs_n - 1 : a, b < 0 ? g.xs_n - 1 : b);
 }
 
 // a 16-byte C-PML entry (constant during a launch)
@@ -307,8 +309,8 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 template <int RPT>
 __device__ __forceinline__ void prefetch_x(const Geo &g, int iw, int2 xs, const float *a, const float *b)
 {
-    const int x = max(xs.x, xs.y);
-    if (x < 0) return;
+    const int x = min(xs.x, xs.y);
+    if (x == g.xs_n - 1) return;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
         const int o = min(iw + r, g.nz - 1) * g.xs_n + x;
@@ -327,20 +329,18 @@ __device__ __forceinline__ void prefetch_z(const Geo &g, int iw, int jb, const f
         prefetch_l1(b + zs * g.P + jb);
     }
 }
-// a row's memories of the columns jb, jb + 1 in an x strip.  Columns outside
-// the strips load some valid element: their coefficients are (0, 0, 1).
-__device__ __forceinline__ float2 mem_x(const float *row, int2 xs)
-{
-    return make_float2(row[max(xs.x, 0)], row[max(xs.y, 0)]);
-}
+// a row's memories of the columns jb, jb + 1 in an x strip.  Outside the strips
+// the coefficients are (0, 0, 1) and the memory 0, not some other column's: that
+// could be infinite, and 0 times it is no zero.
+__device__ __forceinline__ float2 mem_x(const float *row, int2 xs) { return make_float2(row[xs.x], row[xs.y]); }
 
 // C-PML of a pair of x-derivatives on one row (c0, c1: the columns' (b, a, 1/k),
 // old: their memories, p: the memory's row) / of z-derivatives (p: the pair's memory)
-__device__ __forceinline__ void pml_x2(float2 &d, const float4 &c0, const float4 &c1, int2 xs, float2 old, float *p)
+__device__ __forceinline__ void pml_x2(const Geo &g, float2 &d, const float4 &c0, const float4 &c1, int2 xs, float2 old, float *p)
 {
     const float p0 = c0.x * old.x + c0.y * d.x, p1 = c1.x * old.y + c1.y * d.y;
-    if (xs.x >= 0) p[xs.x] = p0;
-    if (xs.y >= 0) p[xs.y] = p1;
+    if (xs.x < g.xs_n - 1) p[xs.x] = p0;
+    if (xs.y < g.xs_n - 1) p[xs.y] = p1;
     d = make_float2(d.x * c0.z + p0, d.y * c1.z + p1);
 }
 __device__ __forceinline__ void pml_z2(float2 &d, const float4 &zc, float2 old, float *p)
@@ -350,10 +350,10 @@ __device__ __forceinline__ void pml_z2(float2 &d, const float4 &zc, float2 old, 
     d = fma2(d, dup2(zc.z), pn);
 }
 // transposed C-PML of a pair (the memory kept as phi = psi / (dt / d)): x' = (1/k + a) x + a phi, phi' = b (x + phi)
-__device__ __forceinline__ void adj_x2(float2 &v, const float4 &c0, const float4 &c1, int2 xs, float2 phi, float *p)
+__device__ __forceinline__ void adj_x2(const Geo &g, float2 &v, const float4 &c0, const float4 &c1, int2 xs, float2 phi, float *p)
 {
-    if (xs.x >= 0) p[xs.x] = c0.x * (v.x + phi.x);
-    if (xs.y >= 0) p[xs.y] = c1.x * (v.y + phi.y);
+    if (xs.x < g.xs_n - 1) p[xs.x] = c0.x * (v.x + phi.x);
+    if (xs.y < g.xs_n - 1) p[xs.y] = c1.x * (v.y + phi.y);
     v = make_float2((c0.z + c0.y) * v.x + c0.y * phi.x, (c1.z + c1.y) * v.y + c1.y * phi.y);
 }
 __device__ __forceinline__ void adj_z2(float2 &v, const float4 &zc, float2 phi, float *p)
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         float *pSXZz = pz_ptr(g, PZ, s, PZ_SXZ), *pSZZ = pz_ptr(g, PZ, s, PZ_SZZ);
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
-            int2 xs = make_int2(-1, -1);
+            int2 xs = make_int2(g.xs_n - 1, g.xs_n - 1);
             const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 if (XB) {
                     const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
                     const float2 m0 = mem_x(pSXX + i * g.xs_n, xs), m1 = mem_x(pSXZx + i * g.xs_n, xs);
-                    pml_x2(dxx, c0, c1, xs, m0, pSXX + i * g.xs_n);
-                    pml_x2(dxxz, c0, c1, xs, m1, pSXZx + i * g.xs_n);
+                    pml_x2(g, dxx, c0, c1, xs, m0, pSXX + i * g.xs_n);
+                    pml_x2(g, dxxz, c0, c1, xs, m1, pSXZx + i * g.xs_n);
                 }
                 if (GUARD) {
                     const float4 zc = ldt(g.pmz + i);
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         float *snap_s = out.snap ? out.snap + ((long long)s * out.slots + out.slot) * g.snf * g.nd : nullptr;
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
-            int2 xs = make_int2(-1, -1);
+            int2 xs = make_int2(g.xs_n - 1, g.xs_n - 1);
             const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
@@ -655,8 +655,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                 if (XB) {
                     const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
                     const float2 m0 = mem_x(pDXU + i * g.xs_n, xs), m1 = mem_x(pDXV + i * g.xs_n, xs);
-                    pml_x2(dxu, c0, c1, xs, m0, pDXU + i * g.xs_n);
-                    if (!last) pml_x2(dxv, c0, c1, xs, m1, pDXV + i * g.xs_n);
+                    pml_x2(g, dxu, c0, c1, xs, m0, pDXU + i * g.xs_n);
+                    if (!last) pml_x2(g, dxv, c0, c1, xs, m1, pDXV + i * g.xs_n);
                 }
                 if (GUARD) {
                     if (g.fs && i == 0) {
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         float *fZXZ = pz_ptr(g, PZ, s, PZ_NFWD + PZA_ZXZ), *fZZ = pz_ptr(g, PZ, s, PZ_NFWD + PZA_ZZ);
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
-            int2 xs = make_int2(-1, -1);
+            int2 xs = make_int2(g.xs_n - 1, g.xs_n - 1);
             const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
@@ -950,8 +950,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                         if (XB) {
                             const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
                             const float2 m0 = mem_x(fXX + i * g.xs_n, xs), m1 = mem_x(fXXZ + i * g.xs_n, xs);
-                            adj_x2(vXX, c0, c1, xs, m0, fXX + i * g.xs_n);
-                            adj_x2(vXXZ, c0, c1, xs, m1, fXXZ + i * g.xs_n);
+                            adj_x2(g, vXX, c0, c1, xs, m0, fXX + i * g.xs_n);
+                            adj_x2(g, vXXZ, c0, c1, xs, m1, fXXZ + i * g.xs_n);
                         }
                         const long long b = (long long)i * g.wxp + band_x(g, jb);
                         *reinterpret_cast<float2 *>(iXX + b) = vXX;
@@ -1164,7 +1164,7 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
         const float *aZXZ = (bx || bz) ? S + 2 * SNA : aXX, *aXXZ = (bx || bz) ? S + 3 * SNA : aZZ;
         auto rows = [&](auto gd, auto xb) -> bool {
             constexpr bool GUARD = decltype(gd)::value, XB = decltype(xb)::value;
-            int2 xs = make_int2(-1, -1);
+            int2 xs = make_int2(g.xs_n - 1, g.xs_n - 1);
             const int e0 = XB ? tab_at(jb, g.nx) : 0, e1 = XB ? tab_at(jb + 1, g.nx) : 0;   // the columns' table entries
             if (XB) {
                 xs = xstrip_pair(g, jb);
@@ -1278,8 +1278,8 @@ __global__ void __launch_bounds__(TX *NW, NW == 8 ? 2 : 1)
                             float *fDXU = px_ptr(g, PX, s, PX_NFWD + PXA_DXU), *fDXV = px_ptr(g, PX, s, PX_NFWD + PXA_DXV);
                             const float4 c0 = ldt(g.pmx + jb), c1 = ldt(g.pmx + jb + 1);
                             const float2 m0 = mem_x(fDXU + i * g.xs_n, xs), m1 = mem_x(fDXV + i * g.xs_n, xs);
-                            adj_x2(d, c0, c1, xs, m0, fDXU + i * g.xs_n);
-                            adj_x2(v, c0, c1, xs, m1, fDXV + i * g.xs_n);
+                            adj_x2(g, d, c0, c1, xs, m0, fDXU + i * g.xs_n);
+                            adj_x2(g, v, c0, c1, xs, m1, fDXV + i * g.xs_n);
                         }
                         const long long b = (long long)i * g.wxp + band_x(g, jb);
                         float *ix = im.xa + (long long)s * 2 * g.txs + b;

@@ -254,7 +254,7 @@ Plan make_plan(const stfwi_desc *d, int k, int G)
     p.nz = d->free_surface ? d->nz_dom + (long long)d->pad : d->nz_dom + 2LL * d->pad;
     p.P = (p.nx + 31) / 32 * 32;
     p.nd = (long long)d->nz_dom * d->nx_dom;
-    p.xs_n = 2LL * d->pad;
+    p.xs_n = 2LL * d->pad + 1;   // and a memory that stays zero (xstrip_pair)
     p.zs_n = d->free_surface ? d->pad : 2LL * d->pad;
     const long long S = d->max_shots;
     p.fields = (size_t)2 * S * F_N * p.nz * p.P * sizeof(float);

@@ -149,3 +149,34 @@ def test_sharded_cuda_path_two_gloo_ranks_equal_one_process(tmp_path):
         # and 2: FP32 sums over a block's shots round differently
         assert abs(float(d["loss"]) / r_loss - 1) < 1e-6
         assert _rel(d["g_vs"], r_vs) < 1e-5 and _rel(d["g_vp"], r_vp) < 1e-5
+
+
+@pytest.mark.parametrize("fd,tiles", [(8, (16, 16)), (4, (8, 8)), (2, (16, 8))])
+def test_a_nan_spreads_no_faster_than_the_stencil(fd, tiles):
+    """A NaN in the wavelet of a source at the left (right) edge reaches the
+    C-PML strip at once.  A step carries it fd cells (fd / 2 into the
+    velocities, fd / 2 on into the stresses): traces farther away are finite."""
+    import torch
+    from stfwi_b200 import Solver
+    nz, nx, pad, nt, n0, dx, dt = 30, 220, 8, 24, 4, 10.0, 1.0e-3
+    vp = np.full((nz, nx), 2500.0)
+    rx, rz = (a.ravel().astype(np.int32) for a in np.meshgrid(np.arange(nx), [9, 10, 11]))
+    wav = O.ricker(np.arange(nt) * dt, 25.0, 0.02) * 1e9
+    wav[n0] = np.nan
+    sx = np.array([0, 0, nx - 1, nx - 1])
+    S = Solver(nz, nx, dx, dx, dt, nt, 25.0, pad, len(rx), 4, fd_order=fd, free_surface=True, want_gradient=False)
+    S.set_tile_rows(*tiles)
+    S.set_receivers(rx, rz)
+    S.set_shots(sx, [10] * 4, ["force", "moment"] * 2, wav.astype(np.float32))
+    S.set_model(vp / 1.8 * np.ones((nz, nx)), vp, np.full((nz, nx), 2000.0))
+    S.forward()
+    rec = torch.empty((4, 4, nt, len(rx)), device="cuda")
+    S.lib.stfwi_get_records(S.h, rec.data_ptr(), None)
+    torch.cuda.synchronize()
+    S.close()
+    finite = np.isfinite(rec.cpu().numpy())
+    away = np.abs(rx[None, :] - sx[:, None])[:, None, None, :]
+    steps = np.maximum(np.arange(nt) - n0 + 1, 0)[None, None, :, None]
+    reach = np.broadcast_to((away <= fd * steps) & (steps > 0), finite.shape)
+    assert not finite[:, :, n0 + 1:][reach[:, :, n0 + 1:]].all()      # the NaN was there
+    assert finite[~reach].all(), int((~finite & ~reach).sum())
