@@ -24,7 +24,6 @@ namespace stfwi {
 
 constexpr int TX = 32;            // lanes of a warp across the tile
 constexpr int NWARP = 8;          // warps per block
-constexpr int NTHR = TX * NWARP;  // threads per block
 
 // psi (C-PML memory) arrays per shot: x-strips and z-strips
 enum { PX_SXX = 0, PX_SXZ, PX_DXU, PX_DXV, PX_NFWD };
@@ -82,8 +81,6 @@ struct Images {
 struct Mat {
     const float *B, *L2M, *L, *M;   // padded grid [nz][P]
     const float *Lr;                // row 0 of -L/L2M [P] (free surface)
-    const float *bx, *ax, *ikx;     // per column [nx]
-    const float *bz, *az, *ikz;     // per row [nz]
 };
 
 struct Shots {

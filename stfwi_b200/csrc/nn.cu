@@ -44,6 +44,7 @@
 namespace stfwi {
 namespace nn {
 
+constexpr int SMS = 148;                 // SMs of a B200, which the grids are cut for
 constexpr int CONV_THREADS = 128;
 constexpr int STAGES = 4;
 constexpr int PIPE_THREADS = 192;         // four epilogue warps (one per quarter of the TMEM lanes), a loader, an issuer
@@ -1031,7 +1032,7 @@ ConvPlan conv_plan(int n, int h, int w, int cin, int cout, int kc)
             // as many CTAs per SM as tensor memory and shared memory hold
             const size_t cap = occ == 1 ? 227 * 1024 : sm_smem / occ - 1024;
             if (occ * cols > 512 || fixed + 4 * a > cap) continue;
-            const double want = occ * 148.0 / ((double)n * (w / 128) * (cout / bn));
+            const double want = (double)occ * SMS / ((double)n * (w / 128) * (cout / bn));
             p.strips = want < 1 ? 1 : want > h ? h : (int)want;
             p.rows = (h + p.strips - 1) / p.strips;
             if (p.rows < ROWS_MIN) break;
@@ -1049,7 +1050,7 @@ ConvPlan conv_plan(int n, int h, int w, int cin, int cout, int kc)
     // chip (us at batch 1, 128 -> 128 at 40 x 128: 14.8 -> 13.2, 256 -> 256 at 20 x 64: 22 -> 19)
     p = ConvPlan();
     p.bn = cout % 128 == 0 ? 128 : cout % 64 == 0 ? 64 : cout % 32 == 0 ? 32 : 16;
-    while (p.bn > 16 && 2.0 * ((double)n * h * w / 128) * (cout / p.bn) <= 148) p.bn /= 2;
+    while (p.bn > 16 && 2.0 * ((double)n * h * w / 128) * (cout / p.bn) <= SMS) p.bn /= 2;
     p.smem = conv_smem(kc, p.bn);
     return p;
 }
@@ -1110,7 +1111,7 @@ int conv_common(const void *x, int n, int h, int w, int cin, const void *wt, int
 unsigned blocks_for(size_t n, int threads)
 {
     size_t b = (n + threads - 1) / threads;
-    return (unsigned)(b < 1 ? 1 : b > 4 * 148 * 8 ? 4 * 148 * 8 : b);
+    return (unsigned)(b < 1 ? 1 : b > 4 * SMS * 8 ? 4 * SMS * 8 : b);
 }
 
 // grid of a row kernel: rows x parts of a row of `per_row` thread items, about four items a thread
@@ -1187,7 +1188,7 @@ int stfwi_nn_conv3x3_wgrad(const void *x, const void *dz, int n, int h, int w, i
     // (Three tiles a CTA and one CTA per SM took 833 us in all, but moved gradients of 12
     // images of 320 x 1024 by up to 8e-5 of their norm; this keeps them within 8e-7.)
     const int tiles = 9 * ((cout + 127) / 128) * g.ci_tiles;
-    int splits = (4 * 148 + tiles - 1) / tiles;
+    int splits = (4 * SMS + tiles - 1) / tiles;
     if (splits > g.chunks) splits = g.chunks;
     if (splits < 1) splits = 1;
     g.chunks_per_split = (g.chunks + splits - 1) / splits;
@@ -1285,7 +1286,7 @@ int stfwi_nn_head_loss_grad(const void *y, size_t npix, int c, const float *wt, 
 {
     if (c % 16 || c > 64) return nn_fail(STFWI_ERR_INVALID, "head: channels must be a multiple of 16, <= 64");
     unsigned blocks = blocks_for(npix, 256);
-    if (blocks > 1184) blocks = 1184;
+    if (blocks > 8 * SMS) blocks = 8 * SMS;
     auto go = [&](auto kern) {
         kern<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const __nv_bfloat16 *>(y), npix, wt, out, target, wgt, inv_norm, static_cast<__nv_bfloat16 *>(dz),
@@ -1307,7 +1308,7 @@ int stfwi_nn_bias_grad(const void *dz, size_t npix, int c, float *db, void *stre
     const int threads = 256;
     const bool v8 = c % 8 == 0 && aligned16(dz);
     unsigned blocks = blocks_for(npix * c / (v8 ? 128 : 64), threads);
-    if (blocks > 8 * 148) blocks = 8 * 148;
+    if (blocks > 8 * SMS) blocks = 8 * SMS;
     // at least one whole pixel's channels among the threads of the grid
     if (blocks * threads < (unsigned)c) blocks = (c + threads - 1) / threads;
     (v8 ? k_bias_grad<8> : k_bias_grad<1>)<<<blocks, threads, c * sizeof(float), static_cast<cudaStream_t>(stream)>>>(

@@ -84,21 +84,4 @@ template <int FD, class CA, class CB> __device__ __forceinline__ float a_tdm(con
     return d;
 }
 
-// forward C-PML (fwi/forward.py:107-112): psi' = b psi + a D ; D' = D/k + psi'
-__device__ __forceinline__ float pml_fwd_pre(float D, float b, float a, float ik, float old, float *psi)
-{
-    const float pn = b * old + a * D;
-    *psi = pn;
-    return D * ik + pn;
-}
-
-// transposed C-PML on a staged value x with the memory kept in the scaled
-// form phi = psi / (dt / d) of the adjoint step (so the step's factor drops
-// out): returns (1/k + a) x + a phi and stores the new memory b (x + phi)
-__device__ __forceinline__ float pml_adj4(float x, float b, float a, float ik, float phi, float *dst)
-{
-    *dst = b * (x + phi);
-    return (ik + a) * x + a * phi;
-}
-
 }  // namespace stfwi

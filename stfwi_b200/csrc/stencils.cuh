@@ -334,7 +334,8 @@ __device__ __forceinline__ void prefetch_z(const Geo &g, int iw, int jb, const f
 // could be infinite, and 0 times it is no zero.
 __device__ __forceinline__ float2 mem_x(const float *row, int2 xs) { return make_float2(row[xs.x], row[xs.y]); }
 
-// C-PML of a pair of x-derivatives on one row (c0, c1: the columns' (b, a, 1/k),
+// C-PML (fwi/forward.py:107-112: psi' = b psi + a D, D' = D/k + psi') of a pair
+// of x-derivatives on one row (c0, c1: the columns' (b, a, 1/k),
 // old: their memories, p: the memory's row) / of z-derivatives (p: the pair's memory)
 __device__ __forceinline__ void pml_x2(const Geo &g, float2 &d, const float4 &c0, const float4 &c1, int2 xs, float2 old, float *p)
 {

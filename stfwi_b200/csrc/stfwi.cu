@@ -49,7 +49,6 @@ struct stfwi_handle {
     // model
     float *vs = nullptr, *vp = nullptr, *rho = nullptr;     // physical [nd]
     float *B = nullptr, *L2M = nullptr, *L = nullptr, *M = nullptr, *Lr = nullptr;
-    float *bx = nullptr, *ax = nullptr, *ikx = nullptr, *bz = nullptr, *az = nullptr, *ikz = nullptr;
     float *vpmax = nullptr;
     float *MATS = nullptr;  // [4][nz][P]: B, L2M, L, M
     bool model_set = false;
@@ -320,8 +319,7 @@ __global__ void k_vpmax(const float *vp, long long n, float *out)
 // C-PML profiles (fwi/forward.py:35-104), as 1-D arrays: the reference's
 // 2-D coefficient arrays are constant along rows (x) / columns (z).
 __global__ void k_pml(int nz, int nx, int nz_dom, int pad, int fs, double dx, double dt, double fc,
-                      const float *vpmax, float *bx, float *ax, float *ikx, float *bz, float *az,
-                      float *ikz, float4 *pmx, float4 *pmz)
+                      const float *vpmax, float4 *pmx, float4 *pmz)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const double Lp = pad * dx;
@@ -330,34 +328,30 @@ __global__ void k_pml(int nz, int nx, int nz_dom, int pad, int fs, double dx, do
     d0f = d0f * (float)log(1e-3);
     d0f = d0f / (float)(2.0 * Lp);
     const double d0 = d0f;
-    auto coef = [&](int i, float *b, float *a, float *ik) {
-        if (i < 0) { *b = 1.f; *a = 0.f; *ik = 1.f; return; }
+    // (b, a, 1/k) at depth i of a strip and a fourth value, (0, 0, 1) outside
+    auto coef = [&](int i, float w) -> float4 {
+        if (i < 0) return make_float4(0.f, 0.f, 1.f, w);
         const double dist = (i + 1) * dx / Lp;
         const double dd = d0 * (dist * dist), kk = 1.0 + (2.0 - 1.0) * (dist * dist);
         const double al = M_PI * fc * (1.0 - dist);
         const double bb = exp(-(dd / kk + al) * dt);
         const double den = kk * (dd + kk * al);
-        *b = (float)bb;
-        *a = (float)(den > 1e-10 ? dd * (bb - 1.0) / den : 0.0);
-        *ik = (float)(1.0 / kk);
+        return make_float4((float)bb, (float)(den > 1e-10 ? dd * (bb - 1.0) / den : 0.0), (float)(1.0 / kk), w);
     };
     if (t < nx) {
         int i = -1;
         if (t < pad) i = pad - 1 - t;
         else if (t >= nx - pad) i = t - (nx - pad);
-        coef(i, bx + t, ax + t, ikx + t);
-        pmx[t] = i < 0 ? make_float4(0.f, 0.f, 1.f, 0.f) : make_float4(bx[t], ax[t], ikx[t], 0.f);
+        pmx[t] = coef(i, 0.f);
     }
     if (t < nz) {
         int i = -1;
         const int bottom = fs ? nz_dom : pad + nz_dom;
         if (t >= bottom) i = t - bottom;
         else if (!fs && t < pad) i = pad - 1 - t;
-        coef(i, bz + t, az + t, ikz + t);
         // the z-strip index: bottom strip first, then the top one
         const int zs = i < 0 ? -1 : t >= bottom ? t - bottom : pad + t;
-        pmz[t] = i < 0 ? make_float4(0.f, 0.f, 1.f, __int_as_float(-1))
-                       : make_float4(bz[t], az[t], ikz[t], __int_as_float(zs));
+        pmz[t] = coef(i, __int_as_float(zs));
     }
 }
 
@@ -607,7 +601,7 @@ __global__ void k_finalize(Geo g, int groups, int accp, const double *acc, const
 
 Mat mat_of(stfwi_handle *h)
 {
-    return Mat{h->B, h->L2M, h->L, h->M, h->Lr, h->bx, h->ax, h->ikx, h->bz, h->az, h->ikz};
+    return Mat{h->B, h->L2M, h->L, h->M, h->Lr};
 }
 Shots shots_of(stfwi_handle *h)
 {
@@ -1439,8 +1433,6 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     bool ok = true;
     ok &= alloc((void **)&h->vs, nd * 4) && alloc((void **)&h->vp, nd * 4) && alloc((void **)&h->rho, nd * 4);
     ok &= alloc((void **)&h->MATS, 4 * NP * 4) && alloc((void **)&h->Lr, p.P * 4);
-    ok &= alloc((void **)&h->bx, p.P * 4) && alloc((void **)&h->ax, p.P * 4) && alloc((void **)&h->ikx, p.P * 4);
-    ok &= alloc((void **)&h->bz, p.nz * 4) && alloc((void **)&h->az, p.nz * 4) && alloc((void **)&h->ikz, p.nz * 4);
     ok &= alloc((void **)&h->vpmax, 16) && alloc((void **)&h->status, 16);
     ok &= alloc((void **)&h->sx, S * 4) && alloc((void **)&h->sz, S * 4) && alloc((void **)&h->stype, S * 4) &&
           alloc((void **)&h->spos, S * sizeof(int4));
@@ -1568,7 +1560,7 @@ stfwi_status stfwi_set_model(stfwi_handle *h, const float *vs, const float *vp, 
     k_vpmax<<<1, 1024, 0, st>>>(h->vp, g.nd, h->vpmax);
     const int nmax = std::max(g.nx, g.nz);
     k_pml<<<(nmax + 127) / 128, 128, 0, st>>>(g.nz, g.nx, g.nz_dom, g.pad, g.fs, h->d.dx, h->d.dt, h->d.fc,
-                                              h->vpmax, h->bx, h->ax, h->ikx, h->bz, h->az, h->ikz, h->pmx, h->pmz);
+                                              h->vpmax, h->pmx, h->pmz);
     CK(h, cudaGetLastError());
     h->model_set = true;
     if (h->shots_set) {
