@@ -426,9 +426,11 @@ def main():
     roof["frac_of_nominal_7700"] = achieved / 7700.0
     roof["step_frac_of_nominal_7700"] = roof["step_achieved"] / 7700.0
     # stencil launches: 2 per forward step and 2 per adjoint step, once per
-    # chain of the pass; plus set-up, misfit, finalize
-    chains = min(args.chains or 2, ns)
-    launches = 4 * nt * chains + 6
+    # chain of the pass (at most one for each run of shots of its second
+    # kernel); plus set-up, misfit, finalize
+    per_block = schedule or {}
+    chains = [min(args.chains or 2, -(-ns // per_block.get(k, args.shot_group or 1))) for k in ("fwd_str", "adj_b")]
+    launches = 2 * nt * sum(chains) + 6
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

@@ -52,9 +52,9 @@ struct stfwi_handle {
     float *vpmax = nullptr;
     float *MATS = nullptr;  // [4][nz][P]: B, L2M, L, M
     bool model_set = false;
-    // tensor maps of the staged tiles and per-kernel shot groups
+    // tensor maps of the staged tiles and shots per block of each kernel
     int sms = 148;
-    int accp = 5;   // accumulator planes per shot group (7 with the density terms)
+    int accp = 5;   // accumulator planes per run of shots (7 with the density terms)
     CUtensorMap tmS{}, tmV{}, tmE{}, tmP{};        // halo boxes: stresses, velocities; one adjoint field (adj_a, adj_b tiles)
     CUtensorMap tmUo{}, tmSo{}, tmPQo{}, tmEo{};   // own-cell boxes
     CUtensorMap tmXa{}, tmZa{}, tmXb{}, tmZb{};    // halo boxes of the image bands
@@ -113,7 +113,7 @@ struct stfwi_handle {
     bool stored = false;  // last forward kept its strain history
 
     cudaStream_t hs = nullptr;
-    // a pass split into chains over the shot groups: the chains it may use
+    // a pass split into chains over the runs of shots: the chains it may use
     // (1-4, stfwi_set_chains), the chains of the pass being recorded, and
     // the streams of chains 1.. (chain 0 runs on the pass's own stream)
     int chains = 2;
