@@ -191,22 +191,17 @@ int level_runs(int n, int run)
 // the default rule's runs are single shots (at most 60 MB in all: there are fewer
 // than 3.2 tiles and shots for each block that the device holds), else one for
 // two shots; or as many as the descriptor's runs.  `narrow`: one for two shots
-// at most, where memory is short.
-int acc_groups_of(const stfwi_desc *d, int sms, bool narrow)
+// at most, where memory is short.  The SM count is a B200's: the plan is made
+// without a device (stfwi_workspace_bytes).
+int acc_groups_of(const stfwi_desc *d, bool narrow)
 {
+    constexpr int sms = 148;
     const int n = d->max_shots;
     if (d->shot_group > 0) return (n + d->shot_group - 1) / d->shot_group;
     if (narrow) return (n + 1) / 2;
     const long long rows = d->nz_dom + (d->free_surface ? 1LL : 2LL) * d->pad;
     const long long tiles = ((d->nx_dom + 2LL * d->pad + TX4 - 1) / TX4) * ((rows + 15) / 16);
     return level_runs(n, std::min(2, default_run(tiles * n, sms, RUN_ADJ_B)));
-}
-
-int sm_count(int device)
-{
-    int n = 148;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) cudaGetLastError();
-    return n;
 }
 
 // Image bands of the adjoint: the columns (rows) that the boxes of the tiles
@@ -1338,9 +1333,7 @@ size_t stfwi_workspace_bytes(const stfwi_desc *d)
 {
     if (!d || d->nt < 1) return 0;
     const int k = d->ckpt_interval > 0 ? std::min(d->ckpt_interval, d->nt) : d->nt;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    return make_plan(d, k, acc_groups_of(d, sm_count(dev), false)).total();
+    return make_plan(d, k, acc_groups_of(d, false)).total();
 }
 
 const char *stfwi_last_error(const stfwi_handle *h) { return h ? h->err.c_str() : "null handle"; }
@@ -1369,12 +1362,12 @@ stfwi_status stfwi_create(const stfwi_desc *d, stfwi_handle **out)
     // history plan: every step if it fits, else the longest checkpoint
     // segment that fits (the recompute costs one forward whatever k is)
     int k = d->nt;
-    h->sms = sm_count(h->device);
-    h->acc_groups = acc_groups_of(d, h->sms, false);
+    cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
+    h->acc_groups = acc_groups_of(d, false);
     if (d->want_gradient) {
         if (d->ckpt_interval > 0) k = std::min(d->ckpt_interval, d->nt);
         // fewer groups before fewer steps
-        if ((double)make_plan(d, k, h->acc_groups).total() > budget) h->acc_groups = acc_groups_of(d, h->sms, true);
+        if ((double)make_plan(d, k, h->acc_groups).total() > budget) h->acc_groups = acc_groups_of(d, true);
         if (d->ckpt_interval <= 0 && (double)make_plan(d, k, h->acc_groups).total() > budget) {
             k = 0;
             for (int kk = d->nt - 1; kk >= 1; --kk)
